@@ -803,3 +803,26 @@ def test_a_last_round_of_few_tiles_becomes_a_product_of_its_own(ops16, T, F, K):
         assert _rel(got[mode][0], want) < 6e-3
         assert _rel(got[mode][1], want_s) < 2e-5
     ops16.check_errors()
+
+
+# --------------------------------------------------------------------------- the float32 product and attention by size
+@pytest.mark.parametrize("M,N,K", [(1, 4, 4), (1, 2050, 130), (2, 33, 2048), (3, 1000, 513), (5, 96, 96), (8, 12000, 260),
+                                   (9, 64, 20), (16, 5000, 36), (17, 70, 16), (31, 4096, 100), (33, 65, 15), (33, 4100, 2049),
+                                   (64, 64, 1024), (65, 129, 777), (130, 30000, 24), (700, 2048, 48), (129, 1, 1)])
+def test_float32_products_at_the_edges_of_their_kernels(ops32, M, N, K):
+    """Rows by lanes (1, 2, 4 and 8 rows a warp, K shared by a block's warps or not), tiles with K in 1, 2 and 8 parts, whole and
+    ragged, rows that 16-byte loads can and cannot take; stored, added and scaled.  A float32 sum of K products in any order is
+    within K 2^-24 of the sum of their magnitudes (first order); the addition and the scale round once more each."""
+    g = torch.Generator(device="cuda").manual_seed(31)
+    for shift in (0, 1):                                       # rows that start one value behind a 16-byte boundary
+        x = torch.randn(M * K + 1, device="cuda", generator=g)[shift:shift + M * K].view(M, K)
+        w = torch.randn(N, K, device="cuda", generator=g)
+        lw = ops32.prepare_linear([w])
+        ref = x.double() @ w.double().T
+        bound = (K + 4) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T) + 1e-30
+        assert ((ops32.linear(x, lw).double() - ref).abs() <= bound).all()
+        assert ((ops32.linear(x, lw, scale=0.5).double() - 0.5 * ref).abs() <= bound).all()
+        acc = torch.randn(M, N, device="cuda", generator=g)
+        want = acc.double() + ref
+        ops32.linear(x, lw, accumulate_into=acc)
+        assert ((acc.double() - want).abs() <= bound + 2.0 ** -23 * want.abs()).all()
