@@ -311,3 +311,13 @@ __device__ __forceinline__ int64_t rb_page_offset(const RbPagedLayer& c, int slo
   const int page = c.page_table[(int64_t)slot * c.max_pages + pos / c.page_size];
   return (((int64_t)page * c.n_kv_heads + kvh) * c.page_size + pos % c.page_size) * c.head_dim;
 }
+// The same for a page size of 2^shift, without the divisions (shift < 0: any page size).
+__device__ __forceinline__ int64_t rb_page_offset(const RbPagedLayer& c, int shift, int slot, int pos, int kvh) {
+#ifndef RB_CHECKED
+  if (shift >= 0) {
+    const int page = c.page_table[(int64_t)slot * c.max_pages + (pos >> shift)];
+    return ((((int64_t)page * c.n_kv_heads + kvh) << shift) + (pos & ((1 << shift) - 1))) * c.head_dim;
+  }
+#endif
+  return rb_page_offset(c, slot, pos, kvh);
+}

@@ -826,3 +826,44 @@ def test_float32_products_at_the_edges_of_their_kernels(ops32, M, N, K):
         want = acc.double() + ref
         ops32.linear(x, lw, accumulate_into=acc)
         assert ((acc.double() - want).abs() <= bound + 2.0 ** -23 * want.abs()).all()
+
+
+@pytest.mark.parametrize("H,Kh,D,page,lengths,decode", [(4, 2, 30, 64, [5, 1], False), (2, 1, 64, 48, [130], False),
+                                                        (32, 4, 64, 64, [300, 17], True), (3, 3, 129, 16, [70, 1], True),
+                                                        (1, 1, 1024, 64, [20], False), (2, 2, 260, 64, [40, 33], True),
+                                                        (16, 16, 96, 64, [200], False)])
+def test_float32_attention_by_groups_of_lanes(ops32, H, Kh, D, page, lengths, decode):
+    """Every number of lanes a key, pairs shared by 1 to 8 warps, pages of any size, with a window, kept positions, sinks and a
+    soft cap, against float64.  Scores are sums of D float32 products of magnitude up to about 5, softmax weights e^score:
+    relative error (D + 4) 2^-24 x 5, twice (numerator and denominator), plus the sums over the keys."""
+    from ctypes import c_void_p
+    g = torch.Generator(device="cuda").manual_seed(32)
+    mp = (max(lengths) + page - 1) // page
+    S = len(lengths)
+    k = torch.randn(S * mp, Kh, page, D, device="cuda", generator=g)
+    v = torch.randn(S * mp, Kh, page, D, device="cuda", generator=g)
+    table = torch.randperm(S * mp, device="cuda", generator=g).to(torch.int32).view(S, mp).contiguous()
+    rows = [(s, p) for s, n in enumerate(lengths) for p in ([n - 1] if decode else range(n))]
+    slot = torch.tensor([r[0] for r in rows], dtype=torch.int32, device="cuda")
+    pos = torch.tensor([r[1] for r in rows], dtype=torch.int32, device="cuda")
+    T = len(rows)
+    q = torch.randn(T, H, D, device="cuda", generator=g)
+    sinks = torch.randn(H, device="cuda", generator=g)
+    ptr = lambda t: c_void_p(t.data_ptr() if t is not None else 0)
+    flat_k, flat_v = (t[table.long()].transpose(2, 3).reshape(S, mp * page, Kh, D).double() for t in (k, v))
+    for window, keep, sink, cap in ((0, 0, None, 0.0), (11, 0, sinks, 0.0), (7, 3, None, 2.0)):
+        out = torch.empty_like(q)
+        ops32.lib.call("rb_attention_next", ptr(sink), cap, keep, launches=0)
+        ops32.lib.call("rb_attention_simple", ptr(out), ptr(q), 0, ptr(k), ptr(v), ptr(table), mp, page, ptr(pos), ptr(slot), T,
+                       H, Kh, D, D ** -0.5, window, ops32._stream())
+        kk, vv = (t[slot.long()].repeat_interleave(H // Kh, dim=2) for t in (flat_k, flat_v))      # [T, positions, H, D]
+        s = torch.einsum("thd,tphd->thp", q.double(), kk) * D ** -0.5
+        if cap:
+            s = cap * torch.tanh(s / cap)
+        at = torch.arange(mp * page, device="cuda")[None]
+        see = (at <= pos[:, None]) & (((pos[:, None] - at < window) | (at < keep)) if window else True)
+        s = s.masked_fill(~see[:, None], -math.inf)
+        if sink is not None:
+            s = torch.cat([s, sink.double()[None, :, None].expand(T, H, 1)], dim=2)
+        want = torch.einsum("thp,tphd->thd", torch.softmax(s, -1)[..., :mp * page], vv)
+        assert _rel(out, want) < (20 * (D + 4) + max(lengths)) * 2.0 ** -24
