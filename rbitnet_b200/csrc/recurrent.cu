@@ -319,9 +319,9 @@ template <int P, int R>
 __global__ void __launch_bounds__(128) matrix_memory_kernel(
     float* __restrict__ o_out, const float* __restrict__ proj, int64_t ld, int q_off, int k_off, int v_off, int i_off,
     int f_off, const float* __restrict__ i_bias, const float* __restrict__ f_bias, float cap, float q_scale,
-    float floor_add, float* __restrict__ C_state, float* __restrict__ n_state, float* __restrict__ m_state,
-    const int* __restrict__ seq_first, const int* __restrict__ seq_count, const int* __restrict__ tok_slot, int H, int D,
-    int Dv, int vec4) {
+    float floor_add, float* __restrict__ C_state, const float* __restrict__ n_state, const float* __restrict__ m_state,
+    float* __restrict__ moved, const int* __restrict__ seq_first, const int* __restrict__ seq_count,
+    const int* __restrict__ tok_slot, int H, int D, int Dv, int vec4) {
   rb_pdl_launch_dependents();
   extern __shared__ __align__(16) float sm[];
   constexpr int Dp = P * R;
@@ -387,7 +387,7 @@ __global__ void __launch_bounds__(128) matrix_memory_kernel(
   stage(0, 0);
   float Cr[R], nr[R];
   float* Cs = C_state + ((int64_t)slot * H + h) * D * Dv;
-  float* ns = n_state + ((int64_t)slot * H + h) * D;
+  const float* ns = n_state + ((int64_t)slot * H + h) * D;
 #pragma unroll
   for (int r = 0; r < R; ++r) {
     const int d = part + P * r;
@@ -488,14 +488,26 @@ __global__ void __launch_bounds__(128) matrix_memory_kernel(
     }
     __syncthreads();                       // the buffer may be filled again
   }
+  // n and m belong to all blocks of the (run, head), and a block may begin when another has ended: the new ones are left
+  // beside the state, and the kernel after this one takes them over.
+  float* left = moved + ((int64_t)blockIdx.x * H + h) * (D + 1);
 #pragma unroll
   for (int r = 0; r < R; ++r) {
     const int d = part + P * r;
     if (live && d < D) Cs[(int64_t)j * D + d] = Cr[r];
-    if (blockIdx.z == 0 && col == 0 && d < D) ns[d] = nr[r];
+    if (blockIdx.z == 0 && col == 0 && d < D) left[d] = nr[r];
   }
-  if (blockIdx.z == 0 && threadIdx.x == 0) m_state[(int64_t)slot * H + h] = *s_m;
+  if (blockIdx.z == 0 && threadIdx.x == 0) left[D] = *s_m;
 }
+
+// n and m of the runs' heads as matrix_memory_kernel left them ([run][H][D + 1]), for the state.
+struct Moved {
+  const float* from = nullptr;
+  float *n_state = nullptr, *m_state = nullptr;
+  const int *tok_slot = nullptr, *seq_first = nullptr;
+  int n_seq = 0, H = 0, D = 0;
+};
+thread_local Moved t_moved;            // for this thread's next head_norm_gate_kernel
 
 // Per (token, head): o / rms(o) over the head's Dv values, times the weight, times sigmoid(gate) (gate_silu: times
 // gate * sigmoid(gate)).  One warp each.  gate: the projections' rows, at column g_off.  The weight has H * Dv
@@ -503,9 +515,18 @@ __global__ void __launch_bounds__(128) matrix_memory_kernel(
 template <typename TI, typename TO>
 __global__ void head_norm_gate_kernel(TO* __restrict__ out, const float* __restrict__ o, const float* __restrict__ w,
                                       const TI* __restrict__ proj, int64_t ld, int g_off, int n_rows, int H, int Dv,
-                                      float eps, int w_shared, int gate_silu) {
+                                      float eps, int w_shared, int gate_silu, Moved moved) {
   rb_pdl_launch_dependents();
   rb_pdl_wait();
+  if (moved.from != nullptr) {
+    const int per = moved.D + 1;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < moved.n_seq * moved.H * per; i += gridDim.x * blockDim.x) {
+      const int rh = i / per, d = i - rh * per, run = rh / moved.H;
+      const int64_t to = (int64_t)moved.tok_slot[moved.seq_first != nullptr ? moved.seq_first[run] : run] * moved.H + rh % moved.H;
+      if (d < moved.D) moved.n_state[to * moved.D + d] = moved.from[i];
+      else moved.m_state[to] = moved.from[i];
+    }
+  }
   const int lane = threadIdx.x & 31;
   const int64_t item = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (item >= (int64_t)n_rows * H) return;
@@ -652,7 +673,7 @@ RB_EXPORT int rb_matrix_memory_lanes(int D) {
 template <int P, int R>
 static int launch_matrix_memory(float* o_out, const float* proj, int64_t ld, int q_off, int k_off, int v_off, int i_off,
                                 int f_off, const float* i_bias, const float* f_bias, float cap, float q_scale,
-                                float floor_add, float* C_state, float* n_state, float* m_state, const int* seq_first,
+                                float floor_add, float* C_state, float* n_state, float* m_state, float* moved, const int* seq_first,
                                 const int* seq_count, const int* tok_slot, int n_seq, int H, int D, int Dv,
                                 cudaStream_t stream) {
   // fewer columns per block while the blocks are too few to give every SM several: the work of a token is a
@@ -670,18 +691,22 @@ static int launch_matrix_memory(float* o_out, const float* proj, int64_t ld, int
   if (smem > 48 * 1024 && once.first())
     RB_CUDA(cudaFuncSetAttribute(matrix_memory_kernel<P, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
   RB_LAUNCH("matrix_memory_kernel", (matrix_memory_kernel<P, R>), grid, threads, smem, stream, o_out, proj, ld, q_off, k_off,
-            v_off, i_off, f_off, i_bias, f_bias, cap, q_scale, floor_add, C_state, n_state, m_state, seq_first, seq_count,
+            v_off, i_off, f_off, i_bias, f_bias, cap, q_scale, floor_add, C_state, n_state, m_state, moved, seq_first, seq_count,
             tok_slot, H, D, Dv, vec4);
   RB_CHECK_LAUNCH("rb_matrix_memory");
+  t_moved = Moved{moved, n_state, m_state, tok_slot, seq_first, n_seq, H, D};
   return 0;
 }
 
+// moved: [n_seq][H][D + 1] floats.  The runs' new n and m are left there, and this thread's next rb_head_norm_gate moves the
+// state on to them.
 RB_EXPORT int rb_matrix_memory(float* o_out, const void* proj, int64_t ld, int proj_dtype, int q_off, int k_off, int v_off,
                                int i_off, int f_off, const float* i_bias, const float* f_bias, float cap, float q_scale,
-                               float floor_add, float* C_state, float* n_state, float* m_state, const int* seq_first,
-                               const int* seq_count, const int* tok_slot, int n_seq, int H, int D, int Dv,
+                               float floor_add, float* C_state, float* n_state, float* m_state, float* moved,
+                               const int* seq_first, const int* seq_count, const int* tok_slot, int n_seq, int H, int D, int Dv,
                                cudaStream_t stream) {
   if (n_seq == 0) return 0;
+  RB_REQUIRE((int64_t)n_seq * H * (D + 1) <= 0x7fffffff, "rb_matrix_memory: %d runs: too many for one launch", n_seq);
   RB_REQUIRE(H > 0 && D > 0 && Dv > 0 && D <= 512, "rb_matrix_memory: bad sizes H=%d D=%d Dv=%d (D up to 512)", H, D, Dv);
   RB_REQUIRE(cap > 0.f, "rb_matrix_memory: the gates' cap must be positive");
   RB_REQUIRE(proj_dtype == RB_F32, "rb_matrix_memory: the projections are float32 rows (found dtype %d)", proj_dtype);
@@ -689,7 +714,7 @@ RB_EXPORT int rb_matrix_memory(float* o_out, const void* proj, int64_t ld, int p
   const int per = (D + P - 1) / P;
 #define GO(PP, RR)                                                                                                    \
   return launch_matrix_memory<PP, RR>(o_out, (const float*)proj, ld, q_off, k_off, v_off, i_off, f_off, i_bias, f_bias, \
-                                      cap, q_scale, floor_add, C_state, n_state, m_state, seq_first, seq_count,       \
+                                      cap, q_scale, floor_add, C_state, n_state, m_state, moved, seq_first, seq_count, \
                                       tok_slot, n_seq, H, D, Dv, stream)
   switch (P) {
     case 1: GO(1, 8);
@@ -709,12 +734,14 @@ RB_EXPORT int rb_matrix_memory(float* o_out, const void* proj, int64_t ld, int p
 RB_EXPORT int rb_head_norm_gate(void* out, int out_dtype, const float* o, const float* w, const void* proj, int64_t ld,
                                 int proj_dtype, int g_off, int T, int H, int Dv, float eps, int w_shared, int gate_silu,
                                 cudaStream_t stream) {
+  const Moved moved = t_moved;
+  t_moved = Moved();
   if (T == 0) return 0;
   const int64_t items = (int64_t)T * H;
   const int blocks = (int)((items + 3) / 4);
 #define LAUNCH(TI, TO)                                                                                              \
   RB_LAUNCH("head_norm_gate_kernel", (head_norm_gate_kernel<TI, TO>), blocks, 128, 0, stream, (TO*)out, o, w,        \
-            (const TI*)proj, ld, g_off, T, H, Dv, eps, w_shared, gate_silu)
+            (const TI*)proj, ld, g_off, T, H, Dv, eps, w_shared, gate_silu, moved)
   if (proj_dtype == RB_F32 && out_dtype == RB_F32) LAUNCH(float, float);
   else if (proj_dtype == RB_F32 && out_dtype == RB_BF16) LAUNCH(float, __nv_bfloat16);
   else if (proj_dtype == RB_BF16 && out_dtype == RB_BF16) LAUNCH(__nv_bfloat16, __nv_bfloat16);

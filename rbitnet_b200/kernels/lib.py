@@ -57,7 +57,8 @@ _SIGNATURES = {
     "rb_gated_step": [P, I, P, L, I, I, I, P, P, P, P, P, P, P, P, F, P, P, P, P, I, I, I, I, P],
     "rb_gated_step_max_rows": [],
     "rb_gated_scan": [P, I, P, P, P, P, P, F, P, L, I, I, I, P, P, P, P, P, P, P, P, I, I, I, I, I, P],
-    "rb_matrix_memory": [P, P, L, I, I, I, I, I, I, P, P, F, F, F, P, P, P, P, P, P, I, I, I, I, P],
+    "rb_matrix_memory": [P, P, L, I, I, I, I, I, I, P, P, F, F, F, P, P, P, P, P, P, P, I, I, I, I, P],
+    "rb_matrix_memory_chunked": [P, P, L, I, I, I, I, I, P, P, F, F, F, P, P, P, P, P, P, P, P, P, I, I, I, I, I, P, P],
     "rb_matrix_memory_lanes": [I],
     "rb_head_norm_gate": [P, I, P, P, P, L, I, I, I, I, I, F, I, I, P],
     "rb_rmsnorm_grouped": [P, I, P, P, I, I, I, F, P],
@@ -142,6 +143,7 @@ class KernelLibrary:
         self.declare("rb_gemm_tc_workspace_bytes", [], restype=ctypes.c_longlong)
         self.declare("rb_gated_delta_chunk_floats", [I, I], restype=ctypes.c_longlong)
         self.declare("rb_ssd_chunk_floats", [I, I], restype=ctypes.c_longlong)
+        self.declare("rb_matrix_memory_chunk_floats", [I, I, I, I], restype=ctypes.c_longlong)
         self.declare("rb_gemm_tc_set_workspace", [P, L])
         self.declare("rb_gemm_tc_plan", [I, I, I, I, I, I, P])
         self.declare("rb_gemm_tc_share_for_test", [I])

@@ -173,6 +173,10 @@ class CudaOps:
         self.gla_in_chunks = True
         #: in bfloat16 mode a state-space mixer takes runs of several tokens in chunks of 64 (else token by token)
         self.ssd_in_chunks = True
+        #: a matrix memory takes runs of several tokens in chunks of 64 (else token by token) from so many tokens on: of a
+        #: run on average, and of the step.  Us token by token and in chunks, 8 heads of 128 x 256: one run of 32 tokens 19,
+        #: 39; of 100 46, 45; of 300 117, 72; 16 runs of 16 tokens 60, 77; of 32 105, 86
+        self.memory_in_chunks, self.memory_chunks_from = True, (24, 128)
         #: a decode step's delta rule (convolution to gate) is one kernel while rows x heads fit the SMs
         self.fuse_delta_step = True
         #: tensor-core products of more than 256 tokens may share a weight tile's inner dimension
@@ -770,10 +774,21 @@ class CudaOps:
         first, count, _, n_seq = self._runs(meta)
         at = p.offsets()
         o = torch.empty((T, H * Dv), dtype=torch.float32, device=self.device)
-        self.lib.call("rb_matrix_memory", _ptr(o), _ptr(proj), proj.stride(0), F32, at["q"], at["k"], at["v"], at["i"],
-                      at["f"], _ptr(p.i_bias), _ptr(p.f_bias), float(p.gate_cap), float(D) ** -0.5, float(p.floor),
-                      _ptr(state["C"]), _ptr(state["n"]), _ptr(state["m"]), _ptr(first), _ptr(count), _ptr(meta.tok_slot),
-                      n_seq, H, D, Dv, self._stream())
+        bias = (_ptr(p.i_bias), _ptr(p.f_bias), float(p.gate_cap), float(D) ** -0.5, float(p.floor))
+        kept = (_ptr(state["C"]), _ptr(state["n"]), _ptr(state["m"]))
+        per_run, per_step = self.memory_chunks_from
+        if first is not None and self.memory_in_chunks and T >= per_run * n_seq and T >= per_step:
+            run0, rows, lens, n_chunks = self._delta_chunks(meta, 64)
+            scratch = torch.empty((self.lib.raw("rb_matrix_memory_chunk_floats")(n_chunks, H, D, Dv),), dtype=torch.float32,
+                                  device=self.device)
+            self.lib.call("rb_matrix_memory_chunked", _ptr(o), _ptr(proj), proj.stride(0), at["q"], at["k"], at["v"], at["i"],
+                          at["f"], *bias, *kept, _ptr(first), _ptr(count), _ptr(run0), _ptr(rows), _ptr(lens),
+                          _ptr(meta.tok_slot), n_seq, n_chunks, H, D, Dv, _ptr(scratch), self._stream(), launches=4)
+        else:
+            moved = torch.empty((n_seq, H, D + 1), dtype=torch.float32, device=self.device)
+            self.lib.call("rb_matrix_memory", _ptr(o), _ptr(proj), proj.stride(0), F32, at["q"], at["k"], at["v"], at["i"],
+                          at["f"], *bias, *kept, _ptr(moved), _ptr(first), _ptr(count), _ptr(meta.tok_slot), n_seq, H, D, Dv,
+                          self._stream())
         out = torch.empty((T, H * Dv), dtype=self.dtype, device=self.device)
         self.lib.call("rb_head_norm_gate", _ptr(out), self.code, _ptr(o), _ptr(p.norm_w), _ptr(proj), proj.stride(0), F32,
                       at["g"], T, H, Dv, float(p.norm_eps), 0, 0, self._stream())

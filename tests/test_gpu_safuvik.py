@@ -242,6 +242,49 @@ def test_matrix_memory_kernel(ops32, H, D, Dv):
         assert float(state["C"][0].abs().max()) == 0.0 and float(state["C"][2].abs().max()) == 0.0
 
 
+@pytest.mark.parametrize("H,D,Dv,lengths", [(2, 16, 24, [64, 1, 65]), (1, 7, 5, [130]), (3, 64, 64, [63, 200, 17]),
+                                            (2, 100, 68, [129, 128]), (8, 128, 256, [90] * 16), (1, 260, 40, [70, 3])])
+@pytest.mark.parametrize("chunks", [True, False])
+def test_matrix_memory_of_several_runs(ops32, H, D, Dv, lengths, chunks):
+    """Runs of unequal lengths side by side (as many as fill the GPU several times over among them), in chunks of 64 at their
+    edges and token by token, in two portions and a decode step for all, against the plain function run by run.  The bound is
+    that of the test above: float32 sums over D and over the tokens, through a quotient and a norm."""
+    from rbitnet_b200.parts.recurrent import MatrixMemory
+    g = torch.Generator().manual_seed(H * 1000 + D + len(lengths))
+    E = 32
+    part = MatrixMemory(E, H, D, Dv, gate_cap=6.0, norm_eps=1e-5)
+    w = {k: torch.randn(*shape, generator=g, dtype=torch.float64) * (0.3 if len(shape) > 1 else 1.0)
+         for k, (shape, _) in part.weight_shapes().items()}
+    w["f.b"] = w["f.b"] + 3.0
+    part.bind({k: v.float().cuda() for k, v in w.items()}, ops32)
+    hs = [torch.randn(n + 1, E, generator=g, dtype=torch.float64) for n in lengths]
+    want = [plain.matrix_memory(w, {"heads": H, "dim": D, "vdim": Dv, "gate_cap": 6.0}, h, 1e-5) for h in hs]
+    state = {k: torch.zeros((len(lengths) + 2, *n.shape), device="cuda") for k, n in part.state_need().items()}
+
+    class Ctx:
+        ops = ops32
+
+        def state_view(self, entry):
+            return state
+    got = [[] for _ in lengths]
+    before = ops32.memory_in_chunks, ops32.memory_chunks_from
+    ops32.memory_in_chunks, ops32.memory_chunks_from = chunks, (1, 1)
+    try:
+        for ends in ([n // 2 for n in lengths], lengths, [n + 1 for n in lengths]):
+            bring = [(i, sum(len(x) for x in got[i]), e) for i, e in enumerate(ends)]
+            bring = [(i, a, e) for i, a, e in bring if e > a]
+            ctx = Ctx()
+            ctx.meta = _meta(ops32, [(i + 1, a, e - a) for i, a, e in bring])
+            out = part.forward(ctx, torch.cat([hs[i][a:e] for i, a, e in bring]).float().cuda(), 0)
+            for (i, _, _), rows in zip(bring, out.cpu().split([e - a for _, a, e in bring])):
+                got[i].append(rows)
+    finally:
+        ops32.memory_in_chunks, ops32.memory_chunks_from = before
+    for rows, one in zip(got, want):
+        assert rel_err(torch.cat(rows), one) <= 2e-4
+    assert float(state["C"][0].abs().max()) == 0.0 and float(state["C"][-1].abs().max()) == 0.0
+
+
 @pytest.mark.parametrize("W,B,K", [(48, 3, 3), (32, 1, 2), (200, 5, 4), (24, 2, 1)])
 def test_gated_recurrence_kernels(ops32, W, B, K):
     from rbitnet_b200.parts.recurrent import GatedLinearRecurrence
