@@ -22,6 +22,7 @@ import torch
 
 from ..parts.base import CacheNeed, StateNeed
 from .allocator import SlotBook, CacheFull, ContextOverflow  # noqa: F401
+from .upload import upload
 
 PAGE_SIZE = 64
 
@@ -102,12 +103,16 @@ class SequenceCache:
             self._state_names[entry] = list(named) if named is not None else None
             for key, one in (((entry, n), v) for n, v in named.items()) if named is not None else ((entry, need),):
                 self.states[key] = torch.zeros((self.n_slots, *one.shape), dtype=one.dtype, device=device)
+        by_dtype: Dict[torch.dtype, list] = {}
+        for st in self.states.values():
+            by_dtype.setdefault(st.dtype, []).append(st)
+        self._states_by_dtype = list(by_dtype.values())
 
     # ---- slots
     def alloc(self) -> int:
         slot = self.book.alloc()
-        for st in self.states.values():
-            st[slot].zero_()
+        for group in self._states_by_dtype:
+            torch._foreach_zero_([st[slot] for st in group])      # one launch for all of a type
         return slot
 
     def free(self, slot: int) -> None:
@@ -137,7 +142,10 @@ class SequenceCache:
         book = self.book
         page, pages, length, most = book.page_size, book.pages, book.length, book.max_seq
         for s in slots:
-            want = length[s] + 1
+            have = length[s]
+            if have % page and have < most:
+                continue                     # the page that holds the last position holds the next one too
+            want = have + 1
             if want > most:
                 self.reserve(s, 1)           # raises ContextOverflow
                 continue
@@ -148,12 +156,15 @@ class SequenceCache:
 
     def advance_one_each(self, slots) -> None:
         """After ``reserve_one_each``: every slot holds one position more."""
-        length = self.book.length
+        length, page = self.book.length, self.book.page_size
         for s in slots:
             length[s] += 1
         if self.book.has_windows:
+            # a page falls behind a window of w keys when the next token's first key, length - w + 1, begins a page
+            first = {(w - 1) % page for w in self.book.windows if w}
             for s in slots:
-                self.book.release_behind_window(s)
+                if length[s] % page in first:
+                    self.book.release_behind_window(s)
 
     def fits(self, lengths, prompts=None) -> bool:
         """Whether new sequences that grow to these lengths fit beside what is live now.  With
@@ -171,14 +182,19 @@ class SequenceCache:
     def upload_tables(self) -> None:
         """Bring the device page tables up to date (rows that changed since the last call)."""
         for g, grp in enumerate(self.groups):
-            for slot in sorted(grp.dirty):
-                n = len(self.book.pages[slot][g]) if slot in self.book.pages else 0
-                if n:
-                    # a pageable copy: staged by the driver before it returns, so the
-                    # host row may change again at once.  (Entries of pages that were given back
-                    # behind a window keep their old number: no kernel reads that far back.)
-                    grp.table[slot, :n].copy_(torch.from_numpy(grp.table_host[slot, :n].copy()))
+            slots = [s for s in sorted(grp.dirty) if s in self.book.pages and self.book.pages[s][g]]
             grp.dirty.clear()
+            if not slots:
+                continue
+            # (Entries of pages that were given back behind a window keep their old number: no kernel reads that far back.)
+            lo, hi = slots[0], slots[-1] + 1
+            if hi - lo <= 2 * len(slots):
+                # neighbours in one copy; rows between them that have not changed get the values they have
+                grp.table[lo:hi].copy_(upload(grp.table_host[lo:hi], grp.table.device))
+            else:
+                for s in slots:
+                    n = len(self.book.pages[s][g])
+                    grp.table[s, :n].copy_(upload(grp.table_host[s, :n], grp.table.device))
 
     # ---- views
     def view(self, entry: int) -> CacheLayerView:

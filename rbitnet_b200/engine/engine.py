@@ -19,7 +19,7 @@ import numpy as np
 import torch
 
 from .. import models  # noqa: F401  (registers the architectures)
-from ..cache import SequenceCache, PAGE_SIZE
+from ..cache import SequenceCache, PAGE_SIZE, upload
 from ..config import ModelConfig, load_config, get_architecture, config_from_dict, ConfigError
 from ..weights import read_model_tensors, random_tensors
 from .generate import GenerationLoop, GenerationResult
@@ -168,22 +168,33 @@ class Engine:
         ``captured``: a step of one token per sequence runs as the captured decode step that
         ``generate`` uses (CUDA graph, padding rows, arg-max sampling whose ids are dropped) instead of
         kernel by kernel, so that its logits can be compared too."""
-        if captured and self.use_graphs and entries and all(len(e.tokens) == 1 for e in entries):
-            slots = [e.slot for e in entries]
-            if len(set(slots)) != len(slots):
+        if captured and self.use_graphs and entries:
+            # one pass over the entries: the host's time between two steps is the GPU's too
+            slots, tokens, rows, wants = [], [], [], True
+            for i, e in enumerate(entries):
+                if len(e.tokens) != 1:
+                    return self.stepper.step(entries)
+                slots.append(e.slot)
+                tokens.append(int(e.tokens[0]))
+                if len(e.want):
+                    rows.append(i)
+                    wants = wants and len(e.want) == 1 and e.want[0] == 0
+            n = len(slots)
+            if len(set(slots)) != n:
                 raise ValueError("a slot appears twice in one step")
             V = self.model.vocab_size
-            for e in entries:
-                if not 0 <= int(e.tokens[0]) < V:
-                    raise ValueError(f"slot {e.slot}: token id out of range (vocabulary {V})")
-                if any(w != 0 for w in e.want):
-                    raise ValueError(f"slot {e.slot}: wanted place is not among its 1 tokens")
-            n = len(entries)
-            self._decode_step([(e.slot, list(e.tokens)) for e in entries], [0.0] * n, [0.0] * n)
-            rows = [i for i, e in enumerate(entries) if len(e.want)]
-            if not rows:
-                return None
-            return self._last_graph.logits[rows].clone()
+            if min(tokens) < 0 or max(tokens) >= V or not wants:
+                for e, token in zip(entries, tokens):
+                    if not 0 <= token < V:
+                        raise ValueError(f"slot {e.slot}: token id out of range (vocabulary {V})")
+                    if any(w != 0 for w in e.want):
+                        raise ValueError(f"slot {e.slot}: wanted place is not among its 1 tokens")
+            ticket = self._launch_rows(slots, tokens, [0.0] * n, [0.0] * n)
+            logits = self._last_graph.logits
+            # asked for before the wait below, so that the copy's launch is not one more thing the GPU waits for
+            out = None if not rows else (logits[:n].clone() if len(rows) == n else logits[rows])
+            self._decode_fetch(ticket)
+            return out
         return self.stepper.step(entries)
 
     def decode_graph(self, batch: int):
@@ -207,11 +218,12 @@ class Engine:
         before, whose tokens and positions that step left on the device (only the uniform numbers are
         copied), which is how a step is launched before the ids of the step before it have been read.
         The sequences' lengths move on at once."""
-        if feed is not None:
-            slots = [s for s, _ in feed]
-            tokens = [t[0] for _, t in feed]
-        else:
-            slots = self._last_slots
+        if feed is None:
+            return self._launch_rows(self._last_slots, None, temperatures, uniforms)
+        return self._launch_rows([s for s, _ in feed], [t[0] for _, t in feed], temperatures, uniforms)
+
+    def _launch_rows(self, slots, tokens, temperatures, uniforms):
+        """The same with the sequences and their tokens (None: the ones on the device) as two lists."""
         n = len(slots)
         positions = self.cache.lengths(slots)
         self.cache.reserve_one_each(slots)
@@ -223,8 +235,8 @@ class Engine:
             uniforms += [0.0] * extra
         self.cache.upload_tables()
         g = self.decode_graph(batch)
-        if feed is not None or g.graph is None:
-            if feed is None:
+        if tokens is not None or g.graph is None:
+            if tokens is None:
                 raise RuntimeError("a decode step without tokens needs the captured step of the launch before it")
             # rows of the padding sequence fill the step up: they rewrite its position 0 and their results are dropped
             g.stage(slots + [self._pad_slot] * extra, tokens + [0] * extra, positions + [0] * extra,
@@ -259,7 +271,7 @@ class Engine:
             return self._decode_step(feed, temperatures, uniforms)   # the error word comes back with the ids
         entries = [StepEntry(slot, toks, [len(toks) - 1]) for slot, toks in feed]
         logits = self.stepper.step(entries)
-        params = torch.from_numpy(np.asarray([temperatures, uniforms], dtype=np.float32)).to(self.ops.device)
+        params = upload(np.asarray([temperatures, uniforms], dtype=np.float32), self.ops.device)
         ids = self.ops.sample(logits, params[0], params[1]).tolist()
         if hasattr(self.ops, "check_errors"):
             self.ops.check_errors()

@@ -18,6 +18,8 @@ from typing import List, Optional, Sequence
 import numpy as np
 import torch
 
+from ..cache.upload import upload
+
 
 @dataclass
 class StepEntry:
@@ -76,7 +78,7 @@ def build_meta(chunks: List[SeqChunk], tokens: np.ndarray, want_rows: np.ndarray
         slot[c.offset:c.offset + c.n_new] = c.slot
     R = int(want_rows.shape[0])
     packed = np.concatenate([tokens.astype(np.int32), pos, slot, want_rows.astype(np.int32)])
-    dev = torch.from_numpy(packed).to(device)       # pageable copy: staged before the call returns
+    dev = upload(packed, device)
     meta = StepMeta(dev[0:T], dev[T:2 * T], dev[2 * T:3 * T], dev[3 * T:3 * T + R], T, R, chunks,
                     all(c.n_new == 1 for c in chunks),
                     max((c.start + c.n_new for c in chunks), default=0))
@@ -94,6 +96,7 @@ class Stepper:
         order of the entries and of each entry's ``want``; None if nothing is wanted."""
         V = self.model.vocab_size
         seen = set()
+        arrays = []
         for e in entries:
             if len(e.tokens) < 1:
                 raise ValueError(f"slot {e.slot}: a step needs at least one token per sequence")
@@ -103,6 +106,7 @@ class Stepper:
             toks = np.asarray(e.tokens)
             if toks.min() < 0 or toks.max() >= V:
                 raise ValueError(f"slot {e.slot}: token id out of range (vocabulary {V})")
+            arrays.append(toks.astype(np.int32))
             for w in e.want:
                 if not 0 <= w < len(e.tokens):
                     raise ValueError(f"slot {e.slot}: wanted place {w} is not among its {len(e.tokens)} tokens")
@@ -128,8 +132,7 @@ class Stepper:
                 outputs.append(out)
             batch, batch_tokens, batch_want, rows = [], [], [], 0
 
-        for e in entries:
-            toks = np.asarray(e.tokens, dtype=np.int32)
+        for e, toks in zip(entries, arrays):
             base = self.cache.length(e.slot)
             want = sorted(e.want)
             if list(want) != list(e.want):

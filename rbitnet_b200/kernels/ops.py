@@ -16,6 +16,7 @@ from typing import List, Optional
 
 import torch
 
+from ..cache.upload import upload
 from .lib import load, KernelError
 
 F32, BF16 = 0, 1
@@ -185,7 +186,9 @@ class CudaOps:
 
     # ------------------------------------------------------------------ helpers
     def _stream(self):
-        return c_void_p(torch.cuda.current_stream(self.device).cuda_stream)
+        # the current stream's handle itself: making a torch.cuda.Stream of it costs a launch's host time again
+        index = self.device.index
+        return c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index))
 
     def _check(self, t: torch.Tensor, dtype, what: str):
         if t.dtype != dtype or not t.is_cuda or not t.is_contiguous():
@@ -614,7 +617,7 @@ class CudaOps:
                 for i in range(0, c.n_new, tokens_per_tile):
                     tok0.append(c.offset + i)
                     ntok.append(min(tokens_per_tile, c.n_new - i))
-            dev = torch.from_numpy(np.asarray([tok0, ntok], dtype=np.int32)).to(self.device)
+            dev = upload(np.asarray([tok0, ntok], dtype=np.int32), self.device)
             meta.extra[key] = (dev[0], dev[1], len(tok0))
         return meta.extra[key]
 
@@ -730,7 +733,7 @@ class CudaOps:
             for i, c in enumerate(meta.seqs):
                 packed[i], packed[n + i] = c.offset, c.n_new
                 packed[2 * n + c.offset:2 * n + c.offset + c.n_new] = c.offset
-            dev = torch.from_numpy(packed).to(self.device)
+            dev = upload(packed, self.device)
             meta.extra[key] = (dev[:n], dev[n:2 * n], dev[2 * n:], n)
         return meta.extra[key]
 
@@ -806,7 +809,7 @@ class CudaOps:
                 for a in range(0, c.n_new, size):
                     rows.append(c.offset + a)
                     lens.append(min(size, c.n_new - a))
-            dev = torch.from_numpy(np.asarray(run0 + rows + lens, dtype=np.int32)).to(self.device)
+            dev = upload(np.asarray(run0 + rows + lens, dtype=np.int32), self.device)
             n, k = len(run0), len(rows)
             meta.extra[key] = (dev[:n], dev[n:n + k], dev[n + k:], k)
         return meta.extra[key]
