@@ -1227,7 +1227,7 @@ RB_EXPORT int rb_gemm_tc_norm_parts(int n_out) { return 4 * ((n_out + BM - 1) / 
 // C (+)= X W^T on the tensor cores.
 //   epilogue 0: C[tokens, n_out] = alpha * product, c_dtype float32 or bfloat16
 //   epilogue 1: C (float32) += alpha * product
-//   (epilogues 0 and 1 with 2..8 splits: the CTAs of a tile form a cluster and each adds up a share
+//   (every epilogue with 2..8 splits: the CTAs of a tile form a cluster and each adds up a share
 //    of the token columns through distributed shared memory, in split order; token tile <= 64)
 //   epilogue 3: W holds, for every 16 output features, 16 gate rows followed by their 16 up rows
 //               (n_out rows in all, a multiple of 32); C[tokens, n_features] = silu(gate)*up

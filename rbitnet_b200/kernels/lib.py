@@ -48,6 +48,8 @@ _SIGNATURES = {
     "rb_route_select_scored": [P, P, P, P, I, I, I, I, I, I, I, P, P],
     "rb_routed_tiles": [I, I, I],
     "rb_routed_plan": [P, P, P, P, I, I, I, I, I, P],
+    "rb_routed_place": [P, P, P, P, L, I, P, P, I, I, I, I, I, I, P],
+    "rb_routed_place_pairs": [],
     "rb_routed_gather": [P, P, L, I, P, I, I, P],
     "rb_routed_combine": [P, L, P, P, L, I, P, P, I, I, I, I, P],
     "rb_gemm_grouped_simple": [P, L, I, P, L, P, L, I, P, I, I, I, I, P],

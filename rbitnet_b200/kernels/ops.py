@@ -170,6 +170,10 @@ class CudaOps:
         self.router_tc_from = 1
         #: products with one matrix per head of many rows run on the tensor cores where the sizes allow it
         self.per_head_on_tensor_cores = True
+        #: gated products of few tokens cut K into parts as the others do
+        self.split_gated = True
+        #: the plan and the gather of a step's few (token, choice) pairs are one kernel
+        self.place_few_pairs = True
         #: so does gated linear attention
         self.gla_in_chunks = True
         #: in bfloat16 mode a state-space mixer takes runs of several tokens in chunks of 64 (else token by token)
@@ -399,6 +403,16 @@ class CudaOps:
         tokens; else up to 8, so that every SM streams a piece of W)."""
         return self.lib.raw("rb_gemm_tc_splits")(T, N, K)
 
+    def _gated_splits(self, T: int, N: int, K: int):
+        """(parts of K, token tile) of a gated product.  Us whole and in parts: 2,816 rows of 2,048, 8 parts: 1 token 11.1, 5.4,
+        64 tokens 15.0, 8.4; 4 parts: 128 tokens 17.2, 11.2; 3,584 rows of 4,096, 8 parts: 8 tokens 19.7, 8.3.  Two parts
+        only beside tiles of 128 and more tokens (3,584 rows, 192 tokens: 25.7, 22.9): 11,264 rows of 2,048 in two parts
+        take 12.8 us for 13.1 alone, no less in a step, and 20.9 for 17.2 with 64 tokens."""
+        splits = self._k_splits(T, N, K) if self.split_gated else 1
+        if splits < 4 and not (splits >= 2 and T > 64):
+            return 1, 0
+        return splits, 64 if T > 64 else 0
+
     def _tensor_core_ok(self, x: torch.Tensor, w: torch.Tensor) -> bool:
         """The tcgen05 product takes bfloat16 operands whose rows TMA can address: inner size and
         row strides multiples of 8 elements, 16-byte aligned bases.  Anything else runs on the
@@ -437,8 +451,8 @@ class CudaOps:
             if weight.bias is not None:
                 self.lib.call("rb_gemm_tc_bias", _ptr(weight.bias), launches=0)
             self.lib.call("rb_gemm_tc", _ptr(out), out.stride(0), self.code, _ptr(x), x.stride(0), T,
-                          _ptr(weight.w), weight.w.stride(0), rows, rows, weight.n_in, 3, weight.inner, 1, 0,
-                          1.0, self._stream())
+                          _ptr(weight.w), weight.w.stride(0), rows, rows, weight.n_in, 3, weight.inner,
+                          *self._gated_splits(T, rows, weight.n_in), 1.0, self._stream())
             return out
         if act is not None:
             if isinstance(x, NormedRows):
@@ -463,8 +477,8 @@ class CudaOps:
             if pending is not None:
                 self._pending_norm(pending)
             self.lib.call("rb_gemm_tc", _ptr(out), out.stride(0), self.code, _ptr(x), x.stride(0), T,
-                          _ptr(weight.w), weight.w.stride(0), rows, rows, weight.n_in, 3, weight.inner, 1, 0,
-                          1.0, self._stream())
+                          _ptr(weight.w), weight.w.stride(0), rows, rows, weight.n_in, 3, weight.inner,
+                          *self._gated_splits(T, rows, weight.n_in), 1.0, self._stream())
             return out
         gu = self.linear(x, LinearWeight(weight.w, rows, weight.n_in))
         self.lib.call("rb_silu_mul", _ptr(out), _ptr(gu), self.code, self.code, T, weight.inner, gu.stride(0),
@@ -1318,14 +1332,14 @@ class CudaOps:
               keep: int, router_tc: Optional[LinearWeight] = None):
         """(ids int32 [T, top], weights float32 [T, top]): softmax of the float32 router product over all outputs; the
         ``top`` largest scores plus ``correction`` among the outputs of the ``keep`` best of ``groups`` equal groups;
-        the weights are the scores themselves.  ``router_tc``: what ``prepare_router`` gave (many tokens then take the
-        tensor-core product for the sums)."""
+        the weights are the scores themselves.  ``router_tc``: what ``prepare_router`` gave (the sums then come from the
+        tensor-core product, for one token too: 17 us with both in one kernel, 8 for the two)."""
         self._check(h, self.dtype, "route input")
         T, K = h.shape
         n = router.shape[0]
         ids = torch.empty((T, top), dtype=torch.int32, device=self.device)
         weights = torch.empty((T, top), dtype=torch.float32, device=self.device)
-        if T >= 64 and router_tc is not None and self._tensor_core_ok(h, router_tc.w):
+        if T >= self.router_tc_from and router_tc is not None and self._tensor_core_ok(h, router_tc.w):
             z = self.linear(h, router_tc, out_dtype=torch.float32)
             self.lib.call("rb_route_select", _ptr(ids), _ptr(weights), _ptr(z), _ptr(correction), T, n, int(top), int(groups),
                           int(keep), self._stream())
@@ -1371,10 +1385,17 @@ class CudaOps:
             rows = n_tiles * tile
             plan = torch.empty((pairs + rows + n_tiles,), dtype=torch.int32, device=self.device)
             pos, row_token, tile_group = plan[:pairs], plan[pairs:pairs + rows], plan[pairs + rows:]
-            self.lib.call("rb_routed_plan", _ptr(pos), _ptr(row_token), _ptr(tile_group), _ptr(ids), pairs, top, n_experts,
-                          tile, n_tiles, self._stream())
             xp = torch.empty((rows, E), dtype=self.dtype, device=self.device)
-            if weight_on_input:
+            place = self.place_few_pairs and pairs <= self.lib.raw("rb_routed_place_pairs")()
+            if place:
+                self.lib.call("rb_routed_place", _ptr(xp), _ptr(pos), _ptr(tile_group), _ptr(h), h.stride(0), self.code, _ptr(ids),
+                              _ptr(weights if weight_on_input else None), pairs, top, n_experts, tile, n_tiles, E, self._stream())
+            else:
+                self.lib.call("rb_routed_plan", _ptr(pos), _ptr(row_token), _ptr(tile_group), _ptr(ids), pairs, top, n_experts,
+                              tile, n_tiles, self._stream())
+            if place:
+                pass
+            elif weight_on_input:
                 self.lib.call("rb_routed_gather_scaled", _ptr(xp), _ptr(h), h.stride(0), self.code, _ptr(row_token), _ptr(pos),
                               _ptr(weights), top, rows, E, self._stream())
             else:

@@ -1,5 +1,6 @@
 """The Vaderax decoder on the GPU: the package's kernels against the plain implementation (whole models in both
 dtypes, the same cases as on the CPU), and each new kernel alone against the plain functions."""
+import ctypes
 import math
 
 import numpy as np
@@ -197,6 +198,72 @@ def test_routed_experts(dtype, T, E, F, n_experts, identity, top):
     before = x.clone()
     part.forward(ctx, h.to(dtype).cuda(), accumulate_into=x)
     assert rel_err((x - before).cpu(), want) <= (1e-5 if dtype == torch.float32 else 2e-2)
+    ops.check_errors()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("weighed", [False, True])
+@pytest.mark.parametrize("T,E,n_experts,top,tile", [(1, 64, 1, 1, 16), (1, 2048, 40, 4, 16), (8, 100, 33, 3, 16), (64, 36, 5, 4, 64),
+                                                    (64, 64, 70, 4, 32), (51, 1032, 3, 5, 16)])
+def test_few_pairs_are_placed_as_many_are(dtype, weighed, T, E, n_experts, top, tile):
+    """rb_routed_place against the plan and the gather: the same tiles for the same experts, every pair's row in one of its
+    expert's rows (in the pairs' order), the same values, zeros elsewhere; identity experts among the ids."""
+    ops = _ops(dtype)
+    g = torch.Generator().manual_seed(T * 100 + E + top)
+    ids = torch.stack([torch.randperm(max(n_experts + 2, top), generator=g)[:top] for _ in range(T)]).to(torch.int32).cuda()
+    weights = torch.rand(T, top, generator=g).cuda()
+    h = torch.randn(T, E, generator=g).to(dtype).cuda()
+    pairs = T * top
+    n_tiles = ops.lib.raw("rb_routed_tiles")(pairs, n_experts, tile)
+    rows = n_tiles * tile
+    ptr = lambda t: ctypes.c_void_p(t.data_ptr() if t is not None else 0)
+    new = lambda *shape, dt=torch.int32: torch.full(shape, -7, dtype=dt, device="cuda")
+    code = 0 if dtype == torch.float32 else 1
+    pos, row_token, groups, xp = new(pairs), new(rows), new(n_tiles), new(rows, E, dt=dtype)
+    ops.lib.call("rb_routed_plan", ptr(pos), ptr(row_token), ptr(groups), ptr(ids), pairs, top, n_experts, tile, n_tiles, ops._stream())
+    if weighed:
+        ops.lib.call("rb_routed_gather_scaled", ptr(xp), ptr(h), h.stride(0), code, ptr(row_token), ptr(pos), ptr(weights), top,
+                     rows, E, ops._stream())
+    else:
+        ops.lib.call("rb_routed_gather", ptr(xp), ptr(h), h.stride(0), code, ptr(row_token), rows, E, ops._stream())
+    pos2, groups2, xp2 = new(pairs), new(n_tiles), new(rows, E, dt=dtype)
+    ops.lib.call("rb_routed_place", ptr(xp2), ptr(pos2), ptr(groups2), ptr(h), h.stride(0), code, ptr(ids),
+                 ptr(weights if weighed else None), pairs, top, n_experts, tile, n_tiles, E, ops._stream())
+    assert torch.equal(groups, groups2)
+    flat = ids.flatten().tolist()
+    at, at2 = pos.tolist(), pos2.tolist()
+    assert [p < 0 for p in at] == [p < 0 for p in at2] == [e >= n_experts for e in flat]
+    taken = [p for p in at2 if p >= 0]
+    assert len(set(taken)) == len(taken)
+    for e in range(n_experts):
+        mine = [p for p, i in zip(at2, flat) if i == e]
+        assert mine == sorted(mine) and sorted(mine) == sorted(p for p, i in zip(at, flat) if i == e)
+    kept = torch.tensor([p >= 0 for p in at])
+    assert torch.equal(xp.cpu()[pos.cpu()[kept].long()], xp2.cpu()[pos2.cpu()[kept].long()])
+    empty = torch.ones(rows, dtype=torch.bool)
+    empty[pos2.cpu()[kept].long()] = False
+    assert float(xp2.cpu()[empty].abs().max()) == 0.0
+
+
+@pytest.mark.parametrize("T,inner,E", [(1, 96, 1024), (16, 1408, 2048), (17, 200, 1032), (64, 48, 1024), (65, 1408, 2048), (200, 96, 4096)])
+@pytest.mark.parametrize("act", [None, (1.702, 7.0, 1.0), "gelu_tanh", "relu"])
+def test_gated_products_with_parts_of_k(T, inner, E, act):
+    """Parts of K in a cluster against K whole: both round the same float32 value once, so a value differs by one step of bfloat16
+    (2^-8 of it) where the sums' last bits decide; with room for the sums' own error, K 2^-24 of their magnitudes."""
+    ops = _ops(torch.bfloat16)
+    g = torch.Generator().manual_seed(T + inner)
+    x = torch.randn(T, E, generator=g).to(torch.bfloat16).cuda()
+    w = ops.prepare_gate_up(*(torch.randn(inner, E, generator=g).to(torch.bfloat16).cuda() / E ** 0.5 for _ in range(2)))
+    before = ops.split_gated
+    try:
+        ops.split_gated = True
+        assert ops._gated_splits(T, w.w.shape[0], E)[0] > 1
+        parts = ops.gated_linear(x, w, act).float()
+        ops.split_gated = False
+        whole = ops.gated_linear(x, w, act).float()
+    finally:
+        ops.split_gated = before
+    assert ((parts - whole).abs() <= 2.0 ** -7 * whole.abs() + 64 * E * 2.0 ** -24).all()
     ops.check_errors()
 
 
