@@ -216,8 +216,11 @@ int launch_delta(dim3 grid, size_t smem, cudaStream_t stream, float* o, const fl
 // One token per sequence: a block per (row, head) does everything between the stacked product and the output product:
 // the convolution of the head's q, k and v channels from the ring of last inputs (and the ring's new row), SiLU, the
 // unit vectors, beta and the decay, one step of the memory for all of the head's value columns (a column on P lanes of
-// R rows each), the norm over the head's outputs, the weight and the SiLU gate.  q and k of a key head are made again by
-// every value head that reads it; the first of them writes their ring rows.
+// R rows each, in neighbouring groups of four), the norm over the head's outputs, the weight and the SiLU gate.  q and k of
+// a key head are made again by every value head that reads it; the first of them writes their ring rows.
+// What bounds it is its chain of loads, sums and barriers: the memory is asked for before the convolution, 16 bytes a
+// lane, every warp makes the sums over q and k for itself, and two barriers are left (2 sequences of 16 heads of 128 x 128:
+// 22.5 us of a step before, 10.5 now).
 template <int R>
 __global__ void __launch_bounds__(1024) delta_step_kernel(
     void* __restrict__ out, int out_bf16, const float* __restrict__ proj, int64_t ld, int g_off, int b_off, int a_off,
@@ -230,54 +233,75 @@ __global__ void __launch_bounds__(1024) delta_step_kernel(
   float* qs = s_step;            // [D]
   float* ks = qs + D;            // [D]
   float* vs = ks + D;            // [Dv]
-  const int t = blockIdx.x, h = blockIdx.y, kvh = h / (H / G), tid = threadIdx.x;
+  const int t = blockIdx.x, h = blockIdx.y, kvh = h / (H / G), tid = threadIdx.x, lane = tid & 31;
   const int C = 2 * G * D + H * Dv;
+  const int p = tid % P, col = tid / P;
+  const bool live = col < Dv;
+  const float a_log = A_log[h], a_bias = dt_bias[h], w_col = live ? norm_w[col] : 0.f;
   rb_pdl_wait();
   const int slot = tok_slot[t], pos = tok_pos[t];
   const float* row = proj + (int64_t)t * ld;
+  // this lane's rows of its column: 4 (p + P g) + {0..3}
+  float* mine = state + (((int64_t)slot * H + h) * Dv + (live ? col : 0)) * D;
+  const bool vec = (D & 3) == 0 && ((uintptr_t)state & 15) == 0;
+  float S[R];
+#pragma unroll
+  for (int g = 0; g < R / 4; ++g) {
+    const int d = 4 * (p + P * g);
+    float v[4] = {0.f, 0.f, 0.f, 0.f};
+    if (live) {
+      if (vec) {
+        if (d < D) rb_load4(mine + d, v);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (d + i < D) v[i] = mine[d + i];
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) S[4 * g + i] = v[i];
+  }
+  const float b_in = row[b_off + h], a_in = row[a_off + h], gate = live && p == 0 ? row[g_off + h * Dv + col] : 0.f;
   const bool writes_qk = h % (H / G) == 0;
   for (int i = tid; i < 2 * D + Dv; i += blockDim.x) {
     const int ch = i < D ? kvh * D + i : (i < 2 * D ? (G + kvh) * D + (i - D) : 2 * G * D + h * Dv + (i - 2 * D));
     const float x0 = row[ch];
     float acc = taps[(int64_t)ch * K + (K - 1)] * x0;
-    for (int d = 1; d < K; ++d) {
-      if (pos - d < 0) break;
-      acc = fmaf(taps[(int64_t)ch * K + (K - 1 - d)], tail[((int64_t)slot * K + (pos - d) % K) * C + ch], acc);
-    }
+#pragma unroll 4
+    for (int d = 1; d < K; ++d)
+      if (pos - d >= 0)
+        acc = fmaf(taps[(int64_t)ch * K + (K - 1 - d)], tail[((int64_t)slot * K + (pos - d) % K) * C + ch], acc);
     if (K > 1 && (i >= 2 * D || writes_qk)) tail[((int64_t)slot * K + pos % K) * C + ch] = x0;
     s_step[i] = acc * sigmoid_(acc);
   }
   __syncthreads();
-  float sq = 0.f, sk = 0.f;
-  for (int d = tid; d < D; d += blockDim.x) { sq = fmaf(qs[d], qs[d], sq); sk = fmaf(ks[d], ks[d], sk); }
-  sq = rb_block_sum(sq, scratch);
-  sk = rb_block_sum(sk, scratch);
-  const float rq = q_scale / sqrtf(sq + unit_eps), rk = 1.0f / sqrtf(sk + unit_eps);
-  float dot = 0.f;
-  for (int d = tid; d < D; d += blockDim.x) {
-    const float a = qs[d] * rq, b = ks[d] * rk;
-    qs[d] = a;
-    ks[d] = b;
+  // |q|^2, |k|^2 and q . k, by every warp for itself
+  float sq = 0.f, sk = 0.f, dot = 0.f;
+  for (int d = lane; d < D; d += 32) {
+    const float a = qs[d], b = ks[d];
+    sq = fmaf(a, a, sq);
+    sk = fmaf(b, b, sk);
     dot = fmaf(a, b, dot);
   }
-  dot = rb_block_sum(dot, scratch);          // (its barriers also make the finished q and k visible)
-  const float beta = sigmoid_(row[b_off + h]);
-  const float g = expf(-expf(A_log[h]) * softplus_(row[a_off + h] + dt_bias[h]));
-  const int p = tid % P, col = tid / P;
-  const bool live = col < Dv;
+  sq = rb_warp_sum(sq);
+  sk = rb_warp_sum(sk);
+  const float rq = q_scale / sqrtf(sq + unit_eps), rk = 1.0f / sqrtf(sk + unit_eps);
+  dot = rb_warp_sum(dot) * rq * rk;
+  const float beta = sigmoid_(b_in);
+  const float g = expf(-expf(a_log) * softplus_(a_in + a_bias));
   float o = 0.f;
   {
     // every thread walks this part, also those beyond the head's columns (with zeros): the lanes of a warp meet in the
     // shuffles below
-    float* mine = state + (((int64_t)slot * H + h) * Dv + (live ? col : 0)) * D;
-    float S[R];
-    float rsum = 0.f, psum = 0.f;
+    constexpr bool KEEP = R <= 16;                   // k's values stay in registers where there is room for them
+    float rsum = 0.f, psum = 0.f, kd[KEEP ? R : 1];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-      const int d = p * R + r;
-      const bool in = live && d < D;
-      S[r] = in ? mine[d] : 0.f;
-      rsum = fmaf(S[r], in ? ks[d] : 0.f, rsum);
+      const int d = 4 * (p + P * (r / 4)) + r % 4;
+      const bool in = d < D;
+      const float k = in ? ks[d] : 0.f;
+      if (KEEP) kd[r] = k;
+      rsum = fmaf(S[r], k, rsum);
       psum = fmaf(S[r], in ? qs[d] : 0.f, psum);
     }
     for (int off = P >> 1; off > 0; off >>= 1) {
@@ -285,20 +309,33 @@ __global__ void __launch_bounds__(1024) delta_step_kernel(
       psum += __shfl_xor_sync(0xffffffffu, psum, off);
     }
     if (live) {
-      const float w = beta * (vs[col] - g * rsum);
+      const float w = beta * (vs[col] - g * (rsum * rk)), wk = w * rk;
 #pragma unroll
-      for (int r = 0; r < R; ++r) {
-        const int d = p * R + r;
-        if (d < D) mine[d] = fmaf(ks[d], w, g * S[r]);
+      for (int x = 0; x < R / 4; ++x) {
+        const int d = 4 * (p + P * x);
+        float v[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[i] = fmaf(KEEP ? kd[4 * x + i] : (d + i < D ? ks[d + i] : 0.f), wk, g * S[4 * x + i]);
+        if (vec) {
+          if (d < D) rb_store4(mine + d, v);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            if (d + i < D) mine[d + i] = v[i];
+        }
       }
-      o = fmaf(w, dot, g * psum);
+      o = fmaf(w, dot, g * (psum * rq));
     }
   }
-  const float ss = rb_block_sum(live && p == 0 ? o * o : 0.f, scratch);
+  // the norm over the head's outputs: the warps' sums of squares, added up by every thread in the same order
+  float ss = rb_warp_sum(live && p == 0 ? o * o : 0.f);
+  if (lane == 0) scratch[tid >> 5] = ss;
+  __syncthreads();
   if (live && p == 0) {
+    ss = 0.f;
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) ss += scratch[w];
     const float r = 1.0f / sqrtf(ss / (float)Dv + norm_eps);
-    const float gate = row[g_off + h * Dv + col];
-    const float y = o * r * norm_w[col] * (gate * sigmoid_(gate));
+    const float y = o * r * w_col * (gate * sigmoid_(gate));
     const int64_t at = ((int64_t)t * H + h) * Dv + col;
     if (out_bf16) ((__nv_bfloat16*)out)[at] = __float2bfloat16_rn(y);
     else ((float*)out)[at] = y;

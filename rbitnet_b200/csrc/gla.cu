@@ -11,7 +11,10 @@
 // gla_scan_kernel    a block per (run, head, tile of value columns).  A column lies on P lanes, each holding R = 16
 //                    channels of it in registers; a chunk of rows' q, k and alpha is staged in shared memory for all
 //                    the block's columns; per row a lane does R decays, R updates and R products, and log2 P
-//                    exchanges finish a column's output.  Token by token: the plain form.
+//                    exchanges finish a column's output.  Token by token: the plain form, and a decode step's: then it
+//                    is bound by reading and writing the memory, whose channels the lanes of a column take in neighbouring
+//                    groups of four, 16 bytes an access (8 sequences of 8 heads of 128 x 256: 17.5 us a
+//                    step with channels p R + r and an access each, 4.9 so).
 // gla_chunk_*        runs of several tokens in chunks of 32, the chain in time only from chunk to chunk (below).
 // gla_step_kernel    a decode step in one launch: decays, the memory's step, the norm per head and the gate.
 #include "rb_common.cuh"
@@ -78,10 +81,25 @@ __global__ void __launch_bounds__(128) gla_scan_kernel(float* __restrict__ o, co
   const int first = seq_first != nullptr ? seq_first[run] : run;
   const int n = seq_count != nullptr ? seq_count[run] : 1;
   const int slot = tok_slot[first];
-  float S[GLA_R];
-  float* mine = state + (((int64_t)slot * H + head) * Dv + j) * D + p * GLA_R;
+  float S[GLA_R];                                  // channels 4 (p + P g) + {0..3}, g = 0..3
+  float* mine = state + (((int64_t)slot * H + head) * Dv + j) * D;
+  const bool vec = (D & 3) == 0 && ((uintptr_t)state & 15) == 0;
 #pragma unroll
-  for (int r = 0; r < GLA_R; ++r) S[r] = (j < Dv && p * GLA_R + r < D) ? mine[r] : 0.f;
+  for (int g = 0; g < GLA_R / 4; ++g) {
+    const int d = 4 * (p + P * g);
+    float v[4] = {0.f, 0.f, 0.f, 0.f};
+    if (j < Dv) {
+      if (vec) {
+        if (d < D) rb_load4(mine + d, v);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (d + i < D) v[i] = mine[d + i];
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) S[4 * g + i] = v[i];
+  }
   for (int t0 = 0; t0 < n; t0 += GLA_CHUNK) {
     const int nt = min(GLA_CHUNK, n - t0);
     __syncthreads();
@@ -104,9 +122,10 @@ __global__ void __launch_bounds__(128) gla_scan_kernel(float* __restrict__ o, co
       float acc = 0.f;
 #pragma unroll
       for (int r4 = 0; r4 < GLA_R; r4 += 4) {
-        const float4 a = *reinterpret_cast<const float4*>(&s_a[i][p * GLA_R + r4]);
-        const float4 k = *reinterpret_cast<const float4*>(&s_k[i][p * GLA_R + r4]);
-        const float4 q = *reinterpret_cast<const float4*>(&s_q[i][p * GLA_R + r4]);
+        const int d = 4 * p + P * r4;
+        const float4 a = *reinterpret_cast<const float4*>(&s_a[i][d]);
+        const float4 k = *reinterpret_cast<const float4*>(&s_k[i][d]);
+        const float4 q = *reinterpret_cast<const float4*>(&s_q[i][d]);
         S[r4 + 0] = fmaf(a.x, S[r4 + 0], k.x * v); acc = fmaf(S[r4 + 0], q.x, acc);
         S[r4 + 1] = fmaf(a.y, S[r4 + 1], k.y * v); acc = fmaf(S[r4 + 1], q.y, acc);
         S[r4 + 2] = fmaf(a.z, S[r4 + 2], k.z * v); acc = fmaf(S[r4 + 2], q.z, acc);
@@ -117,9 +136,19 @@ __global__ void __launch_bounds__(128) gla_scan_kernel(float* __restrict__ o, co
       if (p == 0 && j < Dv) o[((int64_t)(first + t0 + i) * H + head) * Dv + j] = acc;
     }
   }
+  if (j >= Dv) return;
 #pragma unroll
-  for (int r = 0; r < GLA_R; ++r)
-    if (j < Dv && p * GLA_R + r < D) mine[r] = S[r];
+  for (int g = 0; g < GLA_R / 4; ++g) {
+    const int d = 4 * (p + P * g);
+    const float v[4] = {S[4 * g], S[4 * g + 1], S[4 * g + 2], S[4 * g + 3]};
+    if (vec) {
+      if (d < D) rb_store4(mine + d, v);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (d + i < D) mine[d + i] = v[i];
+    }
+  }
 }
 
 template <int P>
