@@ -368,6 +368,7 @@ __global__ void __launch_bounds__(128) delta_chunk_prepare_kernel(
   float* As = Qs + CH * KS;                      // [32][33]: the system's matrix below the diagonal
   float* Lc = As + CH * 33;                      // [32]
   float* Bt = Lc + CH;                           // [32]
+  float* Be = Bt + CH;                           // [32]: beta e^L
   const int chunk = blockIdx.x, h = blockIdx.y, kvh = h / (H / G);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   rb_pdl_wait();
@@ -394,6 +395,7 @@ __global__ void __launch_bounds__(128) delta_chunk_prepare_kernel(
     }
     Lc[lane] = l;
     Bt[lane] = lane < m ? beta[(int64_t)(row0 + lane) * H + h] : 0.f;
+    Be[lane] = Bt[lane] * expf(l);
   }
   __syncthreads();
   {
@@ -424,20 +426,25 @@ __global__ void __launch_bounds__(128) delta_chunk_prepare_kernel(
     if (tid < CH) Lg[((int64_t)chunk * H + h) * CH + tid] = Lc[tid];
   }
   __syncthreads();
-  // one column of the right-hand side per thread and turn: forward substitution down its 32 rows
+  // One column of the right-hand side per thread and turn: its 32 values are asked for together, then forward substitution;
+  // a row that is finished goes into all rows below it at once, so that the chain is 32 steps long and not 496.
   float* Wo = Wg + ((int64_t)chunk * H + h) * CH * D;
   float* Uo = Utg + ((int64_t)chunk * H + h) * CH * Dv;
   for (int c = tid; c < D + Dv; c += 128) {
     float X[CH];
+    if (c < D) {
 #pragma unroll
-    for (int i = 0; i < CH; ++i) {
-      float acc;
-      if (c < D) acc = Bt[i] * expf(Lc[i]) * Ks[i * KS + c];
-      else acc = i < m ? Bt[i] * u[(int64_t)(row0 + i) * ldu + v_off + (c - D)] : 0.f;
+      for (int i = 0; i < CH; ++i) X[i] = Be[i] * Ks[i * KS + c];
+    } else {
 #pragma unroll
-      for (int j = 0; j < i; ++j) acc = fmaf(-As[i * 33 + j], X[j], acc);
-      X[i] = acc;
+      for (int i = 0; i < CH; ++i) X[i] = i < m ? u[(int64_t)(row0 + i) * ldu + v_off + (c - D)] : 0.f;
+#pragma unroll
+      for (int i = 0; i < CH; ++i) X[i] *= Bt[i];
     }
+#pragma unroll
+    for (int j = 0; j < CH; ++j)
+#pragma unroll
+      for (int i = j + 1; i < CH; ++i) X[i] = fmaf(-As[i * 33 + j], X[j], X[i]);
     if (c < D) {
 #pragma unroll
       for (int i = 0; i < CH; ++i) Wo[i * D + c] = X[i];
@@ -448,14 +455,15 @@ __global__ void __launch_bounds__(128) delta_chunk_prepare_kernel(
   }
 }
 
-// grid (runs, H, tiles of CT = 16 value columns), 256 threads (eight warps: two per scheduler, so that one's
-// shared-memory loads run under the other's multiply-adds).  Shared memory: two buffers of a chunk's W, q, k
-// [32][D] each, M [32][32] and L [32], filled a chunk ahead with cp.async; the memory's tile S [D][16], U [32][16] and
-// the chunk's 2 x 32 exponentials.
-constexpr int CCT = 16;
-constexpr int SCAN_NT = 256;              // threads: 16 columns by SCAN_G groups of rows
-constexpr int SCAN_G = SCAN_NT / CCT;      // 16
-constexpr int SCAN_R = CH / SCAN_G;        // rows of a chunk per thread: 2
+// grid (runs, H, tiles of 32 value columns), 512 threads.  A run is a chain of its chunks, so what counts is a chunk's time
+// on one SM: S0's products with W and with q, then the memory's step beside the outputs.  Warps 0..7 make W S0 (U) and the
+// memory's step, warps 8..15 q S0 and the outputs; a thread makes 4 x 4 values, so that a multiply-add costs an eighth of a
+// 16-byte shared-memory load (values by value it was 0.75 loads, and 10.6 us a chunk of 128 x 128 with 16 columns a
+// block, where it is 4.8 now with 32).  Shared memory: two buffers of a chunk's W, q, k [32][D] each, M [32][32] and L [32], filled a chunk
+// ahead with cp.async; the memory's tile S [D][32], of which warps 0..7 also hold their values in registers; U [32][32],
+// U weighted for the memory's step, and the chunk's 32 exponentials.
+constexpr int CCT = 32;
+constexpr int SCAN_NT = 512;
 __device__ __forceinline__ void cp_async16_or_zeros(void* dst, const void* src, bool real) {
   const int bytes = real ? 16 : 0;            // fewer source bytes than 16: the rest is filled with zeros
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(bytes)
@@ -470,13 +478,19 @@ __global__ void __launch_bounds__(SCAN_NT) delta_chunk_scan_kernel(
   rb_pdl_launch_dependents();
   extern __shared__ __align__(16) float s_scan[];
   const int per_buf = 3 * CH * D + CH * CH + CH;
-  float* Ss = s_scan + 2 * per_buf;   // [D][16]
-  float* Us = Ss + D * CCT;           // [32][16]
-  float* Es = Us + CH * CCT;          // [32]: e^{L_i}
-  float* Fs = Es + CH;                // [32]: e^{L_end - L_j}
+  float* Ss = s_scan + 2 * per_buf;   // [D][32]
+  float* Us = Ss + D * CCT;           // [32][32]: U
+  float* Vs = Us + CH * CCT;          // [32][32]: e^{L_end - L_j} U_j
+  float* Es = Vs + CH * CCT;          // [32]: e^{L_i}
   const int run = blockIdx.x, h = blockIdx.y, kvh = h / (H / G), col0 = blockIdx.z * CCT;
-  const int tid = threadIdx.x, c = tid & 15, g8 = tid >> 4;          // column of the tile; one of SCAN_G groups of rows
-  const bool live = col0 + c < Dv;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const bool second = warp >= 8;                 // q's product and the outputs
+  // products with S0: rows 4 (warp mod 8) + {0..3}, columns 4 ct + {0..3}; the sum over d is shared by four lanes, and lane
+  // part `ks` ends up with row 4 (warp mod 8) + ks.  (Eight neighbouring lanes, whose 16-byte loads are served together,
+  // share a row of S0: with neighbours in different rows all four would meet in the same banks.)
+  const int ks = lane >> 3, ct = lane & 7, rows = 4 * (warp & 7), mine_row = rows + ks;
+  // the memory's step: rows 4 dt + {0..3}, columns 4 cs + {0..3}
+  const int cs = tid & 7, dt = tid >> 3;
   rb_pdl_wait();
   const int first = seq_first[run], n = seq_count[run], chunk0 = run_chunk0[run];
   const int slot = tok_slot[first];
@@ -504,9 +518,17 @@ __global__ void __launch_bounds__(SCAN_NT) delta_chunk_scan_kernel(
   copy_chunk(0, 0);
   cp_async_commit();
   float* mine = state + (((int64_t)slot * H + h) * Dv + col0) * D;      // [column][D]
-  for (int i = tid; i < D * CCT; i += SCAN_NT) {
-    const int cc = i / D, d = i - cc * D;
-    Ss[d * CCT + cc] = col0 + cc < Dv ? mine[(int64_t)cc * D + d] : 0.f;
+  const bool steps = !second && 4 * dt < D;      // this thread moves values of the memory on
+  float S[4][4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const bool in = steps && col0 + 4 * cs + j < Dv;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) S[i][j] = in ? mine[(int64_t)(4 * cs + j) * D + 4 * dt + i] : 0.f;
+  }
+  if (steps) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(Ss + (4 * dt + i) * CCT + 4 * cs) = make_float4(S[i][0], S[i][1], S[i][2], S[i][3]);
   }
   for (int ci = 0, buf = 0; ci < n_chunks; ++ci, buf ^= 1) {
     const int row0 = first + ci * CH, m = min(CH, n - ci * CH);
@@ -525,66 +547,112 @@ __global__ void __launch_bounds__(SCAN_NT) delta_chunk_scan_kernel(
     const float* Ms = Kc + CH * D;
     const float* Ls = Ms + CH * CH;
     // asked for now, used after the products
-    const float* Ut = Utg + item * CH * Dv;
-    float ut[SCAN_R];
+    float ut[4] = {0.f, 0.f, 0.f, 0.f};
+    if (!second) {
+      const float* Ut = Utg + (item * CH + mine_row) * Dv + col0 + 4 * ct;
 #pragma unroll
-    for (int r = 0; r < SCAN_R; ++r) ut[r] = live ? Ut[(int64_t)(g8 + SCAN_G * r) * Dv + col0 + c] : 0.f;
-    if (tid < CH) {
-      Es[tid] = expf(Ls[tid]);
-      Fs[tid] = expf(Ls[CH - 1] - Ls[tid]);
+      for (int j = 0; j < 4; ++j)
+        if (col0 + 4 * ct + j < Dv) ut[j] = Ut[j];
     }
-    // rows i = g8 + SCAN_G r (r < SCAN_R) of column c:  W S and Q S
-    float ws[SCAN_R], qs[SCAN_R];
+    if (tid < CH) Es[tid] = expf(Ls[tid]);
+    // four rows of W (of q) times S0
+    float acc[4][4];
 #pragma unroll
-    for (int r = 0; r < SCAN_R; ++r) ws[r] = qs[r] = 0.f;
-    for (int d = 0; d < D; d += 4) {
-      const float s0 = Ss[d * CCT + c], s1 = Ss[(d + 1) * CCT + c], s2 = Ss[(d + 2) * CCT + c], s3 = Ss[(d + 3) * CCT + c];
+    for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int r = 0; r < SCAN_R; ++r) {
-        const int i = g8 + SCAN_G * r;
-        const float4 w4 = *reinterpret_cast<const float4*>(Ws + i * D + d);
-        const float4 q4 = *reinterpret_cast<const float4*>(Qs + i * D + d);
-        ws[r] = fmaf(w4.x, s0, fmaf(w4.y, s1, fmaf(w4.z, s2, fmaf(w4.w, s3, ws[r]))));
-        qs[r] = fmaf(q4.x, s0, fmaf(q4.y, s1, fmaf(q4.z, s2, fmaf(q4.w, s3, qs[r]))));
-      }
-    }
+      for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+    const float* A = (second ? Qs : Ws) + rows * D;
+#pragma unroll 2
+    for (int d = 4 * ks; d < D; d += 16) {
+      float4 a[4], b[4];
 #pragma unroll
-    for (int r = 0; r < SCAN_R; ++r) Us[(g8 + SCAN_G * r) * CCT + c] = ut[r] - ws[r];
-    __syncthreads();
-    // the chunk's outputs: e^{L_i} (Q S)_i + sum_{j <= i} M_ij U_j
+      for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const float4*>(A + i * D + d);
 #pragma unroll
-    for (int r = 0; r < SCAN_R; ++r) {
-      const int i = g8 + SCAN_G * r;
-      float acc = Es[i] * qs[r];
-      for (int j = 0; j <= i; ++j) acc = fmaf(Ms[i * CH + j], Us[j * CCT + c], acc);
-      if (live && i < m) o[((int64_t)(row0 + i) * H + h) * Dv + col0 + c] = acc;
-    }
-    // the memory moves on: S <- e^{L_end} S + sum_j e^{L_end - L_j} k_j U_j, rows d = d0 + g8 + SCAN_G r of column c
-    const float keep = Es[CH - 1];
-    for (int d0 = 0; d0 < D; d0 += 8 * SCAN_G) {
-      float acc[8];
+      for (int x = 0; x < 4; ++x) b[x] = *reinterpret_cast<const float4*>(Ss + (d + x) * CCT + 4 * ct);
 #pragma unroll
-      for (int r = 0; r < 8; ++r) acc[r] = 0.f;
-      for (int j = 0; j < CH; ++j) {
-        const float uj = Fs[j] * Us[j * CCT + c];
+      for (int i = 0; i < 4; ++i) {
+        const float ai[4] = {a[i].x, a[i].y, a[i].z, a[i].w};
 #pragma unroll
-        for (int r = 0; r < 8; ++r) {
-          const int d = d0 + g8 + SCAN_G * r;
-          if (d < D) acc[r] = fmaf(Kc[j * D + d], uj, acc[r]);
+        for (int x = 0; x < 4; ++x) {
+          acc[i][0] = fmaf(ai[x], b[x].x, acc[i][0]);
+          acc[i][1] = fmaf(ai[x], b[x].y, acc[i][1]);
+          acc[i][2] = fmaf(ai[x], b[x].z, acc[i][2]);
+          acc[i][3] = fmaf(ai[x], b[x].w, acc[i][3]);
         }
       }
-      // (every thread read the old S in the products above, before the barrier that followed them)
+    }
+    // the four lanes' shares: after two exchanges lane ks has row ks
+    float sum[4];
 #pragma unroll
-      for (int r = 0; r < 8; ++r) {
-        const int d = d0 + g8 + SCAN_G * r;
-        if (d < D) Ss[d * CCT + c] = fmaf(keep, Ss[d * CCT + c], acc[r]);
+    for (int j = 0; j < 4; ++j) {
+      const float k0 = (ks & 1) ? acc[1][j] : acc[0][j], s0 = (ks & 1) ? acc[0][j] : acc[1][j];
+      const float k1 = (ks & 1) ? acc[3][j] : acc[2][j], s1 = (ks & 1) ? acc[2][j] : acc[3][j];
+      const float r0 = k0 + __shfl_xor_sync(0xffffffffu, s0, 8), r1 = k1 + __shfl_xor_sync(0xffffffffu, s1, 8);
+      sum[j] = ((ks & 2) ? r1 : r0) + __shfl_xor_sync(0xffffffffu, (ks & 2) ? r0 : r1, 16);
+    }
+    if (!second) {
+      const float f = expf(Ls[CH - 1] - Ls[mine_row]);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) sum[j] = ut[j] - sum[j];
+      *reinterpret_cast<float4*>(Us + mine_row * CCT + 4 * ct) = make_float4(sum[0], sum[1], sum[2], sum[3]);
+      *reinterpret_cast<float4*>(Vs + mine_row * CCT + 4 * ct) = make_float4(f * sum[0], f * sum[1], f * sum[2], f * sum[3]);
+    }
+    __syncthreads();                  // U is there, and every thread has read the old S
+    if (second) {
+      // the chunk's outputs: e^{L_i} (q S0)_i + sum_{j <= i} M_ij U_j (M is zero above the diagonal)
+      const float e = Es[mine_row];
+      float out[4] = {e * sum[0], e * sum[1], e * sum[2], e * sum[3]};
+#pragma unroll 4
+      for (int j = 0; j < CH; j += 4) {
+        const float4 m4 = *reinterpret_cast<const float4*>(Ms + mine_row * CH + j);
+        const float mj[4] = {m4.x, m4.y, m4.z, m4.w};
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+          const float4 u4 = *reinterpret_cast<const float4*>(Us + (j + x) * CCT + 4 * ct);
+          out[0] = fmaf(mj[x], u4.x, out[0]);
+          out[1] = fmaf(mj[x], u4.y, out[1]);
+          out[2] = fmaf(mj[x], u4.z, out[2]);
+          out[3] = fmaf(mj[x], u4.w, out[3]);
+        }
       }
+      if (mine_row < m) {
+        float* to = o + ((int64_t)(row0 + mine_row) * H + h) * Dv + col0 + 4 * ct;
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (col0 + 4 * ct + j < Dv) to[j] = out[j];
+      }
+    } else if (steps) {
+      // the memory moves on: S <- e^{L_end} S + sum_j k_j e^{L_end - L_j} U_j
+      const float keep = Es[CH - 1];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) S[i][j] *= keep;
+#pragma unroll 4
+      for (int j = 0; j < CH; ++j) {
+        const float4 k4 = *reinterpret_cast<const float4*>(Kc + j * D + 4 * dt);
+        const float4 u4 = *reinterpret_cast<const float4*>(Vs + j * CCT + 4 * cs);
+        const float ki[4] = {k4.x, k4.y, k4.z, k4.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          S[i][0] = fmaf(ki[i], u4.x, S[i][0]);
+          S[i][1] = fmaf(ki[i], u4.y, S[i][1]);
+          S[i][2] = fmaf(ki[i], u4.z, S[i][2]);
+          S[i][3] = fmaf(ki[i], u4.w, S[i][3]);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(Ss + (4 * dt + i) * CCT + 4 * cs) = make_float4(S[i][0], S[i][1], S[i][2], S[i][3]);
     }
     __syncthreads();                  // before the copies of the chunk after the next overwrite this buffer, and U and the exponentials change
   }
-  for (int i = tid; i < D * CCT; i += SCAN_NT) {
-    const int cc = i / D, d = i - cc * D;
-    if (col0 + cc < Dv) mine[(int64_t)cc * D + d] = Ss[d * CCT + cc];
+  if (steps) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (col0 + 4 * cs + j < Dv) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) mine[(int64_t)(4 * cs + j) * D + 4 * dt + i] = S[i][j];
+      }
   }
 }
 
@@ -659,14 +727,14 @@ RB_EXPORT int rb_gated_delta_chunked(float* o, const float* u, int64_t ldu, cons
   float* Mg = Utg + items * CH * Dv;
   float* Lg = Mg + items * CH * CH;
   RB_REQUIRE(n_chunks <= 2147483647 / 1 && H <= 65535, "rb_gated_delta_chunked: too many heads");
-  const size_t smem_a = (size_t)(2 * CH * (D + 4) + CH * 33 + 2 * CH) * sizeof(float);
-  const size_t smem_b = (size_t)(2 * (3 * CH * D + CH * CH + CH) + D * CCT + CH * CCT + 2 * CH) * sizeof(float);
+  const size_t smem_a = (size_t)(2 * CH * (D + 4) + CH * 33 + 3 * CH) * sizeof(float);
+  const size_t smem_b = (size_t)(2 * (3 * CH * D + CH * CH + CH) + D * CCT + 2 * CH * CCT + CH) * sizeof(float);
   static RbOncePerDevice configured;
   if (configured.first()) {
     RB_CUDA(cudaFuncSetAttribute(delta_chunk_prepare_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
-    RB_CUDA(cudaFuncSetAttribute(delta_chunk_scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024));
+    RB_CUDA(cudaFuncSetAttribute(delta_chunk_scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 132 * 1024));
   }
-  RB_REQUIRE(smem_a <= 64 * 1024 && smem_b <= 128 * 1024, "rb_gated_delta_chunked: key size %d needs too much shared memory", D);
+  RB_REQUIRE(smem_a <= 64 * 1024 && smem_b <= 132 * 1024, "rb_gated_delta_chunked: key size %d needs too much shared memory", D);
   RB_LAUNCH("delta_chunk_prepare_kernel", (delta_chunk_prepare_kernel), dim3(n_chunks, H), 128, smem_a, stream, Wg, Utg, Mg, Lg, u,
             ldu, beta, log_decay, chunk_row, chunk_len, H, G, D, Dv);
   RB_CHECK_LAUNCH("rb_gated_delta_chunked");

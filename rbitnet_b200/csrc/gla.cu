@@ -174,8 +174,8 @@ int launch_scan(float* o, const float* rows, int64_t ld, int q_off, int k_off, i
 // (chunk, head) at once; the second walks a run's chunks with the memory: two small products per chunk.  A chunk's
 // missing tokens (the run's end) count as decay 1 and k = q = v = 0.
 constexpr int GCH = 32;          // tokens of a chunk
-constexpr int GCT = 16;          // value columns of a block of the second kernel
-constexpr int GSCAN_NT = 256;
+constexpr int GCT = 32;          // value columns of a block of the second kernel
+constexpr int GSCAN_NT = 512;
 
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
@@ -272,9 +272,12 @@ __global__ void __launch_bounds__(128) gla_chunk_prepare_kernel(float* __restric
   for (int d = tid; d < D; d += 128) Eo[d] = expf(Bs[(GCH - 1) * KS + d]);
 }
 
-// grid (runs, H, tiles of 16 value columns), 256 threads.  Shared memory: two buffers of a chunk's item (as the first
-// kernel left it) and the tile's values [32][16], filled a chunk ahead with cp.async; the memory's tile S [16][D + 4]
-// twice: a chunk reads one and writes the other, so that its read-out and its update need no barrier between them.
+// grid (runs, H, tiles of 32 value columns), 512 threads.  A run is a chain of its chunks, so what counts is a chunk's time on
+// one SM.  Warps 0..7 move the memory on, 4 x 4 values a thread that stay in registers and are left in shared memory for the
+// others; warps 8..15 make the outputs from what the chunk starts from, beside them.  Shared memory: two buffers of a
+// chunk's item (as the first kernel left it) and the tile's values [32][32], filled a chunk ahead with cp.async; the memory's
+// tile S [D][32] twice: a chunk reads one and writes the other, so that a chunk has one barrier.
+// (With 16 columns and a value or two a thread: 4.6 us a chunk of 128 channels, 3.2 now.)
 __global__ void __launch_bounds__(GSCAN_NT) gla_chunk_scan_kernel(
     float* __restrict__ o, const float* __restrict__ scratch, const float* __restrict__ rows, int64_t ld, int v_off,
     float* __restrict__ state, const int* __restrict__ seq_first, const int* __restrict__ seq_count,
@@ -283,11 +286,17 @@ __global__ void __launch_bounds__(GSCAN_NT) gla_chunk_scan_kernel(
   extern __shared__ __align__(16) float s_gscan[];
   const int item_floats = gla_item_floats(D);
   const int per_buf = item_floats + GCH * GCT;
-  const int SS = D + 4;
-  float* Sa = s_gscan + 2 * per_buf;    // [16][D + 4]: the memory as this chunk finds it
-  float* Sb = Sa + GCT * SS;            // the memory as this chunk leaves it (the two change places after every chunk)
+  float* Sa = s_gscan + 2 * per_buf;    // [D][32]: the memory as this chunk finds it
+  float* Sb = Sa + D * GCT;             // the memory as this chunk leaves it (the two change places after every chunk)
   const int run = blockIdx.x, h = blockIdx.y, col0 = blockIdx.z * GCT;
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const bool second = warp >= 8;        // the outputs
+  // outputs: rows 4 (warp - 8) + {0..3}, columns 4 ct + {0..3}; the sum over the channels is shared by four lanes, and part
+  // ks ends up with row 4 (warp - 8) + ks.  (Eight neighbouring lanes, whose 16-byte loads are served together, read one row
+  // of S.)
+  const int ks = lane >> 3, ct = lane & 7, r0 = 4 * (warp & 7), mine_row = r0 + ks;
+  // the memory's step: channels 4 dt + {0..3}, columns 4 cs + {0..3}
+  const int cs = tid & 7, dt = tid >> 3;
   rb_pdl_wait();
   const int first = seq_first[run], n = seq_count[run], chunk0 = run_chunk0[run];
   const int slot = tok_slot[first];
@@ -297,7 +306,7 @@ __global__ void __launch_bounds__(GSCAN_NT) gla_chunk_scan_kernel(
     float* dst = s_gscan + (size_t)buf * per_buf;
     for (int i = tid; i < (item_floats >> 2); i += GSCAN_NT) cp_async16(dst + 4 * i, src + 4 * i);
     if (tid < GCH * GCT / 4) {
-      const int j = tid >> 2, c4 = (tid & 3) << 2;
+      const int j = tid >> 3, c4 = (tid & 7) << 2;
       const bool real = j < m && col0 + c4 < Dv;
       const float* v = real ? rows + (int64_t)(row0 + j) * ld + v_off + h * Dv + col0 + c4 : rows;
       cp_async16_or_zeros(dst + item_floats + j * GCT + c4, v, real);
@@ -307,12 +316,16 @@ __global__ void __launch_bounds__(GSCAN_NT) gla_chunk_scan_kernel(
   copy_chunk(0, 0);
   cp_async_commit();
   float* mine = state + (((int64_t)slot * H + h) * Dv + col0) * D;      // [column][D]
-  for (int i = tid; i < D * GCT; i += GSCAN_NT) {
-    const int cc = i / D, d = i - cc * D;
-    Sa[cc * SS + d] = col0 + cc < Dv ? mine[(int64_t)cc * D + d] : 0.f;
+  const bool steps = !second && 4 * dt < D;
+  float S[4][4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) S[i][j] = steps && col0 + 4 * cs + j < Dv ? mine[(int64_t)(4 * cs + j) * D + 4 * dt + i] : 0.f;
+  if (steps) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(Sa + (4 * dt + i) * GCT + 4 * cs) = make_float4(S[i][0], S[i][1], S[i][2], S[i][3]);
   }
-  const int c = tid & 15, g = tid >> 4;              // read-out: column c, rows g and g + 16
-  const int dq = (tid & 31) << 2, cp = (tid >> 5) << 1;   // update: channels dq .. dq + 3 of columns cp and cp + 1
   for (int ci = 0, buf = 0; ci < n_chunks; ++ci, buf ^= 1) {
     const int row0 = first + ci * GCH, m = min(GCH, n - ci * GCH);
     cp_async_wait<0>();
@@ -329,60 +342,93 @@ __global__ void __launch_bounds__(GSCAN_NT) gla_chunk_scan_kernel(
     const float* Ms = Kt + GCH * D;
     const float* Es = Ms + GCH * GCH;
     const float* Vs = Qt + item_floats;
-    {
-      float acc0 = 0.f, acc1 = 0.f;
-      const float* s = Ss + c * SS;
-      const float* q0 = Qt + g * D;
-      const float* q1 = Qt + (g + 16) * D;
-      for (int d = 0; d < D; d += 4) {
-        const float4 s4 = *reinterpret_cast<const float4*>(s + d);
-        const float4 a4 = *reinterpret_cast<const float4*>(q0 + d);
-        const float4 b4 = *reinterpret_cast<const float4*>(q1 + d);
-        acc0 = fmaf(a4.x, s4.x, fmaf(a4.y, s4.y, fmaf(a4.z, s4.z, fmaf(a4.w, s4.w, acc0))));
-        acc1 = fmaf(b4.x, s4.x, fmaf(b4.y, s4.y, fmaf(b4.z, s4.z, fmaf(b4.w, s4.w, acc1))));
-      }
-      // M is zero above its diagonal, so both rows take all 32 columns: a loop of fixed length whose loads run ahead
-      const float4* m0 = reinterpret_cast<const float4*>(Ms + g * GCH);
-      const float4* m1 = reinterpret_cast<const float4*>(Ms + (g + 16) * GCH);
+    if (second) {
+      float acc[4][4];
 #pragma unroll
-      for (int j4 = 0; j4 < GCH / 4; ++j4) {
-        const float4 a4 = m0[j4], b4 = m1[j4];
-        const float v0 = Vs[(4 * j4 + 0) * GCT + c], v1 = Vs[(4 * j4 + 1) * GCT + c];
-        const float v2 = Vs[(4 * j4 + 2) * GCT + c], v3 = Vs[(4 * j4 + 3) * GCT + c];
-        acc0 = fmaf(a4.x, v0, fmaf(a4.y, v1, fmaf(a4.z, v2, fmaf(a4.w, v3, acc0))));
-        acc1 = fmaf(b4.x, v0, fmaf(b4.y, v1, fmaf(b4.z, v2, fmaf(b4.w, v3, acc1))));
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+      const float* A = Qt + r0 * D;
+#pragma unroll 2
+      for (int d = 4 * ks; d < D; d += 16) {
+        float4 a[4], b[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const float4*>(A + i * D + d);
+#pragma unroll
+        for (int x = 0; x < 4; ++x) b[x] = *reinterpret_cast<const float4*>(Ss + (d + x) * GCT + 4 * ct);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float ai[4] = {a[i].x, a[i].y, a[i].z, a[i].w};
+#pragma unroll
+          for (int x = 0; x < 4; ++x) {
+            acc[i][0] = fmaf(ai[x], b[x].x, acc[i][0]);
+            acc[i][1] = fmaf(ai[x], b[x].y, acc[i][1]);
+            acc[i][2] = fmaf(ai[x], b[x].z, acc[i][2]);
+            acc[i][3] = fmaf(ai[x], b[x].w, acc[i][3]);
+          }
+        }
       }
-      if (col0 + c < Dv) {
-        if (g < m) o[((int64_t)(row0 + g) * H + h) * Dv + col0 + c] = acc0;
-        if (g + 16 < m) o[((int64_t)(row0 + g + 16) * H + h) * Dv + col0 + c] = acc1;
+      // the four lanes' shares: after two exchanges lane part ks has its row
+      float out[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float k0 = (ks & 1) ? acc[1][j] : acc[0][j], s0 = (ks & 1) ? acc[0][j] : acc[1][j];
+        const float k1 = (ks & 1) ? acc[3][j] : acc[2][j], s1 = (ks & 1) ? acc[2][j] : acc[3][j];
+        const float v0 = k0 + __shfl_xor_sync(0xffffffffu, s0, 8), v1 = k1 + __shfl_xor_sync(0xffffffffu, s1, 8);
+        out[j] = ((ks & 2) ? v1 : v0) + __shfl_xor_sync(0xffffffffu, (ks & 2) ? v0 : v1, 16);
       }
-    }
-    // the memory moves on into the other buffer, so that no thread waits here for the read-outs of the others
-    if (dq < D) {
-      float4 a0 = make_float4(0.f, 0.f, 0.f, 0.f), a1 = a0;
-#pragma unroll 8
+      // M is zero above its diagonal: a loop of fixed length whose loads run ahead
+#pragma unroll 4
+      for (int j = 0; j < GCH; j += 4) {
+        const float4 m4 = *reinterpret_cast<const float4*>(Ms + mine_row * GCH + j);
+        const float mj[4] = {m4.x, m4.y, m4.z, m4.w};
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+          const float4 v4 = *reinterpret_cast<const float4*>(Vs + (j + x) * GCT + 4 * ct);
+          out[0] = fmaf(mj[x], v4.x, out[0]);
+          out[1] = fmaf(mj[x], v4.y, out[1]);
+          out[2] = fmaf(mj[x], v4.z, out[2]);
+          out[3] = fmaf(mj[x], v4.w, out[3]);
+        }
+      }
+      if (mine_row < m) {
+        float* to = o + ((int64_t)(row0 + mine_row) * H + h) * Dv + col0 + 4 * ct;
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (col0 + 4 * ct + j < Dv) to[j] = out[j];
+      }
+    } else if (steps) {
+      // S <- diag(e^{B_end}) S + sum_j Kt_j v_j
+      const float4 e4 = *reinterpret_cast<const float4*>(Es + 4 * dt);
+      const float e[4] = {e4.x, e4.y, e4.z, e4.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) S[i][j] *= e[i];
+#pragma unroll 4
       for (int j = 0; j < GCH; ++j) {
-        const float4 k4 = *reinterpret_cast<const float4*>(Kt + j * D + dq);
-        const float2 v2 = *reinterpret_cast<const float2*>(Vs + j * GCT + cp);
-        a0.x = fmaf(k4.x, v2.x, a0.x); a0.y = fmaf(k4.y, v2.x, a0.y); a0.z = fmaf(k4.z, v2.x, a0.z); a0.w = fmaf(k4.w, v2.x, a0.w);
-        a1.x = fmaf(k4.x, v2.y, a1.x); a1.y = fmaf(k4.y, v2.y, a1.y); a1.z = fmaf(k4.z, v2.y, a1.z); a1.w = fmaf(k4.w, v2.y, a1.w);
+        const float4 k4 = *reinterpret_cast<const float4*>(Kt + j * D + 4 * dt);
+        const float4 v4 = *reinterpret_cast<const float4*>(Vs + j * GCT + 4 * cs);
+        const float ki[4] = {k4.x, k4.y, k4.z, k4.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          S[i][0] = fmaf(ki[i], v4.x, S[i][0]);
+          S[i][1] = fmaf(ki[i], v4.y, S[i][1]);
+          S[i][2] = fmaf(ki[i], v4.z, S[i][2]);
+          S[i][3] = fmaf(ki[i], v4.w, S[i][3]);
+        }
       }
-      const float4 e4 = *reinterpret_cast<const float4*>(Es + dq);
-      float4 x = *reinterpret_cast<const float4*>(Ss + cp * SS + dq);
-      float4 y = *reinterpret_cast<const float4*>(Ss + (cp + 1) * SS + dq);
-      float4* s0 = reinterpret_cast<float4*>(Sn + cp * SS + dq);
-      float4* s1 = reinterpret_cast<float4*>(Sn + (cp + 1) * SS + dq);
-      x.x = fmaf(e4.x, x.x, a0.x); x.y = fmaf(e4.y, x.y, a0.y); x.z = fmaf(e4.z, x.z, a0.z); x.w = fmaf(e4.w, x.w, a0.w);
-      y.x = fmaf(e4.x, y.x, a1.x); y.y = fmaf(e4.y, y.y, a1.y); y.z = fmaf(e4.z, y.z, a1.z); y.w = fmaf(e4.w, y.w, a1.w);
-      *s0 = x;
-      *s1 = y;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(Sn + (4 * dt + i) * GCT + 4 * cs) = make_float4(S[i][0], S[i][1], S[i][2], S[i][3]);
     }
   }
-  __syncthreads();
-  const float* Se = (n_chunks & 1) ? Sb : Sa;
-  for (int i = tid; i < D * GCT; i += GSCAN_NT) {
-    const int cc = i / D, d = i - cc * D;
-    if (col0 + cc < Dv) mine[(int64_t)cc * D + d] = Se[cc * SS + d];
+  if (steps) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (col0 + 4 * cs + j < Dv) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) mine[(int64_t)(4 * cs + j) * D + 4 * dt + i] = S[i][j];
+      }
   }
 }
 
@@ -463,7 +509,7 @@ RB_EXPORT int rb_gla_chunked(float* o, const float* rows, int64_t ld, int q_off,
                  (uintptr_t)scratch % 16 == 0 && (uintptr_t)log_alpha % 16 == 0,
              "rb_gla_chunked: bad sizes H=%d D=%d Dv=%d", H, D, Dv);
   const size_t smem_a = (size_t)(3 * GCH * (D + 4)) * sizeof(float);
-  const size_t smem_b = (size_t)(2 * (gla_item_floats(D) + GCH * GCT) + 2 * GCT * (D + 4)) * sizeof(float);
+  const size_t smem_b = (size_t)(2 * (gla_item_floats(D) + GCH * GCT) + 2 * GCT * D) * sizeof(float);
   static RbOncePerDevice configured;
   if (configured.first()) {
     RB_CUDA(cudaFuncSetAttribute(gla_chunk_prepare_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
