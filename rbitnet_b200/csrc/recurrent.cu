@@ -56,6 +56,75 @@ __global__ void conv_causal_kernel(float* __restrict__ u, const TI* __restrict__
   }
 }
 
+// The same for many float32 rows: a thread keeps the last K inputs of four neighbouring channels in registers while it goes
+// down a block's rows, so that an input is read once and not K times, 16 bytes a load, eight rows on their way at a time.  The
+// same sums in the same order.  Bound by the bytes of its rows (2,048 rows of 2,048 channels, K 4: 33 us before, 7.9 now; about 2,500 of 4,096 80 and 39;
+// the rows alone take 5 and 12).
+constexpr int CONV_ROWS = 16, CONV_AHEAD = 8;
+template <int K>
+__global__ void __launch_bounds__(128) conv_causal_rows_kernel(float* __restrict__ u, const float* __restrict__ x, int64_t ldx, int x_off,
+                                                               const float* __restrict__ x_bias, const float* __restrict__ taps,
+                                                               const float* __restrict__ conv_bias, const float* __restrict__ tail,
+                                                               const int* __restrict__ tok_first, const int* __restrict__ tok_slot,
+                                                               const int* __restrict__ tok_pos, int T, int C, int silu) {
+  rb_pdl_launch_dependents();
+  const int c = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
+  if (c >= C) return;
+  float w[K][4], b[4], xb[4], hist[K][4];                // hist[d]: the input (with its bias) d rows back; d = 0: this row's
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    b[i] = conv_bias != nullptr ? conv_bias[c + i] : 0.f;
+    xb[i] = x_bias != nullptr ? x_bias[c + i] : 0.f;
+#pragma unroll
+    for (int d = 0; d < K; ++d) w[d][i] = taps[(int64_t)(c + i) * K + K - 1 - d];
+  }
+  rb_pdl_wait();
+  const int t0 = blockIdx.x * CONV_ROWS, t1 = min(T, t0 + CONV_ROWS);
+  int run = -1;
+  for (int ta = t0; ta < t1; ta += CONV_AHEAD) {
+    float in[CONV_AHEAD][4];
+#pragma unroll
+    for (int r = 0; r < CONV_AHEAD; ++r)
+      if (ta + r < t1) rb_load4(x + (int64_t)(ta + r) * ldx + x_off + c, in[r]);
+#pragma unroll
+    for (int r = 0; r < CONV_AHEAD; ++r) {
+      const int t = ta + r;
+      if (t >= t1) break;
+      const int first = tok_first != nullptr ? tok_first[t] : t;
+      if (first != run) {                                // a new run, or the block's first row: fetch the rows before
+        run = first;
+        const int slot = tok_slot[t], pos = tok_pos[t];
+#pragma unroll
+        for (int d = 1; d < K; ++d) {
+          if (t - d >= first) {
+            rb_load4(x + (int64_t)(t - d) * ldx + x_off + c, hist[d]);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) hist[d][i] += xb[i];
+          } else if (pos - d < 0) {
+            hist[d][0] = hist[d][1] = hist[d][2] = hist[d][3] = 0.f;
+          } else {
+            rb_load4(tail + ((int64_t)slot * K + (pos - d) % K) * C + c, hist[d]);
+          }
+        }
+      }
+      float y[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        hist[0][i] = in[r][i] + xb[i];
+        float acc = b[i];
+#pragma unroll
+        for (int d = 0; d < K; ++d) acc = fmaf(w[d][i], hist[d][i], acc);
+        y[i] = silu ? acc * sigmoidf_(acc) : acc;
+      }
+      rb_store4(u + (int64_t)t * C + c, y);
+#pragma unroll
+      for (int d = K - 1; d > 0; --d)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) hist[d][i] = hist[d - 1][i];
+    }
+  }
+}
+
 // The ring of a convolution's last inputs moves on to the end of every run: the inputs (with their bias) of the
 // run's last K-1 positions go to their rows.  For a mixer whose recurrence kernel does not do this itself.
 template <typename TI>
@@ -551,6 +620,17 @@ RB_EXPORT int rb_conv_causal(float* u, const void* x, int64_t ldx, int x_off, in
   if (T == 0) return 0;
   RB_REQUIRE(C > 0 && K >= 1, "rb_conv_causal: bad sizes C=%d K=%d", C, K);
   const int threads = 128;
+  // Enough rows to give every SM several blocks: rows through registers, where 16-byte accesses are possible (below that,
+  // and for other sizes, a thread per row and channel).
+  if (x_dtype == RB_F32 && T >= 64 && K >= 2 && K <= 4 && C % 4 == 0 && ldx % 4 == 0 && x_off % 4 == 0 && (uintptr_t)x % 16 == 0 &&
+      (uintptr_t)u % 16 == 0 && (uintptr_t)tail % 16 == 0 && (C / 4 + threads - 1) / threads <= 65535) {
+    const dim3 rgrid((T + CONV_ROWS - 1) / CONV_ROWS, (C / 4 + threads - 1) / threads);
+#define ROWS(KK) RB_LAUNCH("conv_causal_rows_kernel", (conv_causal_rows_kernel<KK>), rgrid, threads, 0, stream, u, (const float*)x, ldx, x_off, x_bias, taps, conv_bias, tail, tok_first, tok_slot, tok_pos, T, C, silu)
+    if (K == 2) ROWS(2); else if (K == 3) ROWS(3); else ROWS(4);
+#undef ROWS
+    RB_CHECK_LAUNCH("rb_conv_causal");
+    return 0;
+  }
   int by = (C + threads - 1) / threads;
   if (by > 64) by = 64;
   const int per_block = T >= 512 ? CONV_TOKENS : 1;

@@ -242,6 +242,35 @@ def test_matrix_memory_kernel(ops32, H, D, Dv):
         assert float(state["C"][0].abs().max()) == 0.0 and float(state["C"][2].abs().max()) == 0.0
 
 
+@pytest.mark.parametrize("C,K,lengths,start", [(64, 4, [40, 1, 2, 60], 0), (4, 2, [64], 5), (516, 3, [15, 17, 33, 3], 2), (1024, 4, [700], 1),
+                                               (64, 4, [1] * 70, 3)])
+def test_convolution_of_many_rows(ops32, C, K, lengths, start):
+    """Rows through registers against a row and channel a thread (63 rows at most at a time), bit for bit: runs that begin inside
+    a block's rows, in the middle of a sequence (inputs from the ring) and at its start, with biases and SiLU."""
+    from ctypes import c_void_p
+    g = torch.Generator(device="cuda").manual_seed(C + K)
+    S, T = len(lengths), sum(lengths)
+    x = torch.randn(T, C + 8, device="cuda", generator=g)
+    taps, b, xb = torch.randn(C, K, device="cuda", generator=g), torch.randn(C, device="cuda", generator=g), torch.randn(C, device="cuda", generator=g)
+    tail = torch.randn(S, K, C, device="cuda", generator=g)
+    rows = [(i, sum(lengths[:i]), j) for i, n in enumerate(lengths) for j in range(n)]
+    dev = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    first, slot, pos = dev([r[1] for r in rows]), dev([r[0] for r in rows]), dev([start + r[2] for r in rows])
+    ptr = lambda t: c_void_p(t.data_ptr())
+    outs = []
+    for misaligned in (False, True):                     # the second call's rows start one value behind a 16-byte boundary
+        buf = torch.zeros(T * (C + 8) + 1, device="cuda")
+        src = buf[1:] if misaligned else buf[:-1]
+        src.copy_(x.flatten())
+        u = torch.empty(T, C, device="cuda")
+        for silu, bias in ((1, b), (0, None)):
+            ops32.lib.call("rb_conv_causal", ptr(u), ptr(src), C + 8, 4, 0, ptr(xb) if bias is not None else c_void_p(0), ptr(taps),
+                           ptr(b) if bias is not None else c_void_p(0), ptr(tail), ptr(first), ptr(slot), ptr(pos), T, C, K, silu,
+                           ops32._stream())
+            outs.append(u.clone())
+    assert torch.equal(outs[0], outs[2]) and torch.equal(outs[1], outs[3])
+
+
 @pytest.mark.parametrize("H,D,Dv,lengths", [(2, 16, 24, [64, 1, 65]), (1, 7, 5, [130]), (3, 64, 64, [63, 200, 17]),
                                             (2, 100, 68, [129, 128]), (8, 128, 256, [90] * 16), (1, 260, 40, [70, 3])])
 @pytest.mark.parametrize("chunks", [True, False])
