@@ -182,6 +182,8 @@ class CudaOps:
         #: run on average, and of the step.  Us token by token and in chunks, 8 heads of 128 x 256: one run of 32 tokens 19,
         #: 39; of 100 46, 45; of 300 117, 72; 16 runs of 16 tokens 60, 77; of 32 105, 86
         self.memory_in_chunks, self.memory_chunks_from = True, (24, 128)
+        #: and with at most this much scratch (a memory per chunk and head: 1 GiB; 8,192 tokens of 8 heads of 256 x 512 take 0.6)
+        self.memory_scratch_floats = 1 << 28
         #: a decode step's delta rule (convolution to gate) is one kernel while rows x heads fit the SMs
         self.fuse_delta_step = True
         #: tensor-core products of more than 256 tokens may share a weight tile's inner dimension
@@ -794,10 +796,13 @@ class CudaOps:
         bias = (_ptr(p.i_bias), _ptr(p.f_bias), float(p.gate_cap), float(D) ** -0.5, float(p.floor))
         kept = (_ptr(state["C"]), _ptr(state["n"]), _ptr(state["m"]))
         per_run, per_step = self.memory_chunks_from
-        if first is not None and self.memory_in_chunks and T >= per_run * n_seq and T >= per_step:
+        chunked = first is not None and self.memory_in_chunks and T >= per_run * n_seq and T >= per_step
+        if chunked:
             run0, rows, lens, n_chunks = self._delta_chunks(meta, 64)
-            scratch = torch.empty((self.lib.raw("rb_matrix_memory_chunk_floats")(n_chunks, H, D, Dv),), dtype=torch.float32,
-                                  device=self.device)
+            floats = self.lib.raw("rb_matrix_memory_chunk_floats")(n_chunks, H, D, Dv)
+            chunked = floats <= self.memory_scratch_floats
+        if chunked:
+            scratch = torch.empty((floats,), dtype=torch.float32, device=self.device)
             self.lib.call("rb_matrix_memory_chunked", _ptr(o), _ptr(proj), proj.stride(0), at["q"], at["k"], at["v"], at["i"],
                           at["f"], *bias, *kept, _ptr(first), _ptr(count), _ptr(run0), _ptr(rows), _ptr(lens),
                           _ptr(meta.tok_slot), n_seq, n_chunks, H, D, Dv, _ptr(scratch), self._stream(), launches=4)
