@@ -406,6 +406,30 @@ def test_retention_part(H, D, Dv, dims, chunks):
     ops.check_errors()
 
 
+@pytest.mark.parametrize("T", [32, 75])
+@pytest.mark.parametrize("H,D,Dv", [(2, 16, 24), (1, 128, 64), (2, 100, 36)])
+def test_a_chunk_rounds_once_at_the_memorys_size(H, D, Dv, T):
+    """A large memory that forgets nothing (every factor is exactly 1) and T small updates.  A chunk of 32 tokens may round the
+    memory once, 2^-24 of it at most; its own sum of 32 products rounds 32 times at the products' size."""
+    from rbitnet_b200.parts.retention import Retention
+    ops = _ops(torch.float32)
+    g = torch.Generator(device="cuda").manual_seed(H * 1000 + D + T)
+    part = Retention(32, H, D, Dv, [1.0] * H, 1e-5)
+    part.bind({k: torch.zeros(shape, device="cuda") for k, (shape, _) in part.weight_shapes().items()}, ops)
+    S0 = 1000.0 * torch.randn(3, H, Dv, D, device="cuda", generator=g)
+    state = {"S": S0.clone()}
+    proj = torch.randn(T, 2 * H * D + 2 * H * Dv, device="cuda", generator=g)
+    at = part.offsets()
+    k = proj[:, at["k"]:at["k"] + H * D].double().view(T, H, D)
+    v = proj[:, at["v"]:at["v"] + H * Dv].double().view(T, H, Dv)
+    ops.retention(proj, part, state, _meta(ops, [(1, 0, T)]))
+    want = S0[1].double() + torch.einsum("thv,thd->hvd", v, k)
+    sums = torch.einsum("thv,thd->hvd", v.abs(), k.abs())
+    bound = 2.0 ** -24 * (-(-T // 32) * (S0[1].double().abs() + sums) + 33 * sums)
+    assert ((state["S"][1].double() - want).abs() <= bound).all()
+    assert torch.equal(state["S"][0], S0[0]) and torch.equal(state["S"][2], S0[2])
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("H,D,R,Dv,C", [(4, 16, 8, 8, 24), (2, 24, 4, 40, 12), (8, 64, 16, 64, 80), (4, 32, 32, 32, 96),
                                         (1, 8, 2, 8, 200), (2, 64, 64, 16, 64), (16, 16, 16, 32, 240)])
