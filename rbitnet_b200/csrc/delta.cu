@@ -622,12 +622,14 @@ __global__ void __launch_bounds__(SCAN_NT) delta_chunk_scan_kernel(
           if (col0 + 4 * ct + j < Dv) to[j] = out[j];
       }
     } else if (steps) {
-      // the memory moves on: S <- e^{L_end} S + sum_j k_j e^{L_end - L_j} U_j
+      // the memory moves on: S <- e^{L_end} S + sum_j k_j e^{L_end - L_j} U_j, the chunk's sum from zero, so that a chunk rounds
+      // at the memory's size once and not 33 times
       const float keep = Es[CH - 1];
+      float add[4][4];
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) S[i][j] *= keep;
+        for (int j = 0; j < 4; ++j) add[i][j] = 0.f;
 #pragma unroll 4
       for (int j = 0; j < CH; ++j) {
         const float4 k4 = *reinterpret_cast<const float4*>(Kc + j * D + 4 * dt);
@@ -635,12 +637,16 @@ __global__ void __launch_bounds__(SCAN_NT) delta_chunk_scan_kernel(
         const float ki[4] = {k4.x, k4.y, k4.z, k4.w};
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          S[i][0] = fmaf(ki[i], u4.x, S[i][0]);
-          S[i][1] = fmaf(ki[i], u4.y, S[i][1]);
-          S[i][2] = fmaf(ki[i], u4.z, S[i][2]);
-          S[i][3] = fmaf(ki[i], u4.w, S[i][3]);
+          add[i][0] = fmaf(ki[i], u4.x, add[i][0]);
+          add[i][1] = fmaf(ki[i], u4.y, add[i][1]);
+          add[i][2] = fmaf(ki[i], u4.z, add[i][2]);
+          add[i][3] = fmaf(ki[i], u4.w, add[i][3]);
         }
       }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) S[i][j] = fmaf(keep, S[i][j], add[i][j]);
 #pragma unroll
       for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(Ss + (4 * dt + i) * CCT + 4 * cs) = make_float4(S[i][0], S[i][1], S[i][2], S[i][3]);
     }

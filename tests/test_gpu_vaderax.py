@@ -324,6 +324,45 @@ def test_gated_delta_kernels(H, G, D, Dv, K, chunks, one_launch):
         assert float(state["S"][0].abs().max()) == 0.0 and float(state["S"][2].abs().max()) == 0.0
 
 
+@pytest.mark.parametrize("T", [32, 75])
+@pytest.mark.parametrize("H,G,D,Dv", [(2, 1, 16, 24), (1, 1, 128, 64), (2, 2, 100, 33)])
+def test_a_chunk_of_the_delta_rule_rounds_once_at_the_memorys_size(H, G, D, Dv, T):
+    """A large memory that forgets nothing, unit keys and a beta of 2^-12, so that the updates are small: a chunk of 32 tokens may
+    round the memory once, 2^-24 of it at most.  The updates' own error: u = beta (v - S^T k) is off by at most (D + 40) 2^-24 of
+    beta sum |S k| and of itself, and is summed with |k| <= 1 over the run; a factor of 2 for the exponentials and the products
+    of the system's small matrix."""
+    import ctypes
+    ops = _ops(torch.float32)
+    g = torch.Generator(device="cuda").manual_seed(H * 1000 + D + T)
+    S0 = 1000.0 * torch.randn(3, H, Dv, D, device="cuda", generator=g)
+    state = S0.clone()
+    qk = torch.nn.functional.normalize(torch.randn(T, 2 * G, D, device="cuda", generator=g).double(), dim=-1).float()
+    v = torch.randn(T, H, Dv, device="cuda", generator=g)
+    u = torch.cat([qk.view(T, -1), v.view(T, -1)], dim=1).contiguous()
+    beta = torch.full((T, H), 2.0 ** -12, device="cuda")
+    log_decay = torch.zeros(T, H, device="cuda")
+    meta = _meta(ops, [(1, 0, T)])
+    first, count, _, runs = ops._runs(meta)
+    run0, row, length, n_chunks = ops._delta_chunks(meta)
+    o = torch.empty(T, H * Dv, device="cuda")
+    scratch = torch.empty(n_chunks * H * ops.lib.raw("rb_gated_delta_chunk_floats")(D, Dv), device="cuda")
+    ptr = lambda t: ctypes.c_void_p(t.data_ptr())
+    u = torch.nn.functional.pad(u, (0, -u.shape[1] % 4)).contiguous()         # rows that start on 16 bytes
+    ops.lib.call("rb_gated_delta_chunked", ptr(o), ptr(u), u.stride(0), ptr(beta), ptr(log_decay), ptr(state), ptr(scratch), ptr(first),
+                 ptr(count), ptr(run0), ptr(row), ptr(length), ptr(meta.tok_slot), runs, n_chunks, H, G, D, Dv, ops._stream())
+    S = S0[1].double()                                                       # [H, Dv, D]
+    slack = torch.zeros_like(S)
+    for t in range(T):
+        k = qk[t, G:].double().repeat_interleave(H // G, 0)                  # [H, D]
+        new = 2.0 ** -12 * (v[t].double() - torch.einsum("hvd,hd->hv", S, k))
+        size = 2.0 ** -12 * (v[t].double().abs() + torch.einsum("hvd,hd->hv", S.abs(), k.abs()))
+        S = S + new[:, :, None] * k[:, None, :]
+        slack += 2 * (D + 40) * size.unsqueeze(2) * k.abs().unsqueeze(1)
+    bound = 2.0 ** -24 * (-(-T // 32) * (torch.maximum(S0[1].double().abs(), S.abs()) + slack / (D + 40)) + slack)
+    assert ((state[1].double() - S).abs() <= bound).all()
+    assert torch.equal(state[0], S0[0]) and torch.equal(state[2], S0[2])
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("H,Kh,D,Dv,rot", [(4, 2, 32, 16, 8), (2, 2, 16, 40, 16), (3, 1, 24, 24, 0), (4, 2, 64, 64, 32), (2, 1, 128, 96, 64),
                                            (1, 1, 200, 8, 2)])
