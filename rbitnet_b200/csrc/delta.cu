@@ -599,22 +599,30 @@ __global__ void __launch_bounds__(SCAN_NT) delta_chunk_scan_kernel(
     }
     __syncthreads();                  // U is there, and every thread has read the old S
     if (second) {
-      // the chunk's outputs: e^{L_i} (q S0)_i + sum_{j <= i} M_ij U_j (M is zero above the diagonal)
+      // the chunk's outputs: e^{L_i} (q S0)_i + sum_{j <= i} M_ij U_j.  Tokens after row i are left out and not multiplied by
+      // zeros: one of them that is infinite would turn the tokens before it into NaN.
       const float e = Es[mine_row];
       float out[4] = {e * sum[0], e * sum[1], e * sum[2], e * sum[3]};
+      auto take = [&](int j, float mj) {
+        const float4 u4 = *reinterpret_cast<const float4*>(Us + j * CCT + 4 * ct);
+        out[0] = fmaf(mj, u4.x, out[0]);
+        out[1] = fmaf(mj, u4.y, out[1]);
+        out[2] = fmaf(mj, u4.z, out[2]);
+        out[3] = fmaf(mj, u4.w, out[3]);
+      };
 #pragma unroll 4
-      for (int j = 0; j < CH; j += 4) {
+      for (int j = 0; j < rows; j += 4) {                // the groups of four before this warp's rows
         const float4 m4 = *reinterpret_cast<const float4*>(Ms + mine_row * CH + j);
-        const float mj[4] = {m4.x, m4.y, m4.z, m4.w};
-#pragma unroll
-        for (int x = 0; x < 4; ++x) {
-          const float4 u4 = *reinterpret_cast<const float4*>(Us + (j + x) * CCT + 4 * ct);
-          out[0] = fmaf(mj[x], u4.x, out[0]);
-          out[1] = fmaf(mj[x], u4.y, out[1]);
-          out[2] = fmaf(mj[x], u4.z, out[2]);
-          out[3] = fmaf(mj[x], u4.w, out[3]);
-        }
+        take(j, m4.x);
+        take(j + 1, m4.y);
+        take(j + 2, m4.z);
+        take(j + 3, m4.w);
       }
+      const float4 m4 = *reinterpret_cast<const float4*>(Ms + mine_row * CH + rows);
+      const float mj[4] = {m4.x, m4.y, m4.z, m4.w};
+#pragma unroll
+      for (int x = 0; x < 4; ++x)
+        if (x <= ks) take(rows + x, mj[x]);
       if (mine_row < m) {
         float* to = o + ((int64_t)(row0 + mine_row) * H + h) * Dv + col0 + 4 * ct;
 #pragma unroll

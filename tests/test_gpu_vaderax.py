@@ -363,6 +363,28 @@ def test_a_chunk_of_the_delta_rule_rounds_once_at_the_memorys_size(H, G, D, Dv, 
     assert torch.equal(state[0], S0[0]) and torch.equal(state[2], S0[2])
 
 
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+def test_a_token_that_is_not_finite_leaves_the_ones_before_it(bad):
+    """The delta rule in chunks, one value of one token infinite or NaN: that token and later ones of its sequence may become
+    anything, the tokens before it and the other sequence stay as they are."""
+    from rbitnet_b200.parts.delta import GatedDeltaRule
+    ops = _ops(torch.float32)
+    g = torch.Generator(device="cuda").manual_seed(41)
+    H, G, D, Dv, K, T, at = 4, 2, 32, 40, 2, 70, 45
+    part = GatedDeltaRule(16, H, G, D, Dv, K, norm_eps=1e-5)
+    part.bind({k: 0.3 * torch.randn(shape, device="cuda", generator=g) for k, (shape, _) in part.weight_shapes().items()}, ops)
+    proj = torch.randn(2 * T, 2 * G * D + 2 * H * Dv + 2 * H, device="cuda", generator=g)
+    outs = []
+    for value in (None, bad):
+        rows = proj.clone()
+        if value is not None:
+            rows[at, 2 * G * D + 3] = value                        # a value channel of head 0
+        state = {k: torch.zeros((2, *n.shape), device="cuda") for k, n in part.state_need().items()}
+        outs.append(ops.gated_delta(rows, part, state, _meta(ops, [(0, 0, T), (1, 0, T)])))
+    assert torch.isfinite(outs[0]).all() and not torch.isfinite(outs[1][at]).all()
+    assert torch.equal(outs[0][:at], outs[1][:at]) and torch.equal(outs[0][T:], outs[1][T:])
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("H,Kh,D,Dv,rot", [(4, 2, 32, 16, 8), (2, 2, 16, 40, 16), (3, 1, 24, 24, 0), (4, 2, 64, 64, 32), (2, 1, 128, 96, 64),
                                            (1, 1, 200, 8, 2)])
