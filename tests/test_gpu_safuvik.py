@@ -314,6 +314,42 @@ def test_matrix_memory_of_several_runs(ops32, H, D, Dv, lengths, chunks):
     assert float(state["C"][0].abs().max()) == 0.0 and float(state["C"][-1].abs().max()) == 0.0
 
 
+@pytest.mark.parametrize("D,Dv,T", [(128, 64, 128), (256, 64, 300), (256, 40, 130)])
+def test_matrix_memory_in_chunks_is_as_exact_as_token_by_token(ops32, D, Dv, T):
+    """Both forms against float64 on the same rows, the mean over six draws of the error's 2-norm.  Token by token a value is the
+    sum of D products, D / 32 to a lane; in chunks it is the sum of 64 + D, which must not cost more."""
+    from rbitnet_b200.parts.recurrent import MatrixMemory
+    H, E = 4, 8
+    part = MatrixMemory(E, H, D, Dv, gate_cap=15.0, norm_eps=1e-5)
+    part.bind({k: torch.full(shape, 4.0 if k == "f.b" else 1.0, device="cuda") for k, (shape, _) in part.weight_shapes().items()}, ops32)
+    at, meta = part.offsets(), _meta(ops32, [(0, 0, T)])
+    errors = {True: [], False: []}
+    before = ops32.memory_in_chunks
+    for seed in range(6):
+        g = torch.Generator(device="cuda").manual_seed(seed)
+        proj = torch.randn(T, 2 * H * D + 2 * H * Dv + 2 * H, device="cuda", generator=g)
+        q, k = (proj[:, at[n]:at[n] + H * D].double().view(T, H, D) for n in "qk")
+        v, gate = (proj[:, at[n]:at[n] + H * Dv].double().view(T, H, Dv) for n in "vg")
+        i, f = (15.0 * torch.tanh((proj[:, at[n]:at[n] + H].double() + b) / 15.0) for n, b in (("i", 1.0), ("f", 4.0)))
+        F = torch.nn.functional.logsigmoid(f).cumsum(0)                                  # [T, H]
+        m = F + torch.cummax(i - F, 0).values.clamp(min=0.0)
+        later = torch.ones(T, T, dtype=torch.bool, device="cuda").triu(1)[:, :, None]
+        weight = torch.exp(((F - m)[:, None] + (i - F)[None]).masked_fill(later, -math.inf))
+        scores = torch.einsum("thd,shd->tsh", q, k) * D ** -0.5 * weight
+        o = torch.einsum("tsh,shv->thv", scores, v)
+        o = o / (torch.maximum(scores.sum(1).abs(), torch.exp(-m)) + part.floor)[:, :, None]
+        want = o / (o.pow(2).mean(-1, keepdim=True) + 1e-5).sqrt() * torch.sigmoid(gate)
+        for chunks in (True, False):
+            ops32.memory_in_chunks = chunks
+            state = {n: torch.zeros((1, *s.shape), device="cuda") for n, s in part.state_need().items()}
+            try:
+                got = ops32.matrix_memory(proj, part, state, meta).double().view(T, H, Dv)
+            finally:
+                ops32.memory_in_chunks = before
+            errors[chunks].append(float((got - want).norm() / want.norm()))
+    assert sum(errors[True]) <= 1.05 * sum(errors[False]), errors
+
+
 @pytest.mark.parametrize("W,B,K", [(48, 3, 3), (32, 1, 2), (200, 5, 4), (24, 2, 1)])
 def test_gated_recurrence_kernels(ops32, W, B, K):
     from rbitnet_b200.parts.recurrent import GatedLinearRecurrence
