@@ -170,6 +170,49 @@ __device__ __forceinline__ void multiply(float (&acc)[8][4], const float* x, con
       for (int j = 0; j < 4; ++j) acc[i][j] += part[i][j];
   }
 }
+// The same for x that is zero for k behind the row (a chunk's scores): later tokens are left out of a row's sum and not
+// multiplied by zeros, since one of them that is infinite would turn the tokens before it into NaN.
+__device__ __forceinline__ void multiply_below(float (&acc)[8][4], const float* x, const float* y, int tx, int ty) {
+#pragma unroll
+  for (int g = 0; g < 2; ++g) {
+    const int r0 = 32 * g + 4 * ty;                      // this group's first row: every k before it, then k = row by row
+    float part[4][4];
+    auto clear = [&]() {
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) part[i][j] = 0.f;
+    };
+    auto add = [&]() {
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[4 * g + i][j] += part[i][j];
+    };
+    auto take = [&](int k, int first) {
+      float a[4], b[4];
+      rb_load4(x + k * PITCH + r0, a);
+      rb_load4(y + k * PITCH + tx * 4, b);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (i >= first) part[i][j] = fmaf(a[i], b[j], part[i][j]);
+    };
+    clear();
+    if (g == 1) {
+#pragma unroll 4
+      for (int k = 0; k < 32; ++k) take(k, 0);
+      add();
+      clear();
+    }
+#pragma unroll 4
+    for (int k = 32 * g; k < r0; ++k) take(k, 0);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) take(r0 + e, e);
+    add();
+  }
+}
 __device__ __forceinline__ int row_of(int i, int ty) { return i / 4 * 32 + ty * 4 + i % 4; }
 
 // grid (chunks, H, 1 + tiles of 64 value columns x tiles of 64 rows).  The first z makes the chunk's scores.
@@ -304,7 +347,7 @@ __global__ void __launch_bounds__(NT, 5) memory_chunk_out_kernel(Memory a, float
   stage<true>(x, a.scores + at * CH * CH, CH, CH, 0, CH, true, nullptr);
   stage<false>(y, base + a.v_off + h * a.Dv, a.ld, rows, j0, a.Dv, a.vec, nullptr);
   __syncthreads();
-  multiply(acc, x, y, tx, ty);
+  multiply_below(acc, x, y, tx, ty);
 #pragma unroll 8
   for (int k = half; k < CH; k += 2) sum += x[k * PITCH + t];
   for (int d0 = 0; d0 < a.D; d0 += CH) {

@@ -350,6 +350,27 @@ def test_matrix_memory_in_chunks_is_as_exact_as_token_by_token(ops32, D, Dv, T):
     assert sum(errors[True]) <= 1.05 * sum(errors[False]), errors
 
 
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+def test_a_token_that_is_not_finite_leaves_the_ones_before_it(ops32, bad):
+    """The matrix memory in chunks, one value of one token infinite or NaN: that token and later ones of its sequence may become
+    anything, the tokens before it and the other sequence stay as they are."""
+    from rbitnet_b200.parts.recurrent import MatrixMemory
+    H, D, Dv, T, at = 2, 40, 72, 150, 101
+    g = torch.Generator(device="cuda").manual_seed(43)
+    part = MatrixMemory(16, H, D, Dv, gate_cap=15.0, norm_eps=1e-5)
+    part.bind({k: 0.3 * torch.randn(shape, device="cuda", generator=g) for k, (shape, _) in part.weight_shapes().items()}, ops32)
+    proj = torch.randn(2 * T, 2 * H * D + 2 * H * Dv + 2 * H, device="cuda", generator=g)
+    outs = []
+    for value in (None, bad):
+        rows = proj.clone()
+        if value is not None:
+            rows[at, part.offsets()["v"] + 5] = value               # a value of head 0
+        state = {n: torch.zeros((2, *s.shape), device="cuda") for n, s in part.state_need().items()}
+        outs.append(ops32.matrix_memory(rows, part, state, _meta(ops32, [(0, 0, T), (1, 0, T)])))
+    assert torch.isfinite(outs[0]).all() and not torch.isfinite(outs[1][at]).all()
+    assert torch.equal(outs[0][:at], outs[1][:at]) and torch.equal(outs[0][T:], outs[1][T:])
+
+
 @pytest.mark.parametrize("W,B,K", [(48, 3, 3), (32, 1, 2), (200, 5, 4), (24, 2, 1)])
 def test_gated_recurrence_kernels(ops32, W, B, K):
     from rbitnet_b200.parts.recurrent import GatedLinearRecurrence
