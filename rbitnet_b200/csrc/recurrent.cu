@@ -569,14 +569,13 @@ __global__ void __launch_bounds__(128) matrix_memory_kernel(
   if (blockIdx.z == 0 && threadIdx.x == 0) left[D] = *s_m;
 }
 
-// n and m of the runs' heads as matrix_memory_kernel left them ([run][H][D + 1]), for the state.
+// n and m of the runs' heads as matrix_memory_kernel left them ([run][H][D + 1]), for the state; from null: none.
 struct Moved {
   const float* from = nullptr;
   float *n_state = nullptr, *m_state = nullptr;
   const int *tok_slot = nullptr, *seq_first = nullptr;
   int n_seq = 0, H = 0, D = 0;
 };
-thread_local Moved t_moved;            // for this thread's next head_norm_gate_kernel
 
 // Per (token, head): o / rms(o) over the head's Dv values, times the weight, times sigmoid(gate) (gate_silu: times
 // gate * sigmoid(gate)).  One warp each.  gate: the projections' rows, at column g_off.  The weight has H * Dv
@@ -584,17 +583,16 @@ thread_local Moved t_moved;            // for this thread's next head_norm_gate_
 template <typename TI, typename TO>
 __global__ void head_norm_gate_kernel(TO* __restrict__ out, const float* __restrict__ o, const float* __restrict__ w,
                                       const TI* __restrict__ proj, int64_t ld, int g_off, int n_rows, int H, int Dv,
-                                      float eps, int w_shared, int gate_silu, Moved moved) {
+                                      float eps, int w_shared, int gate_silu, int norm_blocks, Moved moved) {
   rb_pdl_launch_dependents();
   rb_pdl_wait();
-  if (moved.from != nullptr) {
-    const int per = moved.D + 1;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < moved.n_seq * moved.H * per; i += gridDim.x * blockDim.x) {
-      const int rh = i / per, d = i - rh * per, run = rh / moved.H;
-      const int64_t to = (int64_t)moved.tok_slot[moved.seq_first != nullptr ? moved.seq_first[run] : run] * moved.H + rh % moved.H;
-      if (d < moved.D) moved.n_state[to * moved.D + d] = moved.from[i];
-      else moved.m_state[to] = moved.from[i];
-    }
+  const int move = (int)blockIdx.x - norm_blocks;         // the blocks behind those take n and m over, one (run, head) each
+  if (move >= 0) {
+    const int64_t to = (int64_t)moved.tok_slot[moved.seq_first != nullptr ? moved.seq_first[move / moved.H] : move / moved.H] * moved.H + move % moved.H;
+    const float* from = moved.from + (int64_t)move * (moved.D + 1);
+    for (int d = threadIdx.x; d < moved.D; d += blockDim.x) moved.n_state[to * moved.D + d] = from[d];
+    if (threadIdx.x == 0) moved.m_state[to] = from[moved.D];
+    return;
   }
   const int lane = threadIdx.x & 31;
   const int64_t item = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -750,6 +748,23 @@ RB_EXPORT int rb_matrix_memory_lanes(int D) {
   return P;
 }
 
+static int head_norm_gate(void* out, int out_dtype, const float* o, const float* w, const void* proj, int64_t ld, int proj_dtype,
+                          int g_off, int T, int H, int Dv, float eps, int w_shared, int gate_silu, const Moved& moved,
+                          cudaStream_t stream) {
+  const int64_t items = (int64_t)T * H;
+  const int norm_blocks = (int)((items + 3) / 4), blocks = norm_blocks + (moved.from != nullptr ? moved.n_seq * moved.H : 0);
+#define LAUNCH(TI, TO)                                                                                              \
+  RB_LAUNCH("head_norm_gate_kernel", (head_norm_gate_kernel<TI, TO>), blocks, 128, 0, stream, (TO*)out, o, w,        \
+            (const TI*)proj, ld, g_off, T, H, Dv, eps, w_shared, gate_silu, norm_blocks, moved)
+  if (proj_dtype == RB_F32 && out_dtype == RB_F32) LAUNCH(float, float);
+  else if (proj_dtype == RB_F32 && out_dtype == RB_BF16) LAUNCH(float, __nv_bfloat16);
+  else if (proj_dtype == RB_BF16 && out_dtype == RB_BF16) LAUNCH(__nv_bfloat16, __nv_bfloat16);
+  else RB_FAIL("rb_head_norm_gate: unsupported dtypes %d -> %d", proj_dtype, out_dtype);
+#undef LAUNCH
+  RB_CHECK_LAUNCH("rb_head_norm_gate");
+  return 0;
+}
+
 template <int P, int R>
 static int launch_matrix_memory(float* o_out, const float* proj, int64_t ld, int q_off, int k_off, int v_off, int i_off,
                                 int f_off, const float* i_bias, const float* f_bias, float cap, float q_scale,
@@ -774,26 +789,17 @@ static int launch_matrix_memory(float* o_out, const float* proj, int64_t ld, int
             v_off, i_off, f_off, i_bias, f_bias, cap, q_scale, floor_add, C_state, n_state, m_state, moved, seq_first, seq_count,
             tok_slot, H, D, Dv, vec4);
   RB_CHECK_LAUNCH("rb_matrix_memory");
-  t_moved = Moved{moved, n_state, m_state, tok_slot, seq_first, n_seq, H, D};
   return 0;
 }
 
-// moved: [n_seq][H][D + 1] floats.  The runs' new n and m are left there, and this thread's next rb_head_norm_gate moves the
-// state on to them.
-RB_EXPORT int rb_matrix_memory(float* o_out, const void* proj, int64_t ld, int proj_dtype, int q_off, int k_off, int v_off,
-                               int i_off, int f_off, const float* i_bias, const float* f_bias, float cap, float q_scale,
-                               float floor_add, float* C_state, float* n_state, float* m_state, float* moved,
-                               const int* seq_first, const int* seq_count, const int* tok_slot, int n_seq, int H, int D, int Dv,
-                               cudaStream_t stream) {
-  if (n_seq == 0) return 0;
-  RB_REQUIRE((int64_t)n_seq * H * (D + 1) <= 0x7fffffff, "rb_matrix_memory: %d runs: too many for one launch", n_seq);
-  RB_REQUIRE(H > 0 && D > 0 && Dv > 0 && D <= 512, "rb_matrix_memory: bad sizes H=%d D=%d Dv=%d (D up to 512)", H, D, Dv);
-  RB_REQUIRE(cap > 0.f, "rb_matrix_memory: the gates' cap must be positive");
-  RB_REQUIRE(proj_dtype == RB_F32, "rb_matrix_memory: the projections are float32 rows (found dtype %d)", proj_dtype);
+static int matrix_memory_steps(float* o_out, const float* proj, int64_t ld, int q_off, int k_off, int v_off, int i_off, int f_off,
+                               const float* i_bias, const float* f_bias, float cap, float q_scale, float floor_add,
+                               float* C_state, float* n_state, float* m_state, float* moved, const int* seq_first,
+                               const int* seq_count, const int* tok_slot, int n_seq, int H, int D, int Dv, cudaStream_t stream) {
   const int P = rb_matrix_memory_lanes(D);
   const int per = (D + P - 1) / P;
 #define GO(PP, RR)                                                                                                    \
-  return launch_matrix_memory<PP, RR>(o_out, (const float*)proj, ld, q_off, k_off, v_off, i_off, f_off, i_bias, f_bias, \
+  return launch_matrix_memory<PP, RR>(o_out, proj, ld, q_off, k_off, v_off, i_off, f_off, i_bias, f_bias, \
                                       cap, q_scale, floor_add, C_state, n_state, m_state, moved, seq_first, seq_count, \
                                       tok_slot, n_seq, H, D, Dv, stream)
   switch (P) {
@@ -811,22 +817,30 @@ RB_EXPORT int rb_matrix_memory(float* o_out, const void* proj, int64_t ld, int p
 #undef GO
 }
 
+// The memory's steps and, after them, the norm per head and the gate (rb_head_norm_gate on o_out with norm_w, g_off, norm_eps),
+// whose kernel also moves the state on to the n and m that the first one has left in moved, [n_seq][H][D + 1] floats.  T: the
+// rows of all runs.
+RB_EXPORT int rb_matrix_memory(void* out, int out_dtype, float* o_out, const void* proj, int64_t ld, int proj_dtype, int q_off,
+                               int k_off, int v_off, int g_off, int i_off, int f_off, const float* i_bias, const float* f_bias,
+                               float cap, float q_scale, float floor_add, const float* norm_w, float norm_eps, float* C_state,
+                               float* n_state, float* m_state, float* moved, const int* seq_first, const int* seq_count,
+                               const int* tok_slot, int T, int n_seq, int H, int D, int Dv, cudaStream_t stream) {
+  if (n_seq == 0) return 0;
+  RB_REQUIRE(T >= n_seq && ((int64_t)T + n_seq) * H <= 0x7fffffff, "rb_matrix_memory: %d runs of %d rows: too many for one launch", n_seq, T);
+  RB_REQUIRE(out_dtype == RB_F32 || out_dtype == RB_BF16, "rb_matrix_memory: unknown dtype %d", out_dtype);
+  RB_REQUIRE(H > 0 && D > 0 && Dv > 0 && D <= 512, "rb_matrix_memory: bad sizes H=%d D=%d Dv=%d (D up to 512)", H, D, Dv);
+  RB_REQUIRE(cap > 0.f, "rb_matrix_memory: the gates' cap must be positive");
+  RB_REQUIRE(proj_dtype == RB_F32, "rb_matrix_memory: the projections are float32 rows (found dtype %d)", proj_dtype);
+  const int rc = matrix_memory_steps(o_out, (const float*)proj, ld, q_off, k_off, v_off, i_off, f_off, i_bias, f_bias, cap, q_scale,
+                                     floor_add, C_state, n_state, m_state, moved, seq_first, seq_count, tok_slot, n_seq, H, D, Dv, stream);
+  if (rc != 0) return rc;
+  return head_norm_gate(out, out_dtype, o_out, norm_w, proj, ld, proj_dtype, g_off, T, H, Dv, norm_eps, 0, 0,
+                        Moved{moved, n_state, m_state, tok_slot, seq_first, n_seq, H, D}, stream);
+}
+
 RB_EXPORT int rb_head_norm_gate(void* out, int out_dtype, const float* o, const float* w, const void* proj, int64_t ld,
                                 int proj_dtype, int g_off, int T, int H, int Dv, float eps, int w_shared, int gate_silu,
                                 cudaStream_t stream) {
-  const Moved moved = t_moved;
-  t_moved = Moved();
   if (T == 0) return 0;
-  const int64_t items = (int64_t)T * H;
-  const int blocks = (int)((items + 3) / 4);
-#define LAUNCH(TI, TO)                                                                                              \
-  RB_LAUNCH("head_norm_gate_kernel", (head_norm_gate_kernel<TI, TO>), blocks, 128, 0, stream, (TO*)out, o, w,        \
-            (const TI*)proj, ld, g_off, T, H, Dv, eps, w_shared, gate_silu, moved)
-  if (proj_dtype == RB_F32 && out_dtype == RB_F32) LAUNCH(float, float);
-  else if (proj_dtype == RB_F32 && out_dtype == RB_BF16) LAUNCH(float, __nv_bfloat16);
-  else if (proj_dtype == RB_BF16 && out_dtype == RB_BF16) LAUNCH(__nv_bfloat16, __nv_bfloat16);
-  else RB_FAIL("rb_head_norm_gate: unsupported dtypes %d -> %d", proj_dtype, out_dtype);
-#undef LAUNCH
-  RB_CHECK_LAUNCH("rb_head_norm_gate");
-  return 0;
+  return head_norm_gate(out, out_dtype, o, w, proj, ld, proj_dtype, g_off, T, H, Dv, eps, w_shared, gate_silu, Moved(), stream);
 }

@@ -793,6 +793,7 @@ class CudaOps:
         first, count, _, n_seq = self._runs(meta)
         at = p.offsets()
         o = torch.empty((T, H * Dv), dtype=torch.float32, device=self.device)
+        out = torch.empty((T, H * Dv), dtype=self.dtype, device=self.device)
         bias = (_ptr(p.i_bias), _ptr(p.f_bias), float(p.gate_cap), float(D) ** -0.5, float(p.floor))
         kept = (_ptr(state["C"]), _ptr(state["n"]), _ptr(state["m"]))
         per_run, per_step = self.memory_chunks_from
@@ -801,17 +802,16 @@ class CudaOps:
             run0, rows, lens, n_chunks = self._delta_chunks(meta, 64)
             floats = self.lib.raw("rb_matrix_memory_chunk_floats")(n_chunks, H, D, Dv)
             chunked = floats <= self.memory_scratch_floats
-        if chunked:
-            scratch = torch.empty((floats,), dtype=torch.float32, device=self.device)
-            self.lib.call("rb_matrix_memory_chunked", _ptr(o), _ptr(proj), proj.stride(0), at["q"], at["k"], at["v"], at["i"],
-                          at["f"], *bias, *kept, _ptr(first), _ptr(count), _ptr(run0), _ptr(rows), _ptr(lens),
-                          _ptr(meta.tok_slot), n_seq, n_chunks, H, D, Dv, _ptr(scratch), self._stream(), launches=4)
-        else:
+        if not chunked:
             moved = torch.empty((n_seq, H, D + 1), dtype=torch.float32, device=self.device)
-            self.lib.call("rb_matrix_memory", _ptr(o), _ptr(proj), proj.stride(0), F32, at["q"], at["k"], at["v"], at["i"],
-                          at["f"], *bias, *kept, _ptr(moved), _ptr(first), _ptr(count), _ptr(meta.tok_slot), n_seq, H, D, Dv,
-                          self._stream())
-        out = torch.empty((T, H * Dv), dtype=self.dtype, device=self.device)
+            self.lib.call("rb_matrix_memory", _ptr(out), self.code, _ptr(o), _ptr(proj), proj.stride(0), F32, at["q"], at["k"],
+                          at["v"], at["g"], at["i"], at["f"], *bias, _ptr(p.norm_w), float(p.norm_eps), *kept, _ptr(moved),
+                          _ptr(first), _ptr(count), _ptr(meta.tok_slot), T, n_seq, H, D, Dv, self._stream(), launches=2)
+            return out
+        scratch = torch.empty((floats,), dtype=torch.float32, device=self.device)
+        self.lib.call("rb_matrix_memory_chunked", _ptr(o), _ptr(proj), proj.stride(0), at["q"], at["k"], at["v"], at["i"],
+                      at["f"], *bias, *kept, _ptr(first), _ptr(count), _ptr(run0), _ptr(rows), _ptr(lens),
+                      _ptr(meta.tok_slot), n_seq, n_chunks, H, D, Dv, _ptr(scratch), self._stream(), launches=4)
         self.lib.call("rb_head_norm_gate", _ptr(out), self.code, _ptr(o), _ptr(p.norm_w), _ptr(proj), proj.stride(0), F32,
                       at["g"], T, H, Dv, float(p.norm_eps), 0, 0, self._stream())
         return out

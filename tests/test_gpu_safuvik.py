@@ -426,3 +426,49 @@ def test_limited_gated_activation(dtype, T, fused):
     assert rel_err(got.cpu(), want) <= (1e-5 if dtype == torch.float32 else 2e-2)
     # the limit is in use: without it the result differs
     assert rel_err(plain.clamped_feed_forward(w, {"limit": 100.0}, h), want) > 0.05
+
+
+@pytest.mark.parametrize("lengths", [[1, 1, 1], [20, 3]])
+def test_a_failed_allocation_leaves_no_store_behind(ops32, lengths, monkeypatch):
+    """An allocation that fails inside the matrix memory (token by token), whichever it is: the memory is as it was before the call,
+    and what another mixer does next on the same thread does not change it.  The call after that is whole."""
+    from rbitnet_b200.parts.recurrent import MatrixMemory
+    from rbitnet_b200.parts.retention import Retention
+    H, D, Dv, E = 2, 24, 40, 16
+    g = torch.Generator(device="cuda").manual_seed(47)
+    part = MatrixMemory(E, H, D, Dv, gate_cap=6.0, norm_eps=1e-5)
+    part.bind({k: 0.3 * torch.randn(shape, device="cuda", generator=g) for k, (shape, _) in part.weight_shapes().items()}, ops32)
+    other = Retention(E, 2, 8, 8, [0.9, 0.5], 1e-5)
+    other.bind({k: 0.3 * torch.randn(shape, device="cuda", generator=g) for k, (shape, _) in other.weight_shapes().items()}, ops32)
+    T, n = sum(lengths), len(lengths)
+    proj = torch.randn(T, 2 * H * D + 2 * H * Dv + 2 * H, device="cuda", generator=g)
+    meta = _meta(ops32, [(i, 4, c) for i, c in enumerate(lengths)])
+    start = {k: torch.randn((n, *s.shape), device="cuda", generator=g) for k, s in part.state_need().items()}
+    good = {k: v.clone() for k, v in start.items()}
+    want = ops32.matrix_memory(proj, part, good, meta)
+    real = torch.empty
+    for which in range(10):
+        state = {k: v.clone() for k, v in start.items()}
+        calls = []
+
+        def failing(*a, **k):
+            calls.append(1)
+            if len(calls) == which + 1:
+                raise torch.OutOfMemoryError("planted")
+            return real(*a, **k)
+        monkeypatch.setattr(torch, "empty", failing)
+        try:
+            ops32.matrix_memory(proj, part, state, meta)
+            failed = False
+        except torch.OutOfMemoryError:
+            failed = True
+        finally:
+            monkeypatch.setattr(torch, "empty", real)
+        if not failed:
+            break
+        rows = torch.randn(2, 4 * 16, device="cuda", generator=g)
+        ops32.retention(rows, other, {"S": torch.zeros(2, 2, 8, 8, device="cuda")}, _meta(ops32, [(0, 0, 1), (1, 0, 1)]))
+        assert all(torch.equal(state[k], start[k]) for k in start), which
+        assert torch.equal(ops32.matrix_memory(proj, part, state, meta), want)
+        assert all(torch.equal(state[k], good[k]) for k in start)
+    assert not failed and which >= 2
