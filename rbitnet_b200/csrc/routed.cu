@@ -163,6 +163,9 @@ __global__ void __launch_bounds__(256) route_kernel(int* __restrict__ ids, float
   const int per_token = 2 * n + 2 * groups;
   const int t0 = blockIdx.x * TB;
   const int nt = min(TB, T - t0);
+  // the router's matrix does not depend on the kernel before: its lines are asked for, into L2, before the wait for it
+  for (int64_t i = blockIdx.x + (int64_t)gridDim.x * threadIdx.x; i * 32 < (int64_t)n * K; i += (int64_t)gridDim.x * blockDim.x)
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(Wr + i * 32));
   rb_pdl_wait();
   if (TB == 1 && vec) {
     // one token: a warp makes four of its outputs at once, so that four rows of Wr are asked for together

@@ -424,3 +424,28 @@ def test_attention_part(dtype, H, Kh, D, Dv, rot):
             cache.advance(slot, b - a)
         assert rel_err(torch.cat(outs).cpu(), want) <= (2e-5 if dtype == torch.float32 else 3e-2), cuts
     ops.check_errors()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("T,K,n,top,groups,keep", [(1, 2048, 32, 4, 1, 1), (8, 4096, 30, 4, 1, 1), (63, 1024, 33, 5, 3, 2), (9, 1030, 17, 2, 1, 1),
+                                                   (5, 516, 64, 8, 8, 3), (2, 64, 1600, 3, 1, 1)])
+def test_the_routers_sums_of_few_tokens(dtype, T, K, n, top, groups, keep):
+    """The softmax router for fewer than 64 tokens: the bits of the kernel that makes the sums (lanes over k, FFMA) and chooses, also
+    where a tensor-core product could make them, whose sums are 2 to 5 times further from float64.
+    Against float64: a lane adds K / 32 products one after the other and the lanes' sums meet in five more, errors that walk to
+    (sqrt(K / 64) + sqrt(5)) 2^-24 of the products' 2-norm; four times that for the largest of T x top values, and 16
+    roundings for the softmax.  A router that is too large for the kernel that chooses from sums in memory is still taken."""
+    ops = _ops(dtype)
+    g = torch.Generator(device="cuda").manual_seed(T + K + n)
+    h = torch.randn(T, K, device="cuda", generator=g).to(dtype)
+    router = (torch.randn(n, K, device="cuda", generator=g) / K ** 0.5).to(torch.bfloat16).float()
+    ids, weights = torch.empty(T, top, dtype=torch.int32, device="cuda"), torch.empty(T, top, device="cuda")
+    ptr = lambda t: ctypes.c_void_p(t.data_ptr() if t is not None else 0)
+    ops.lib.call("rb_route", ptr(ids), ptr(weights), ptr(h), h.stride(0), 0 if dtype == torch.float32 else 1, ptr(router), ptr(None), T, K,
+                 n, top, groups, keep, ptr(None), ops._stream())
+    got_ids, got = ops.route(h, router, None, top, groups, keep, ops.prepare_router(router))
+    assert torch.equal(got_ids, ids) and torch.equal(got, weights)
+    want = torch.softmax(h.double() @ router.double().T, -1).gather(1, ids.long())
+    size = (h.double().square() @ router.double().square().T).max(1, keepdim=True).values.sqrt()
+    bound = 4 * 2.0 ** -24 * (((K / 64) ** 0.5 + 5 ** 0.5) * size + 16)
+    assert ((weights.double() - want).abs() <= bound * want).all()
