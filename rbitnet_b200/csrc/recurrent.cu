@@ -56,12 +56,14 @@ __global__ void conv_causal_kernel(float* __restrict__ u, const TI* __restrict__
   }
 }
 
-// The same for many float32 rows: a thread keeps the last K inputs of four neighbouring channels in registers while it goes
-// down a block's rows, so that an input is read once and not K times, 16 bytes a load, eight rows on their way at a time.  The
-// same sums in the same order.  Bound by the bytes of its rows (2,048 rows of 2,048 channels, K 4: 33 us before, 7.9 now; about 2,500 of 4,096 80 and 39;
-// the rows alone take 5 and 12).
-constexpr int CONV_ROWS = 16, CONV_AHEAD = 8;
-template <int K>
+// The same for float32 rows that a thread takes ROWS of, one after the other: it keeps the last K inputs of four neighbouring
+// channels in registers, so that an input is read once and not K times, 16 bytes a load, eight rows on their way at a time.  The
+// same sums in the same order.  Bound by the bytes of its rows, and by a block's chain of rows where there are few (a run's first
+// row there waits for its slot and position, then for the ring).  One run of 2,048 channels, K 4, us with a thread per row and
+// channel and with 2, 4, 8, 16 rows: 64 rows 3.6; 3.2 3.8 5.3 8.6; 300 rows 7.1; 6.6 4.5 5.8 8.7; 1,024 rows 17; 15 9.9 7.1 9.7;
+// 4,096 rows 55; 53 34 26 21.
+constexpr int CONV_AHEAD = 8;
+template <int K, int ROWS>
 __global__ void __launch_bounds__(128) conv_causal_rows_kernel(float* __restrict__ u, const float* __restrict__ x, int64_t ldx, int x_off,
                                                                const float* __restrict__ x_bias, const float* __restrict__ taps,
                                                                const float* __restrict__ conv_bias, const float* __restrict__ tail,
@@ -79,7 +81,7 @@ __global__ void __launch_bounds__(128) conv_causal_rows_kernel(float* __restrict
     for (int d = 0; d < K; ++d) w[d][i] = taps[(int64_t)(c + i) * K + K - 1 - d];
   }
   rb_pdl_wait();
-  const int t0 = blockIdx.x * CONV_ROWS, t1 = min(T, t0 + CONV_ROWS);
+  const int t0 = blockIdx.x * ROWS, t1 = min(T, t0 + ROWS);
   int run = -1;
   for (int ta = t0; ta < t1; ta += CONV_AHEAD) {
     float in[CONV_AHEAD][4];
@@ -612,20 +614,33 @@ __global__ void head_norm_gate_kernel(TO* __restrict__ out, const float* __restr
 
 }  // namespace
 
+// Rows that a thread of the causal convolution takes one after the other, where 16-byte accesses are possible; 0: a thread per row
+// and channel.  That is while its blocks are up to six an SM (64 rows of 512 channels 2.9 us, 3.4 with two rows a thread; of
+// 2,048 channels 4.2 and 3.7); from 512 rows on its blocks take eight rows each, which is never faster.  Else as many rows as still
+// leave every SM four blocks, which are what an SM holds.
+RB_EXPORT int rb_conv_rows(int T, int C, int K) {
+  const int64_t sms = rb_sm_count(), columns = (C / 4 + 127) / 128;
+  if (K < 2 || K > 4 || C % 4 != 0 || columns > 65535 || (T < 512 && (int64_t)T * ((C + 127) / 128) < 6 * sms)) return 0;
+  int rows = 2;
+  while (rows < 16 && (T + rows - 1) / rows * columns > 4 * sms) rows *= 2;
+  return rows;
+}
+
 RB_EXPORT int rb_conv_causal(float* u, const void* x, int64_t ldx, int x_off, int x_dtype, const float* x_bias,
                              const float* taps, const float* conv_bias, const float* tail, const int* tok_first,
                              const int* tok_slot, const int* tok_pos, int T, int C, int K, int silu, cudaStream_t stream) {
   if (T == 0) return 0;
   RB_REQUIRE(C > 0 && K >= 1, "rb_conv_causal: bad sizes C=%d K=%d", C, K);
   const int threads = 128;
-  // Enough rows to give every SM several blocks: rows through registers, where 16-byte accesses are possible (below that,
-  // and for other sizes, a thread per row and channel).
-  if (x_dtype == RB_F32 && T >= 64 && K >= 2 && K <= 4 && C % 4 == 0 && ldx % 4 == 0 && x_off % 4 == 0 && (uintptr_t)x % 16 == 0 &&
-      (uintptr_t)u % 16 == 0 && (uintptr_t)tail % 16 == 0 && (C / 4 + threads - 1) / threads <= 65535) {
-    const dim3 rgrid((T + CONV_ROWS - 1) / CONV_ROWS, (C / 4 + threads - 1) / threads);
-#define ROWS(KK) RB_LAUNCH("conv_causal_rows_kernel", (conv_causal_rows_kernel<KK>), rgrid, threads, 0, stream, u, (const float*)x, ldx, x_off, x_bias, taps, conv_bias, tail, tok_first, tok_slot, tok_pos, T, C, silu)
-    if (K == 2) ROWS(2); else if (K == 3) ROWS(3); else ROWS(4);
-#undef ROWS
+  const int rows = rb_conv_rows(T, C, K);
+  if (rows > 0 && x_dtype == RB_F32 && ldx % 4 == 0 && x_off % 4 == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)u % 16 == 0 &&
+      (uintptr_t)tail % 16 == 0) {
+    const dim3 rgrid((T + rows - 1) / rows, (C / 4 + threads - 1) / threads);
+#define GO(KK, RR) RB_LAUNCH("conv_causal_rows_kernel", (conv_causal_rows_kernel<KK, RR>), rgrid, threads, 0, stream, u, (const float*)x, ldx, x_off, x_bias, taps, conv_bias, tail, tok_first, tok_slot, tok_pos, T, C, silu)
+#define OF_ROWS(KK) do { if (rows == 2) GO(KK, 2); else if (rows == 4) GO(KK, 4); else if (rows == 8) GO(KK, 8); else GO(KK, 16); } while (0)
+    if (K == 2) OF_ROWS(2); else if (K == 3) OF_ROWS(3); else OF_ROWS(4);
+#undef OF_ROWS
+#undef GO
     RB_CHECK_LAUNCH("rb_conv_causal");
     return 0;
   }

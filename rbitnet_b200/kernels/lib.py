@@ -33,6 +33,7 @@ _SIGNATURES = {
     "rb_head_gate": [P, P, P, L, I, I, I, I, I, I, P],
     "rb_gated_act": [P, P, I, I, I, I, L, I, I, F, F, F, P, P],
     "rb_tanh_norm": [P, I, P, P, P, F, I, I, P],
+    "rb_conv_rows": [I, I, I],
     "rb_conv_causal": [P, P, L, I, I, P, P, P, P, P, P, P, I, I, I, I, P],
     "rb_conv_tail_update": [P, P, L, I, I, P, P, P, P, P, I, I, I, P],
     "rb_delta_prepare": [P, L, P, L, I, I, P, P, P, P, P, P, I, I, I, I, F, F, P],

@@ -128,3 +128,20 @@ def test_plan_of_a_product_of_many_tokens(lib):
                     if p["blocks_per_team"]:
                         assert p["teams"] * p["token_tiles"] <= sms
                         assert p["teams"] * p["blocks_per_team"] >= w_tiles * blocks > (p["teams"] - 1) * p["blocks_per_team"]
+
+
+def test_rows_of_the_convolution_fill_the_sms(lib):
+    """A thread takes several rows only where enough blocks are left: never fewer than half of four an SM, or two rows."""
+    rows, sms = lib.raw("rb_conv_rows"), lib.raw("rb_device_sm_count")()
+    for C in (4, 64, 512, 1536, 2048, 4096, 8192):
+        for T in (1, 16, 63, 64, 100, 128, 256, 511, 512, 1000, 2048, 100000):
+            r = rows(T, C, 4)
+            assert r in (0, 2, 4, 8, 16)
+            blocks = -(-T // max(r, 1)) * -(-C // 512)
+            assert r <= 2 or blocks >= sms, (T, C, r)               # (64 rows of 2,048 channels in 16 blocks took 8.6 us, 3.2 in 128)
+            if T >= 512:
+                assert r >= 2
+            if r == 0:
+                assert T * -(-C // 128) < 6 * sms
+    assert rows(2048, 2048, 4) == 16 and rows(64, 2048, 4) == 2 and rows(16, 2048, 4) == 0
+    assert rows(2048, 2047, 4) == 0 and rows(2048, 2048, 5) == 0 and rows(2048, 2048, 1) == 0

@@ -243,20 +243,24 @@ def test_matrix_memory_kernel(ops32, H, D, Dv):
 
 
 @pytest.mark.parametrize("C,K,lengths,start", [(64, 4, [40, 1, 2, 60], 0), (4, 2, [64], 5), (516, 3, [15, 17, 33, 3], 2), (1024, 4, [700], 1),
-                                               (64, 4, [1] * 70, 3)])
+                                               (64, 4, [1] * 70, 3), (2048, 4, None, 9), (8192, 3, [70, 1, 130], 2), (2048, 2, [2100], 0),
+                                               (64, 4, [513], 6), (4096, 4, [300, 1, 1, 1, 40], 3), (1024, 4, [1] * 600, 8)])
 def test_convolution_of_many_rows(ops32, C, K, lengths, start):
-    """Rows through registers against a row and channel a thread (63 rows at most at a time), bit for bit: runs that begin inside
-    a block's rows, in the middle of a sequence (inputs from the ring) and at its start, with biases and SiLU."""
+    """Two to sixteen rows a thread against a thread per row and channel (which rows that 16-byte loads cannot take get), bit for bit:
+    runs that begin inside a block's rows, in the middle of a sequence (inputs from the ring) and at its start, rows that are their
+    own runs without a table of runs (lengths None: 130 of them), with biases and SiLU."""
     from ctypes import c_void_p
     g = torch.Generator(device="cuda").manual_seed(C + K)
+    alone = lengths is None
+    lengths = lengths or [1] * 130
     S, T = len(lengths), sum(lengths)
     x = torch.randn(T, C + 8, device="cuda", generator=g)
     taps, b, xb = torch.randn(C, K, device="cuda", generator=g), torch.randn(C, device="cuda", generator=g), torch.randn(C, device="cuda", generator=g)
     tail = torch.randn(S, K, C, device="cuda", generator=g)
     rows = [(i, sum(lengths[:i]), j) for i, n in enumerate(lengths) for j in range(n)]
     dev = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
-    first, slot, pos = dev([r[1] for r in rows]), dev([r[0] for r in rows]), dev([start + r[2] for r in rows])
-    ptr = lambda t: c_void_p(t.data_ptr())
+    first, slot, pos = None if alone else dev([r[1] for r in rows]), dev([r[0] for r in rows]), dev([start + r[2] for r in rows])
+    ptr = lambda t: c_void_p(t.data_ptr() if t is not None else 0)
     outs = []
     for misaligned in (False, True):                     # the second call's rows start one value behind a 16-byte boundary
         buf = torch.zeros(T * (C + 8) + 1, device="cuda")
