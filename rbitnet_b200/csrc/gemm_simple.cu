@@ -193,11 +193,22 @@ cudaError_t launch_parts(int n_parts, void (*kernel)(KArgs...), dim3 grid, dim3 
 // Parts of K for so many tiles.  K 2,048, us in 1, 2, 4, 8 parts (148 SMs): 32 tiles 98 50 40 30; 224 tiles 220 122 108 109;
 // 352 tiles 235 185 164 159; 704 tiles 317 299 302 312; 1,232 tiles 530 497 515 533; 5,632 tiles 2,218 2,215 2,324 2,404:
 // many parts even out what the SMs hold while the tiles are few, and cost their exchange once there are enough.
+// The exchange costs as much as a block of K.  That is nothing beside a long K, but below 512 it decides: there the parts are those
+// with the least of (waves of four blocks an SM, where one that is not full counts 0.4 and 0.6 of its share) x (blocks of K a
+// part, and one for the exchange).  K 128: 128 tiles 10.1 10.9 8.9 14.0; 320 tiles 19.3 20.5 20.7 30.6; 1,024 tiles 37.6 43.1
+// 51.9 86.8; 2,048 tiles 66 78 98 168.  K 64, 1,024 tiles: 23 30 41 41.
 int tile_parts(int64_t tiles, int K, int sms) {
   const int blocks = (K + LK - 1) / LK;
-  int p = tiles <= 3 * (int64_t)sms ? 8 : (tiles < 20 * (int64_t)sms ? 2 : 1);
-  while (p > blocks) p /= 2;
-  return p;
+  if (K >= 512) return tiles <= 3 * (int64_t)sms ? 8 : (tiles < 20 * (int64_t)sms ? 2 : 1);
+  int best = 1;
+  double least = 0;
+  for (int p = 1; p <= 8 && p <= blocks; p *= 2) {
+    const int64_t all = tiles * p, wave = 4 * (int64_t)sms;
+    const double rest = (double)(all % wave) / wave, waves = (double)(all / wave) + (rest > 0 ? 0.4 + 0.6 * rest : 0);
+    const double time = waves * ((double)blocks / p + (p > 1 ? 1 : 0));
+    if (p == 1 || time < least) { best = p; least = time; }
+  }
+  return best;
 }
 
 // ---- few rows
@@ -357,6 +368,10 @@ Tail take_tail() {
   return t;
 }
 
+// Few rows by lanes: W is read once for eight of them.  Against tiles, us: 2,048 x 2,048 with 16, 32 rows 10, 17 and 30, 31;
+// 11,264 x 2,048 with 16, 20, 32 rows 83, 97, 125 and 86, 87, 87; so more than 16 rows only where the outputs are few.
+bool few_rows(int M, int N) { return M <= 16 || (M <= 32 && N <= 4096); }
+
 }  // namespace
 
 // The next rb_gemm_simple, rb_gemm_simple_batched or rb_per_head_few_rows call of this thread adds bias[n] (float32, or
@@ -392,6 +407,12 @@ RB_EXPORT int rb_per_head_few_rows(void* C, int64_t ldc, int c_dtype, const void
   return 0;
 }
 
+// Into how many parts K is cut for this product (1: not; 0: few rows, which are not made by tiles).
+RB_EXPORT int rb_gemm_simple_parts(int M, int N, int K, int n_batch) {
+  if (few_rows(M, N)) return 0;
+  return tile_parts((int64_t)((N + TILE - 1) / TILE) * ((M + TILE - 1) / TILE) * n_batch, K, rb_sm_count());
+}
+
 // a_dtype: dtype of A and W; c_dtype: dtype of C.  accumulate: C += instead of C =.
 // alpha multiplies the finished sum (1.0 leaves it as it is).
 // n_batch products at once: product z reads A + z*batch_a and W + z*batch_w and writes C + z*batch_c
@@ -415,9 +436,7 @@ RB_EXPORT int rb_gemm_simple_batched(void* C, int64_t ldc, int c_dtype, const vo
     else RB_FAIL("rb_gemm_simple: unsupported dtypes a=%d c=%d", a_dtype, c_dtype);             \
   } while (0)
   const int sms = rb_sm_count();
-  // Few rows by lanes: W is read once for eight of them.  Against tiles, us: 2,048 x 2,048 with 16, 32 rows 10, 17 and 30,
-  // 31; 11,264 x 2,048 with 16, 20, 32 rows 83, 97, 125 and 86, 87, 87; so more than 16 rows only where the outputs are few.
-  if (M <= 16 || (M <= 32 && N <= 4096)) {
+  if (few_rows(M, N)) {
     const int rm = M <= 1 ? 1 : (M <= 2 ? 2 : (M <= 4 ? 4 : 8));
     const int groups = (N + ROW_N - 1) / ROW_N, ys = (M + rm - 1) / rm;
     const bool share = (int64_t)groups * ys * n_batch < (int64_t)sms * 16;

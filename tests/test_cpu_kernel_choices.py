@@ -145,3 +145,19 @@ def test_rows_of_the_convolution_fill_the_sms(lib):
                 assert T * -(-C // 128) < 6 * sms
     assert rows(2048, 2048, 4) == 16 and rows(64, 2048, 4) == 2 and rows(16, 2048, 4) == 0
     assert rows(2048, 2047, 4) == 0 and rows(2048, 2048, 5) == 0 and rows(2048, 2048, 1) == 0
+
+
+def test_parts_of_the_float32_product(lib):
+    """Cluster sizes that the blocks of K (16 values each) suffice for; many tiles of a short K stay whole (2,048 tiles of K 128 took
+    78 us in two parts, 66 whole), few tiles of a long K are cut."""
+    parts, sms = lib.raw("rb_gemm_simple_parts"), lib.raw("rb_device_sm_count")()
+    for M in (17, 33, 64, 130, 300, 512, 1024, 2048, 8192):
+        for N in (1, 64, 256, 2048, 5000, 8192):
+            for K in (1, 16, 17, 48, 64, 100, 128, 256, 511, 512, 2048, 11008):
+                p = parts(M, N, K, 1)
+                assert p in ((0,) if M <= 32 and N <= 4096 else (1, 2, 4, 8)) and p <= -(-K // 16), (M, N, K, p)
+                tiles = -(-M // 64) * -(-N // 64)
+                if K <= 256 and tiles >= 6 * sms:
+                    assert p in (0, 1), (M, N, K, p)
+    assert parts(64, 2048, 2048, 1) == 8 and parts(2048, 2048, 2048, 1) == 2 and parts(2048, 11264, 2048, 1) == 1
+    assert parts(300, 256, 128, 16) == 1 and parts(100, 256, 128, 16) == 4 and parts(1, 1, 1, 1) == 0

@@ -808,9 +808,10 @@ def test_a_last_round_of_few_tiles_becomes_a_product_of_its_own(ops16, T, F, K):
 # --------------------------------------------------------------------------- the float32 product and attention by size
 @pytest.mark.parametrize("M,N,K", [(1, 4, 4), (1, 2050, 130), (2, 33, 2048), (3, 1000, 513), (5, 96, 96), (8, 12000, 260),
                                    (9, 64, 20), (16, 5000, 36), (17, 70, 16), (31, 4096, 100), (33, 65, 15), (33, 4100, 2049),
-                                   (64, 64, 1024), (65, 129, 777), (130, 30000, 24), (700, 2048, 48), (129, 1, 1)])
+                                   (64, 64, 1024), (65, 129, 777), (130, 30000, 24), (700, 2048, 48), (129, 1, 1),
+                                   (40, 5000, 100), (70, 200, 64), (256, 2048, 200), (130, 4100, 254)])
 def test_float32_products_at_the_edges_of_their_kernels(ops32, M, N, K):
-    """Rows by lanes (1, 2, 4 and 8 rows a warp, K shared by a block's warps or not), tiles with K in 1, 2 and 8 parts, whole and
+    """Rows by lanes (1, 2, 4 and 8 rows a warp, K shared by a block's warps or not), tiles with K in 1, 2, 4 and 8 parts, whole and
     ragged, rows that 16-byte loads can and cannot take; stored, added and scaled.  A float32 sum of K products in any order is
     within K 2^-24 of the sum of their magnitudes (first order); the addition and the scale round once more each."""
     g = torch.Generator(device="cuda").manual_seed(31)
