@@ -73,8 +73,9 @@ __global__ void __launch_bounds__(TILE_THREADS, 4) gemm_tile_kernel(
   W += blockIdx.z * batch_w;
   __shared__ __align__(16) float sm[2 * 2 * LK * PITCH];   // [buffer][A, W][LK][PITCH]; at the end [TILE][PITCH], this part's sums
   static_assert(2 * 2 * LK >= TILE, "a tile's sums fit the buffers");
-  const int part = blockIdx.x % n_parts;
-  const int m0 = blockIdx.y * TILE, n0 = blockIdx.x / n_parts * TILE;
+  // blockIdx.x counts parts, tiles of a row of tiles and rows of tiles: y would end at 65,535
+  const int part = blockIdx.x % n_parts, tile = blockIdx.x / n_parts, tiles_n = (N + TILE - 1) / TILE;
+  const int m0 = tile / tiles_n * TILE, n0 = tile % tiles_n * TILE;
   const int n_blocks = (K + LK - 1) / LK;
   const int k_first = (int)((int64_t)n_blocks * part / n_parts) * LK;
   const int k_end = min(K, (int)((int64_t)n_blocks * (part + 1) / n_parts) * LK);
@@ -454,8 +455,8 @@ RB_EXPORT int rb_gemm_simple_batched(void* C, int64_t ldc, int c_dtype, const vo
   } else {
     const int64_t tiles_n = (N + TILE - 1) / TILE, tiles_m = (M + TILE - 1) / TILE;
     const int parts = tile_parts(tiles_n * tiles_m * n_batch, K, sms);
-    RB_REQUIRE(tiles_m <= 65535 && tiles_n * parts <= 0x7fffffff, "rb_gemm_simple: M=%d N=%d: too large for one launch", M, N);
-    const dim3 grid((unsigned)(tiles_n * parts), (unsigned)tiles_m, n_batch);
+    RB_REQUIRE(tiles_n * tiles_m * parts <= 0x7fffffff, "rb_gemm_simple: M=%d N=%d: too large for one launch", M, N);
+    const dim3 grid((unsigned)(tiles_n * tiles_m * parts), 1, n_batch);
 #define GO(VEC, TA, TC)                                                                                                 \
   do {                                                                                                                  \
     const cudaError_t e = launch_parts(parts, gemm_tile_kernel<VEC, TA, TC>, grid, TILE_THREADS, stream, (TC*)C, ldc, (const TA*)A, lda, (const TA*)W, ldw, M, N, K, accumulate, alpha, tail, batch_c, batch_a, batch_w, parts); \

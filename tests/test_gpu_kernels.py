@@ -829,6 +829,19 @@ def test_float32_products_at_the_edges_of_their_kernels(ops32, M, N, K):
         assert ((acc.double() - want).abs() <= bound + 2.0 ** -23 * want.abs()).all()
 
 
+def test_float32_product_of_more_rows_than_a_grids_second_dimension(ops32):
+    """65,536 and more rows of tiles (64 rows each).  The bound is that of the test above."""
+    M, N, K = 65536 * 64 + 5, 128, 4
+    g = torch.Generator(device="cuda").manual_seed(33)
+    x = torch.randn(M, K, device="cuda", generator=g)
+    w = torch.randn(N, K, device="cuda", generator=g)
+    got = ops32.linear(x, ops32.prepare_linear([w]))
+    for a in (0, M // 2, M - 70):
+        rows = x[a:a + 70].double()
+        bound = (K + 4) * 2.0 ** -24 * (rows.abs() @ w.double().abs().T) + 1e-30
+        assert ((got[a:a + 70].double() - rows @ w.double().T).abs() <= bound).all()
+
+
 @pytest.mark.parametrize("H,Kh,D,page,lengths,decode", [(4, 2, 30, 64, [5, 1], False), (2, 1, 64, 48, [130], False),
                                                         (32, 4, 64, 64, [300, 17], True), (3, 3, 129, 16, [70, 1], True),
                                                         (1, 1, 1024, 64, [20], False), (2, 2, 260, 64, [40, 33], True),
