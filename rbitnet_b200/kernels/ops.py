@@ -28,6 +28,19 @@ def _ptr(t: Optional[torch.Tensor]):
     return c_void_p(t.data_ptr()) if t is not None else c_void_p(0)
 
 
+def memory_chunks_pay(longest: int, tokens: int, chunks: int, heads: int, dim: int, value_dim: int) -> bool:
+    """Whether a step's runs (``tokens`` in all, ``longest`` the longest of them, ``chunks`` chunks of 64) go through a matrix memory
+    sooner in chunks than token by token: microseconds of the two forms on one B200, from runs of 16 to 500 tokens, 1 to 64 of
+    them, and memories of 16 x 24 to 512 x 512 (the choice is within 1 % of the better form on average; never more than 1.1 times
+    token by token).  Token by token a run is a chain of its tokens, at least; many runs are bound by the memory's updates.
+    In chunks there are four kernels with the chain of 64 + ``dim`` products in them, then every chunk's memory."""
+    a_token = 0.3 if dim <= 64 else 0.4 if dim <= 128 else 1.0 if dim <= 256 else 2.0
+    memory = heads * dim * value_dim
+    by_token = max(5.0 + a_token * longest, tokens * memory / (1.3e6 if dim <= 256 else 0.65e6))
+    in_chunks = max(27.0, 15.0 + 0.22 * dim) + chunks * (0.15 + memory / 80e3)
+    return in_chunks < by_token
+
+
 @dataclass
 class LinearWeight:
     """A weight matrix [out, in] made ready for ``linear``."""
@@ -178,10 +191,9 @@ class CudaOps:
         self.gla_in_chunks = True
         #: in bfloat16 mode a state-space mixer takes runs of several tokens in chunks of 64 (else token by token)
         self.ssd_in_chunks = True
-        #: a matrix memory takes runs of several tokens in chunks of 64 (else token by token) from so many tokens on: of a
-        #: run on average, and of the step.  Us token by token and in chunks, 8 heads of 128 x 256: one run of 32 tokens 19,
-        #: 39; of 100 46, 45; of 300 117, 72; 16 runs of 16 tokens 60, 77; of 32 105, 86
-        self.memory_in_chunks, self.memory_chunks_from = True, (24, 128)
+        #: a matrix memory takes runs of several tokens in chunks of 64 (else token by token) where ``memory_chunks_pay`` says so,
+        #: or (not None) from so many tokens on, of a run on average and of the step
+        self.memory_in_chunks, self.memory_chunks_from = True, None
         #: and with at most this much scratch (a memory per chunk and head: 1 GiB; 8,192 tokens of 8 heads of 256 x 512 take 0.6)
         self.memory_scratch_floats = 1 << 28
         #: a decode step's delta rule (convolution to gate) is one kernel while rows x heads fit the SMs
@@ -796,12 +808,10 @@ class CudaOps:
         out = torch.empty((T, H * Dv), dtype=self.dtype, device=self.device)
         bias = (_ptr(p.i_bias), _ptr(p.f_bias), float(p.gate_cap), float(D) ** -0.5, float(p.floor))
         kept = (_ptr(state["C"]), _ptr(state["n"]), _ptr(state["m"]))
-        per_run, per_step = self.memory_chunks_from
-        chunked = first is not None and self.memory_in_chunks and T >= per_run * n_seq and T >= per_step
+        chunked = first is not None and self.memory_in_chunks and self._memory_chunks_chosen(meta, n_seq, H, D, Dv)
         if chunked:
             run0, rows, lens, n_chunks = self._delta_chunks(meta, 64)
             floats = self.lib.raw("rb_matrix_memory_chunk_floats")(n_chunks, H, D, Dv)
-            chunked = floats <= self.memory_scratch_floats
         if not chunked:
             moved = torch.empty((n_seq, H, D + 1), dtype=torch.float32, device=self.device)
             self.lib.call("rb_matrix_memory", _ptr(out), self.code, _ptr(o), _ptr(proj), proj.stride(0), F32, at["q"], at["k"],
@@ -815,6 +825,19 @@ class CudaOps:
         self.lib.call("rb_head_norm_gate", _ptr(out), self.code, _ptr(o), _ptr(p.norm_w), _ptr(proj), proj.stride(0), F32,
                       at["g"], T, H, Dv, float(p.norm_eps), 0, 0, self._stream())
         return out
+
+    def _memory_chunks_chosen(self, meta, n_seq: int, H: int, D: int, Dv: int) -> bool:
+        """Whether the step's runs go through a matrix memory in chunks of 64: by time, and if the scratch is allowed."""
+        key = ("memory_chunks", H, D, Dv, self.memory_chunks_from, self.memory_scratch_floats)
+        if key not in meta.extra:
+            longest = max(c.n_new for c in meta.seqs)
+            chunks = sum(-(-c.n_new // 64) for c in meta.seqs)
+            if self.memory_chunks_from is None:
+                wanted = memory_chunks_pay(longest, meta.n_tokens, chunks, H, D, Dv)
+            else:
+                wanted = meta.n_tokens >= self.memory_chunks_from[0] * n_seq and meta.n_tokens >= self.memory_chunks_from[1]
+            meta.extra[key] = wanted and self.lib.raw("rb_matrix_memory_chunk_floats")(chunks, H, D, Dv) <= self.memory_scratch_floats
+        return meta.extra[key]
 
     def _delta_chunks(self, meta, size: int = 32):
         """The step's runs cut into chunks of ``size`` rows (device int32: per run its first chunk; per chunk its first

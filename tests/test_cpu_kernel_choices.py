@@ -161,3 +161,18 @@ def test_parts_of_the_float32_product(lib):
                     assert p in (0, 1), (M, N, K, p)
     assert parts(64, 2048, 2048, 1) == 8 and parts(2048, 2048, 2048, 1) == 2 and parts(2048, 11264, 2048, 1) == 1
     assert parts(300, 256, 128, 16) == 1 and parts(100, 256, 128, 16) == 4 and parts(1, 1, 1, 1) == 0
+
+
+def test_when_a_matrix_memory_goes_in_chunks():
+    """The longest run decides where the runs are few, not their average; small memories and short runs stay token by token."""
+    from rbitnet_b200.kernels.ops import memory_chunks_pay
+
+    def pays(lengths, H, D, Dv):
+        return memory_chunks_pay(max(lengths), sum(lengths), sum(-(-n // 64) for n in lengths), H, D, Dv)
+    assert pays([2048], 8, 128, 256) and pays([2048], 8, 256, 512) and pays([300], 4, 64, 64)
+    assert pays([2000] + [1] * 90, 8, 128, 256)                     # one long prompt beside 90 decoding rows
+    assert not pays([24] * 6, 8, 128, 256)                          # 30 us token by token, 49 in chunks
+    assert not pays([48] * 16, 4, 64, 64) and not pays([64] * 16, 2, 16, 24)
+    assert pays([64] * 16, 8, 128, 256) and not pays([16] * 64, 8, 128, 256)
+    for size in ((8, 128, 256), (2, 512, 512), (1, 1, 1)):
+        assert not pays([2], *size) and not pays([1, 1, 2], *size)
