@@ -812,13 +812,16 @@ class CudaOps:
         if chunked:
             run0, rows, lens, n_chunks = self._delta_chunks(meta, 64)
             floats = self.lib.raw("rb_matrix_memory_chunk_floats")(n_chunks, H, D, Dv)
+            try:
+                scratch = torch.empty((floats,), dtype=torch.float32, device=self.device)
+            except torch.OutOfMemoryError:
+                chunked = False                  # beside a cache that fills the memory: slower, but without the scratch
         if not chunked:
             moved = torch.empty((n_seq, H, D + 1), dtype=torch.float32, device=self.device)
             self.lib.call("rb_matrix_memory", _ptr(out), self.code, _ptr(o), _ptr(proj), proj.stride(0), F32, at["q"], at["k"],
                           at["v"], at["g"], at["i"], at["f"], *bias, _ptr(p.norm_w), float(p.norm_eps), *kept, _ptr(moved),
                           _ptr(first), _ptr(count), _ptr(meta.tok_slot), T, n_seq, H, D, Dv, self._stream(), launches=2)
             return out
-        scratch = torch.empty((floats,), dtype=torch.float32, device=self.device)
         self.lib.call("rb_matrix_memory_chunked", _ptr(o), _ptr(proj), proj.stride(0), at["q"], at["k"], at["v"], at["i"],
                       at["f"], *bias, *kept, _ptr(first), _ptr(count), _ptr(run0), _ptr(rows), _ptr(lens),
                       _ptr(meta.tok_slot), n_seq, n_chunks, H, D, Dv, _ptr(scratch), self._stream(), launches=4)

@@ -476,3 +476,30 @@ def test_a_failed_allocation_leaves_no_store_behind(ops32, lengths, monkeypatch)
         assert torch.equal(ops32.matrix_memory(proj, part, state, meta), want)
         assert all(torch.equal(state[k], good[k]) for k in start)
     assert not failed and which >= 2
+
+
+def test_a_prompt_without_room_for_the_chunks_scratch(ops32, monkeypatch):
+    """Where the chunked form's scratch cannot be had the prompt goes token by token, with that form's bits."""
+    from rbitnet_b200.parts.recurrent import MatrixMemory
+    H, D, Dv, T = 2, 64, 48, 300
+    g = torch.Generator(device="cuda").manual_seed(53)
+    part = MatrixMemory(16, H, D, Dv, gate_cap=6.0, norm_eps=1e-5)
+    part.bind({k: 0.3 * torch.randn(shape, device="cuda", generator=g) for k, (shape, _) in part.weight_shapes().items()}, ops32)
+    proj = torch.randn(T, 2 * H * D + 2 * H * Dv + 2 * H, device="cuda", generator=g)
+    floats = ops32.lib.raw("rb_matrix_memory_chunk_floats")(-(-T // 64), H, D, Dv)
+    real, refused, results = torch.empty, [], []
+
+    def no_room(*a, **k):
+        if a and a[0] == (floats,):
+            refused.append(1)
+            raise torch.OutOfMemoryError("planted")
+        return real(*a, **k)
+    for chunks, empty in ((False, real), (True, no_room)):
+        state = {k: torch.zeros((1, *s.shape), device="cuda") for k, s in part.state_need().items()}
+        monkeypatch.setattr(ops32, "memory_in_chunks", chunks)
+        monkeypatch.setattr(torch, "empty", empty)
+        out = ops32.matrix_memory(proj, part, state, _meta(ops32, [(0, 0, T)]))
+        monkeypatch.setattr(torch, "empty", real)
+        results.append((out, state))
+    assert refused == [1] and torch.equal(results[0][0], results[1][0])
+    assert all(torch.equal(results[0][1][k], results[1][1][k]) for k in results[0][1])
