@@ -28,6 +28,21 @@ def _ptr(t: Optional[torch.Tensor]):
     return c_void_p(t.data_ptr()) if t is not None else c_void_p(0)
 
 
+def gated_parts(T: int, N: int, K: int, parts: int, sms: int) -> int:
+    """Parts of K of a gated product of T tokens and N weight rows (gate and up), from those that would give every SM a piece of the
+    weights.  Us whole and in parts: 2,816 rows of 2,048, 8 parts: 1 token 11.1, 5.4, 64 tokens 15.0, 8.4; 4 parts: 128 tokens
+    17.2, 11.2; 3,584 rows of 4,096, 8 parts: 8 tokens 19.7, 8.3.
+    Two parts only beside tiles of 128 and more tokens, and for a K of 4,096 and more: 3,584 rows of 4,096, 192 tokens 26.5, 22.2;
+    but 5,632 rows of 2,048, 65 tokens 15.3, 17.3, of 1,024 11.1, 15.1; 192 rows of 512 8.7, 13.0.
+    More than 32 tokens' sums cost as much as a short K where the parts are well more than the SMs: 8,192 rows of 1,024 in 4
+    parts, 17 tokens 8.4, 7.3, 48 tokens 9.7, 10.5."""
+    if parts < 4:
+        return parts if parts >= 2 and T > 64 and K >= 4096 else 1
+    if K < 2048 and T > 32 and 2 * -(-N // 128) * parts > 3 * sms:
+        return 1
+    return parts
+
+
 def memory_chunks_pay(longest: int, tokens: int, chunks: int, heads: int, dim: int, value_dim: int) -> bool:
     """Whether a step's runs (``tokens`` in all, ``longest`` the longest of them, ``chunks`` chunks of 64) go through a matrix memory
     sooner in chunks than token by token: microseconds of the two forms on one B200, from runs of 16 to 500 tokens, 1 to 64 of
@@ -418,14 +433,9 @@ class CudaOps:
         return self.lib.raw("rb_gemm_tc_splits")(T, N, K)
 
     def _gated_splits(self, T: int, N: int, K: int):
-        """(parts of K, token tile) of a gated product.  Us whole and in parts: 2,816 rows of 2,048, 8 parts: 1 token 11.1, 5.4,
-        64 tokens 15.0, 8.4; 4 parts: 128 tokens 17.2, 11.2; 3,584 rows of 4,096, 8 parts: 8 tokens 19.7, 8.3.  Two parts
-        only beside tiles of 128 and more tokens (3,584 rows, 192 tokens: 25.7, 22.9): 11,264 rows of 2,048 in two parts
-        take 12.8 us for 13.1 alone, no less in a step, and 20.9 for 17.2 with 64 tokens."""
-        splits = self._k_splits(T, N, K) if self.split_gated else 1
-        if splits < 4 and not (splits >= 2 and T > 64):
-            return 1, 0
-        return splits, 64 if T > 64 else 0
+        """(parts of K, token tile) of a gated product: those of ``gated_parts``, and tiles of 64 tokens at most beside them."""
+        parts = gated_parts(T, N, K, self._k_splits(T, N, K), self.lib.raw("rb_device_sm_count")()) if self.split_gated else 1
+        return parts, 64 if parts > 1 and T > 64 else 0
 
     def _tensor_core_ok(self, x: torch.Tensor, w: torch.Tensor) -> bool:
         """The tcgen05 product takes bfloat16 operands whose rows TMA can address: inner size and

@@ -176,3 +176,13 @@ def test_when_a_matrix_memory_goes_in_chunks():
     assert pays([64] * 16, 8, 128, 256) and not pays([16] * 64, 8, 128, 256)
     for size in ((8, 128, 256), (2, 512, 512), (1, 1, 1)):
         assert not pays([2], *size) and not pays([1, 1, 2], *size)
+
+
+def test_parts_of_a_gated_product():
+    """Two parts of a short K and many parts' sums of many tokens are left out: each was slower than the product whole."""
+    from rbitnet_b200.kernels.ops import gated_parts
+    assert gated_parts(1, 2816, 2048, 8, 148) == 8 and gated_parts(64, 2816, 2048, 8, 148) == 8
+    assert gated_parts(192, 3584, 4096, 2, 148) == 2 and gated_parts(64, 3584, 4096, 2, 148) == 1
+    assert gated_parts(65, 192, 512, 2, 148) == 1 and gated_parts(192, 5632, 1024, 2, 148) == 1 and gated_parts(65, 5632, 2048, 2, 148) == 1
+    assert gated_parts(48, 8192, 1024, 4, 148) == 1 and gated_parts(17, 8192, 1024, 4, 148) == 4 and gated_parts(48, 5632, 1024, 4, 148) == 4
+    assert gated_parts(300, 2816, 2048, 1, 148) == 1

@@ -246,14 +246,21 @@ def test_few_pairs_are_placed_as_many_are(dtype, weighed, T, E, n_experts, top, 
 
 
 @pytest.mark.parametrize("T,inner,E", [(1, 96, 1024), (16, 1408, 2048), (17, 200, 1032), (64, 48, 1024), (65, 1408, 2048), (200, 96, 4096)])
-@pytest.mark.parametrize("act", [None, (1.702, 7.0, 1.0), "gelu_tanh", "relu"])
+@pytest.mark.parametrize("act", [None, (1.702, 7.0, 1.0), "gelu_tanh", "relu", "biases", "norm"])
 def test_gated_products_with_parts_of_k(T, inner, E, act):
     """Parts of K in a cluster against K whole: both round the same float32 value once, so a value differs by one step of bfloat16
-    (2^-8 of it) where the sums' last bits decide; with room for the sums' own error, K 2^-24 of their magnitudes."""
+    (2^-8 of it) where the sums' last bits decide; with room for the sums' own error, K 2^-24 of their magnitudes.  Also with biases, and on rows whose norm is pending (as a product
+    of up to 16 tokens takes them)."""
+    from rbitnet_b200.kernels.ops import NormedRows
+    kind, act = act, None if act in ("biases", "norm") else act
     ops = _ops(torch.bfloat16)
     g = torch.Generator().manual_seed(T + inner)
     x = torch.randn(T, E, generator=g).to(torch.bfloat16).cuda()
-    w = ops.prepare_gate_up(*(torch.randn(inner, E, generator=g).to(torch.bfloat16).cuda() / E ** 0.5 for _ in range(2)))
+    biases = [torch.randn(inner, generator=g).cuda() for _ in range(2)] if kind == "biases" else []
+    w = ops.prepare_gate_up(*(torch.randn(inner, E, generator=g).to(torch.bfloat16).cuda() / E ** 0.5 for _ in range(2)), *biases)
+    if kind == "norm":
+        rows, gw = torch.randn(T, E, generator=g).cuda(), torch.rand(E, generator=g).cuda() + 0.5
+        x = NormedRows(rows, gw, 1e-5, (rows * gw).to(torch.bfloat16), rows.square().sum(-1)[None].contiguous())
     before = ops.split_gated
     try:
         ops.split_gated = True
