@@ -183,18 +183,16 @@ class SequenceCache:
         """Bring the device page tables up to date (rows that changed since the last call)."""
         for g, grp in enumerate(self.groups):
             slots = [s for s in sorted(grp.dirty) if s in self.book.pages and self.book.pages[s][g]]
-            grp.dirty.clear()
-            if not slots:
-                continue
             # (Entries of pages that were given back behind a window keep their old number: no kernel reads that far back.)
-            lo, hi = slots[0], slots[-1] + 1
-            if hi - lo <= 2 * len(slots):
+            if slots and slots[-1] + 1 - slots[0] <= 2 * len(slots):
+                lo, hi = slots[0], slots[-1] + 1
                 # neighbours in one copy; rows between them that have not changed get the values they have
                 grp.table[lo:hi].copy_(upload(grp.table_host[lo:hi], grp.table.device))
             else:
                 for s in slots:
                     n = len(self.book.pages[s][g])
                     grp.table[s, :n].copy_(upload(grp.table_host[s, :n], grp.table.device))
+            grp.dirty.clear()                    # once they have been copied: a copy that fails is made up for by the next call
 
     # ---- views
     def view(self, entry: int) -> CacheLayerView:

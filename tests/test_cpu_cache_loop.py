@@ -1,6 +1,7 @@
 """The cache's bookkeeping and the generation loop's decisions (no GPU)."""
 import random
 
+import numpy as np
 import pytest
 import torch
 
@@ -396,3 +397,55 @@ def test_loop_that_launches_ahead_gives_the_same_results(case):
     assert sorted(seen[True]) == sorted(seen[False])
     for r in range(len(script)):                                  # per request the tokens come in order
         assert [t for q, t in seen[True] if q == r] == outs[True][r].tokens
+
+
+def test_an_uploaded_array_may_change():
+    from rbitnet_b200.cache import upload
+    a = np.arange(12, dtype=np.int32)
+    t = upload(a, "cpu")
+    a[:] = -1
+    assert t.tolist() == list(range(12))
+
+
+def test_page_tables_follow_the_host_rows(monkeypatch):
+    """Rows that changed reach the device's table whether they are neighbours (one copy) or far apart (one each), also after a copy
+    that failed."""
+    import rbitnet_b200.cache.cache as module
+    rng = random.Random(1)
+    cache = SequenceCache({0: CacheNeed(1, 8), 1: CacheNeed(1, 8, window=20)}, reads={}, state_needs={}, max_tokens=16 * 200, max_seq=128,
+                          dtype=torch.float32, device="cpu", page_size=16, n_slots=24)
+    live, real, copies = [], module.upload, []
+
+    def counted(array, device):
+        copies.append(array.shape)
+        if rng.random() < 0.2:
+            raise torch.OutOfMemoryError("planted")
+        return real(array, device)
+    monkeypatch.setattr(module, "upload", counted)
+    shapes = set()
+    for _ in range(400):
+        if len(live) < 20 and rng.random() < 0.4:
+            live.append(cache.alloc())
+        elif live and rng.random() < 0.15:
+            cache.free(live.pop(rng.randrange(len(live))))
+        for s in live:
+            if rng.random() < rng.choice((0.05, 0.9)):
+                n = min(rng.randint(1, 20), 128 - cache.length(s))
+                try:
+                    if n > 0:
+                        cache.reserve(s, n)
+                        cache.advance(s, n)
+                except CacheFull:
+                    pass
+        try:
+            cache.upload_tables()
+        except torch.OutOfMemoryError:
+            continue
+        shapes |= {len(c) for c in copies}
+        copies.clear()
+        for g, grp in enumerate(cache.groups):
+            for s in live:
+                pages = cache.book.pages[s][g]
+                assert [p for p in grp.table[s, :len(pages)].tolist()] == grp.table_host[s, :len(pages)].tolist()
+                assert all(p in (-1, t) for p, t in zip(pages, grp.table[s].tolist()))
+    assert shapes == {1, 2}

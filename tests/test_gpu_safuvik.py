@@ -503,3 +503,30 @@ def test_a_prompt_without_room_for_the_chunks_scratch(ops32, monkeypatch):
         results.append((out, state))
     assert refused == [1] and torch.equal(results[0][0], results[1][0])
     assert all(torch.equal(results[0][1][k], results[1][1][k]) for k in results[0][1])
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_many_sequences_give_the_same_bits_again(dtype):
+    """Sixteen unequal prompts in one step, then captured decode steps for all: matrix memories whose blocks are several times what the
+    GPU holds at once, so that blocks of one (sequence, head) run at different times.  A second engine gives the same bits, and
+    float32 logits are the plain model's."""
+    from rbitnet_b200.engine.step import StepEntry
+    from safuvik_tiny import memory_layer, dense
+    cfg = {"architecture": "Safuvik", "vocab": 80, "width": 128, "norm": {"eps": 1e-5}, "streams": 2, "logit_scale": 0.5,
+           "layers": [memory_layer(16, 64, 128, 10.0, dense(96, 2.0)), memory_layer(8, 128, 256, 10.0, None)]}
+    tensors = make_tensors(cfg, seed=21)
+    lengths = [3, 17, 40, 1, 26, 9, 33, 2, 12, 65, 5, 21, 30, 8, 14, 48]
+    steps = 4
+    toks = [tokens_for(cfg, n + steps, 60 + i) for i, n in enumerate(lengths)]
+    runs = []
+    for _ in range(2):
+        eng = engine_maker(dtype)(cfg, tensors, max_tokens=64 * 64, graphs=True)
+        slots = [eng.new_sequence() for _ in lengths]
+        out = [eng.step([StepEntry(s, t[:n], [n - 1]) for s, t, n in zip(slots, toks, lengths)]).float().cpu()]
+        for k in range(steps):
+            out.append(eng.step([StepEntry(s, [t[n + k]], [0]) for s, t, n in zip(slots, toks, lengths)], captured=True).float().cpu())
+        runs.append(torch.stack(out))                                # [1 + steps, sequences, vocab]
+    assert torch.equal(runs[0], runs[1])
+    if dtype == "float32":
+        for i, (t, n) in enumerate(zip(toks, lengths)):
+            assert rel_err(runs[0][:, i], plain.forward(cfg, tensors, t, torch.float64)[n - 1:n + steps]) <= TOL[dtype], i
