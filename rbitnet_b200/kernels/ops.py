@@ -43,16 +43,19 @@ def gated_parts(T: int, N: int, K: int, parts: int, sms: int) -> int:
     return parts
 
 
-def memory_chunks_pay(longest: int, tokens: int, chunks: int, heads: int, dim: int, value_dim: int) -> bool:
+def memory_chunks_pay(longest: int, tokens: int, chunks: int, heads: int, dim: int, value_dim: int, sms: int = 148) -> bool:
     """Whether a step's runs (``tokens`` in all, ``longest`` the longest of them, ``chunks`` chunks of 64) go through a matrix memory
     sooner in chunks than token by token: microseconds of the two forms on one B200, from runs of 16 to 500 tokens, 1 to 64 of
-    them, and memories of 16 x 24 to 512 x 512 (the choice is within 1 % of the better form on average; never more than 1.1 times
-    token by token).  Token by token a run is a chain of its tokens, at least; many runs are bound by the memory's updates.
-    In chunks there are four kernels with the chain of 64 + ``dim`` products in them, then every chunk's memory."""
-    a_token = 0.3 if dim <= 64 else 0.4 if dim <= 128 else 1.0 if dim <= 256 else 2.0
+    them, and memories of 16 x 24 to 512 x 512 (within 1 % of the better form on average, and at most a tenth over token by
+    token).  Token by token a run is a chain of its tokens, at least; many runs are bound by the memory's updates.  In chunks the
+    waves of blocks count, five to an SM: of the outputs, each 64 + ``dim`` products long, and of the sums; then the bytes of
+    every chunk's memory."""
+    a_token = 0.27 if dim <= 64 else 0.4 if dim <= 128 else 1.0 if dim <= 256 else 2.0
     memory = heads * dim * value_dim
     by_token = max(5.0 + a_token * longest, tokens * memory / (1.3e6 if dim <= 256 else 0.65e6))
-    in_chunks = max(27.0, 15.0 + 0.22 * dim) + chunks * (0.15 + memory / 80e3)
+    tiles, rows = -(-value_dim // 64), -(-dim // 64)
+    waves = lambda blocks: -(-chunks * heads * blocks // (5 * sms))
+    in_chunks = 10.0 + 9.8 * waves(tiles) * (1 + dim / 64) + 1.6 * waves(1 + tiles * rows) + chunks * (0.25 + 9.7e-6 * memory)
     return in_chunks < by_token
 
 
@@ -846,7 +849,7 @@ class CudaOps:
             longest = max(c.n_new for c in meta.seqs)
             chunks = sum(-(-c.n_new // 64) for c in meta.seqs)
             if self.memory_chunks_from is None:
-                wanted = memory_chunks_pay(longest, meta.n_tokens, chunks, H, D, Dv)
+                wanted = memory_chunks_pay(longest, meta.n_tokens, chunks, H, D, Dv, self.lib.raw("rb_device_sm_count")())
             else:
                 wanted = meta.n_tokens >= self.memory_chunks_from[0] * n_seq and meta.n_tokens >= self.memory_chunks_from[1]
             meta.extra[key] = wanted and self.lib.raw("rb_matrix_memory_chunk_floats")(chunks, H, D, Dv) <= self.memory_scratch_floats

@@ -171,6 +171,7 @@ def test_when_a_matrix_memory_goes_in_chunks():
         return memory_chunks_pay(max(lengths), sum(lengths), sum(-(-n // 64) for n in lengths), H, D, Dv)
     assert pays([2048], 8, 128, 256) and pays([2048], 8, 256, 512) and pays([300], 4, 64, 64)
     assert pays([2000] + [1] * 90, 8, 128, 256)                     # one long prompt beside 90 decoding rows
+    assert pays([200] + [1] * 7, 8, 256, 512)                       # 256 us token by token, 164 in chunks
     assert not pays([24] * 6, 8, 128, 256)                          # 30 us token by token, 49 in chunks
     assert not pays([48] * 16, 4, 64, 64) and not pays([64] * 16, 2, 16, 24)
     assert pays([64] * 16, 8, 128, 256) and not pays([16] * 64, 8, 128, 256)
