@@ -45,10 +45,10 @@ __device__ __forceinline__ float rescale(float m, float to) { return m == -INFIN
 
 // L lanes a key, Q groups of four values a lane; `share` warps of the block for a (token, head) pair.
 template <typename T, bool VEC, int L, int Q>
-__global__ void __launch_bounds__(WARPS * 32) attn_simple_kernel(T* __restrict__ out, const T* __restrict__ q,
-                                                         RbPagedLayer cache, int page_shift, const int* __restrict__ tok_pos,
-                                                         const int* __restrict__ tok_slot, int n_tokens, int H,
-                                                         float scale, int window, const float* __restrict__ sinks,
+__global__ void __launch_bounds__(WARPS * 32) attn_simple_kernel(T* out, const T* q,
+                                                         RbPagedLayer cache, int page_shift, const int* tok_pos,
+                                                         const int* tok_slot, int n_tokens, int H,
+                                                         float scale, int window, const float* sinks,
                                                          float softcap, int keep, int share) {
   constexpr int KEYS = 32 / L;
   extern __shared__ float parts[];                     // share > 1: [WARPS][D + 2]

@@ -357,8 +357,8 @@ __global__ void __launch_bounds__(WARPS * 32) attn_tiled_kernel(AttnParams p) {
 }
 
 // Merges the partials of a split decode in split order.
-__global__ void attn_combine_kernel(__nv_bfloat16* __restrict__ out, const float* __restrict__ part_o,
-                                    const float* __restrict__ part_ml, int n_splits, int D) {
+__global__ void attn_combine_kernel(__nv_bfloat16* out, const float* part_o,
+                                    const float* part_ml, int n_splits, int D) {
   rb_pdl_launch_dependents();
   rb_pdl_wait();
   // One thread per output value.  The parts are taken 16 at a time with all their loads issued

@@ -22,11 +22,11 @@ __device__ __forceinline__ float softplus_(float v) { return fmaxf(v, 0.f) + log
 // u: rows [T, 2 G D + H Dv] (q heads, k heads, v heads) after the convolution and its activation; q and k are
 // normalised in place.  proj: the projections' float32 rows with b at column b_off and a at column a_off.
 // Leaves beta, decay and its logarithm [T, H], and kq [T, G] (the product k . q of the finished vectors).
-__global__ void __launch_bounds__(128) delta_prepare_kernel(float* __restrict__ u, int64_t ldu, const float* __restrict__ proj,
-                                                            int64_t ld, int b_off, int a_off, const float* __restrict__ A_log,
-                                                            const float* __restrict__ dt_bias, float* __restrict__ beta,
-                                                            float* __restrict__ decay, float* __restrict__ log_decay,
-                                                            float* __restrict__ kq, int H, int G, int D, float q_scale,
+__global__ void __launch_bounds__(128) delta_prepare_kernel(float* u, int64_t ldu, const float* proj,
+                                                            int64_t ld, int b_off, int a_off, const float* A_log,
+                                                            const float* dt_bias, float* beta,
+                                                            float* decay, float* log_decay,
+                                                            float* kq, int H, int G, int D, float q_scale,
                                                             float unit_eps) {
   rb_pdl_launch_dependents();
   rb_pdl_wait();
@@ -77,9 +77,9 @@ template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile(
 
 template <int P, int R, int NT>
 __global__ void __launch_bounds__(NT) gated_delta_kernel(
-    float* __restrict__ o, const float* __restrict__ u, int64_t ldu, const float* __restrict__ beta,
-    const float* __restrict__ decay, const float* __restrict__ kq, float* __restrict__ state,
-    const int* __restrict__ seq_first, const int* __restrict__ seq_count, const int* __restrict__ tok_slot, int H, int G,
+    float* o, const float* u, int64_t ldu, const float* beta,
+    const float* decay, const float* kq, float* state,
+    const int* seq_first, const int* seq_count, const int* tok_slot, int H, int G,
     int D, int Dv, int TT, int vec16) {
   rb_pdl_launch_dependents();
   constexpr int CT = NT / P;              // value columns of this block
@@ -223,10 +223,10 @@ int launch_delta(dim3 grid, size_t smem, cudaStream_t stream, float* o, const fl
 // 22.5 us of a step before, 10.5 now).
 template <int R>
 __global__ void __launch_bounds__(1024) delta_step_kernel(
-    void* __restrict__ out, int out_bf16, const float* __restrict__ proj, int64_t ld, int g_off, int b_off, int a_off,
-    const float* __restrict__ taps, const float* __restrict__ A_log, const float* __restrict__ dt_bias,
-    const float* __restrict__ norm_w, float* __restrict__ state, float* __restrict__ tail, const int* __restrict__ tok_slot,
-    const int* __restrict__ tok_pos, int H, int G, int D, int Dv, int K, int P, float q_scale, float unit_eps, float norm_eps) {
+    void* out, int out_bf16, const float* proj, int64_t ld, int g_off, int b_off, int a_off,
+    const float* taps, const float* A_log, const float* dt_bias,
+    const float* norm_w, float* state, float* tail, const int* tok_slot,
+    const int* tok_pos, int H, int G, int D, int Dv, int K, int P, float q_scale, float unit_eps, float norm_eps) {
   rb_pdl_launch_dependents();
   extern __shared__ __align__(16) float s_step[];
   __shared__ float scratch[33];
@@ -357,9 +357,9 @@ constexpr int CH = 32;
 // grid (chunks, H), 128 threads.  chunk_row[c]: the chunk's first row; chunk_len[c]: its tokens (1..32).
 // Scratch per (chunk, head): W [32][D], Ut [32][Dv], M [32][32], L [32].
 __global__ void __launch_bounds__(128) delta_chunk_prepare_kernel(
-    float* __restrict__ Wg, float* __restrict__ Utg, float* __restrict__ Mg, float* __restrict__ Lg,
-    const float* __restrict__ u, int64_t ldu, const float* __restrict__ beta, const float* __restrict__ log_decay,
-    const int* __restrict__ chunk_row, const int* __restrict__ chunk_len, int H, int G, int D, int Dv) {
+    float* Wg, float* Utg, float* Mg, float* Lg,
+    const float* u, int64_t ldu, const float* beta, const float* log_decay,
+    const int* chunk_row, const int* chunk_len, int H, int G, int D, int Dv) {
   rb_pdl_launch_dependents();
   extern __shared__ __align__(16) float s_prep[];
   const int KS = D + 4;                          // row stride of k and q
@@ -471,10 +471,10 @@ __device__ __forceinline__ void cp_async16_or_zeros(void* dst, const void* src, 
 }
 
 __global__ void __launch_bounds__(SCAN_NT) delta_chunk_scan_kernel(
-    float* __restrict__ o, const float* __restrict__ Wg, const float* __restrict__ Utg, const float* __restrict__ Mg,
-    const float* __restrict__ Lg, const float* __restrict__ u, int64_t ldu, float* __restrict__ state,
-    const int* __restrict__ seq_first, const int* __restrict__ seq_count, const int* __restrict__ run_chunk0,
-    const int* __restrict__ tok_slot, int H, int G, int D, int Dv) {
+    float* o, const float* Wg, const float* Utg, const float* Mg,
+    const float* Lg, const float* u, int64_t ldu, float* state,
+    const int* seq_first, const int* seq_count, const int* run_chunk0,
+    const int* tok_slot, int H, int G, int D, int Dv) {
   rb_pdl_launch_dependents();
   extern __shared__ __align__(16) float s_scan[];
   const int per_buf = 3 * CH * D + CH * CH + CH;

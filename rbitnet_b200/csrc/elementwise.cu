@@ -46,8 +46,8 @@ RB_EXPORT int rb_is_checked_build() {
 // An id outside [0, V) is refused on the host before the launch; the kernel
 // writes zeros for one rather than read outside the table.
 template <typename TW>
-__global__ void embed_kernel(float* __restrict__ out, const TW* __restrict__ table,
-                             const int* __restrict__ ids, int E, int V, float scale) {
+__global__ void embed_kernel(float* out, const TW* table,
+                             const int* ids, int E, int V, float scale) {
   rb_pdl_launch_dependents();
   rb_pdl_wait();
   // four values per thread and the whole row in flight at once: the rows come from anywhere in a
@@ -112,7 +112,7 @@ template <> __device__ __forceinline__ void store4<__nv_bfloat16>(__nv_bfloat16*
 
 // VEC: the width is a multiple of 4 and rows are read and written four values at a time.
 template <typename TO, bool VEC>
-__global__ void rmsnorm_kernel(TO* __restrict__ out, const float* __restrict__ x, const float* __restrict__ w,
+__global__ void rmsnorm_kernel(TO* out, const float* x, const float* w,
                                int E, float eps) {
   rb_pdl_launch_dependents();
   rb_pdl_wait();
@@ -151,7 +151,7 @@ __global__ void rmsnorm_kernel(TO* __restrict__ out, const float* __restrict__ x
 // Rows of up to 4*NV*blockDim values (a multiple of 4) kept in registers: every load of a row
 // is in flight before the first is used, and nothing goes through shared memory.
 template <typename TO, int NV>
-__global__ void rmsnorm_reg_kernel(TO* __restrict__ out, const float* __restrict__ x, const float* __restrict__ w,
+__global__ void rmsnorm_reg_kernel(TO* out, const float* x, const float* w,
                                    int E, float eps) {
   rb_pdl_launch_dependents();
   __shared__ float scratch[33];
@@ -237,8 +237,8 @@ RB_EXPORT int rb_rmsnorm(void* out, int out_dtype, const float* x, const float* 
 // out = w * tanh(alpha * x) + b, value by value.  A thread keeps its V columns (their w and b in registers) and takes
 // every gridDim.y-th row.
 template <typename TO, int V>
-__global__ void __launch_bounds__(256) tanh_norm_kernel(TO* __restrict__ out, const float* __restrict__ x,
-                                                        const float* __restrict__ w, const float* __restrict__ b,
+__global__ void __launch_bounds__(256) tanh_norm_kernel(TO* out, const float* x,
+                                                        const float* w, const float* b,
                                                         float alpha, int T, int E) {
   rb_pdl_launch_dependents();
   const int e = (blockIdx.x * blockDim.x + threadIdx.x) * V;
@@ -286,8 +286,8 @@ RB_EXPORT int rb_tanh_norm(void* out, int out_dtype, const float* x, const float
 // out = (x - mean) / sqrt(var + eps) * w + b, var the mean of the squared deviations; float32 sums, two passes over
 // the row (the second over the deviations).  One block per row.
 template <typename TO>
-__global__ void __launch_bounds__(256) layernorm_kernel(TO* __restrict__ out, const float* __restrict__ x,
-                                                        const float* __restrict__ w, const float* __restrict__ b, int E,
+__global__ void __launch_bounds__(256) layernorm_kernel(TO* out, const float* x,
+                                                        const float* w, const float* b, int E,
                                                         float eps) {
   rb_pdl_launch_dependents();
   __shared__ float scratch[33];
@@ -305,8 +305,8 @@ __global__ void __launch_bounds__(256) layernorm_kernel(TO* __restrict__ out, co
 
 // The same with the row held in registers (NV groups of four values a thread, 16-byte accesses): the row is read once.
 template <typename TO, int NV>
-__global__ void __launch_bounds__(256) layernorm_reg_kernel(TO* __restrict__ out, const float* __restrict__ x,
-                                                            const float* __restrict__ w, const float* __restrict__ b, int E,
+__global__ void __launch_bounds__(256) layernorm_reg_kernel(TO* out, const float* x,
+                                                            const float* w, const float* b, int E,
                                                             float eps) {
   rb_pdl_launch_dependents();
   __shared__ float scratch[33];
@@ -376,7 +376,7 @@ RB_EXPORT int rb_layernorm(void* out, int out_dtype, const float* x, const float
 }
 
 // ---------------------------------------------------------------- x += y, float32
-__global__ void add_rows_kernel(float* __restrict__ x, const float* __restrict__ y, int64_t n) {
+__global__ void add_rows_kernel(float* x, const float* y, int64_t n) {
   rb_pdl_launch_dependents();
   rb_pdl_wait();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) x[i] += y[i];
@@ -400,9 +400,9 @@ RB_EXPORT int rb_add_rows(float* x, const float* y, long long n, cudaStream_t st
 // layer that reads another layer's cache).  Only the first rot_dim values of a head are
 // rotated (pairs (2i,2i+1) or (i, i+rot_dim/2) among them); the rest pass unchanged.
 template <typename T>
-__global__ void rotate_append_kernel(T* __restrict__ q_out, const T* __restrict__ qkv, int64_t qkv_stride,
-                                     const float* __restrict__ inv_freq, const int* __restrict__ tok_pos,
-                                     const int* __restrict__ tok_slot, RbPagedLayer cache, int H, int write_kv,
+__global__ void rotate_append_kernel(T* q_out, const T* qkv, int64_t qkv_stride,
+                                     const float* inv_freq, const int* tok_pos,
+                                     const int* tok_slot, RbPagedLayer cache, int H, int write_kv,
                                      int interleaved, int heads_per_block, int rot_dim) {
   rb_pdl_launch_dependents();
   const int t = blockIdx.x;
@@ -454,8 +454,8 @@ __global__ void rotate_append_kernel(T* __restrict__ q_out, const T* __restrict_
 // and walks over the heads with 16-byte loads and stores; values are copied 16 bytes at a time.
 constexpr int ROWS_MAX_PAIRS = 256;      // head sizes up to 512 take the many-token kernel
 __global__ void __launch_bounds__(1024) rotate_append_rows_kernel(
-    __nv_bfloat16* __restrict__ q_out, const __nv_bfloat16* __restrict__ qkv, int64_t qkv_stride,
-    const float* __restrict__ inv_freq, const int* __restrict__ tok_pos, const int* __restrict__ tok_slot,
+    __nv_bfloat16* q_out, const __nv_bfloat16* qkv, int64_t qkv_stride,
+    const float* inv_freq, const int* tok_pos, const int* tok_slot,
     RbPagedLayer cache, int H, int write_kv, int interleaved) {
   rb_pdl_launch_dependents();
   rb_pdl_wait();
@@ -577,7 +577,7 @@ RB_EXPORT int rb_rotate_append(void* q_out, const void* qkv, int64_t qkv_stride,
 // values, B of gate followed by the B of up for the same features (the row order the tensor-core
 // gated product wants of its weights); `ld` is the row length of gu.
 template <typename T, typename TI>
-__global__ void silu_mul_kernel(T* __restrict__ out, const TI* __restrict__ gu, int64_t n, int F, int64_t ld, int block) {
+__global__ void silu_mul_kernel(T* out, const TI* gu, int64_t n, int F, int64_t ld, int block) {
   rb_pdl_launch_dependents();
   rb_pdl_wait();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -613,8 +613,8 @@ RB_EXPORT int rb_silu_mul(void* out, const void* gate_up, int dtype, int in_dtyp
 }
 
 // ---------------------------------------------------------------- row gather (float32 residual rows)
-__global__ void gather_rows_kernel(float* __restrict__ out, const float* __restrict__ x,
-                                   const int* __restrict__ rows, int E) {
+__global__ void gather_rows_kernel(float* out, const float* x,
+                                   const int* rows, int E) {
   rb_pdl_launch_dependents();
   rb_pdl_wait();
   // one element (or one group of four) per thread: the copies of a row are all in flight together
@@ -642,9 +642,9 @@ RB_EXPORT int rb_gather_rows(float* out, const float* x, const int* rows, int R,
 // position moves on by one, so that steps can follow one another without the host.  Only the first
 // *n_live rows move (n_live null: all B): rows behind them belong to the padding sequence, which
 // rewrites its position 0 at every step.
-__global__ void decode_advance_kernel(int* __restrict__ token_ids, int* __restrict__ tok_pos,
-                                      const int* __restrict__ sampled, int B, const int* __restrict__ n_live,
-                                      const int* flag_a, const int* flag_b, int* __restrict__ flag_out) {
+__global__ void decode_advance_kernel(int* token_ids, int* tok_pos,
+                                      const int* sampled, int B, const int* n_live,
+                                      const int* flag_a, const int* flag_b, int* flag_out) {
   rb_pdl_launch_dependents();
   rb_pdl_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -691,9 +691,9 @@ __device__ __forceinline__ void rb_angle_sincos(int pos, double freq, float magn
 
 template <typename T>
 __global__ void __launch_bounds__(256) norm_rotate_append_kernel(
-    T* __restrict__ q_out, const T* __restrict__ proj, int64_t ld, const float* __restrict__ q_norm_w,
-    const float* __restrict__ k_norm_w, float eps, const double* __restrict__ freq, float magnitude,
-    const int* __restrict__ tok_pos, const int* __restrict__ tok_slot, RbPagedLayer cache, int H, int D, int Dv,
+    T* q_out, const T* proj, int64_t ld, const float* q_norm_w,
+    const float* k_norm_w, float eps, const double* freq, float magnitude,
+    const int* tok_pos, const int* tok_slot, RbPagedLayer cache, int H, int D, int Dv,
     int rot_dim, int interleaved, int write_kv, int heads_per_block) {
   rb_pdl_launch_dependents();
   __shared__ float scratch[33];
@@ -766,9 +766,9 @@ __global__ void __launch_bounds__(256) norm_rotate_append_kernel(
 // multiples of 8, interleaved pairs, 16-byte aligned rows): a thread takes eight neighbouring values at a time, which
 // hold four whole pairs, with one 16-byte load and one 16-byte store.
 __global__ void __launch_bounds__(256) norm_rotate_append_rows_kernel(
-    __nv_bfloat16* __restrict__ q_out, const __nv_bfloat16* __restrict__ proj, int64_t ld, const float* __restrict__ q_norm_w,
-    const float* __restrict__ k_norm_w, float eps, const double* __restrict__ freq, float magnitude,
-    const int* __restrict__ tok_pos, const int* __restrict__ tok_slot, RbPagedLayer cache, int H, int D, int Dv,
+    __nv_bfloat16* q_out, const __nv_bfloat16* proj, int64_t ld, const float* q_norm_w,
+    const float* k_norm_w, float eps, const double* freq, float magnitude,
+    const int* tok_pos, const int* tok_slot, RbPagedLayer cache, int H, int D, int Dv,
     int rot_dim, int heads_per_block) {
   rb_pdl_launch_dependents();
   __shared__ float scratch[33];
@@ -858,8 +858,8 @@ __global__ void __launch_bounds__(256) norm_rotate_append_rows_kernel(
 constexpr int HN_MAX = 16;
 template <typename T, int NG>      // NG: groups of 32 values a head's cache row holds at most
 __global__ void __launch_bounds__(256) rotate_headnorm_append_kernel(
-    T* __restrict__ q_out, const T* __restrict__ proj, int64_t ld, float eps, const double* __restrict__ freq, float magnitude,
-    const int* __restrict__ tok_pos, const int* __restrict__ tok_slot, RbPagedLayer cache, int n_tokens, int H, int D, int Dv,
+    T* q_out, const T* proj, int64_t ld, float eps, const double* freq, float magnitude,
+    const int* tok_pos, const int* tok_slot, RbPagedLayer cache, int n_tokens, int H, int D, int Dv,
     int rot_dim, int interleaved, int write_kv, int heads_per_block) {
   rb_pdl_launch_dependents();
   extern __shared__ float s_sincos[];              // rot_dim/2 sines, then as many cosines, of this token's position
@@ -995,7 +995,7 @@ RB_EXPORT int rb_norm_rotate_append(void* q_out, const void* proj, int64_t ld, i
 // Dc wide and applies one gate value per head (no gate: gate == null), or one per value (per_value:
 // gate[t*ldg + h*Dv + j]).
 template <typename T>
-__global__ void head_gate_kernel(T* __restrict__ out, const T* __restrict__ a, const T* __restrict__ gate, int64_t ldg,
+__global__ void head_gate_kernel(T* out, const T* a, const T* gate, int64_t ldg,
                                  int64_t n, int H, int Dv, int Dc, int per_value) {
   rb_pdl_launch_dependents();
   rb_pdl_wait();
@@ -1010,8 +1010,8 @@ __global__ void head_gate_kernel(T* __restrict__ out, const T* __restrict__ a, c
 }
 
 // The same for bfloat16 rows in groups of eight values (Dv and Dc multiples of 8, 16-byte aligned rows).
-__global__ void head_gate_rows_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ a,
-                                      const __nv_bfloat16* __restrict__ gate, int64_t ldg, int64_t n8, int H, int Dv, int Dc,
+__global__ void head_gate_rows_kernel(__nv_bfloat16* out, const __nv_bfloat16* a,
+                                      const __nv_bfloat16* gate, int64_t ldg, int64_t n8, int H, int Dv, int Dc,
                                       int per_value) {
   rb_pdl_launch_dependents();
   rb_pdl_wait();
@@ -1081,8 +1081,8 @@ RB_EXPORT int rb_head_gate(void* out, const void* a, const void* gate, int64_t l
 //         g/2 * (1 + tanh(...)) written with one exponential
 // bias (or null): a number per column of gu, added first.  Row layouts as rb_silu_mul.
 template <typename T, typename TI>
-__global__ void gated_act_kernel(T* __restrict__ out, const TI* __restrict__ gu, int64_t n, int F, int64_t ld, int block,
-                                 int kind, float alpha, float limit, float shift, const float* __restrict__ bias) {
+__global__ void gated_act_kernel(T* out, const TI* gu, int64_t n, int F, int64_t ld, int block,
+                                 int kind, float alpha, float limit, float shift, const float* bias) {
   rb_pdl_launch_dependents();
   rb_pdl_wait();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -1130,3 +1130,27 @@ RB_EXPORT int rb_gated_act(void* out, const void* gate_up, int dtype, int in_dty
 }
 
 RB_CHECK_READER(elementwise)
+
+namespace {
+__global__ void late_copy_kernel(float4* dst, const float4* src, long long n, long long delay_ns) {
+  rb_pdl_launch_dependents();
+  rb_pdl_wait();
+  long long t0, t;
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
+  for (int i = 0; i < 1000000; ++i) {                    // (the delay ends the wait long before the count does)
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    if (t - t0 >= delay_ns) break;
+    __nanosleep(200);
+  }
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) dst[i] = src[i];
+}
+}  // namespace
+
+// For tests: lets the next kernel begin at once, and writes what it reads only after the delay (at most 2 ms).  Sizes in multiples
+// of 16 bytes.
+RB_EXPORT int rb_late_copy_for_test(void* dst, const void* src, long long bytes, long long delay_ns, cudaStream_t stream) {
+  RB_REQUIRE(bytes > 0 && bytes % 16 == 0 && delay_ns >= 0 && delay_ns <= 2000000, "rb_late_copy_for_test: %lld bytes, %lld ns", bytes, delay_ns);
+  RB_LAUNCH("late_copy_kernel", (late_copy_kernel), 8, 128, 0, stream, (float4*)dst, (const float4*)src, bytes / 16, delay_ns);
+  RB_CHECK_LAUNCH("rb_late_copy_for_test");
+  return 0;
+}

@@ -39,7 +39,7 @@ constexpr int TILE = 64, LK = 16, PITCH = TILE + 4, TILE_THREADS = 128;
 
 // Four finished neighbours of a row.
 template <typename TC>
-__device__ __forceinline__ void leave4(TC* __restrict__ C, int64_t ldc, int M, int N, int m, int n, float (&v)[4], int accumulate,
+__device__ __forceinline__ void leave4(TC* C, int64_t ldc, int M, int N, int m, int n, float (&v)[4], int accumulate,
                                        float alpha, const Tail& tail) {
   if (m >= M) return;
   TC* p = C + (int64_t)m * ldc + n;
@@ -63,7 +63,7 @@ __device__ __forceinline__ void leave4(TC* __restrict__ C, int64_t ldc, int M, i
 
 template <bool VEC, typename TA, typename TC>
 __global__ void __launch_bounds__(TILE_THREADS, 4) gemm_tile_kernel(
-    TC* __restrict__ C, int64_t ldc, const TA* __restrict__ A, int64_t lda, const TA* __restrict__ W, int64_t ldw, int M, int N,
+    TC* C, int64_t ldc, const TA* A, int64_t lda, const TA* W, int64_t ldw, int M, int N,
     int K, int accumulate, float alpha, Tail tail, int64_t batch_c, int64_t batch_a, int64_t batch_w, int n_parts) {
   constexpr int FETCH = TILE * LK / 4 / TILE_THREADS;      // groups of four values a thread fetches of each operand
   rb_pdl_launch_dependents();
@@ -222,7 +222,7 @@ int tile_parts(int64_t tiles, int K, int sms) {
 constexpr int ROW_N = 4, ROW_WARPS = 4;
 template <int RM, bool SHARE, bool VEC, typename TA, typename TC>
 __global__ void __launch_bounds__(ROW_WARPS * 32) gemm_rows_kernel(
-    TC* __restrict__ C, int64_t ldc, const TA* __restrict__ A, int64_t lda, const TA* __restrict__ W, int64_t ldw, int M, int N,
+    TC* C, int64_t ldc, const TA* A, int64_t lda, const TA* W, int64_t ldw, int M, int N,
     int K, int accumulate, float alpha, Tail tail, int64_t batch_c, int64_t batch_a, int64_t batch_w) {
   constexpr int V = VEC ? 4 : 1, TURN = RM == 8 ? 2 : 4;
   constexpr int STRIDE = 32 * V * (SHARE ? ROW_WARPS : 1);
@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(ROW_WARPS * 32) gemm_rows_kernel(
 constexpr int FEW_ROWS = 8, FEW_OUTS = 4, FEW_WARPS = 4;
 template <typename TA, typename TC, bool VEC>
 __global__ void __launch_bounds__(FEW_WARPS * 32) per_head_few_rows_kernel(
-    TC* __restrict__ C, int64_t ldc, const TA* __restrict__ A, int64_t lda, int head_a, const TA* __restrict__ W, int M, int N,
+    TC* C, int64_t ldc, const TA* A, int64_t lda, int head_a, const TA* W, int M, int N,
     int K, Tail tail) {
   rb_pdl_launch_dependents();
   rb_pdl_wait();

@@ -967,7 +967,7 @@ RB_EXPORT int rb_set_error_flag_for_test(int code) { return rb_file_set_error_fl
 // up, records `code` and the kernel returns.  This is the bounded wait of the product and attention
 // kernels (same function, their limit is two seconds) run to its end on purpose, in a kernel that
 // does nothing else.
-__global__ void wait_probe_kernel(unsigned long long limit_ns, int code, int* __restrict__ gave_up) {
+__global__ void wait_probe_kernel(unsigned long long limit_ns, int code, int* gave_up) {
   __shared__ uint64_t bar;
   if (threadIdx.x == 0) {
     mbar_init(&bar, 1);
@@ -979,8 +979,8 @@ __global__ void wait_probe_kernel(unsigned long long limit_ns, int code, int* __
 
 // The same for the wait on a count in global memory (a tile's finished parts): `word` holds zero and
 // nobody ever stores the one that the thread waits for.
-__global__ void count_wait_probe_kernel(const int* __restrict__ word, unsigned long long limit_ns, int code,
-                                        int* __restrict__ gave_up) {
+__global__ void count_wait_probe_kernel(const int* word, unsigned long long limit_ns, int code,
+                                        int* gave_up) {
   if (threadIdx.x == 0) {
     const bool ok = wait_for_count(word, 1, code, limit_ns);
     if (gave_up != nullptr) *gave_up = ok ? 0 : 1;

@@ -27,9 +27,9 @@ __device__ __forceinline__ float softplus_(float v) { return v > 20.f ? v : log1
 
 // A block takes GLA_DT rows and 128 channels at a time: a channel's row of A2 is read once for all of them.
 constexpr int GLA_DT = 8;
-__global__ void __launch_bounds__(128) gla_decay_kernel(float* __restrict__ alpha, const float* __restrict__ rows, int64_t ld,
-                                                        int a_off, const float* __restrict__ A2,
-                                                        const float* __restrict__ bias, int T, int C, int rank,
+__global__ void __launch_bounds__(128) gla_decay_kernel(float* alpha, const float* rows, int64_t ld,
+                                                        int a_off, const float* A2,
+                                                        const float* bias, int T, int C, int rank,
                                                         float inv_tau, int as_log) {
   rb_pdl_launch_dependents();
   rb_pdl_wait();
@@ -62,11 +62,11 @@ __global__ void __launch_bounds__(128) gla_decay_kernel(float* __restrict__ alph
 }
 
 template <int P>
-__global__ void __launch_bounds__(128) gla_scan_kernel(float* __restrict__ o, const float* __restrict__ rows, int64_t ld,
-                                                       int q_off, int k_off, int v_off, const float* __restrict__ alpha,
-                                                       float q_scale, float* __restrict__ state,
-                                                       const int* __restrict__ seq_first, const int* __restrict__ seq_count,
-                                                       const int* __restrict__ tok_slot, int H, int D, int Dv,
+__global__ void __launch_bounds__(128) gla_scan_kernel(float* o, const float* rows, int64_t ld,
+                                                       int q_off, int k_off, int v_off, const float* alpha,
+                                                       float q_scale, float* state,
+                                                       const int* seq_first, const int* seq_count,
+                                                       const int* tok_slot, int H, int D, int Dv,
                                                        int64_t a_ld) {
   rb_pdl_launch_dependents();
   constexpr int COLS = 128 / P;                    // value columns of a block
@@ -192,11 +192,11 @@ __host__ __device__ constexpr int gla_item_floats(int D) { return 2 * GCH * D + 
 
 // grid (chunks, H), 128 threads.  log_alpha: [T, H * D].  Scratch per (chunk, head): Qt [32][D], Kt [32][D], M [32][32],
 // e^{B_end} [D].
-__global__ void __launch_bounds__(128) gla_chunk_prepare_kernel(float* __restrict__ scratch, const float* __restrict__ rows,
+__global__ void __launch_bounds__(128) gla_chunk_prepare_kernel(float* scratch, const float* rows,
                                                                 int64_t ld, int q_off, int k_off,
-                                                                const float* __restrict__ log_alpha, float q_scale,
-                                                                const int* __restrict__ chunk_row,
-                                                                const int* __restrict__ chunk_len, int H, int D,
+                                                                const float* log_alpha, float q_scale,
+                                                                const int* chunk_row,
+                                                                const int* chunk_len, int H, int D,
                                                                 int64_t a_ld) {
   rb_pdl_launch_dependents();
   extern __shared__ __align__(16) float s_gprep[];
@@ -279,9 +279,9 @@ __global__ void __launch_bounds__(128) gla_chunk_prepare_kernel(float* __restric
 // tile S [D][32] twice: a chunk reads one and writes the other, so that a chunk has one barrier.
 // (With 16 columns and a value or two a thread: 4.6 us a chunk of 128 channels, 3.2 now.)
 __global__ void __launch_bounds__(GSCAN_NT) gla_chunk_scan_kernel(
-    float* __restrict__ o, const float* __restrict__ scratch, const float* __restrict__ rows, int64_t ld, int v_off,
-    float* __restrict__ state, const int* __restrict__ seq_first, const int* __restrict__ seq_count,
-    const int* __restrict__ run_chunk0, const int* __restrict__ tok_slot, int H, int D, int Dv) {
+    float* o, const float* scratch, const float* rows, int64_t ld, int v_off,
+    float* state, const int* seq_first, const int* seq_count,
+    const int* run_chunk0, const int* tok_slot, int H, int D, int Dv) {
   rb_pdl_launch_dependents();
   extern __shared__ __align__(16) float s_gscan[];
   const int item_floats = gla_item_floats(D);

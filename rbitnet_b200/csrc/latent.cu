@@ -20,10 +20,10 @@ namespace {
 // A block per token.  STAGED: the row's values wait in shared memory between the sums and the values made from them.
 template <typename T, bool STAGED>
 __global__ void __launch_bounds__(256) latent_norm_append_kernel(
-    T* __restrict__ cq, const float* __restrict__ rows, int64_t ld, int q_off, int kv_off, int q_rank, int kv_rank,
-    int rot_dim, const float* __restrict__ wq, const float* __restrict__ wkv, float eps, const double* __restrict__ freq,
-    float magnitude, int interleaved, RbPagedLayer cache, int width, const int* __restrict__ tok_pos,
-    const int* __restrict__ tok_slot) {
+    T* cq, const float* rows, int64_t ld, int q_off, int kv_off, int q_rank, int kv_rank,
+    int rot_dim, const float* wq, const float* wkv, float eps, const double* freq,
+    float magnitude, int interleaved, RbPagedLayer cache, int width, const int* tok_pos,
+    const int* tok_slot) {
   rb_pdl_launch_dependents();
   __shared__ float scratch[66];
   extern __shared__ float s_mem[];
@@ -74,8 +74,8 @@ __global__ void __launch_bounds__(256) latent_norm_append_kernel(
 constexpr int FEW_ROWS = 8, FEW_OUTS = 4, FEW_WARPS = 4;
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(FEW_WARPS * 32) latent_queries_few_kernel(
-    T* __restrict__ out, const T* __restrict__ q, const T* __restrict__ W, const double* __restrict__ freq, float magnitude,
-    int interleaved, const int* __restrict__ tok_pos, int M, int H, int D, int R, int C, int width, int dot_blocks) {
+    T* out, const T* q, const T* W, const double* freq, float magnitude,
+    int interleaved, const int* tok_pos, int M, int H, int D, int R, int C, int width, int dot_blocks) {
   rb_pdl_launch_dependents();
   rb_pdl_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -145,9 +145,9 @@ __global__ void __launch_bounds__(FEW_WARPS * 32) latent_queries_few_kernel(
 // A block per token: columns C .. width-1 of every head's row.  A thread turns a pair at a time; PAIRS2: two neighbouring
 // pairs of the half layout, whose values lie side by side.
 template <typename T, bool PAIRS2>
-__global__ void __launch_bounds__(256) latent_turn_kernel(T* __restrict__ out, const T* __restrict__ q,
-                                                          const double* __restrict__ freq, float magnitude, int interleaved,
-                                                          const int* __restrict__ tok_pos, int H, int D, int R, int C,
+__global__ void __launch_bounds__(256) latent_turn_kernel(T* out, const T* q,
+                                                          const double* freq, float magnitude, int interleaved,
+                                                          const int* tok_pos, int H, int D, int R, int C,
                                                           int width) {
   rb_pdl_launch_dependents();
   extern __shared__ float s_sincos[];

@@ -42,10 +42,10 @@ struct Memory {
 };
 
 // One warp per (run, head), two tokens a lane; the next chunk's pre-activations are on their way while a chunk is worked on.
-__global__ void __launch_bounds__(128) memory_gates_kernel(Memory a, const float* __restrict__ i_bias, const float* __restrict__ f_bias,
-                                                           float cap, float* __restrict__ m_state, const int* __restrict__ run_chunk0,
-                                                           const int* __restrict__ seq_first, const int* __restrict__ seq_count,
-                                                           const int* __restrict__ tok_slot) {
+__global__ void __launch_bounds__(128) memory_gates_kernel(Memory a, const float* i_bias, const float* f_bias,
+                                                           float cap, float* m_state, const int* run_chunk0,
+                                                           const int* seq_first, const int* seq_count,
+                                                           const int* tok_slot) {
   rb_pdl_launch_dependents();
   const int lane = threadIdx.x & 31, h = blockIdx.y * 4 + (threadIdx.x >> 5);
   if (h >= a.H) return;
@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(128) memory_gates_kernel(Memory a, const float
 // TURN: the rows become the columns (depth = the row's values), else a row stays a row.  What is not there is zero; row r
 // is multiplied by mul[r] (null: 1).
 template <bool TURN>
-__device__ __forceinline__ void stage(float* dst, const float* __restrict__ src, int64_t ld, int rows, int c0, int live, bool vec,
+__device__ __forceinline__ void stage(float* dst, const float* src, int64_t ld, int rows, int c0, int live, bool vec,
                                       const float* mul) {
 #pragma unroll 4
   for (int e = threadIdx.x; e < CH * CH / 4; e += NT) {
@@ -285,9 +285,9 @@ __global__ void __launch_bounds__(NT, 5) memory_chunk_sum_kernel(Memory a) {
 
 // grid (runs, H, pieces); V neighbouring values a thread.
 template <int V>
-__global__ void __launch_bounds__(128) memory_chunk_walk_kernel(Memory a, float* __restrict__ C_state, float* __restrict__ n_state,
-                                                                const int* __restrict__ run_chunk0, const int* __restrict__ seq_first,
-                                                                const int* __restrict__ seq_count, const int* __restrict__ tok_slot) {
+__global__ void __launch_bounds__(128) memory_chunk_walk_kernel(Memory a, float* C_state, float* n_state,
+                                                                const int* run_chunk0, const int* seq_first,
+                                                                const int* seq_count, const int* tok_slot) {
   rb_pdl_launch_dependents();
   rb_pdl_wait();
   const int h = blockIdx.y, chunk0 = run_chunk0[blockIdx.x], chunks = (seq_count[blockIdx.x] + CH - 1) / CH;
@@ -327,7 +327,7 @@ __global__ void __launch_bounds__(128) memory_chunk_walk_kernel(Memory a, float*
 }
 
 // grid (chunks, H, tiles of 64 value columns): scores x v, then (e^(p_t + m0) q) x what the chunk starts from.
-__global__ void __launch_bounds__(NT, 5) memory_chunk_out_kernel(Memory a, float* __restrict__ o_out, float q_scale, float floor_add) {
+__global__ void __launch_bounds__(NT, 5) memory_chunk_out_kernel(Memory a, float* o_out, float q_scale, float floor_add) {
   rb_pdl_launch_dependents();
   __shared__ __align__(16) float x[CH * PITCH], y[CH * PITCH];
   __shared__ float carry[CH], n0[CH], nq[2][CH];

@@ -33,7 +33,7 @@ template <> __device__ __forceinline__ void rb_store_values<__nv_bfloat16>(__nv_
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) round_rows_kernel(T* __restrict__ out, const float* __restrict__ x, int64_t n) {
+__global__ void __launch_bounds__(256) round_rows_kernel(T* out, const float* x, int64_t n) {
   rb_pdl_launch_dependents();
   rb_pdl_wait();
   // four values a thread and turn where the addresses allow 16-byte loads, the rest value by value
@@ -51,9 +51,9 @@ __global__ void __launch_bounds__(256) round_rows_kernel(T* __restrict__ out, co
 
 // A block per row.  VEC: the row is read four values at a time (E a multiple of 4, aligned rows).
 template <typename T, bool VEC>
-__global__ void __launch_bounds__(256) norm_add_kernel(float* __restrict__ x, const float* __restrict__ y,
-                                                       const float* __restrict__ w, float eps, int E,
-                                                       T* __restrict__ rounded) {
+__global__ void __launch_bounds__(256) norm_add_kernel(float* x, const float* y,
+                                                       const float* w, float eps, int E,
+                                                       T* rounded) {
   rb_pdl_launch_dependents();
   __shared__ float scratch[33];
   rb_pdl_wait();
@@ -95,9 +95,9 @@ __global__ void __launch_bounds__(256) norm_add_kernel(float* __restrict__ x, co
 // A block per row: x (+)= y / rms(y) * w, then h = x / rms(x) * w2.  VEC: a thread holds NV times four values of the row in
 // registers (blockDim.x * NV * 4 >= E); else the row goes through memory, each thread its own values.
 template <typename T, bool VEC, int NV>
-__global__ void __launch_bounds__(1024) norm_add_norm_kernel(float* __restrict__ x, const float* __restrict__ y,
-                                                             const float* __restrict__ w, float eps, int E, int fresh,
-                                                             T* __restrict__ h, const float* __restrict__ w2, float eps2) {
+__global__ void __launch_bounds__(1024) norm_add_norm_kernel(float* x, const float* y,
+                                                             const float* w, float eps, int E, int fresh,
+                                                             T* h, const float* w2, float eps2) {
   rb_pdl_launch_dependents();
   __shared__ float scratch[33];
   const int64_t row = blockIdx.x;
@@ -176,8 +176,8 @@ __device__ __forceinline__ float gelu_tanh_(float z) {
 }
 
 template <typename T, typename TT>
-__global__ void __launch_bounds__(256) token_gate_kernel(T* __restrict__ out, const float* __restrict__ a, int64_t lda,
-                                                         const TT* __restrict__ table, const int* __restrict__ ids,
+__global__ void __launch_bounds__(256) token_gate_kernel(T* out, const float* a, int64_t lda,
+                                                         const TT* table, const int* ids,
                                                          int64_t n, int dim) {
   rb_pdl_launch_dependents();
   rb_pdl_wait();
@@ -192,10 +192,10 @@ __global__ void __launch_bounds__(256) token_gate_kernel(T* __restrict__ out, co
 // single: every row is a run of its own (a decode step; rows that pad a captured step may share a slot).  A step of
 // runs of several rows takes two launches (add, then update), because a run's first row reads what its last row writes.
 template <typename TT>
-__global__ void __launch_bounds__(256) embed_pairs_kernel(float* __restrict__ out, const TT* __restrict__ table,
-                                                          const TT* __restrict__ pairs, const int* __restrict__ ids,
-                                                          const int* __restrict__ tok_pos, const int* __restrict__ tok_slot,
-                                                          int* __restrict__ previous, int T, int E, int V, float scale,
+__global__ void __launch_bounds__(256) embed_pairs_kernel(float* out, const TT* table,
+                                                          const TT* pairs, const int* ids,
+                                                          const int* tok_pos, const int* tok_slot,
+                                                          int* previous, int T, int E, int V, float scale,
                                                           int buckets, int mul_prev, int mul_cur, int add, int update,
                                                           int single) {
   rb_pdl_launch_dependents();
@@ -240,7 +240,7 @@ struct QkParams {
 // A block per token.  Shared memory: rot_dim sines and cosines, the C = (H + Kh) D convolved q and k values, a factor
 // per head.
 template <typename T>
-__global__ void __launch_bounds__(1024) qk_prepare_kernel(T* __restrict__ q_out, T* __restrict__ gates_out, QkParams p,
+__global__ void __launch_bounds__(1024) qk_prepare_kernel(T* q_out, T* gates_out, QkParams p,
                                                          RbPagedLayer cache) {
   rb_pdl_launch_dependents();
   __shared__ float scratch[33];
@@ -351,9 +351,9 @@ __global__ void __launch_bounds__(1024) qk_prepare_kernel(T* __restrict__ q_out,
 // (one stream, one head, Dc wide) takes [c / rms(c) * w | turned key part | zeros].
 template <typename T>
 __global__ void __launch_bounds__(256) latent_rotate_append_kernel(
-    T* __restrict__ q_out, const float* __restrict__ rows, int64_t ld, const float* __restrict__ w, float eps,
-    const double* __restrict__ freq, float magnitude, int interleaved, const int* __restrict__ tok_pos,
-    const int* __restrict__ tok_slot, RbPagedLayer cache, int H, int D, int R, int C) {
+    T* q_out, const float* rows, int64_t ld, const float* w, float eps,
+    const double* freq, float magnitude, int interleaved, const int* tok_pos,
+    const int* tok_slot, RbPagedLayer cache, int H, int D, int R, int C) {
   rb_pdl_launch_dependents();
   __shared__ float scratch[33];
   extern __shared__ float s_sincos[];
@@ -395,9 +395,9 @@ __global__ void __launch_bounds__(256) latent_rotate_append_kernel(
 
 // rows[t, col0 + head * D + e], head < n_heads: the first rot_dim values of every head turned by the row's position,
 // in place.  A block per token; a thread owns whole pairs, so nothing is read after it was written.
-__global__ void __launch_bounds__(256) rotate_rows_kernel(float* __restrict__ rows, int64_t ld, int col0, int n_heads, int D,
-                                                          const double* __restrict__ freq, float magnitude, int rot_dim,
-                                                          int interleaved, const int* __restrict__ tok_pos) {
+__global__ void __launch_bounds__(256) rotate_rows_kernel(float* rows, int64_t ld, int col0, int n_heads, int D,
+                                                          const double* freq, float magnitude, int rot_dim,
+                                                          int interleaved, const int* tok_pos) {
   rb_pdl_launch_dependents();
   extern __shared__ float s_sincos[];
   const int t = blockIdx.x;

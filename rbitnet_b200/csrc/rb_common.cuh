@@ -46,6 +46,11 @@ void rb_set_error(const char* fmt, ...);
 // has completed and is visible), and rb_pdl_launch_dependents() as early as it can, so that
 // the next kernel's launch and set-up overlap this kernel's work.  Inside a captured graph the
 // same launches become programmatic edges.
+//
+// No pointer of a kernel is declared restrict.  Behind such a pointer the compiler takes the data for its own, or, if it is
+// const, for constant while the kernel runs, and may load it before the wait, whose clobber says nothing about it: the tiled
+// product of bfloat16 rows without 16-byte loads did so once its loads stood in a row behind the wait, and multiplied what
+// the kernel before it had not written yet.
 __device__ __forceinline__ void rb_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void rb_pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

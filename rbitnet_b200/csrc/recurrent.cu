@@ -28,11 +28,11 @@ __device__ __forceinline__ float gelu_tanh_(float z) {
 // the start of a sequence.  tok_first: row of the first token of the row's run (null: every row is its own run).
 constexpr int CONV_TOKENS = 8;
 template <typename TI>
-__global__ void conv_causal_kernel(float* __restrict__ u, const TI* __restrict__ x, int64_t ldx, int x_off,
-                                   const float* __restrict__ x_bias, const float* __restrict__ taps,
-                                   const float* __restrict__ conv_bias, const float* __restrict__ tail,
-                                   const int* __restrict__ tok_first, const int* __restrict__ tok_slot,
-                                   const int* __restrict__ tok_pos, int n_tokens, int C, int K, int silu, int per_block) {
+__global__ void conv_causal_kernel(float* u, const TI* x, int64_t ldx, int x_off,
+                                   const float* x_bias, const float* taps,
+                                   const float* conv_bias, const float* tail,
+                                   const int* tok_first, const int* tok_slot,
+                                   const int* tok_pos, int n_tokens, int C, int K, int silu, int per_block) {
   rb_pdl_launch_dependents();
   rb_pdl_wait();
   // with many rows a block takes per_block neighbouring rows in turn: the earlier rows a row reads are then mostly in
@@ -64,11 +64,11 @@ __global__ void conv_causal_kernel(float* __restrict__ u, const TI* __restrict__
 // 4,096 rows 55; 53 34 26 21.
 constexpr int CONV_AHEAD = 8;
 template <int K, int ROWS>
-__global__ void __launch_bounds__(128) conv_causal_rows_kernel(float* __restrict__ u, const float* __restrict__ x, int64_t ldx, int x_off,
-                                                               const float* __restrict__ x_bias, const float* __restrict__ taps,
-                                                               const float* __restrict__ conv_bias, const float* __restrict__ tail,
-                                                               const int* __restrict__ tok_first, const int* __restrict__ tok_slot,
-                                                               const int* __restrict__ tok_pos, int T, int C, int silu) {
+__global__ void __launch_bounds__(128) conv_causal_rows_kernel(float* u, const float* x, int64_t ldx, int x_off,
+                                                               const float* x_bias, const float* taps,
+                                                               const float* conv_bias, const float* tail,
+                                                               const int* tok_first, const int* tok_slot,
+                                                               const int* tok_pos, int T, int C, int silu) {
   rb_pdl_launch_dependents();
   const int c = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
   if (c >= C) return;
@@ -130,10 +130,10 @@ __global__ void __launch_bounds__(128) conv_causal_rows_kernel(float* __restrict
 // The ring of a convolution's last inputs moves on to the end of every run: the inputs (with their bias) of the
 // run's last K-1 positions go to their rows.  For a mixer whose recurrence kernel does not do this itself.
 template <typename TI>
-__global__ void conv_tail_kernel(float* __restrict__ tail, const TI* __restrict__ x, int64_t ldx, int x_off,
-                                 const float* __restrict__ x_bias, const int* __restrict__ seq_first,
-                                 const int* __restrict__ seq_count, const int* __restrict__ tok_slot,
-                                 const int* __restrict__ tok_pos, int C, int K) {
+__global__ void conv_tail_kernel(float* tail, const TI* x, int64_t ldx, int x_off,
+                                 const float* x_bias, const int* seq_first,
+                                 const int* seq_count, const int* tok_slot,
+                                 const int* tok_pos, int C, int K) {
   rb_pdl_launch_dependents();
   rb_pdl_wait();
   const int first = seq_first != nullptr ? seq_first[blockIdx.x] : blockIdx.x;
@@ -153,11 +153,11 @@ __global__ void conv_tail_kernel(float* __restrict__ tail, const TI* __restrict_
 // input gate) of the channel's block.  Also moves the convolution's tail on to the end of the run.
 template <typename TI, typename TO>
 __global__ void __launch_bounds__(64) gated_scan_kernel(
-    TO* __restrict__ out, const float* __restrict__ u, const float* __restrict__ gates, const float* __restrict__ gate_r_bias,
-    const float* __restrict__ gate_i_bias, const float* __restrict__ lam, float decay_scale, const TI* __restrict__ xy,
-    int64_t ldxy, int x_off, int y_off, const float* __restrict__ x_bias, const float* __restrict__ y_bias,
-    float* __restrict__ state, float* __restrict__ tail, const int* __restrict__ seq_first,
-    const int* __restrict__ seq_count, const int* __restrict__ tok_slot, const int* __restrict__ tok_pos, int W, int Wb, int K) {
+    TO* out, const float* u, const float* gates, const float* gate_r_bias,
+    const float* gate_i_bias, const float* lam, float decay_scale, const TI* xy,
+    int64_t ldxy, int x_off, int y_off, const float* x_bias, const float* y_bias,
+    float* state, float* tail, const int* seq_first,
+    const int* seq_count, const int* tok_slot, const int* tok_pos, int W, int Wb, int K) {
   rb_pdl_launch_dependents();
   const int c = blockIdx.y * blockDim.x + threadIdx.x;
   if (c >= W) return;
@@ -193,8 +193,8 @@ __global__ void __launch_bounds__(64) gated_scan_kernel(
 
 // ---- long runs: the gates become decays and drives in one pass over all rows, then a scan in chunks of time
 // a = exp(-c softplus(lam) sigmoid(g_r + b_r)) replaces g_r and b = sqrt(1 - a^2) sigmoid(g_i + b_i) u replaces g_i, in place.
-__global__ void gate_prepare_kernel(float* __restrict__ gates, const float* __restrict__ u, const float* __restrict__ gate_r_bias,
-                                    const float* __restrict__ gate_i_bias, const float* __restrict__ lam, float decay_scale,
+__global__ void gate_prepare_kernel(float* gates, const float* u, const float* gate_r_bias,
+                                    const float* gate_i_bias, const float* lam, float decay_scale,
                                     int64_t n, int W, int Wb) {
   rb_pdl_launch_dependents();
   rb_pdl_wait();
@@ -218,10 +218,10 @@ __global__ void gate_prepare_kernel(float* __restrict__ gates, const float* __re
 constexpr int SCAN_CH = 32, SCAN_CHUNKS = 32;
 template <typename TI, typename TO>
 __global__ void __launch_bounds__(SCAN_CH * SCAN_CHUNKS) gated_scan_chunked_kernel(
-    TO* __restrict__ out, const float* __restrict__ ab, const TI* __restrict__ xy, int64_t ldxy, int x_off, int y_off,
-    const float* __restrict__ x_bias, const float* __restrict__ y_bias, float* __restrict__ state, float* __restrict__ tail,
-    const int* __restrict__ seq_first, const int* __restrict__ seq_count, const int* __restrict__ tok_slot,
-    const int* __restrict__ tok_pos, int W, int Wb, int K) {
+    TO* out, const float* ab, const TI* xy, int64_t ldxy, int x_off, int y_off,
+    const float* x_bias, const float* y_bias, float* state, float* tail,
+    const int* seq_first, const int* seq_count, const int* tok_slot,
+    const int* tok_pos, int W, int Wb, int K) {
   rb_pdl_launch_dependents();
   __shared__ float sA[SCAN_CHUNKS][SCAN_CH], sB[SCAN_CHUNKS][SCAN_CH];
   const int lane = threadIdx.x & 31, chunk = threadIdx.x >> 5;
@@ -273,11 +273,11 @@ __global__ void __launch_bounds__(SCAN_CH * SCAN_CHUNKS) gated_scan_chunked_kern
 constexpr int STEP_CH = 8, STEP_MAX_ROWS = 16;
 template <typename TI, typename TO>
 __global__ void __launch_bounds__(32 * STEP_CH) gated_step_kernel(
-    TO* __restrict__ out, const TI* __restrict__ xy, int64_t ldxy, int x_off, int y_off, const float* __restrict__ x_bias,
-    const float* __restrict__ y_bias, const float* __restrict__ taps, const float* __restrict__ conv_bias,
-    const float* __restrict__ w_gates, const float* __restrict__ gate_r_bias, const float* __restrict__ gate_i_bias,
-    const float* __restrict__ lam, float decay_scale, float* __restrict__ state, float* __restrict__ tail,
-    const int* __restrict__ tok_slot, const int* __restrict__ tok_pos, int T, int W, int Wb, int K) {
+    TO* out, const TI* xy, int64_t ldxy, int x_off, int y_off, const float* x_bias,
+    const float* y_bias, const float* taps, const float* conv_bias,
+    const float* w_gates, const float* gate_r_bias, const float* gate_i_bias,
+    const float* lam, float decay_scale, float* state, float* tail,
+    const int* tok_slot, const int* tok_pos, int T, int W, int Wb, int K) {
   rb_pdl_launch_dependents();
   extern __shared__ float s_u[];                 // [T][Wb]
   const int b = blockIdx.x;
@@ -388,11 +388,11 @@ template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile(
 // in shared memory, zeros behind D, so the loop over d needs no test and its addresses are constants.
 template <int P, int R>
 __global__ void __launch_bounds__(128) matrix_memory_kernel(
-    float* __restrict__ o_out, const float* __restrict__ proj, int64_t ld, int q_off, int k_off, int v_off, int i_off,
-    int f_off, const float* __restrict__ i_bias, const float* __restrict__ f_bias, float cap, float q_scale,
-    float floor_add, float* __restrict__ C_state, const float* __restrict__ n_state, const float* __restrict__ m_state,
-    float* __restrict__ moved, const int* __restrict__ seq_first, const int* __restrict__ seq_count,
-    const int* __restrict__ tok_slot, int H, int D, int Dv, int vec4) {
+    float* o_out, const float* proj, int64_t ld, int q_off, int k_off, int v_off, int i_off,
+    int f_off, const float* i_bias, const float* f_bias, float cap, float q_scale,
+    float floor_add, float* C_state, const float* n_state, const float* m_state,
+    float* moved, const int* seq_first, const int* seq_count,
+    const int* tok_slot, int H, int D, int Dv, int vec4) {
   rb_pdl_launch_dependents();
   extern __shared__ __align__(16) float sm[];
   constexpr int Dp = P * R;
@@ -583,8 +583,8 @@ struct Moved {
 // gate * sigmoid(gate)).  One warp each.  gate: the projections' rows, at column g_off.  The weight has H * Dv
 // values, or Dv values that every head uses (w_shared).
 template <typename TI, typename TO>
-__global__ void head_norm_gate_kernel(TO* __restrict__ out, const float* __restrict__ o, const float* __restrict__ w,
-                                      const TI* __restrict__ proj, int64_t ld, int g_off, int n_rows, int H, int Dv,
+__global__ void head_norm_gate_kernel(TO* out, const float* o, const float* w,
+                                      const TI* proj, int64_t ld, int g_off, int n_rows, int H, int Dv,
                                       float eps, int w_shared, int gate_silu, int norm_blocks, Moved moved) {
   rb_pdl_launch_dependents();
   rb_pdl_wait();

@@ -38,9 +38,9 @@ struct RouteWeighing {
 // warp w makes the choice of token w.  Shared memory: per token 2 n + 2 groups floats.
 // One warp: from the token's router sums z[0..n) (shared memory; choice, gscore: n and 2 groups floats of scratch) to
 // its `top` outputs and their weights.
-__device__ __forceinline__ void route_select(float* z, float* choice, float* gscore, const float* __restrict__ correction,
-                                             int n, int top, int groups, int keep, int lane, int* __restrict__ ids,
-                                             float* __restrict__ weights, int64_t t, int scoring = 0,
+__device__ __forceinline__ void route_select(float* z, float* choice, float* gscore, const float* correction,
+                                             int n, int top, int groups, int keep, int lane, int* ids,
+                                             float* weights, int64_t t, int scoring = 0,
                                              RouteWeighing weighing = RouteWeighing()) {
   if (scoring == 2) {
     for (int e = lane; e < n; e += 32) choice[e] = z[e] + (correction != nullptr ? correction[e] : 0.f);
@@ -151,11 +151,11 @@ RouteWeighing take_weighing() {
 constexpr int ROUTE_TB = 8;
 
 template <typename TI>
-__global__ void __launch_bounds__(256) route_kernel(int* __restrict__ ids, float* __restrict__ weights,
-                                                    const TI* __restrict__ h, int64_t ldh,
-                                                    const float* __restrict__ Wr, const float* __restrict__ correction,
+__global__ void __launch_bounds__(256) route_kernel(int* ids, float* weights,
+                                                    const TI* h, int64_t ldh,
+                                                    const float* Wr, const float* correction,
                                                     int T, int K, int n_out, int top, int groups, int keep, int TB, int vec,
-                                                    int scoring, int n_extra, float* __restrict__ extra, RouteWeighing weighing) {
+                                                    int scoring, int n_extra, float* extra, RouteWeighing weighing) {
   rb_pdl_launch_dependents();
   extern __shared__ float s_route[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -240,8 +240,8 @@ __global__ void __launch_bounds__(256) route_kernel(int* __restrict__ ids, float
 // order), then a warp per token for the choice.
 constexpr int RL_TM = 16, RL_TN = 64, RL_TK = 32;
 template <typename TI>
-__global__ void __launch_bounds__(256) route_logits_kernel(float* __restrict__ z, const TI* __restrict__ h, int64_t ldh,
-                                                           const float* __restrict__ Wr, int T, int K, int n) {
+__global__ void __launch_bounds__(256) route_logits_kernel(float* z, const TI* h, int64_t ldh,
+                                                           const float* Wr, int T, int K, int n) {
   rb_pdl_launch_dependents();
   __shared__ float As[RL_TK][RL_TM + 1];
   __shared__ __align__(16) float Ws[RL_TK][RL_TN + 4];
@@ -292,10 +292,10 @@ __global__ void __launch_bounds__(256) route_logits_kernel(float* __restrict__ z
   }
 }
 
-__global__ void __launch_bounds__(128) route_select_kernel(int* __restrict__ ids, float* __restrict__ weights,
-                                                           const float* __restrict__ zg, const float* __restrict__ correction,
+__global__ void __launch_bounds__(128) route_select_kernel(int* ids, float* weights,
+                                                           const float* zg, const float* correction,
                                                            int T, int n, int top, int groups, int keep, int scoring,
-                                                           int n_extra, float* __restrict__ extra, RouteWeighing weighing) {
+                                                           int n_extra, float* extra, RouteWeighing weighing) {
   rb_pdl_launch_dependents();
   extern __shared__ float s_route[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -315,8 +315,8 @@ __global__ void __launch_bounds__(128) route_select_kernel(int* __restrict__ ids
 //   pos [pairs]        the pair's row in the padded buffer (-1: an identity expert)
 //   row_token [rows]   the token whose input row a buffer row holds (-1: padding)
 //   tile_group [tiles] the expert of a tile of rows (-1: none)
-__global__ void __launch_bounds__(1024) plan_kernel(int* __restrict__ pos, int* __restrict__ row_token,
-                                                    int* __restrict__ tile_group, const int* __restrict__ ids,
+__global__ void __launch_bounds__(1024) plan_kernel(int* pos, int* row_token,
+                                                    int* tile_group, const int* ids,
                                                     int pairs, int top, int n_experts, int tile, int n_tiles) {
   rb_pdl_launch_dependents();
   extern __shared__ int s_plan[];       // counts [n_experts], first rows [n_experts]
@@ -358,7 +358,7 @@ __global__ void __launch_bounds__(1024) plan_kernel(int* __restrict__ pos, int* 
 // ---------------------------------------------------------------- gather
 // xp[r, :] = h[row_token[r], :], zeros for padding rows.
 template <typename T>
-__global__ void gather_kernel(T* __restrict__ xp, const T* __restrict__ h, int64_t ldh, const int* __restrict__ row_token,
+__global__ void gather_kernel(T* xp, const T* h, int64_t ldh, const int* row_token,
                               int K) {
   rb_pdl_launch_dependents();
   rb_pdl_wait();
@@ -388,8 +388,8 @@ __global__ void gather_kernel(T* __restrict__ xp, const T* __restrict__ h, int64
 // xp[r, :] = w * h[row_token[r], :] with w the weight of the pair that owns row r (the token's choice j with
 // pos[token, j] == r), rounded to the rows' type; zeros for padding rows.
 template <typename T>
-__global__ void gather_scaled_kernel(T* __restrict__ xp, const T* __restrict__ h, int64_t ldh, const int* __restrict__ row_token,
-                                     const int* __restrict__ pos, const float* __restrict__ weights, int top, int K) {
+__global__ void gather_scaled_kernel(T* xp, const T* h, int64_t ldh, const int* row_token,
+                                     const int* pos, const float* weights, int top, int K) {
   rb_pdl_launch_dependents();
   rb_pdl_wait();
   const int r = blockIdx.x;
@@ -413,9 +413,9 @@ __global__ void gather_scaled_kernel(T* __restrict__ xp, const T* __restrict__ h
 // chosen, rows of 2,048: the two took 5.1 us of a step, this one 2.1; 8 tokens, weighed rows 7.1 and 3.6).
 constexpr int PLACE_PAIRS = 256;
 template <typename T>
-__global__ void __launch_bounds__(256) place_kernel(T* __restrict__ xp, int* __restrict__ pos, int* __restrict__ tile_group,
-                                                    const T* __restrict__ h, int64_t ldh, const int* __restrict__ ids,
-                                                    const float* __restrict__ weights, int pairs, int top, int n_experts, int tile,
+__global__ void __launch_bounds__(256) place_kernel(T* xp, int* pos, int* tile_group,
+                                                    const T* h, int64_t ldh, const int* ids,
+                                                    const float* weights, int pairs, int top, int n_experts, int tile,
                                                     int K, int vec) {
   rb_pdl_launch_dependents();
   extern __shared__ int s_place[];      // ids [PLACE_PAIRS], tiles of every expert [n_experts]
@@ -503,8 +503,8 @@ struct CombineTail {
 
 // x[t, :] (+)= sum_j w[t, j] * (pos[t, j] >= 0 ? y[pos[t, j], :] : h[t, :]), the choices in their order.
 template <typename T>
-__global__ void combine_kernel(float* __restrict__ x, int64_t ldx, const float* __restrict__ y, const T* __restrict__ h,
-                               int64_t ldh, const int* __restrict__ pos, const float* __restrict__ weights, int top, int E,
+__global__ void combine_kernel(float* x, int64_t ldx, const float* y, const T* h,
+                               int64_t ldh, const int* pos, const float* weights, int top, int E,
                                int accumulate, int vec4, CombineTail tail) {
   rb_pdl_launch_dependents();
   rb_pdl_wait();
@@ -573,9 +573,9 @@ __global__ void combine_kernel(float* __restrict__ x, int64_t ldx, const float* 
 constexpr int GM = 64, GN = 64, GK = 16;
 
 template <typename TA, typename TC>
-__global__ void __launch_bounds__(256) gemm_grouped_kernel(TC* __restrict__ C, int64_t ldc, const TA* __restrict__ A,
-                                                          int64_t lda, const TA* __restrict__ W, int64_t ldw,
-                                                          const int* __restrict__ tile_group, int N, int K,
+__global__ void __launch_bounds__(256) gemm_grouped_kernel(TC* C, int64_t ldc, const TA* A,
+                                                          int64_t lda, const TA* W, int64_t ldw,
+                                                          const int* tile_group, int N, int K,
                                                           int square_relu) {
   rb_pdl_launch_dependents();
   rb_pdl_wait();
@@ -630,7 +630,7 @@ __global__ void __launch_bounds__(256) gemm_grouped_kernel(TC* __restrict__ C, i
 
 // ---------------------------------------------------------------- max(v, 0)^2, element by element
 template <typename T>
-__global__ void square_relu_kernel(T* __restrict__ out, const T* __restrict__ in, int64_t n) {
+__global__ void square_relu_kernel(T* out, const T* in, int64_t n) {
   rb_pdl_launch_dependents();
   rb_pdl_wait();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {

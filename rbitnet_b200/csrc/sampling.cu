@@ -23,9 +23,9 @@ constexpr int THREADS = 256;
 
 __device__ __forceinline__ float clean(float v) { return v != v ? -INFINITY : v; }
 
-__global__ void __launch_bounds__(THREADS) sample_stats_kernel(float* __restrict__ stats,
-                                                              const float* __restrict__ logits, int64_t row_stride,
-                                                              int V, int chunk, const float* __restrict__ temperature) {
+__global__ void __launch_bounds__(THREADS) sample_stats_kernel(float* stats,
+                                                              const float* logits, int64_t row_stride,
+                                                              int V, int chunk, const float* temperature) {
   rb_pdl_launch_dependents();
   rb_pdl_wait();
   __shared__ float scratch[33];
@@ -57,11 +57,11 @@ __global__ void __launch_bounds__(THREADS) sample_stats_kernel(float* __restrict
   }
 }
 
-__global__ void __launch_bounds__(THREADS) sample_pick_kernel(int* __restrict__ out, const float* __restrict__ stats,
-                                                             const float* __restrict__ logits, int64_t row_stride,
+__global__ void __launch_bounds__(THREADS) sample_pick_kernel(int* out, const float* stats,
+                                                             const float* logits, int64_t row_stride,
                                                              int V, int chunk, int n_chunks,
-                                                             const float* __restrict__ temperature,
-                                                             const float* __restrict__ uniform) {
+                                                             const float* temperature,
+                                                             const float* uniform) {
   rb_pdl_launch_dependents();
   rb_pdl_wait();
   __shared__ float part[THREADS];

@@ -29,10 +29,10 @@ __device__ __forceinline__ float ssd_silu_fast(float v) { return __fdividef(v, 1
 // u[t, c] = silu(bias[c] + sum_d taps[c, K-1-d] x_(t-d)[c]), zeros before a sequence's start, rows before a run from the
 // ring tail[slot][K][C] (the input of position q in row q mod K).  A block takes `per_block` rows; V channels a thread.
 template <typename TO, int K, int V>
-__global__ void __launch_bounds__(128) ssd_conv_kernel(TO* __restrict__ u, int64_t ldu, const float* __restrict__ x, int64_t ldx,
-                                                       int x_off, const float* __restrict__ taps, const float* __restrict__ bias,
-                                                       const float* __restrict__ tail, const int* __restrict__ tok_first,
-                                                       const int* __restrict__ tok_slot, const int* __restrict__ tok_pos, int T,
+__global__ void __launch_bounds__(128) ssd_conv_kernel(TO* u, int64_t ldu, const float* x, int64_t ldx,
+                                                       int x_off, const float* taps, const float* bias,
+                                                       const float* tail, const int* tok_first,
+                                                       const int* tok_slot, const int* tok_pos, int T,
                                                        int C, int per_block) {
   rb_pdl_launch_dependents();
   const int c = (blockIdx.y * blockDim.x + threadIdx.x) * V;
@@ -110,11 +110,11 @@ __global__ void __launch_bounds__(128) ssd_conv_kernel(TO* __restrict__ u, int64
 
 // Any number of taps, value by value.
 template <typename TO>
-__global__ void __launch_bounds__(128) ssd_conv_any_kernel(TO* __restrict__ u, int64_t ldu, const float* __restrict__ x, int64_t ldx,
-                                                           int x_off, const float* __restrict__ taps,
-                                                           const float* __restrict__ bias, const float* __restrict__ tail,
-                                                           const int* __restrict__ tok_first, const int* __restrict__ tok_slot,
-                                                           const int* __restrict__ tok_pos, int T, int C, int K) {
+__global__ void __launch_bounds__(128) ssd_conv_any_kernel(TO* u, int64_t ldu, const float* x, int64_t ldx,
+                                                           int x_off, const float* taps,
+                                                           const float* bias, const float* tail,
+                                                           const int* tok_first, const int* tok_slot,
+                                                           const int* tok_pos, int T, int C, int K) {
   rb_pdl_launch_dependents();
   rb_pdl_wait();
   const int t = blockIdx.x;
@@ -139,10 +139,10 @@ constexpr int STEP_HELD = 8;            // state rows a thread holds at a time
 // KT: the convolution's taps (0: any number, from K).
 template <int V, int KT>
 __global__ void __launch_bounds__(STEP_NT, 3) ssd_step_kernel(
-    float* __restrict__ out, const float* __restrict__ rows, int64_t ld, int z_off, int x_off, int dt_off,
-    const float* __restrict__ taps, const float* __restrict__ conv_bias, const float* __restrict__ dt_bias,
-    const float* __restrict__ A_log, const float* __restrict__ D_skip, float* __restrict__ state, float* __restrict__ tail,
-    const int* __restrict__ tok_slot, const int* __restrict__ tok_pos, int H, int P, int N, int G, int K_, int cols) {
+    float* out, const float* rows, int64_t ld, int z_off, int x_off, int dt_off,
+    const float* taps, const float* conv_bias, const float* dt_bias,
+    const float* A_log, const float* D_skip, float* state, float* tail,
+    const int* tok_slot, const int* tok_pos, int H, int P, int N, int G, int K_, int cols) {
   rb_pdl_launch_dependents();
   extern __shared__ float s_step[];
   float* sx = s_step;                   // [cols] x
@@ -290,9 +290,9 @@ constexpr int SCAN_ROWS = SCAN_NT / SCAN_COLS;
 
 template <typename TU, int R>
 __global__ void __launch_bounds__(SCAN_NT) ssd_scan_kernel(
-    float* __restrict__ out, const TU* __restrict__ u, int64_t ldu, const float* __restrict__ rows, int64_t ld, int z_off, int dt_off,
-    const float* __restrict__ dt_bias, const float* __restrict__ A_log, const float* __restrict__ D_skip, float* __restrict__ state,
-    const int* __restrict__ seq_first, const int* __restrict__ seq_count, const int* __restrict__ tok_slot, int H, int P, int N,
+    float* out, const TU* u, int64_t ldu, const float* rows, int64_t ld, int z_off, int dt_off,
+    const float* dt_bias, const float* A_log, const float* D_skip, float* state,
+    const int* seq_first, const int* seq_count, const int* tok_slot, int H, int P, int N,
     int G) {
   rb_pdl_launch_dependents();
   __shared__ float red[2][SCAN_NT / 32][SCAN_COLS];
@@ -391,7 +391,7 @@ __device__ __forceinline__ void split3(float a, float b, uint32_t& hi, uint32_t&
 }
 
 // One warp: dt and L of the chunk's tokens into s_dt [64] and s_L [64] (float64).
-__device__ __forceinline__ void chunk_decays(const float* __restrict__ rows, int64_t ld, int col, int64_t row0, int m, float a,
+__device__ __forceinline__ void chunk_decays(const float* rows, int64_t ld, int col, int64_t row0, int m, float a,
                                              float dt_bias, double* s_L, float* s_dt, int lane) {
   float d[2];
 #pragma unroll
@@ -415,7 +415,7 @@ __device__ __forceinline__ void chunk_decays(const float* __restrict__ rows, int
 // A tile [64 rows][width] of bfloat16 values from u's columns col.., zeros beyond row m and column `live`.  vec: 16-byte
 // pieces (every column and stride a multiple of 8 values), which are only asked for: see tiles_landed.
 __device__ __forceinline__ void tiles_landed() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-__device__ __forceinline__ void load_tile(__nv_bfloat16* dst, int ldd, int width, const __nv_bfloat16* __restrict__ u, int64_t ldu,
+__device__ __forceinline__ void load_tile(__nv_bfloat16* dst, int ldd, int width, const __nv_bfloat16* u, int64_t ldu,
                                           int64_t row0, int m, int col, int live, bool vec) {
   if (vec) {
     const int w8 = width >> 3;
@@ -438,9 +438,9 @@ __device__ __forceinline__ void load_tile(__nv_bfloat16* dst, int ldd, int width
 // grid (chunks, H, tiles of 64 columns).  sums [chunks][H][N][P], ends [chunks][H].
 template <bool FULL>
 __global__ void __launch_bounds__(CH_NT, 4) ssd_chunk_sum_kernel(
-    float* __restrict__ sums, float* __restrict__ ends, const __nv_bfloat16* __restrict__ u, int64_t ldu,
-    const float* __restrict__ rows, int64_t ld, int dt_off, const float* __restrict__ dt_bias, const float* __restrict__ A_log,
-    const int* __restrict__ chunk_row, const int* __restrict__ chunk_len, int H, int P, int N, int G, int vec) {
+    float* sums, float* ends, const __nv_bfloat16* u, int64_t ldu,
+    const float* rows, int64_t ld, int dt_off, const float* dt_bias, const float* A_log,
+    const int* chunk_row, const int* chunk_len, int H, int P, int N, int G, int vec) {
   rb_pdl_launch_dependents();
   extern __shared__ __align__(16) uint8_t s_bytes[];
   const int NP = (N + 15) & ~15, LDB = NP + 8;
@@ -520,13 +520,13 @@ __global__ void __launch_bounds__(CH_NT, 4) ssd_chunk_sum_kernel(
 // grid (runs, H, pieces of a state), 128 threads, V values each: sums[chunk] <- the state the chunk starts from; and
 // the ring of the convolution's last inputs is brought up to the run's end (tail [n_slots, K, C], null with one tap).
 template <int V>
-__global__ void __launch_bounds__(128) ssd_chunk_walk_kernel(float* __restrict__ sums, const float* __restrict__ ends,
-                                                             float* __restrict__ state, const int* __restrict__ seq_first,
-                                                             const int* __restrict__ seq_count,
-                                                             const int* __restrict__ run_chunk0, const int* __restrict__ tok_slot,
-                                                             int H, int64_t NP_, float* __restrict__ tail,
-                                                             const float* __restrict__ rows, int64_t ld, int x_off,
-                                                             const int* __restrict__ tok_pos, int C, int K) {
+__global__ void __launch_bounds__(128) ssd_chunk_walk_kernel(float* sums, const float* ends,
+                                                             float* state, const int* seq_first,
+                                                             const int* seq_count,
+                                                             const int* run_chunk0, const int* tok_slot,
+                                                             int H, int64_t NP_, float* tail,
+                                                             const float* rows, int64_t ld, int x_off,
+                                                             const int* tok_pos, int C, int K) {
   rb_pdl_launch_dependents();
   const int run = blockIdx.x, h = blockIdx.y;
   const int64_t e = ((int64_t)blockIdx.z * 128 + threadIdx.x) * V;
@@ -580,10 +580,10 @@ __global__ void __launch_bounds__(128) ssd_chunk_walk_kernel(float* __restrict__
 // grid (chunks, H, tiles of 64 columns).  starts: what the walk left.  out [T, H * P] = v (see the top of the file).
 template <bool FULL>
 __global__ void __launch_bounds__(CH_NT, 3) ssd_chunk_out_kernel(
-    float* __restrict__ out, const float* __restrict__ starts, const __nv_bfloat16* __restrict__ u, int64_t ldu,
-    const float* __restrict__ rows, int64_t ld, int z_off, int dt_off, const float* __restrict__ dt_bias,
-    const float* __restrict__ A_log, const float* __restrict__ D_skip, const int* __restrict__ chunk_row,
-    const int* __restrict__ chunk_len, int H, int P, int N, int G, int vec) {
+    float* out, const float* starts, const __nv_bfloat16* u, int64_t ldu,
+    const float* rows, int64_t ld, int z_off, int dt_off, const float* dt_bias,
+    const float* A_log, const float* D_skip, const int* chunk_row,
+    const int* chunk_len, int H, int P, int N, int G, int vec) {
   rb_pdl_launch_dependents();
   extern __shared__ __align__(16) uint8_t s_bytes[];
   const int NP = (N + 15) & ~15, LDB = NP + 8;

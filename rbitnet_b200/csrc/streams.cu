@@ -159,7 +159,7 @@ __global__ void __launch_bounds__(256) stream_step_kernel(StreamStepArgs a) {
 }
 
 // X[t][k][:] = x[t][:] for every stream k
-__global__ void streams_expand_kernel(float* __restrict__ X, const float* __restrict__ x, int s, int E) {
+__global__ void streams_expand_kernel(float* X, const float* x, int s, int E) {
   rb_pdl_launch_dependents();
   rb_pdl_wait();
   const int t = blockIdx.x;
@@ -170,7 +170,7 @@ __global__ void streams_expand_kernel(float* __restrict__ X, const float* __rest
 }
 
 // out[r][:] = sum_k X[r][k][:], streams added in ascending order
-__global__ void streams_sum_kernel(float* __restrict__ out, const float* __restrict__ X, int s, int E) {
+__global__ void streams_sum_kernel(float* out, const float* X, int s, int E) {
   rb_pdl_launch_dependents();
   rb_pdl_wait();
   const int t = blockIdx.x;

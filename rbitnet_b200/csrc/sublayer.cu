@@ -29,8 +29,8 @@ __device__ __forceinline__ void store4(__nv_bfloat16* d, float a, float b, float
 }
 
 template <typename TO>
-__global__ void __launch_bounds__(256) rmsnorm_grouped_kernel(TO* __restrict__ out, const float* __restrict__ x,
-                                                              const float* __restrict__ w, int E, int groups, float eps,
+__global__ void __launch_bounds__(256) rmsnorm_grouped_kernel(TO* out, const float* x,
+                                                              const float* w, int E, int groups, float eps,
                                                               int vec) {
   rb_pdl_launch_dependents();
   rb_pdl_wait();
@@ -88,9 +88,9 @@ __global__ void __launch_bounds__(256) rmsnorm_grouped_kernel(TO* __restrict__ o
 // position 0).  With `update` (every row is its own run) the row also goes into the ring at its position: the rows it
 // read lie at other positions of the ring.
 template <typename T>
-__global__ void input_filter_kernel(T* __restrict__ out, const T* __restrict__ h, const float* __restrict__ taps,
-                                    float* __restrict__ ring, const int* __restrict__ tok_first,
-                                    const int* __restrict__ tok_slot, const int* __restrict__ tok_pos, int n_tokens, int C,
+__global__ void input_filter_kernel(T* out, const T* h, const float* taps,
+                                    float* ring, const int* tok_first,
+                                    const int* tok_slot, const int* tok_pos, int n_tokens, int C,
                                     int K, int update, int per_block) {
   rb_pdl_launch_dependents();
   rb_pdl_wait();
@@ -147,11 +147,11 @@ template <> struct FilterVec<__nv_bfloat16, 8> {
 };
 
 template <typename T, int V, int KM>
-__global__ void __launch_bounds__(256) input_filter_vec_kernel(T* __restrict__ out, const T* __restrict__ h,
-                                                               const float* __restrict__ taps, float* __restrict__ ring,
-                                                               const int* __restrict__ tok_first,
-                                                               const int* __restrict__ tok_slot,
-                                                               const int* __restrict__ tok_pos, int n_tokens, int C, int K,
+__global__ void __launch_bounds__(256) input_filter_vec_kernel(T* out, const T* h,
+                                                               const float* taps, float* ring,
+                                                               const int* tok_first,
+                                                               const int* tok_slot,
+                                                               const int* tok_pos, int n_tokens, int C, int K,
                                                                int update, int per_block) {
   rb_pdl_launch_dependents();
   const int c0 = (blockIdx.y * blockDim.x + threadIdx.x) * V;
@@ -198,13 +198,13 @@ __global__ void __launch_bounds__(256) input_filter_vec_kernel(T* __restrict__ o
 // the norm in groups of the new x (h), and the filter on h from the ring (hf), whose row at the token's position
 // becomes h.  A block of eight warps per row and part of the row.
 template <typename TO>
-__global__ void __launch_bounds__(256) norm_filter_rows_kernel(TO* __restrict__ h, TO* __restrict__ hf, float* __restrict__ x,
-                                                               const float* __restrict__ y, const float* __restrict__ g,
-                                                               int64_t ldg, const float* __restrict__ bias,
-                                                               const float* __restrict__ w, int E, int groups, float eps,
-                                                               const float* __restrict__ taps, float* __restrict__ ring,
-                                                               const int* __restrict__ tok_slot,
-                                                               const int* __restrict__ tok_pos, int K) {
+__global__ void __launch_bounds__(256) norm_filter_rows_kernel(TO* h, TO* hf, float* x,
+                                                               const float* y, const float* g,
+                                                               int64_t ldg, const float* bias,
+                                                               const float* w, int E, int groups, float eps,
+                                                               const float* taps, float* ring,
+                                                               const int* tok_slot,
+                                                               const int* tok_pos, int K) {
   rb_pdl_launch_dependents();
   rb_pdl_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
@@ -271,8 +271,8 @@ __global__ void __launch_bounds__(256) norm_filter_rows_kernel(TO* __restrict__ 
 
 // ---------------------------------------------------------------- gated residual
 template <typename TG>
-__global__ void gated_add_kernel(float* __restrict__ x, const float* __restrict__ y, const TG* __restrict__ g, int64_t ldg,
-                                 const float* __restrict__ bias, int64_t n, int E) {
+__global__ void gated_add_kernel(float* x, const float* y, const TG* g, int64_t ldg,
+                                 const float* bias, int64_t n, int E) {
   rb_pdl_launch_dependents();
   rb_pdl_wait();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -283,7 +283,7 @@ __global__ void gated_add_kernel(float* __restrict__ x, const float* __restrict_
   }
 }
 
-__global__ void softcap_kernel(float* __restrict__ v, int64_t n, float cap) {
+__global__ void softcap_kernel(float* v, int64_t n, float cap) {
   rb_pdl_launch_dependents();
   rb_pdl_wait();
   const float inv = 1.0f / cap;
@@ -299,8 +299,8 @@ inline int flat_blocks(int64_t n, int threads) {
 
 // The same for parts of 256 values and more: a block per row and part, NV times four values a thread in registers.
 template <typename TO, int NV>
-__global__ void __launch_bounds__(256) rmsnorm_parts_kernel(TO* __restrict__ out, const float* __restrict__ x,
-                                                            const float* __restrict__ w, int E, int per, float eps) {
+__global__ void __launch_bounds__(256) rmsnorm_parts_kernel(TO* out, const float* x,
+                                                            const float* w, int E, int per, float eps) {
   rb_pdl_launch_dependents();
   __shared__ float scratch[33];
   const int64_t at = (int64_t)blockIdx.x * E + (int64_t)blockIdx.y * per;

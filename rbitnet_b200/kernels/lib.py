@@ -113,6 +113,7 @@ _SIGNATURES = {
     "rb_latent_rotate_append": [P, I, P, L, P, F, P, F, I, P, P, P, P, I, I, I, I, I, I, I, I, P],
     "rb_rotate_rows": [P, L, I, I, I, P, F, I, I, P, I, P],
     "rb_set_error_flag_for_test": [I],
+    "rb_late_copy_for_test": [P, P, L, L, P],
     "rb_wait_probe": [L, I, P, P],
     "rb_count_wait_probe": [P, L, I, P, P],
 }

@@ -187,3 +187,11 @@ def test_parts_of_a_gated_product():
     assert gated_parts(65, 192, 512, 2, 148) == 1 and gated_parts(192, 5632, 1024, 2, 148) == 1 and gated_parts(65, 5632, 2048, 2, 148) == 1
     assert gated_parts(48, 8192, 1024, 4, 148) == 1 and gated_parts(17, 8192, 1024, 4, 148) == 4 and gated_parts(48, 5632, 1024, 4, 148) == 4
     assert gated_parts(300, 2816, 2048, 1, 148) == 1
+
+
+def test_no_pointer_of_a_kernel_is_restrict():
+    """The compiler may load what lies behind a restrict pointer before the wait for the kernel that writes it (rb_common.cuh)."""
+    from pathlib import Path
+    import rbitnet_b200
+    sources = sorted((Path(rbitnet_b200.__file__).parent / "csrc").glob("*.cu*"))
+    assert sources and not [s.name for s in sources if "__restrict" in s.read_text() or "__ldg(" in s.read_text()]
