@@ -167,7 +167,7 @@ __global__ void __launch_bounds__(WARPS * 32) attn_simple_kernel(T* out, const T
     const float mn = fmaxf(m, sinks[h]), c = rescale(m, mn);
     inv = c / (l * c + expf(sinks[h] - mn));
   } else {
-    inv = l > 0.f ? 1.0f / l : 0.f;
+    inv = 1.0f / l;                                    // every score -inf: 0 / 0, no keys that could be weighed
   }
   T* op = out + ((int64_t)t * H + h) * D;
 #pragma unroll

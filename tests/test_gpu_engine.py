@@ -253,3 +253,28 @@ def test_mid_size_prefill_chunks_and_decode(tmp_path, name, dtype):
             row = full[len(p) - 1 + i]
             atol, rtol = TOL[dtype]
             assert float(row[t]) >= float(row.max()) - 2 * (atol + rtol * float(row.abs().max()))
+
+
+def test_uploads_behind_a_busy_stream_and_under_capture():
+    """A host array is overwritten as soon as upload() returns, behind work that keeps the stream busy: the copies hold the values of
+    the call, below and above the size from which arrays go through pinned memory.  Under capture an upload is refused."""
+    import numpy as np
+    from rbitnet_b200.cache import upload
+    busy = torch.randn(4096, 4096, device="cuda")
+    for count in (1, 3, 700, 16 << 10, (16 << 10) + 1, 300_000):             # 4 bytes to 1.2 MB, the border at 64 KiB
+        array = np.empty(count, dtype=np.int32)
+        got = []
+        for _ in range(4):
+            busy @ busy
+        for k in range(20):
+            array[:] = np.arange(count, dtype=np.int32) + k
+            got.append(upload(array, "cuda:0"))
+            array[:] = -1
+        base = torch.arange(count, dtype=torch.int32, device="cuda")
+        assert all(torch.equal(t, base + k) for k, t in enumerate(got)), count
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        with pytest.raises(RuntimeError, match="captured"):
+            upload(np.zeros(4, dtype=np.int32), "cuda:0")
+        busy + 1.0
+    torch.cuda.synchronize()

@@ -881,3 +881,31 @@ def test_float32_attention_by_groups_of_lanes(ops32, H, Kh, D, page, lengths, de
             s = torch.cat([s, sink.double()[None, :, None].expand(T, H, 1)], dim=2)
         want = torch.einsum("thp,tphd->thd", torch.softmax(s, -1)[..., :mp * page], vv)
         assert _rel(out, want) < (20 * (D + 4) + max(lengths)) * 2.0 ** -24
+
+
+@pytest.mark.parametrize("D,T", [(64, 1), (30, 40), (256, 3)])
+def test_float32_attention_with_scores_that_are_not_finite(ops32, D, T):
+    """As a softmax in float64: keys with a score of -inf beside others weigh nothing, wherever they stand; a token whose scores are all
+    -inf, or one of them NaN, has no result (NaN); the other tokens and heads keep theirs."""
+    from ctypes import c_void_p
+    H, page, n = 4, 64, 90
+    g = torch.Generator(device="cuda").manual_seed(37)
+    k, v = (torch.randn(2, H, page, D, device="cuda", generator=g) for _ in range(2))
+    q = torch.rand(T, H, D, device="cuda", generator=g) + 0.5                # positive: an infinite key's score is -inf
+    k[0, 0, :5] = -math.inf                                                   # head 0: the first keys
+    k[:, 1] = -math.inf                                                       # head 1: every key
+    k[0, 2, 3, 0] = math.nan                                                  # head 2: one key NaN
+    table = torch.tensor([[0, 1]], dtype=torch.int32, device="cuda")
+    pos = torch.arange(n - T, n, dtype=torch.int32, device="cuda")
+    slot = torch.zeros(T, dtype=torch.int32, device="cuda")
+    out = torch.empty_like(q)
+    ptr = lambda t: c_void_p(t.data_ptr())
+    ops32.lib.call("rb_attention_simple", ptr(out), ptr(q), 0, ptr(k), ptr(v), ptr(table), 2, page, ptr(pos), ptr(slot), T, H, H, D,
+                   D ** -0.5, 0, ops32._stream())
+    kk, vv = (t.transpose(0, 1).reshape(H, 2 * page, D).double() for t in (k, v))
+    s = torch.einsum("thd,hpd->thp", q.double(), kk) * D ** -0.5
+    s = s.masked_fill((torch.arange(2 * page, device="cuda")[None] > pos[:, None])[:, None], -math.inf)
+    want = torch.einsum("thp,hpd->thd", torch.softmax(s, -1), vv)
+    assert torch.equal(torch.isnan(out), torch.isnan(want)) and torch.isnan(out[:, 1:3]).all()
+    keep = torch.isfinite(want)
+    assert keep[:, [0, 3]].all() and _rel(out[:, [0, 3]], want[:, [0, 3]]) < (20 * (D + 4) + n) * 2.0 ** -24
