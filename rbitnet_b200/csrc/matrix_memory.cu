@@ -381,7 +381,20 @@ __global__ void __launch_bounds__(NT, 5) memory_chunk_out_kernel(Memory a, float
   }
 }
 
+// Blocks of the walk for one (run, head): 128 threads of four values, of one where rows do not allow that.
+int64_t walk_pieces(int D, int Dv) {
+  const int64_t values = (int64_t)Dv * D + D;
+  return ((D % 4 == 0 ? values / 4 : values) + 127) / 128;
+}
+
 }  // namespace
+
+// Whether the chunked form takes heads of this size: the blocks of the sums and of the walk for a head are counted in the grid's third
+// dimension (33 million values a head; 8 million where D is no multiple of four).
+RB_EXPORT int rb_matrix_memory_chunked_takes(int D, int Dv) {
+  const int64_t tiles = (((int64_t)Dv + CH - 1) / CH) * ((D + CH - 1) / CH);
+  return D > 0 && D <= 512 && Dv > 0 && tiles < 65535 && walk_pieces(D, Dv) <= 65535;
+}
 
 // Scratch of the chunked form in floats.
 RB_EXPORT long long rb_matrix_memory_chunk_floats(int n_chunks, int H, int D, int Dv) {
@@ -399,7 +412,7 @@ RB_EXPORT int rb_matrix_memory_chunked(float* o_out, const float* proj, int64_t 
                                        const int* tok_slot, int n_seq, int n_chunks, int H, int D, int Dv, float* scratch,
                                        cudaStream_t stream) {
   if (n_seq == 0) return 0;
-  RB_REQUIRE(H > 0 && H <= 65535 && D > 0 && D <= 512 && Dv > 0 && n_chunks > 0, "rb_matrix_memory_chunked: bad sizes H=%d D=%d Dv=%d (D up to 512)", H, D, Dv);
+  RB_REQUIRE(H > 0 && H <= 65535 && n_chunks > 0 && rb_matrix_memory_chunked_takes(D, Dv), "rb_matrix_memory_chunked: sizes H=%d D=%d Dv=%d are not taken", H, D, Dv);
   RB_REQUIRE(cap > 0.f, "rb_matrix_memory_chunked: the gates' cap must be positive");
   RB_REQUIRE((uintptr_t)scratch % 16 == 0, "rb_matrix_memory_chunked: scratch must be 16-byte aligned");
   const int64_t heads = (int64_t)n_chunks * H;
@@ -417,22 +430,16 @@ RB_EXPORT int rb_matrix_memory_chunked(float* o_out, const float* proj, int64_t 
   a.vec = D % 4 == 0 && Dv % 4 == 0 && ld % 4 == 0 && q_off % 4 == 0 && k_off % 4 == 0 && v_off % 4 == 0 &&
           (uintptr_t)proj % 16 == 0 && (uintptr_t)o_out % 16 == 0 && (uintptr_t)C_state % 16 == 0;
   const int tiles_j = (Dv + CH - 1) / CH, tiles_d = (D + CH - 1) / CH;
-  RB_REQUIRE(tiles_j * tiles_d < 65535, "rb_matrix_memory_chunked: %d value columns: too large for one launch", Dv);
   RB_LAUNCH("memory_gates_kernel", (memory_gates_kernel), dim3(n_seq, (H + 3) / 4), 128, 0, stream, a, i_bias, f_bias, cap, m_state,
             run_chunk0, seq_first, seq_count, tok_slot);
   RB_LAUNCH("memory_chunk_sum_kernel", (memory_chunk_sum_kernel), dim3(n_chunks, H, 1 + tiles_j * tiles_d), NT, 0, stream, a);
-  const int64_t values = (int64_t)Dv * D + D;
-  if (D % 4 == 0) {
-    const int64_t z = (values / 4 + 127) / 128;
-    RB_REQUIRE(z <= 65535, "rb_matrix_memory_chunked: a memory of %d x %d: too large for one launch", D, Dv);
-    RB_LAUNCH("memory_chunk_walk_kernel", (memory_chunk_walk_kernel<4>), dim3(n_seq, H, (int)z), 128, 0, stream, a, C_state, n_state,
+  const dim3 walk(n_seq, H, (unsigned)walk_pieces(D, Dv));
+  if (D % 4 == 0)
+    RB_LAUNCH("memory_chunk_walk_kernel", (memory_chunk_walk_kernel<4>), walk, 128, 0, stream, a, C_state, n_state,
               run_chunk0, seq_first, seq_count, tok_slot);
-  } else {
-    const int64_t z = (values + 127) / 128;
-    RB_REQUIRE(z <= 65535, "rb_matrix_memory_chunked: a memory of %d x %d: too large for one launch", D, Dv);
-    RB_LAUNCH("memory_chunk_walk_kernel", (memory_chunk_walk_kernel<1>), dim3(n_seq, H, (int)z), 128, 0, stream, a, C_state, n_state,
+  else
+    RB_LAUNCH("memory_chunk_walk_kernel", (memory_chunk_walk_kernel<1>), walk, 128, 0, stream, a, C_state, n_state,
               run_chunk0, seq_first, seq_count, tok_slot);
-  }
   RB_LAUNCH("memory_chunk_out_kernel", (memory_chunk_out_kernel), dim3(n_chunks, H, tiles_j), NT, 0, stream, a, o_out, q_scale, floor_add);
   RB_CHECK_LAUNCH("rb_matrix_memory_chunked");
   return 0;

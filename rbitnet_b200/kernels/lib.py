@@ -63,6 +63,7 @@ _SIGNATURES = {
     "rb_gated_scan": [P, I, P, P, P, P, P, F, P, L, I, I, I, P, P, P, P, P, P, P, P, I, I, I, I, I, P],
     "rb_matrix_memory": [P, I, P, P, L, I, I, I, I, I, I, I, P, P, F, F, F, P, F, P, P, P, P, P, P, P, I, I, I, I, I, P],
     "rb_matrix_memory_chunked": [P, P, L, I, I, I, I, I, P, P, F, F, F, P, P, P, P, P, P, P, P, P, I, I, I, I, I, P, P],
+    "rb_matrix_memory_chunked_takes": [I, I],
     "rb_matrix_memory_lanes": [I],
     "rb_head_norm_gate": [P, I, P, P, P, L, I, I, I, I, I, F, I, I, P],
     "rb_rmsnorm_grouped": [P, I, P, P, I, I, I, F, P],

@@ -843,7 +843,8 @@ class CudaOps:
         return out
 
     def _memory_chunks_chosen(self, meta, n_seq: int, H: int, D: int, Dv: int) -> bool:
-        """Whether the step's runs go through a matrix memory in chunks of 64: by time, and if the scratch is allowed."""
+        """Whether the step's runs go through a matrix memory in chunks of 64: by time, and if the kernels take the size and the
+        scratch is allowed."""
         key = ("memory_chunks", H, D, Dv, self.memory_chunks_from, self.memory_scratch_floats)
         if key not in meta.extra:
             longest = max(c.n_new for c in meta.seqs)
@@ -852,7 +853,8 @@ class CudaOps:
                 wanted = memory_chunks_pay(longest, meta.n_tokens, chunks, H, D, Dv, self.lib.raw("rb_device_sm_count")())
             else:
                 wanted = meta.n_tokens >= self.memory_chunks_from[0] * n_seq and meta.n_tokens >= self.memory_chunks_from[1]
-            meta.extra[key] = wanted and self.lib.raw("rb_matrix_memory_chunk_floats")(chunks, H, D, Dv) <= self.memory_scratch_floats
+            meta.extra[key] = wanted and self.lib.raw("rb_matrix_memory_chunked_takes")(D, Dv) != 0 and \
+                self.lib.raw("rb_matrix_memory_chunk_floats")(chunks, H, D, Dv) <= self.memory_scratch_floats
         return meta.extra[key]
 
     def _delta_chunks(self, meta, size: int = 32):

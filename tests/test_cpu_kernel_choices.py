@@ -179,6 +179,21 @@ def test_when_a_matrix_memory_goes_in_chunks():
         assert not pays([2], *size) and not pays([1, 1, 2], *size)
 
 
+@pytest.mark.parametrize("D,Dv,chunks", [(512, 65534, True), (512, 65535, False), (512, 100000, False), (511, 16414, True), (511, 16420, False),
+                                         (4, 64 * 65534, True), (4, 64 * 65534 + 1, False)])
+def test_a_memory_too_large_for_the_chunks_goes_token_by_token(lib, D, Dv, chunks):
+    """Sizes whose sums or whose walk over the chunks would be more than 65,535 blocks a head, which the form that goes token by token
+    takes."""
+    from types import SimpleNamespace
+    from rbitnet_b200.kernels.ops import CudaOps
+    ops = SimpleNamespace(lib=lib, memory_chunks_from=(1, 1), memory_scratch_floats=1 << 40)
+    meta = SimpleNamespace(extra={}, seqs=[SimpleNamespace(n_new=130)], n_tokens=130)
+    assert CudaOps._memory_chunks_chosen(ops, meta, 1, 1, D, Dv) == chunks
+    walk = ((Dv + 1) * D // (4 if D % 4 == 0 else 1) + 127) // 128
+    sums = 1 + -(-Dv // 64) * -(-D // 64)
+    assert (max(walk, sums) <= 65535) == chunks
+
+
 def test_parts_of_a_gated_product():
     """Two parts of a short K and many parts' sums of many tokens are left out: each was slower than the product whole."""
     from rbitnet_b200.kernels.ops import gated_parts
