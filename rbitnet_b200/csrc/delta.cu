@@ -219,8 +219,10 @@ int launch_delta(dim3 grid, size_t smem, cudaStream_t stream, float* o, const fl
 // R rows each, in neighbouring groups of four), the norm over the head's outputs, the weight and the SiLU gate.  q and k of
 // a key head are made again by every value head that reads it; the first of them writes their ring rows.
 // What bounds it is its chain of loads, sums and barriers: the memory is asked for before the convolution, 16 bytes a
-// lane, every warp makes the sums over q and k for itself, and two barriers are left (2 sequences of 16 heads of 128 x 128:
-// 22.5 us of a step before, 10.5 now).
+// lane, every warp makes the sums over q and k for itself, and two barriers are left.  1,024 threads leave 64 registers a
+// thread, and the memory is held across the convolution: R = 16 spills 12 words, R = 32 32 of them.  The kernel in a
+// row of its own launches, us before (rows asked for one by one after the convolution, no spills) and now, 2 sequences: 16 heads
+// of 128 x 128 19.9, 7.6; 8 of 128 x 256 (R = 32) 45.8, 13.9; 8 of 256 x 128 (R = 32) 52.5, 13.3; 8 of 64 x 64 9.1, 6.7; 4 of 100 x 33 7.3, 5.3.
 template <int R>
 __global__ void __launch_bounds__(1024) delta_step_kernel(
     void* out, int out_bf16, const float* proj, int64_t ld, int g_off, int b_off, int a_off,

@@ -409,7 +409,7 @@ __global__ void gather_scaled_kernel(T* xp, const T* h, int64_t ldh, const int* 
 // ---------------------------------------------------------------- plan and gather of few pairs
 // Both in one launch: a block per row of the buffer finds its tile's expert and its own pair from the ids alone (every
 // block counts all of them: a few loads and shared-memory additions), copies the pair's row and leaves its place in pos.
-// An expert's pairs take its rows in their order.  A decode step pays two launches less (1 token, 4 of 32 experts
+// An expert's pairs take its rows in their order.  A decode step pays one launch instead of two (1 token, 4 of 32 experts
 // chosen, rows of 2,048: the two took 5.1 us of a step, this one 2.1; 8 tokens, weighed rows 7.1 and 3.6).
 constexpr int PLACE_PAIRS = 256;
 template <typename T>
