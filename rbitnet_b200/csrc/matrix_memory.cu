@@ -15,8 +15,8 @@
 //   memory_chunk_out_kernel   every chunk's outputs, all at once
 // Every operand, product and sum is float32 (FFMA).  The first form bounds a prompt by its chain of tokens (2,048 tokens of 8
 // heads of 128 x 256: 770 us); here the products are bound by the multiply-adds and the shared memory that feeds them, the
-// walk by the memory's bytes: gates 39, sums and scores 50,
-// walk 20, outputs 82 us (memories of 256 x 512: 1,968 us token by token, 508 in chunks).
+// walk by the memory's bytes: gates 57, sums and scores 54, walk 21, outputs 91 us, each launch by itself with cold caches; about
+// 210 with the norm in a step (memories of 256 x 512: 1,968 us token by token, 508 in chunks before the sums in groups).
 #include "rb_common.cuh"
 
 namespace {
