@@ -8,8 +8,8 @@
 // TMA brings [rows, 64] boxes of W and X with the 128-byte swizzle, which is the canonical
 // K-major layout the instruction's shared-memory descriptors name.
 //
-// Roles in a CTA of 192 threads: warp 0 issues TMA loads into a ring of stages, warp 1 owns the
-// tensor memory and issues tcgen05.mma (one lane), warps 2..5 read the accumulators back with
+// Roles in a CTA of 192 threads (320 for token tiles of 128 and more): warp 0 issues TMA loads into a ring of stages, warp 1 owns the
+// tensor memory and issues tcgen05.mma (one lane), warps 2..5 (2..9) read the accumulators back with
 // tcgen05.ld and write the result.  With token tiles of at most 64 (which the caller asks for up
 // to 256 tokens, where a product is bound by reading W) K may be cut into 2..8 parts: the CTAs
 // of a tile then form a thread-block cluster, and after their products each of them adds up a
@@ -73,6 +73,9 @@ struct QkvTail {
 template <bool BY_TMA> struct OutputMap { using type = CUtensorMap; };
 template <> struct OutputMap<false> { struct type { int none; }; };
 template <int BN, int EPI> constexpr bool leaves_by_tma() { return BN >= 128 && EPI != EPI_QKV; }
+// Tiles that leave by TMA have two groups of four epilogue warps, the others one.
+constexpr int LEAVE_GROUPS = 2, LEAVE_STAGE_BYTES = 16 * 1024;      // staging room of a group
+template <int BN, int EPI> constexpr int block_threads() { return leaves_by_tma<BN, EPI>() ? 64 + 128 * LEAVE_GROUPS : 192; }
 
 struct GemmParams {
   void* C;            // output
@@ -195,7 +198,7 @@ __device__ __forceinline__ void cluster_sync_all() {
 // for waits for nobody, all CTAs of the launch are resident (one per SM at most), and every wait is
 // bounded like the others.  The last part sets the count back to zero.
 template <int BN, int STAGES, int EPI, typename OutT, int MINB>
-__global__ void __launch_bounds__(192, MINB)
+__global__ void __launch_bounds__((block_threads<BN, EPI>()), MINB)
 gemm_wx_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX,
                const __grid_constant__ typename OutputMap<leaves_by_tma<BN, EPI>()>::type tmC, GemmParams p) {
   constexpr int X_TILE_BYTES = BN * BK * 2;
@@ -207,28 +210,38 @@ gemm_wx_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
   constexpr bool SHARED_RANGES = BN >= 128 && EPI == EPI_ADD;     // compiled in for these only
   // Token tiles of 128 and more leave through shared memory: 16 token rows of the tile at a time are
   // staged there and go out as one TMA box (stored, or added to the residual stream by the memory
-  // system), two boxes in flight.  Stores a thread makes itself have one chunk of loads or stores in
+  // system).  Stores a thread makes itself have one chunk of loads or stores in
   // flight per thread, about 8 KB an SM, and an epilogue of a 128 x 256 tile then takes longer than
-  // the products of a short tile.
+  // the products of a short tile.  What bounds the way out is the chain of a box: out of tensor memory, into
+  // shared memory, a barrier of its warps, the box read again before its room is used twice.  So two
+  // groups of four warps take every other box, each with up to four boxes in flight in its 16 KB, and the
+  // next box's values come out of tensor memory while the one before is finished.  With one group and two boxes a
+  // 128 x 256 gated tile took 19 us to leave, more than its products with K 2,048.  11,264 gated rows of 2,048, us before and
+  // now: 600 tokens 50, 30; 2,048 106, 70; 3,001 157, 106; 6,140 279, 195; 2,048 x 2,048 float32 of 3,001 tokens 43, 27.
+  // With K 4,096 the products hide either, and only a launch's last tiles show (2,048 tokens of 28,672 gated rows 343, 337).
+  // (Token tiles of 192 gave a stage of their ring for the room: 90.7 and 91.2 us for 6,144 rows of 4,096, 2,048 tokens.)
   constexpr bool TMA_EPI = leaves_by_tma<BN, EPI>();
+  constexpr int GROUPS = TMA_EPI ? LEAVE_GROUPS : 1;
   // A pending norm of the input rows and what a later norm needs (see GemmParams) are compiled for the
   // 16-token tile only, which is where a step uses them: present in the 64-token tile's kernels, asked
   // for or not, they cost each product of a batch of 64 about half a microsecond.
   constexpr bool PENDING_NORM = BN <= 16;
   constexpr int OUT_COLS = EPI == EPI_GATED ? BM / 2 : BM;          // values per token row of a staged box
-  constexpr int OUT_STAGE_BYTES = 16 * BM * 4;                      // room for 16 rows of float32
+  constexpr int BOX_BYTES = 16 * OUT_COLS * (int)sizeof(OutT);
+  constexpr int BOXES = LEAVE_STAGE_BYTES / BOX_BYTES < 4 ? LEAVE_STAGE_BYTES / BOX_BYTES : 4;
+  static_assert(BOXES >= 2, "a group's boxes alternate");
   static_assert(BN % 16 == 0 && BN >= 16 && BN <= 256, "UMMA N");
   static_assert(WANT_COLS <= 512, "tensor memory has 512 columns");
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  uint8_t* out_stage = smem + (size_t)STAGES * STAGE_BYTES;          // TMA_EPI: two boxes of OUT_STAGE_BYTES
+  uint8_t* out_stage = smem + (size_t)STAGES * STAGE_BYTES;          // TMA_EPI: LEAVE_STAGE_BYTES per group
   __shared__ uint64_t full_bar[STAGES];
   __shared__ uint64_t empty_bar[STAGES];
   __shared__ uint64_t accum_full[NBUF];
   __shared__ uint64_t accum_empty[NBUF];
   __shared__ uint32_t tmem_holder;
-  __shared__ int epi_fail;
+  __shared__ int epi_fail[2];          // per group of epilogue warps
   __shared__ float norm_r[64];         // per token: the factor of a pending norm
 
   rb_pdl_launch_dependents();     // the next kernel may be set up while this one runs
@@ -239,14 +252,14 @@ gemm_wx_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
   const int item_stride = p.cluster ? p.n_items : gridDim.x;
 
   if (threadIdx.x == 0) {
-    epi_fail = 0;
+    epi_fail[0] = epi_fail[1] = 0;
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(&full_bar[s], 1);
       mbar_init(&empty_bar[s], 1);
     }
     for (int b = 0; b < NBUF; ++b) {
       mbar_init(&accum_full[b], 1);
-      mbar_init(&accum_empty[b], 4);     // one arrival per epilogue warp
+      mbar_init(&accum_empty[b], 4 * GROUPS);     // one arrival per epilogue warp
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -397,10 +410,12 @@ gemm_wx_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
       }
     }
   } else {
-    // ------------------------------------------------------------ epilogue (warps 2..5)
+    // ------------------------------------------------------------ epilogue (warps 2..5, or 2..9)
     const int quarter = warp & 3;        // tensor-memory lanes 32*quarter .. +31 belong to this warp
     const int row = quarter * 32 + lane;
-    const bool issuer = warp == 2 && lane == 0;      // the one thread that sends the boxes of TMA_EPI
+    const int group = GROUPS > 1 ? (warp - 2) >> 2 : 0;
+    const bool issuer = ((warp - 2) & 3) == 0 && lane == 0;      // the one thread of a group that sends the boxes of TMA_EPI
+    auto group_sync = [&]() { asm volatile("bar.sync %0, 128;" ::"r"(3 + group) : "memory"); };
     rb_pdl_wait();                       // before C is read or written
     const bool normed = PENDING_NORM && p.norm_ss != nullptr;
     if (normed) {
@@ -450,23 +465,28 @@ gemm_wx_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
       if (lane == 0) ok = mbar_wait(&accum_full[b], (li / NBUF) & 1, 3);
       ok = __shfl_sync(0xffffffffu, ok, 0);
       if (TMA_EPI) {
-        // the four warps meet at barriers below: they go on together or leave together
-        if (!ok && lane == 0) epi_fail = 1;
-        asm volatile("bar.sync 3, 128;" ::: "memory");
-        ok = *(volatile int*)&epi_fail == 0;
+        // a group's four warps meet at barriers below: they go on together or leave together
+        if (!ok && lane == 0) *(volatile int*)&epi_fail[group] = 1;
+        group_sync();
+        ok = *(volatile int*)&epi_fail[group] == 0;
       }
       if (!ok) break;
       tcgen05_fence_after();
-      // columns c .. c+15 of this warp's 32 rows of the accumulator
-      auto load_acc = [&](int c, uint32_t (&r)[16]) {
+      // columns c .. c+15 of this warp's 32 rows of the accumulator: asked for, and waited for
+      auto ask_acc = [&](int c, uint32_t (&r)[16]) {
         __syncwarp();
-        if (nkb > 0) {
-          tmem_ld16(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(b * ACC_COLS + c), r);
-          tmem_ld_wait();
-        } else {
+        tmem_ld16(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(b * ACC_COLS + c), r);
+      };
+      auto have_acc = [&](uint32_t (&r)[16]) {
+        if (TMA_EPI) tmem_ld_wait16(r); else tmem_ld_wait();
+        if (nkb <= 0) {
 #pragma unroll
           for (int j = 0; j < 16; ++j) r[j] = 0u;
         }
+      };
+      auto load_acc = [&](int c, uint32_t (&r)[16]) {
+        ask_acc(c, r);
+        have_acc(r);
       };
       if (p.cluster) {
         // this split's accumulator goes to shared memory (the stage ring is idle now: every MMA
@@ -484,21 +504,25 @@ gemm_wx_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
       }
       if constexpr (TMA_EPI) {
         // A tile whose K is shared: the parts are added to C in the order of their k blocks, so this
-        // part's first box waits until the count of finished parts has reached its own number.
+        // part's first box waits until the count of finished parts has reached its own number.  (Each
+        // group counts its own boxes, which are the same ones in every part.)
         int* finished = nullptr;
         bool must_wait = false;
         if (SHARED_RANGES && s.parts > 1) {
-          finished = p.sk_finished + (int64_t)s.w_tile * p.n_t_tiles + sk_tt;
+          finished = p.sk_finished + ((int64_t)s.w_tile * p.n_t_tiles + sk_tt) * GROUPS + group;
           must_wait = s.part > 0;
         }
+        const int c_end = min(BN, p.n_tokens - t0);
+        const bool any = group * 16 < c_end;
+        uint32_t r[16];
+        if (any) load_acc(group * 16, r);
 #pragma unroll 1
-        for (int c = 0; c < BN; c += 16) {
-          if (t0 + c >= p.n_tokens) break;
-          uint32_t r[16];
-          load_acc(c, r);
+        for (int c = group * 16; c < c_end; c += 16 * GROUPS) {
+          uint32_t next[16];                               // (the last chunk asks for itself again)
+          ask_acc(c + 16 * GROUPS < c_end ? c + 16 * GROUPS : c, next);
           // The 16 token rows of the chunk go to shared memory as [token][OUT_COLS values] and leave as
           // one box; rows and columns beyond the matrix are dropped by the tensor map.
-          OutT* box = reinterpret_cast<OutT*>(out_stage + (n_boxes & 1) * OUT_STAGE_BYTES);
+          OutT* box = reinterpret_cast<OutT*>(out_stage + group * LEAVE_STAGE_BYTES + n_boxes % BOXES * BOX_BYTES);
           ++n_boxes;
           if (EPI == EPI_GATED) {
             // Lanes 0..15 hold gate rows, lanes 16..31 the up rows of the same 16 features (feature =
@@ -525,18 +549,22 @@ gemm_wx_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
             }
           }
           fence_async_shared();
-          if (issuer) bulk_wait_read_all();          // the box before this one has left its half of the staging area
-          asm volatile("bar.sync 3, 128;" ::: "memory");
+          // whoever passes the barrier may write the box that left BOXES - 1 boxes ago
+          if (issuer) bulk_wait_read<BOXES - 2>();
+          group_sync();
           if (issuer) {
             if (must_wait) {
-              if (!wait_for_count(finished, s.part, 4)) epi_fail = 1;     // noticed at the next piece; the results are void
+              if (!wait_for_count(finished, s.part, 4)) *(volatile int*)&epi_fail[group] = 1;     // noticed at the next piece; the results are void
               must_wait = false;
             }
             tma_store_2d(&tmC, box, EPI == EPI_GATED ? n0 / 2 : s.c0 + n0, t0 + c, EPI == EPI_ADD);
             bulk_commit();
           }
+          have_acc(next);
+#pragma unroll
+          for (int j = 0; j < 16; ++j) r[j] = next[j];
         }
-        if (finished != nullptr && issuer) {
+        if (finished != nullptr && issuer && any) {
           // this part is in C: count it, or, as the last part, set the count back for the next launch
           bulk_wait_all();
           asm volatile("fence.proxy.async;" ::: "memory");
@@ -880,7 +908,7 @@ thread_local int t_kernels_launched = 0;     // by this thread's product calls, 
 template <int BN, int STAGES, int EPI, typename OutT, int MINB>
 int launch(const CUtensorMap& tw, const CUtensorMap& tx, const CUtensorMap& tc, const GemmParams& p, cudaStream_t stream) {
   constexpr int stage_bytes = W_TILE_BYTES + BN * BK * 2;
-  constexpr int smem = STAGES * stage_bytes + 1024 + (BN >= 128 ? 2 * 16 * BM * 4 : 0);
+  constexpr int smem = STAGES * stage_bytes + 1024 + (leaves_by_tma<BN, EPI>() ? LEAVE_GROUPS * LEAVE_STAGE_BYTES : 0);
   static_assert(smem * MINB <= 227 * 1024, "shared memory");
   auto kernel = gemm_wx_kernel<BN, STAGES, EPI, OutT, MINB>;
   ++t_kernels_launched;
@@ -894,7 +922,7 @@ int launch(const CUtensorMap& tw, const CUtensorMap& tx, const CUtensorMap& tc, 
     // grid (splits, tiles): the CTAs of one tile are one cluster
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(p.splits, p.n_items / p.splits, 1);
-    cfg.blockDim = dim3(192, 1, 1);
+    cfg.blockDim = dim3(block_threads<BN, EPI>(), 1, 1);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
@@ -915,7 +943,7 @@ int launch(const CUtensorMap& tw, const CUtensorMap& tx, const CUtensorMap& tc, 
     RB_REQUIRE(BN >= 128 && EPI == EPI_ADD && p.n_items <= slots, "rb_gemm_tc: shared ranges with a token tile of %d, %d CTAs", BN, p.n_items);
     grid = p.n_items;                                    // one CTA per team and token tile
   }
-  RB_LAUNCH("kernel", (kernel), grid, 192, smem, stream, tw, tx, out_map, p);
+  RB_LAUNCH("kernel", (kernel), grid, (block_threads<BN, EPI>()), smem, stream, tw, tx, out_map, p);
   RB_CHECK_LAUNCH("rb_gemm_tc");
   return 0;
 }
@@ -929,7 +957,7 @@ int dispatch(int bn, const CUtensorMap& tw, const CUtensorMap& tx, const CUtenso
     case 64: return launch<64, 4, EPI, OutT, 2>(tw, tx, tc, p, stream);
     case 128: return launch<128, 6, EPI, OutT, 1>(tw, tx, tc, p, stream);
     case 160: return launch<160, 5, EPI, OutT, 1>(tw, tx, tc, p, stream);
-    case 192: return launch<192, 5, EPI, OutT, 1>(tw, tx, tc, p, stream);
+    case 192: return launch<192, 4, EPI, OutT, 1>(tw, tx, tc, p, stream);
     case 224: return launch<224, 4, EPI, OutT, 1>(tw, tx, tc, p, stream);
     case 256: return launch<256, 4, EPI, OutT, 1>(tw, tx, tc, p, stream);
   }
@@ -1019,7 +1047,7 @@ RB_EXPORT int rb_gemm_tc_splits(int n_tokens, int n_out, int K) {
 
 // ---------------------------------------------------------------- shared ranges: the plan and the counters
 namespace {
-constexpr int SK_MAX_COUNTS = 1 << 16;             // tiles whose finished parts can be counted
+constexpr int SK_MAX_COUNTS = LEAVE_GROUPS << 16;   // per tile and group of epilogue warps: finished parts
 struct SkWorkspace { void* ptr = nullptr; long long bytes = 0; };
 SkWorkspace g_sk_ws[64];
 std::mutex g_sk_mu;
@@ -1042,7 +1070,7 @@ GemmPlan plan_for_tile(int n_tokens, int n_out, int K, int bn, int sms, bool sha
   GemmPlan pl{bn, 0, 0, (int)n_t, 0.0};
   const long long rounds = (w_tiles * n_t + sms - 1) / sms;
   pl.cost = (double)rounds * item_cost(bn);
-  if (!shared_ok || bn < 128 || n_t > sms || w_tiles * n_t > SK_MAX_COUNTS) return pl;
+  if (!shared_ok || bn < 128 || n_t > sms || w_tiles * n_t > SK_MAX_COUNTS / LEAVE_GROUPS) return pl;
   const double leaving = 12.0 / nkb * bn / 256.0;
   pl.cost += leaving;
   const long long teams = sms / n_t, total = w_tiles * nkb;

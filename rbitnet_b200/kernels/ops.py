@@ -148,7 +148,7 @@ class NormedRows:
 #: freed: the library keeps its address.
 _GEMM_WORKSPACES = {}
 _GEMM_WORKSPACE_SET = set()
-_GEMM_COUNTER_BYTES = 4 << 16
+_GEMM_COUNTER_BYTES = 8 << 16
 
 
 def _give_gemm_workspace(lib, device: torch.device) -> None:
