@@ -31,6 +31,7 @@
 // memory.  The host reads the word with rb_read_error_flag().
 #include "rb_tcgen05.cuh"
 
+#include <algorithm>
 #include <mutex>
 #include <unordered_map>
 #include <string>
@@ -86,6 +87,7 @@ struct GemmParams {
   int n_features;     // EPI_GATED: output columns (W holds 32 rows, 16 gate and 16 up, per 16 of them)
   int kb_per_split;   // 64-wide k blocks per split
   int n_t_tiles;      // token tiles
+  int t_band;         // token tiles of a band: items go through all weight tiles of a band before the next band begins
   int splits;         // parts of K
   int n_items;        // weight tiles * token tiles * splits
   int cluster;        // 1: the splits of a tile form a thread-block cluster and are summed through shared memory
@@ -314,14 +316,24 @@ gemm_wx_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
     if (item >= p.n_items) return false;
     const int split = item % p.splits;
     const int tile = item / p.splits;
-    s.w_tile = tile / p.n_t_tiles;
+    int t_tile;
+    if (BN >= 128) {
+      // bands of t_band token tiles; within a band all weight tiles, the band's token tiles fastest
+      const int per_band = p.n_w_tiles * p.t_band, band = tile / per_band, in_band = tile - band * per_band;
+      const int width = min(p.t_band, p.n_t_tiles - band * p.t_band);
+      s.w_tile = in_band / width;
+      t_tile = band * p.t_band + in_band - s.w_tile * width;
+    } else {                       // (at most a few token tiles; two divisions less in a step's many small products)
+      s.w_tile = tile / p.n_t_tiles;
+      t_tile = tile % p.n_t_tiles;
+    }
     s.n0 = s.w_tile * BM;
-    s.t0 = (tile % p.n_t_tiles) * BN;
+    s.t0 = t_tile * BN;
     s.kb_begin = split * p.kb_per_split;
     s.nkb = max(0, min(nkb_total, s.kb_begin + p.kb_per_split) - s.kb_begin);
     s.w0 = s.n0;
     if (p.tile_group != nullptr) {
-      const int g = p.tile_group[tile % p.n_t_tiles];
+      const int g = p.tile_group[t_tile];
       if (g < 0) s.nkb = 0;
       else s.w0 = g * p.group_rows + s.n0;
     }
@@ -1086,6 +1098,18 @@ GemmPlan plan_for_tile(int n_tokens, int n_out, int K, int bn, int sms, bool sha
   return pl;
 }
 
+// Token tiles of a band (see piece_at): bands of equal size, of at most 16 tiles and 48 MB of X.  The CTAs that run together then
+// share fewer tiles of X and more of W: with all 32 token tiles of 8,192 tokens at once, every round of the SMs fetched 64 MB of X,
+// which the L2 no longer holds from round to round.  8,192 tokens, K 4,096, back to back: 12,288 rows 716 us, in bands of 24, 16,
+// 12, 8, 4 tiles 656, 623, 628, 635, 662; 22,016 rows gated 1,233: 1,156, 1,103, 1,122, 1,136, 1,191; K 11,008, 4,096 rows 674:
+// 640, 630, 610, 608, 616.  16 tiles and fewer are best left as one: 4,096 tokens 722, in bands of 12, 8 750, 746.
+int band_tiles(int n_t, int bn, int K) {
+  const long long tile = (long long)bn * K * 2;
+  const long long most = std::max<long long>(1, std::min<long long>(16, (48ll << 20) / tile));
+  const long long bands = (n_t + most - 1) / most;
+  return (int)((n_t + bands - 1) / bands);
+}
+
 GemmPlan plan_gemm(int n_tokens, int n_out, int K, int token_tile, int sms, bool shared_ok) {
   if (token_tile != 0) return plan_for_tile(n_tokens, n_out, K, token_tile, sms, shared_ok);
   const int bn = n_tokens <= 16 ? 16 : n_tokens <= 32 ? 32 : n_tokens <= 64 ? 64 : n_tokens <= 128 ? 128 : 256;
@@ -1389,6 +1413,7 @@ static int gemm_tc(void* C, int64_t ldc, int c_dtype, const void* X, int64_t ldx
   RB_REQUIRE(norm.out_xb == nullptr || (epilogue == EPI_ADD && p.cluster && bn <= 16),
              "rb_gemm_tc: only an added product of at most 16 tokens whose K is split into a cluster leaves a norm's inputs");
   p.n_w_tiles = n_w_tiles;
+  p.t_band = band_tiles(n_t_tiles, bn, K);
   p.sk_len = plan.sk_len;
   p.sk_finished = (int*)ws.ptr;
   if (p.sk_len > 0) {

@@ -56,3 +56,21 @@ def test_a_last_token_tile_of_few_rows(ops, tile, rest):
             assert _rel(c[:T], 1.0 + 2.0 * ref) < 2e-5 and bool((c[T:] == 1.0).all())
         finally:
             ops.lib.call("rb_gemm_tc_share_for_test", 0, launches=0)
+
+
+@pytest.mark.parametrize("T,N,K,tile", [
+    (16 * 128, 300, 72, 128), (17 * 128 + 5, 300, 72, 128),   # one band of 16 token tiles; two of 9
+    (35 * 128 - 1, 130, 72, 128),                             # three of 12, the last one narrower
+    (33 * 256, 520, 64, 256), (641, 300, 65536, 128)])        # bands held to three tiles by the size of X
+def test_token_tiles_taken_in_bands(ops, T, N, K, tile):
+    g = torch.Generator(device="cuda").manual_seed(T)
+    x = torch.randn(T, K, device="cuda", generator=g).to(BF16)
+    w = (torch.randn(N, K, device="cuda", generator=g) / math.sqrt(K)).to(BF16)
+    ref = x.double() @ w.double().T
+    c = torch.full((T, N), float("nan"), dtype=F32, device="cuda")
+    _product(ops, x, w, c, 0, tile)
+    # sums of K float32 products: their rounding grows with the square root of the k blocks
+    assert _rel(c, ref) < (2e-5 if K < 10000 else 1e-4)
+    c.zero_()
+    _product(ops, x, w, c, 1, tile)
+    assert _rel(c, ref) < (2e-5 if K < 10000 else 1e-4)
