@@ -1,31 +1,15 @@
 // Plain matrix product on the CUDA cores: C[M,N] (+)= alpha * A[M,K] * W[N,K]^T.
 //
-// This is the true 32-bit path's product (FFMA with float32 accumulation, no
-// tensor-core or reduced-precision mode) and the product for shapes that the
-// tensor-core kernel refuses.  W is row-major [out, in], the layout the
+// This is the true 32-bit path's product (FFMA with float32 accumulation; of many rows times a K of 128 and more the tensor cores
+// make it from values split without loss, see gemm_f32_tcgen05.cuh) and the product for shapes that the
+// bfloat16 tensor-core kernel refuses.  W is row-major [out, in], the layout the
 // reference indexes as w[i + o*n_in] (crates/bitnet-core/src/llama/model.rs:67-91),
 // so no weight is transposed at load.  Every sum is float32 and its order is fixed by the kernel that makes it: tiles of
 // outputs add over k in ascending order; a product of few rows adds by lanes (lane l takes every 32nd group of four values)
 // and then over the lanes, and the block's warps where they share K, in a fixed tree.
-#include "rb_common.cuh"
+#include "product_tail.cuh"
 
 namespace {
-
-// What happens to a finished sum before it is stored or added (null: nothing): bias[n] is added, and the value is
-// multiplied by sigmoid(gate[row * ldg + z * gate_batch + n * gate_step]), z the number of the product (a head); a step of
-// 0 is one gate for all of a product's values.
-struct Tail {
-  const float* bias = nullptr;
-  const float* gate = nullptr;
-  int64_t ldg = 0;
-  int64_t gate_batch = 0;
-  int gate_step = 1;
-};
-__device__ __forceinline__ float finished(const Tail& tail, float v, int64_t row, int n, int64_t z) {
-  if (tail.bias != nullptr) v += tail.bias[n];
-  if (tail.gate != nullptr) v *= 1.0f / (1.0f + expf(-tail.gate[row * tail.ldg + z * tail.gate_batch + n * tail.gate_step]));
-  return v;
-}
 
 // ---- tiles of outputs
 // 64 x 64 outputs a block of 128 threads, 8 x 4 a thread.  What bounds it is the multiply-adds and the shared memory that
@@ -407,7 +391,7 @@ RB_EXPORT int rb_per_head_few_rows(void* C, int64_t ldc, int c_dtype, const void
   return 0;
 }
 
-// Into how many parts K is cut for this product (1: not; 0: few rows, which are not made by tiles).
+// Into how many parts plain tiles cut K for this product (1: not; 0: few rows, which are not made by tiles).
 RB_EXPORT int rb_gemm_simple_parts(int M, int N, int K, int n_batch) {
   if (few_rows(M, N)) return 0;
   return tile_parts((int64_t)((N + TILE - 1) / TILE) * ((M + TILE - 1) / TILE) * n_batch, K, rb_sm_count());
@@ -453,6 +437,10 @@ RB_EXPORT int rb_gemm_simple_batched(void* C, int64_t ldc, int c_dtype, const vo
 #undef GO
 #undef ROWS
   } else {
+    const F32Plan plan = a_dtype == RB_F32 && c_dtype == RB_F32 && vec ? rb_f32_tc_plan(M, N, K, n_batch, sms) : F32Plan{0, 0};
+    if (plan.bn > 0)
+      return rb_f32_tc(F32Product{(float*)C, ldc, (const float*)A, lda, (const float*)W, ldw, M, N, K, accumulate, alpha, tail,
+                                  n_batch, batch_c, batch_a, batch_w}, plan, stream);
     const int64_t tiles_n = (N + TILE - 1) / TILE, tiles_m = (M + TILE - 1) / TILE;
     const int parts = tile_parts(tiles_n * tiles_m * n_batch, K, sms);
     RB_REQUIRE(tiles_n * tiles_m * parts <= 0x7fffffff, "rb_gemm_simple: M=%d N=%d: too large for one launch", M, N);

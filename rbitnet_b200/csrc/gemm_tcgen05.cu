@@ -221,7 +221,7 @@ gemm_wx_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
   // 128 x 256 gated tile took 19 us to leave, more than its products with K 2,048.  11,264 gated rows of 2,048, us before and
   // now: 600 tokens 50, 30; 2,048 106, 70; 3,001 157, 106; 6,140 279, 195; 2,048 x 2,048 float32 of 3,001 tokens 43, 27.
   // With K 4,096 the products hide either, and only a launch's last tiles show (2,048 tokens of 28,672 gated rows 343, 337).
-  // (Token tiles of 192 gave a stage of their ring for the room: 90.7 and 91.2 us for 6,144 rows of 4,096, 2,048 tokens.)
+  // (Token tiles of 192 gave a stage of their ring for the room.)
   constexpr bool TMA_EPI = leaves_by_tma<BN, EPI>();
   constexpr int GROUPS = TMA_EPI ? LEAVE_GROUPS : 1;
   // A pending norm of the input rows and what a later norm needs (see GemmParams) are compiled for the
@@ -826,6 +826,12 @@ gemm_wx_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
   }
 }
+
+}  // namespace
+
+#include "gemm_f32_tcgen05.cuh"
+
+namespace {
 
 // ---------------------------------------------------------------- host side
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,

@@ -2,8 +2,9 @@
 package's own CUDA kernels.
 
 ``CudaOps(dtype)`` is the only implementation on the product path.  With
-``torch.float32`` every product is a float32 FFMA sum and every activation,
-cache entry and weight is float32 (no tensor-core or reduced-precision mode).
+``torch.float32`` every product is a float32 sum (by FFMA, or on the tensor cores from values
+split into three bfloat16 parts without loss) and every activation, cache entry and weight is
+float32 (no reduced-precision mode).
 With ``torch.bfloat16`` weights, activations between kernels and the cache are
 bfloat16, while the residual stream, norms, rotation angles, softmax and all
 accumulation stay float32.

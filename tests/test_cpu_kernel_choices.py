@@ -163,6 +163,26 @@ def test_parts_of_the_float32_product(lib):
     assert parts(300, 256, 128, 16) == 1 and parts(100, 256, 128, 16) == 4 and parts(1, 1, 1, 1) == 0
 
 
+def test_float32_products_that_go_to_the_tensor_cores(lib):
+    """Enough outputs to fill the chip and a K of 128 and more, little of it padding; clusters of 1, 2 or 4 parts of whole blocks of K."""
+    import ctypes
+    out = (ctypes.c_int * 2)()
+
+    def plan(M, N, K, Z=1):
+        assert lib.raw("rb_f32_tc_plan_of")(M, N, K, Z, 148, out) == 0
+        return tuple(out)
+    for M in (17, 33, 64, 130, 300, 2048, 8192):
+        for N in (1, 64, 96, 256, 2048, 5000, 30000):
+            for K in (4, 64, 128, 260, 512, 2048, 11008):
+                for Z in (1, 16):
+                    bn, parts = plan(M, N, K, Z)
+                    assert (bn, parts) == (0, 0) or (bn in (64, 128) and parts in (1, 2, 4) and parts <= -(-K // 64)), (M, N, K, Z)
+                    if K < 128 or -(-N // 64) * -(-M // 64) * Z < 16:
+                        assert bn == 0, (M, N, K, Z)
+    assert plan(64, 2048, 2048) == (64, 4) and plan(600, 11264, 2048) == (128, 1) and plan(2048, 4096, 14336) == (128, 2)
+    assert plan(4000, 64, 256, 64) == (0, 0) and plan(2048, 128, 128, 16) == (128, 1) and plan(300, 512, 192) == (0, 0)
+
+
 def test_when_a_matrix_memory_goes_in_chunks():
     """The longest run decides where the runs are few, not their average; small memories and short runs stay token by token."""
     from rbitnet_b200.kernels.ops import memory_chunks_pay

@@ -74,3 +74,89 @@ def test_token_tiles_taken_in_bands(ops, T, N, K, tile):
     c.zero_()
     _product(ops, x, w, c, 1, tile)
     assert _rel(c, ref) < (2e-5 if K < 10000 else 1e-4)
+
+
+# ---------------------------------------------------------------- float32 products of values in three bfloat16 parts
+@pytest.fixture(scope="module")
+def ops32():
+    from rbitnet_b200.kernels.ops import CudaOps
+    return CudaOps(F32, verbose_build=False)
+
+
+def _f32(ops32, x, w, out, accumulate=0, alpha=1.0, batch=1, strides=(0, 0, 0), bias=None, gate=None, want=True):
+    import ctypes
+    from ctypes import c_void_p
+    from rbitnet_b200.kernels.ops import _ptr
+    (M, K), N = (x.shape[0], w.shape[-1]), w.shape[-2]
+    plan = (ctypes.c_int * 2)()
+    ops32.lib.call("rb_f32_tc_plan_of", M, N, K, batch, ops32.lib.raw("rb_device_sm_count")(), plan, launches=0)
+    assert (plan[0] > 0) == want, "these sizes were chosen for the one or the other"
+    if bias is not None or gate is not None:
+        ops32.lib.call("rb_gemm_simple_next", _ptr(bias), _ptr(gate), gate.stride(0) if gate is not None else 0, 0, 1, launches=0)
+    ops32.lib.call("rb_gemm_simple_batched", _ptr(out), out.stride(0), 0, _ptr(x), x.stride(0), _ptr(w), w.stride(-2), 0, M, N, K,
+                   accumulate, float(alpha), batch, *strides, ops32._stream())
+    ops32.check_errors()
+    return plan[0], plan[1]
+
+
+@pytest.mark.parametrize("M,N,K", [(1000, 130, 516), (65, 1000, 2052), (129, 2048, 128), (333, 2500, 132), (600, 2048, 2048),
+                                   (2049, 384, 260), (64, 2048, 5632), (700, 3001, 1028), (300, 300, 1000)])
+def test_float32_products_from_three_parts(ops32, M, N, K):
+    """Rows, weight rows and values of K that fill no tile; K whole and in parts; stored, added, scaled, with bias and gate; rows
+    wider than K.  Per block of 64 values of K the tensor cores cut off at most 68 times 2^-24 of the magnitudes' sum (four sums
+    of 17 values each), adding the blocks rounds once each, and the dropped products of parts are below 2^-25 of theirs."""
+    g = torch.Generator(device="cuda").manual_seed(M)
+    x = torch.randn(M, K + 4, device="cuda", generator=g)[:, :K]
+    w = torch.randn(N, K + 8, device="cuda", generator=g)[:, :K]
+    ref, mag = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    bound = (72 + -(-K // 64)) * 2.0 ** -24 * mag
+    out = torch.full((M + 2, N), 5.0, device="cuda")
+    _f32(ops32, x, w, out[:M])
+    assert ((out[:M].double() - ref).abs() <= bound).all() and bool((out[M:] == 5.0).all())
+    plain = torch.empty((M, N), device="cuda")                 # rows without 16-byte loads: the FFMA tiles
+    x1 = torch.empty(M * (K + 1), device="cuda").view(M, K + 1)[:, 1:].copy_(x)
+    _f32(ops32, x1, w, plain)
+    assert (out[:M].double() - ref).norm() <= (plain.double() - ref).norm()
+    bias, gate = torch.randn(N, device="cuda", generator=g), torch.randn(M, N, device="cuda", generator=g)
+    acc = torch.ones((M, N), device="cuda")
+    _f32(ops32, x, w, acc, accumulate=1, alpha=0.5, bias=bias, gate=gate)
+    s = torch.sigmoid(gate.double())
+    want = 1.0 + (0.5 * ref + bias.double()) * s
+    assert ((acc.double() - want).abs() <= bound + 2.0 ** -21 * (want.abs() + 1.0 + bias.double().abs())).all()
+
+
+def test_float32_products_of_blocks_from_three_parts(ops32):
+    """Sixteen products at once, a fixed distance apart."""
+    g = torch.Generator(device="cuda").manual_seed(5)
+    Z, M, N, K = 16, 333, 128, 128
+    x = torch.randn(M, Z * K, device="cuda", generator=g)
+    w = torch.randn(Z, N, K, device="cuda", generator=g)
+    out = torch.empty(M, Z * N, device="cuda")
+    _f32(ops32, x[:, :K], w[0], out, batch=Z, strides=(N, K, N * K))
+    a = x.double().view(M, Z, K)
+    ref = torch.einsum("mzk,znk->mzn", a, w.double()).reshape(M, Z * N)
+    mag = torch.einsum("mzk,znk->mzn", a.abs(), w.double().abs()).reshape(M, Z * N)
+    assert ((out.double() - ref).abs() <= 74 * 2.0 ** -24 * mag).all()
+
+
+@pytest.mark.parametrize("K", [512, 2048])
+def test_float32_products_that_are_not_finite(ops32, K):
+    """Infinities, NaN, values above the largest bfloat16 and very small ones leave what float32 sums leave."""
+    g = torch.Generator(device="cuda").manual_seed(6)
+    M, N = 128, 1024
+    x = torch.randn(M, K, device="cuda", generator=g)
+    w = torch.randn(N, K, device="cuda", generator=g)
+    x[3, 7], x[5, 9], x[70, 1], w[100, 2] = float("inf"), float("nan"), float("-inf"), float("inf")
+    w[101, 2] = 0.0
+    x[3, 2] = 1.0
+    x[9] = 0.0
+    x[9, 0], w[:, 0] = 3.4e38, w[:, 0].clamp(-0.9, 0.9)         # rounds to infinity as a bfloat16
+    x[10] *= 1e-30
+    out = torch.empty(M, N, device="cuda")
+    _f32(ops32, x, w, out)
+    ref = x.double() @ w.double().T
+    assert torch.equal(torch.isnan(out), torch.isnan(ref))
+    assert torch.equal(torch.isposinf(out), torch.isposinf(ref)) and torch.equal(torch.isneginf(out), torch.isneginf(ref))
+    fin = torch.isfinite(ref)
+    mag = torch.where(torch.isfinite(x), x, 0).double().abs() @ torch.where(torch.isfinite(w), w, 0).double().abs().T
+    assert ((out.double() - ref).abs()[fin] <= ((K + 8) * 2.0 ** -24 * mag)[fin]).all()      # (K: the sums made by FFMA)
