@@ -164,7 +164,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
   float* row_max = reinterpret_cast<float*>(smem + S::OFF_MAX);
 
   rb_pdl_launch_dependents();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, role = rb_uniform_warp();
   // late tiles see the most keys: CTAs start in the order (tile descending, kv head), so the long
   // ones of every kv head run first and the short ones fill the end
   const int tile = p.n_tiles - 1 - (int)blockIdx.y;
@@ -254,94 +254,108 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
     tcgen05_fence_after();
   }
 
-  if (warp == 0) {
+  if (role == 0) {
     // ------------------------------------------------------------ TMA loader
-    if (lane == 0) {
-      for (int kt = kt_begin, j = 0; kt < kt_end; ++kt, ++j) {
-        const int s = j % KV_STAGES;
-        const uint32_t ph = ((j / KV_STAGES) & 1) ^ 1;
-        int row[TILE_KEYS / PIECE];
+    int s = 0;
+    uint32_t ph = 1;
+    for (int kt = kt_begin; kt < kt_end; ++kt) {
+      int row[TILE_KEYS / PIECE];
 #pragma unroll
-        for (int h = 0; h < TILE_KEYS / PIECE; ++h) {      // a tile is two pieces of 64 positions
-          const int key0 = tile_of(kt) * TILE_KEYS + h * PIECE;
-          const int pi = min(key0 / p.page_size, p.max_pages - 1);       // past the sequence: any page, masked later
-          const int page = p.page_table[(int64_t)slot * p.max_pages + pi];
-          row[h] = (page * p.n_kv_heads + kvh) * p.page_size + key0 % p.page_size;
-        }
-        if (!mbar_wait(SHARED ? &v_empty[s] : &k_empty[s], ph, 5)) break;
+      for (int h = 0; h < TILE_KEYS / PIECE; ++h) {      // a tile is two pieces of 64 positions
+        const int key0 = tile_of(kt) * TILE_KEYS + h * PIECE;
+        const int pi = min(key0 / p.page_size, p.max_pages - 1);       // past the sequence: any page, masked later
+        const int page = p.page_table[(int64_t)slot * p.max_pages + pi];
+        row[h] = (page * p.n_kv_heads + kvh) * p.page_size + key0 % p.page_size;
+      }
+      if (!mbar_wait_warp(SHARED ? &v_empty[s] : &k_empty[s], ph, 5)) break;
+      if (elect_one()) {
         mbar_expect_tx(&k_full[s], S::KV_TILE_BYTES);
 #pragma unroll
         for (int b = 0; b < DB; ++b)
 #pragma unroll
           for (int h = 0; h < TILE_KEYS / PIECE; ++h)
             tma_load_2d(smem + S::OFF_K + s * S::KV_TILE_BYTES + b * S::BLOCK + h * (PIECE * 128), &tmK, b * 64, row[h], &k_full[s]);
-        if (SHARED) continue;
-        if (!mbar_wait(&v_empty[s], ph, 5)) break;
-        mbar_expect_tx(&v_full[s], S::KV_TILE_BYTES);
-#pragma unroll
-        for (int b = 0; b < DB; ++b)
-#pragma unroll
-          for (int h = 0; h < TILE_KEYS / PIECE; ++h)
-            tma_load_2d(smem + S::OFF_V + s * S::KV_TILE_BYTES + b * S::BLOCK + h * (PIECE * 128), &tmV, b * 64, row[h], &v_full[s]);
       }
+      __syncwarp();
+      if (!SHARED) {
+        if (!mbar_wait_warp(&v_empty[s], ph, 5)) break;
+        if (elect_one()) {
+          mbar_expect_tx(&v_full[s], S::KV_TILE_BYTES);
+#pragma unroll
+          for (int b = 0; b < DB; ++b)
+#pragma unroll
+            for (int h = 0; h < TILE_KEYS / PIECE; ++h)
+              tma_load_2d(smem + S::OFF_V + s * S::KV_TILE_BYTES + b * S::BLOCK + h * (PIECE * 128), &tmV, b * 64, row[h], &v_full[s]);
+        }
+        __syncwarp();
+      }
+      if (++s == KV_STAGES) { s = 0; ph ^= 1; }
     }
-  } else if (warp == 1) {
+  } else if (role == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      constexpr uint32_t idesc_s = make_idesc_mn(ROWS, TILE_KEYS, 0, 0);   // Q (K-major) x K (K-major)
-      constexpr uint32_t idesc_o = make_idesc_mn(ROWS, D, 0, 1);           // P (K-major) x V (D contiguous)
-      bool ok = true;
-      const int n_tiles = kt_end - kt_begin;
-      // S of tile j goes to S buffer j & 1.  S(j+1) is issued before P V (j), so the tensor cores
-      // work on the next tile's scores while the softmax of this tile runs.
-      auto issue_s = [&](int j) -> bool {
-        const int s = j % KV_STAGES;
-        if (!mbar_wait(&k_full[s], (j / KV_STAGES) & 1, 6)) return false;
-        tcgen05_fence_after();
-        const uint32_t k_addr = smem_u32(smem + S::OFF_K + s * S::KV_TILE_BYTES);
+    constexpr uint32_t idesc_s = make_idesc_mn(ROWS, TILE_KEYS, 0, 0);   // Q (K-major) x K (K-major)
+    constexpr uint32_t idesc_o = make_idesc_mn(ROWS, D, 0, 1);           // P (K-major) x V (D contiguous)
+    const uint64_t dq0 = smem_desc_sw128(smem_u32(smem + S::OFF_Q)), dk0 = smem_desc_sw128(smem_u32(smem + S::OFF_K));
+    const uint64_t dv0 = smem_desc_sw128_mn(smem_u32(smem + S::OFF_V), S::BLOCK);
+    bool ok = true;
+    const int n_tiles = kt_end - kt_begin;
+    // S of tile j goes to S buffer j & 1.  S(j+1) is issued before P V (j), so the tensor cores
+    // work on the next tile's scores while the softmax of this tile runs.
+    int s_stage = 0, v_stage = 0;             // the next tile's stage of keys, of values
+    uint32_t s_phase = 0, v_phase = 0;
+    auto issue_s = [&](int j) -> bool {
+      if (!mbar_wait_warp(&k_full[s_stage], s_phase, 6)) return false;
+      tcgen05_fence_after();
+      const uint64_t dk = dk0 + (uint64_t)(s_stage * (S::KV_TILE_BYTES >> 4));
+      const uint32_t to = tmem_base + (uint32_t)((j & 1) * TILE_KEYS);
+      if (elect_one()) {
 #pragma unroll
         for (int b = 0; b < DB; ++b)
 #pragma unroll
           for (int k4 = 0; k4 < 4; ++k4) {
-            const uint64_t koff = (uint64_t)(k4 * 32 >> 4);
+            const uint64_t off = (uint64_t)(b * (S::BLOCK >> 4) + (k4 * 32 >> 4));
             // A: 16 values of Q = 8 columns of tensor memory; B: the keys' 16 values of block b
             if (Q_SMEM)
-              umma_bf16(tmem_base + (uint32_t)((j & 1) * TILE_KEYS), smem_desc_sw128(smem_u32(smem + S::OFF_Q) + b * S::BLOCK) + koff,
-                        smem_desc_sw128(k_addr + b * S::BLOCK) + koff, idesc_s, (b > 0 || k4 > 0) ? 1u : 0u);
+              umma_bf16(to, dq0 + off, dk + off, idesc_s, (b > 0 || k4 > 0) ? 1u : 0u);
             else
-              umma_bf16_ts(tmem_base + (uint32_t)((j & 1) * TILE_KEYS), tmem_base + (uint32_t)(Q_COL + b * 32 + k4 * 8),
-                         smem_desc_sw128(k_addr + b * S::BLOCK) + koff, idesc_s, (b > 0 || k4 > 0) ? 1u : 0u);
+              umma_bf16_ts(to, tmem_base + (uint32_t)(Q_COL + b * 32 + k4 * 8), dk + off, idesc_s, (b > 0 || k4 > 0) ? 1u : 0u);
           }
         tcgen05_commit(&s_full[j & 1]);
-        if (!SHARED) tcgen05_commit(&k_empty[s]);
-        return true;
-      };
-      if (n_tiles > 0) ok = issue_s(0);
-      for (int j = 0; j < n_tiles && ok; ++j) {
-        // (SHARED with few stages: where the next tile has not landed yet, this tile's P V goes first)
-        const bool first = !SHARED || j + 1 >= n_tiles || mbar_try_wait(&k_full[(j + 1) % KV_STAGES], ((j + 1) / KV_STAGES) & 1, 0u);
-        if (j + 1 < n_tiles && first) ok = issue_s(j + 1);
-        if (!ok) break;
-        const int s = j % KV_STAGES;
-        ok = mbar_wait(p_full, j & 1, 7);                    // P of this tile is in tensor memory
-        if (!ok) break;
-        if (!SHARED) ok = mbar_wait(&v_full[s], (j / KV_STAGES) & 1, 6);
-        if (!ok) break;
-        tcgen05_fence_after();
-        const uint32_t v_addr = smem_u32(smem + S::OFF_V + s * S::KV_TILE_BYTES);
+        if (!SHARED) tcgen05_commit(&k_empty[s_stage]);
+      }
+      __syncwarp();
+      if (++s_stage == KV_STAGES) { s_stage = 0; s_phase ^= 1; }
+      return true;
+    };
+    if (n_tiles > 0) ok = issue_s(0);
+    for (int j = 0; j < n_tiles && ok; ++j) {
+      // (SHARED with few stages: where the next tile has not landed yet, this tile's P V goes first)
+      const bool first = !SHARED || j + 1 >= n_tiles || __all_sync(0xffffffffu, mbar_try_wait(&k_full[s_stage], s_phase, 0u));
+      if (j + 1 < n_tiles && first) ok = issue_s(j + 1);
+      if (!ok) break;
+      ok = mbar_wait_warp(p_full, j & 1, 7);                    // P of this tile is in tensor memory
+      if (!ok) break;
+      if (!SHARED) ok = mbar_wait_warp(&v_full[v_stage], v_phase, 6);
+      if (!ok) break;
+      tcgen05_fence_after();
+      const uint64_t dv = dv0 + (uint64_t)(v_stage * (S::KV_TILE_BYTES >> 4));
+      if (elect_one()) {
 #pragma unroll
         for (int k16 = 0; k16 < TILE_KEYS / 16; ++k16) {
           // A: 16 keys of P = 8 columns of tensor memory, in place of the S buffer of this tile;
           // B: 16 key rows of V (2048 bytes further per step), all D columns: 64-column blocks S::BLOCK apart
           umma_bf16_ts(tmem_base + O_COL, tmem_base + (uint32_t)((j & 1) * TILE_KEYS + k16 * 8),
-                       smem_desc_sw128_mn(v_addr + k16 * 2048, S::BLOCK), idesc_o, (j > 0 || k16 > 0) ? 1u : 0u);
+                       dv + (uint64_t)(k16 * (2048 >> 4)), idesc_o, (j > 0 || k16 > 0) ? 1u : 0u);
         }
-        tcgen05_commit(&v_empty[s]);
+        tcgen05_commit(&v_empty[v_stage]);
         tcgen05_commit(pv_done);
-        if (!first) ok = issue_s(j + 1);
       }
-      tcgen05_commit(o_full);
+      __syncwarp();
+      if (++v_stage == KV_STAGES) { v_stage = 0; v_phase ^= 1; }
+      if (!first) ok = issue_s(j + 1);
     }
+    if (elect_one()) tcgen05_commit(o_full);
+    __syncwarp();
   } else {
     // ------------------------------------------------------------ softmax and output (warps 2..9)
     // Two threads per row: thread (quarter, lane, half) owns row quarter*32 + lane, the 64 keys

@@ -16,9 +16,9 @@
 // values into registers a block ahead, split them, write the parts into the swizzled operand tiles of one of two stages
 // (the planes of a side one below the other, so one instruction reaches two of them: four instructions per 16 values of K) and add up the
 // blocks' sums; one thread issues the products.
-// What bounds it is shared memory: the products' operands and the splitting's stores and loads take 3,000 of a block's 3,500 to
-// 4,000 cycles, the products' arithmetic 1,536.  2,048 x 11,264 outputs with K 2,048: 704 us, 134 TFLOP/s of float32 (FFMA tiles
-// 2,185 us, 43); 2,048 x 4,096 with K 14,336 1,562 (5,500); 600 x 2,048 with K 2,048 70 (146).  Relative error against float64
+// What bounds it is shared memory: the products' operands and the splitting's stores and loads take about 3,000 of a block's 3,300 to
+// 4,000 cycles, the products' arithmetic 1,536.  2,048 x 11,264 outputs with K 2,048: 680 us, 139 TFLOP/s of float32 (FFMA tiles
+// 2,185 us, 43); 2,048 x 4,096 with K 14,336 1,520 (5,500); 600 x 2,048 with K 2,048 69 (146).  Relative error against float64
 // (root mean square): K 128 7.5e-8 (FFMA tiles 2.0e-7), 2,048 1.3e-7 (8.1e-7), 14,336 2.1e-7 (1.5e-6).
 // (Eight warps of twice the values: 987 us for the first, latencies show; all of an accumulator's products in a row: 766.)
 // K in parts: the CTAs of a tile form a cluster, each adds up a share of the token columns from all parts, in order of k.
@@ -65,6 +65,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_kernel(const F32Product p
   __shared__ uint32_t tmem_holder;
   rb_pdl_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const bool issuing = rb_uniform_warp() == 0;
   const int64_t z = blockIdx.z;
   const float* A = p.A + z * p.batch_a;
   const float* W = p.W + z * p.batch_w;
@@ -146,24 +147,27 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_kernel(const F32Product p
     if (lane == 0) mbar_arrive(&full_bar[block & 1]);
   };
   bool ok = true;
-  // one thread issues a block's products once all warps have put their rows
+  // the first warp issues a block's products once all warps have put their rows
+  constexpr uint32_t one = make_idesc(BN), two = make_idesc(2 * BN);
+  constexpr uint64_t K_STEP = UMMA_K * 2 >> 4;
+  const uint64_t first_stage = smem_desc_sw128(smem_u32(smem));
   auto issue = [&](int b) {
-    constexpr uint32_t one = make_idesc(BN), two = make_idesc(2 * BN);
-    constexpr uint64_t K_STEP = UMMA_K * 2 >> 4;
-    if (!mbar_wait(&full_bar[b & 1], (b >> 1) & 1, 2)) return;        // (noticed by everybody's wait for these products)
+    if (!mbar_wait_warp(&full_bar[b & 1], (b >> 1) & 1, 2)) return;        // (noticed by everybody's wait for these products)
     tcgen05_fence_after();
-    const uint32_t stage = smem_u32(smem + (b & 1) * stage_bytes<BN>());
-    const uint32_t hh = tmem_base + (uint32_t)((b & 1) * BN), low = tmem_base + 2 * BN, lowest = tmem_base + 3 * BN;
-    const uint64_t w_h = smem_desc_sw128(stage), w_m = smem_desc_sw128(stage + BM * 128), w_l = smem_desc_sw128(stage + 2 * BM * 128);
-    const uint64_t x_h = smem_desc_sw128(stage + 3 * BM * 128), x_m = smem_desc_sw128(stage + 3 * BM * 128 + BN * 128);
+    const uint32_t hh = tmem_base + (uint32_t)((b & 1) * BN), low = tmem_base + 2 * BN;
+    const uint64_t w_h = first_stage + (uint64_t)((b & 1) * (stage_bytes<BN>() >> 4)), w_m = w_h + (BM * 128 >> 4), w_l = w_m + (BM * 128 >> 4);
+    const uint64_t x_h = w_l + (BM * 128 >> 4), x_m = x_h + (BN * 128 >> 4);
+    if (elect_one()) {
 #pragma unroll
-    for (int k4 = 0; k4 < BK / UMMA_K; ++k4) {
-      umma_bf16(hh, w_h + k4 * K_STEP, x_h + k4 * K_STEP, one, k4 > 0 ? 1u : 0u);
-      umma_bf16(low, w_h + k4 * K_STEP, x_m + k4 * K_STEP, two, b > 0 || k4 > 0 ? 1u : 0u);      // hm and hl
-      umma_bf16(low, w_m + k4 * K_STEP, x_h + k4 * K_STEP, two, 1u);                             // mh and mm
-      umma_bf16(lowest, w_l + k4 * K_STEP, x_h + k4 * K_STEP, one, 1u);                          // lh
+      for (int k4 = 0; k4 < BK / UMMA_K; ++k4) {
+        umma_bf16(hh, w_h + k4 * K_STEP, x_h + k4 * K_STEP, one, k4 > 0 ? 1u : 0u);
+        umma_bf16(low, w_h + k4 * K_STEP, x_m + k4 * K_STEP, two, b > 0 || k4 > 0 ? 1u : 0u);      // hm and hl
+        umma_bf16(low, w_m + k4 * K_STEP, x_h + k4 * K_STEP, two, 1u);                             // mh and mm
+        umma_bf16(low + BN, w_l + k4 * K_STEP, x_h + k4 * K_STEP, one, 1u);                        // lh
+      }
+      tcgen05_commit(&done_bar[b & 1]);
     }
-    tcgen05_commit(&done_bar[b & 1]);
+    __syncwarp();
   };
   const int quarter = warp & 3, c0 = (warp >> 2) * COLS;
   const uint32_t lanes = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)c0;
@@ -176,11 +180,11 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_kernel(const F32Product p
 #pragma unroll
   for (int i = 0; i < X_ROWS; ++i) x[i] = *reinterpret_cast<const float4*>(from_x[i] + k_of(0));
   put(0);
-  if (threadIdx.x == 0) issue(0);
+  if (issuing) issue(0);
   for (int b = 0; ok && b < n_blocks; ++b) {
     if (b + 1 < n_blocks) {
       put(b + 1);                                         // the products of block b - 1, which read that stage, are done
-      if (threadIdx.x == 0) issue(b + 1);
+      if (issuing) issue(b + 1);
     }
     ok = mbar_wait(&done_bar[b & 1], (b >> 1) & 1, 3);
     ok = __all_sync(0xffffffffu, ok);

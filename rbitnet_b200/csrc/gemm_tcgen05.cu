@@ -247,7 +247,7 @@ gemm_wx_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
   __shared__ float norm_r[64];         // per token: the factor of a pending norm
 
   rb_pdl_launch_dependents();     // the next kernel may be set up while this one runs
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, role = rb_uniform_warp();
   const int nkb_total = (p.K + BK - 1) / BK;
   // cluster mode: grid (splits, tiles), one item per CTA, blockIdx.x is the split and the cluster rank
   const int first_item = blockIdx.y * p.splits + blockIdx.x;
@@ -349,77 +349,77 @@ gemm_wx_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
     return true;
   };
 
-  if (warp == 0) {
+  if (role == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
-      uint32_t it = 0;
-      bool ok = true;
-      // the first piece's first stages: W before the wait, X after it
-      int early = 0;
-      Piece s;
-      if (piece_at(0, s)) {
-        early = min(s.nkb, STAGES);
+    bool ok = true;
+    int st = 0;
+    uint32_t phase = 1;                 // of the wait for a free stage: the first round waits for nobody
+    // the first piece's first stages: W before the wait, X after it
+    int early = 0;
+    Piece s;
+    if (piece_at(0, s)) {
+      early = min(s.nkb, STAGES);
+      if (elect_one())
         for (int i = 0; i < early; ++i) {
-          uint8_t* stage = smem + (size_t)i * STAGE_BYTES;
           mbar_expect_tx(&full_bar[i], STAGE_BYTES);
-          const int k = (s.kb_begin + i) * BK;
-          tma_load_2d(stage, &tmW, k, s.w0, &full_bar[i]);
+          tma_load_2d(smem + (size_t)i * STAGE_BYTES, &tmW, (s.kb_begin + i) * BK, s.w0, &full_bar[i]);
         }
-        rb_pdl_wait();
-        for (int i = 0; i < early; ++i) {
-          uint8_t* stage = smem + (size_t)i * STAGE_BYTES;
-          tma_load_2d(stage + W_TILE_BYTES, &tmX, s.x0 + (s.kb_begin + i) * BK, s.t0, &full_bar[i]);
-        }
-      }
-      for (int li = 0; ok && piece_at(li, s); ++li) {
-        int i = 0;
-        if (li == 0) { i = early; it = early; }
-        for (; i < s.nkb; ++i, ++it) {
-          const int st = it % STAGES;
-          const uint32_t phase = (it / STAGES) & 1;
-          ok = mbar_wait(&empty_bar[st], phase ^ 1, 1);
-          if (!ok) break;
-          uint8_t* stage = smem + (size_t)st * STAGE_BYTES;
+      __syncwarp();
+      rb_pdl_wait();
+      if (elect_one())
+        for (int i = 0; i < early; ++i)
+          tma_load_2d(smem + (size_t)i * STAGE_BYTES + W_TILE_BYTES, &tmX, s.x0 + (s.kb_begin + i) * BK, s.t0, &full_bar[i]);
+      __syncwarp();
+      if (early == STAGES) phase = 0; else st = early;
+    }
+    for (int li = 0; ok && piece_at(li, s); ++li) {
+      for (int i = li == 0 ? early : 0; i < s.nkb; ++i) {
+        ok = mbar_wait_warp(&empty_bar[st], phase, 1);
+        if (!ok) break;
+        uint8_t* stage = smem + (size_t)st * STAGE_BYTES;
+        const int k = (s.kb_begin + i) * BK;
+        if (elect_one()) {
           mbar_expect_tx(&full_bar[st], STAGE_BYTES);
-          const int k = (s.kb_begin + i) * BK;
           tma_load_2d(stage, &tmW, k, s.w0, &full_bar[st]);
           tma_load_2d(stage + W_TILE_BYTES, &tmX, s.x0 + k, s.t0, &full_bar[st]);
         }
+        __syncwarp();
+        if (++st == STAGES) { st = 0; phase ^= 1; }
       }
     }
-  } else if (warp == 1) {
+  } else if (role == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      constexpr uint32_t idesc = make_idesc(BN);
-      uint32_t it = 0;
-      bool ok = true;
-      Piece s;
-      for (int li = 0; ok && piece_at(li, s); ++li) {
-        const int nkb = s.nkb;
-        const int b = li % NBUF;
-        ok = mbar_wait(&accum_empty[b], ((li / NBUF) & 1) ^ 1, 4);    // the epilogue has drained this accumulator
+    constexpr uint32_t idesc = make_idesc(BN);
+    const uint64_t dw0 = smem_desc_sw128(smem_u32(smem)), dx0 = smem_desc_sw128(smem_u32(smem) + W_TILE_BYTES);
+    bool ok = true;
+    int st = 0;
+    uint32_t phase = 0;
+    Piece s;
+    for (int li = 0; ok && piece_at(li, s); ++li) {
+      const int nkb = s.nkb;
+      const int b = li % NBUF;
+      ok = mbar_wait_warp(&accum_empty[b], ((li / NBUF) & 1) ^ 1, 4);    // the epilogue has drained this accumulator
+      if (!ok) break;
+      tcgen05_fence_after();
+      const uint32_t acc_addr = tmem_base + (uint32_t)(b * ACC_COLS);
+      for (int i = 0; i < nkb; ++i) {
+        ok = mbar_wait_warp(&full_bar[st], phase, 2);
         if (!ok) break;
         tcgen05_fence_after();
-        const uint32_t acc_addr = tmem_base + (uint32_t)(b * ACC_COLS);
-        for (int i = 0; i < nkb; ++i, ++it) {
-          const int s = it % STAGES;
-          const uint32_t phase = (it / STAGES) & 1;
-          ok = mbar_wait(&full_bar[s], phase, 2);
-          if (!ok) break;
-          tcgen05_fence_after();
-          const uint32_t stage = smem_u32(smem + (size_t)s * STAGE_BYTES);
-          const uint64_t dw = smem_desc_sw128(stage);
-          const uint64_t dx = smem_desc_sw128(stage + W_TILE_BYTES);
+        const uint64_t dw = dw0 + (uint64_t)(st * (STAGE_BYTES >> 4)), dx = dx0 + (uint64_t)(st * (STAGE_BYTES >> 4));
+        if (elect_one()) {
 #pragma unroll
           for (int k4 = 0; k4 < BK / UMMA_K; ++k4) {
-            const uint32_t acc = (i > 0 || k4 > 0) ? 1u : 0u;
             const uint64_t koff = (uint64_t)(k4 * UMMA_K * 2 >> 4);
-            umma_bf16(acc_addr, dw + koff, dx + koff, idesc, acc);
+            umma_bf16(acc_addr, dw + koff, dx + koff, idesc, i > 0 || k4 > 0 ? 1u : 0u);
           }
-          tcgen05_commit(&empty_bar[s]);   // frees the stage when these MMAs have read it
+          tcgen05_commit(&empty_bar[st]);   // frees the stage when these MMAs have read it
         }
-        tcgen05_commit(&accum_full[b]);    // this item's accumulator is complete
+        __syncwarp();
+        if (++st == STAGES) { st = 0; phase ^= 1; }
       }
+      if (elect_one()) tcgen05_commit(&accum_full[b]);    // this item's accumulator is complete
+      __syncwarp();
     }
   } else {
     // ------------------------------------------------------------ epilogue (warps 2..5, or 2..9)

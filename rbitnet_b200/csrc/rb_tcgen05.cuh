@@ -87,6 +87,31 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int co
     }
   }
 }
+// ---- a warp that issues.  One lane of it issues the loads or products, but the warp stays together around that: what a single lane
+// computes behind a branch the compiler takes for different in every lane, and it then moves each address and descriptor into
+// the uniform registers these instructions read, value by value.  A block of K of a product of 16 or 64 tokens (four tcgen05.mma)
+// cost 0.305 us with issuing lanes, loads or no loads, and 0.235 with issuing warps (W from L2, K 16,384, one CTA).
+__device__ __forceinline__ int rb_uniform_warp() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+// true in one lane of the warp
+__device__ __forceinline__ bool elect_one() {
+  uint32_t one;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
+  return one != 0;
+}
+// mbar_wait by a whole warp; the same answer in every lane.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, int code, uint64_t limit_ns = 2000000000ull) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  const uint64_t t0 = global_timer_ns();
+  for (;;) {
+#pragma unroll 1
+    for (int i = 0; i < 1024; ++i)
+      if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    if (__any_sync(0xffffffffu, global_timer_ns() - t0 > limit_ns)) {
+      atomicCAS(&g_error_flag, 0, code);
+      return false;
+    }
+  }
+}
 // Bounded wait for a word in global memory to reach `value` (another CTA of the same launch stores
 // it with release): false, and the error word set to `code`, after `limit_ns`.
 __device__ __forceinline__ bool wait_for_count(const int* word, int value, int code, uint64_t limit_ns = 2000000000ull) {
