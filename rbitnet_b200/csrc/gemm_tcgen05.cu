@@ -276,7 +276,16 @@ gemm_wx_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
   __syncthreads();
   tcgen05_fence_after();
   const uint32_t tmem_base = tmem_holder;
-  if (p.tile_group != nullptr) rb_pdl_wait();      // the tiles' groups are data of the kernel before this one
+  // Grouped rows of small tiles: the tiles' groups are data of the kernel before this one.  Tiles with rows come before those
+  // without, so the items of the former go first, and the CTAs share them out evenly: taken as they lie, 21 of 32 tiles gave a
+  // third of the CTAs three of them and another third one.
+  int n_filled = 0;
+  if (p.tile_group != nullptr) {
+    rb_pdl_wait();
+    if (BN < 128)
+      for (int i = 0; i < p.n_t_tiles; i += blockDim.x)
+        n_filled += __syncthreads_count(i + (int)threadIdx.x < p.n_t_tiles && p.tile_group[i + (int)threadIdx.x] >= 0);
+  }
   // Barriers and tensor memory are ready.  Whoever touches memory that an earlier kernel may
   // still be writing or reading calls rb_pdl_wait() first: the loader before it loads X, the
   // epilogue warps before they touch C.  W is never written, so its first tiles are requested
@@ -323,6 +332,10 @@ gemm_wx_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
       const int width = min(p.t_band, p.n_t_tiles - band * p.t_band);
       s.w_tile = in_band / width;
       t_tile = band * p.t_band + in_band - s.w_tile * width;
+    } else if (p.tile_group != nullptr) {
+      const int filled = p.n_w_tiles * n_filled, rest = p.n_t_tiles - n_filled;
+      if (tile < filled) { s.w_tile = tile / n_filled; t_tile = tile - s.w_tile * n_filled; }
+      else { s.w_tile = (tile - filled) / rest; t_tile = n_filled + (tile - filled) - s.w_tile * rest; }
     } else {                       // (at most a few token tiles; two divisions less in a step's many small products)
       s.w_tile = tile / p.n_t_tiles;
       t_tile = tile % p.n_t_tiles;

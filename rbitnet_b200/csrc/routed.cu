@@ -141,6 +141,66 @@ __device__ __forceinline__ void route_select(float* z, float* choice, float* gsc
   }
 }
 
+// The same for up to 32 outputs, a lane each: the values stay in registers, and a largest one is a reduction of the warp over
+// ordered bits and a ballot instead of ten exchanges.  2 tokens, 32 outputs in 8 groups, with the placing: 9.3 us of a step as above,
+// 5.3 so; 8 tokens without groups 7.4, 4.2.
+// zg: the token's sums; ids, weights: the token's `top` places (in shared or global memory).
+__device__ __forceinline__ void route_select32(const float* zg, const float* correction, int n, int top, int groups, int keep, int lane,
+                                               int* ids, float* weights, int scoring, const RouteWeighing& weighing) {
+  const bool live = lane < n;
+  const float z = live ? zg[lane] : -INFINITY;
+  const float plus = live && correction != nullptr ? correction[lane] : 0.f;
+  float s = z;                                        // what a chosen output weighs
+  if (scoring == 1) {
+    s = 1.0f / (1.0f + expf(-z));
+  } else if (scoring == 0) {
+    const float m = rb_warp_max(z);
+    const float e = live ? expf(z - m) : 0.f;
+    s = e * (1.0f / rb_warp_sum(e));
+  }
+  // bits that order as the values do; 0 for what cannot be chosen (-inf, NaN; +0 and -0 are the same)
+  auto ordered = [](float v) -> uint32_t {
+    if (!(v > -INFINITY)) return 0u;
+    const uint32_t u = __float_as_uint(v + 0.0f);
+    return (u & 0x80000000u) ? ~u : u | 0x80000000u;
+  };
+  uint32_t key = live ? ordered(s + plus) : 0u;
+  if (groups > 1 && keep < groups) {
+    const int per = n / groups, mine = live ? lane / per : groups;
+    // a group's best: the warp's groups reduce side by side (lanes behind the last output are one more)
+    const unsigned all = 0xffffffffu, of_mine = mine < groups ? ((per < 32 ? (1u << per) - 1u : all) << (mine * per)) : all << n;
+    uint32_t best = __reduce_max_sync(of_mine, key);
+    bool kept = false;
+    for (int j = 0; j < keep; ++j) {
+      const uint32_t top_key = __reduce_max_sync(all, best);
+      if (top_key == 0u) break;                       // nothing left to take
+      const int g = (__ffs(__ballot_sync(all, best == top_key)) - 1) / per;
+      if (mine == g) { kept = true; best = 0u; }
+    }
+    if (!kept) key = 0u;
+  }
+  float w = 0.f;
+  int id = 0;
+  for (int j = 0; j < top; ++j) {
+    const uint32_t best = __reduce_max_sync(0xffffffffu, key);
+    const int e = __ffs(__ballot_sync(0xffffffffu, key == best)) - 1;
+    const float v = __shfl_sync(0xffffffffu, s, e);
+    if (lane == j && best != 0u) { id = e; w = v; }
+    if (lane == e) key = 0u;
+  }
+  if (scoring == 2) {
+    const float m = rb_warp_max(lane < top ? w : -INFINITY);
+    const float e = lane < top ? expf(w - m) : 0.f;
+    w = e / rb_warp_sum(e);
+  }
+  if (weighing.normalize || weighing.scale != 1.0f) {
+    float by = weighing.scale;
+    if (weighing.normalize) by /= rb_warp_sum(lane < top ? w : 0.f) + weighing.floor;
+    w *= by;
+  }
+  if (lane < top) { ids[lane] = id; weights[lane] = w; }
+}
+
 thread_local RouteWeighing t_weighing;          // of this thread's next choice
 RouteWeighing take_weighing() {
   const RouteWeighing w = t_weighing;
@@ -235,6 +295,49 @@ __global__ void __launch_bounds__(256) route_kernel(int* ids, float* weights,
   route_select(z, z + n, z + 2 * n, correction, n_out, top, groups, keep, lane, ids, weights, t0 + warp, scoring, weighing);
 }
 
+// Few tokens: a warp makes one output of one token, so that a step's sums run on many SMs, with the same sums as above (lane l
+// takes every 32nd group of four values, then the lanes' shares in a fixed tree).  Up to 2,048 values of the warp's row of Wr are
+// asked for before the wait for the kernel before.  2 tokens, 32 outputs in 8 groups, 2,048 values: the kernel that makes sums and
+// choice in one block a token and the placing took 14.6 + 3.1 us of a step, this and the choice with the placing (below) 3.7 + 5.3;
+// 8 tokens: a tensor-core product with K in 8 parts 3.8, this 4.4 at twice the precision, and less where the kernel before ends early.
+constexpr int SUM_WARPS = 4, SUM_AHEAD = 16;
+template <typename TI>
+__global__ void __launch_bounds__(SUM_WARPS * 32) route_sums_kernel(float* z, const TI* h, int64_t ldh, const float* Wr, int K, int n) {
+  rb_pdl_launch_dependents();
+  const int lane = threadIdx.x & 31, e = blockIdx.x * SUM_WARPS + (threadIdx.x >> 5), t = blockIdx.y;
+  if (e >= n) return;
+  const float* w = Wr + (int64_t)e * K;
+  float ahead[SUM_AHEAD][4];
+#pragma unroll
+  for (int u = 0; u < SUM_AHEAD; ++u) {
+    const int k = lane * 4 + u * 128;
+    if (k < K) rb_load4(w + k, ahead[u]);
+    else ahead[u][0] = ahead[u][1] = ahead[u][2] = ahead[u][3] = 0.f;
+  }
+  rb_pdl_wait();
+  const TI* row = h + (int64_t)t * ldh;
+  float acc = 0.f;
+#pragma unroll
+  for (int u = 0; u < SUM_AHEAD; ++u) {
+    const int k = lane * 4 + u * 128;
+    if (k < K) {
+      float hv[4];
+      rb_load4(row + k, hv);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) acc = fmaf(hv[i], ahead[u][i], acc);
+    }
+  }
+  for (int k = lane * 4 + SUM_AHEAD * 128; k < K; k += 128) {
+    float hv[4], wv[4];
+    rb_load4(row + k, hv);
+    rb_load4(w + k, wv);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) acc = fmaf(hv[i], wv[i], acc);
+  }
+  acc = rb_warp_sum(acc);
+  if (lane == 0) z[(int64_t)t * n + e] = acc;
+}
+
 // Many tokens: the router's sums as a tiled float32 product (16 tokens by 64 outputs a block, k in steps of 32 through
 // shared memory, the next step's values asked for before this one is multiplied; every sum runs over k in ascending
 // order), then a warp per token for the choice.
@@ -304,6 +407,12 @@ __global__ void __launch_bounds__(128) route_select_kernel(int* ids, float* weig
   rb_pdl_wait();
   if (t >= T) return;
   const int64_t ldz = n + n_extra;                     // zg holds the outputs' sums, then the extra rows'
+  if (n <= 32) {
+    for (int i = lane; i < n_extra; i += 32) extra[(int64_t)t * n_extra + i] = zg[(int64_t)t * ldz + n + i];
+    route_select32(zg + (int64_t)t * ldz, correction, n, top, groups, keep, lane, ids + (int64_t)t * top, weights + (int64_t)t * top, scoring,
+                   weighing);
+    return;
+  }
   for (int e = lane; e < n; e += 32) z[e] = zg[(int64_t)t * ldz + e];
   for (int i = lane; i < n_extra; i += 32) extra[(int64_t)t * n_extra + i] = zg[(int64_t)t * ldz + n + i];
   __syncwarp();
@@ -411,70 +520,77 @@ __global__ void gather_scaled_kernel(T* xp, const T* h, int64_t ldh, const int* 
 // block counts all of them: a few loads and shared-memory additions), copies the pair's row and leaves its place in pos.
 // An expert's pairs take its rows in their order.  A decode step pays one launch instead of two (1 token, 4 of 32 experts
 // chosen, rows of 2,048: the two took 5.1 us of a step, this one 2.1; 8 tokens, weighed rows 7.1 and 3.6).
+// A shared expert whose matrices lie behind the others' (group n_experts) takes the first `n_shared` tiles: row r of them is
+// token r's row, unweighted.
 constexpr int PLACE_PAIRS = 256;
+// What a block does with its row once the ids (and, if rows are weighed, the weights) of all pairs are in shared memory.
 template <typename T>
-__global__ void __launch_bounds__(256) place_kernel(T* xp, int* pos, int* tile_group,
-                                                    const T* h, int64_t ldh, const int* ids,
-                                                    const float* weights, int pairs, int top, int n_experts, int tile,
-                                                    int K, int vec) {
-  rb_pdl_launch_dependents();
-  extern __shared__ int s_place[];      // ids [PLACE_PAIRS], tiles of every expert [n_experts]
+__device__ __forceinline__ void place_row(T* xp, int* pos, int* tile_group, const T* h, int64_t ldh, const int* s_ids,
+                                          const float* s_weights, int* counts, int n_tokens, int top, int n_experts, int tile,
+                                          int n_shared, int K, int vec) {
   __shared__ int s_expert, s_rank, s_pair;
-  int* s_ids = s_place;
-  int* counts = s_place + PLACE_PAIRS;
-  const int r = blockIdx.x, mine = r / tile;
-  for (int e = threadIdx.x; e < n_experts; e += blockDim.x) counts[e] = 0;
-  if (threadIdx.x == 0) { s_expert = -1; s_pair = -1; }
-  rb_pdl_wait();
-  __syncthreads();
-  for (int i = threadIdx.x; i < pairs; i += blockDim.x) {
-    const int e = ids[i];
-    s_ids[i] = e;
-    if (e < n_experts) atomicAdd(&counts[e], 1);
-    else if (r == 0) pos[i] = -1;       // an identity expert
-  }
-  __syncthreads();
-  const int lane = threadIdx.x & 31;
-  if (threadIdx.x < 32) {
-    // the expert whose tiles hold this one
-    int before = 0;
-    for (int e0 = 0; e0 < n_experts; e0 += 32) {
-      const int e = e0 + lane, t = e < n_experts ? (counts[e] + tile - 1) / tile : 0;
-      int up_to = t;
+  const int pairs = n_tokens * top, lane = threadIdx.x & 31;
+  const int r = blockIdx.x, mine = r / tile - n_shared;          // the row's tile, counted behind the shared ones
+  int source = -1;                                               // the token whose row this is
+  float w = 1.f;
+  if (mine < 0) {
+    if (r < n_tokens) source = r;
+    if (threadIdx.x == 0 && r % tile == 0) tile_group[r / tile] = n_experts;
+    // (no barrier below is passed: the whole block is here)
+  } else {
+    for (int e = threadIdx.x; e < n_experts; e += blockDim.x) counts[e] = 0;
+    if (threadIdx.x == 0) { s_expert = -1; s_pair = -1; }
+    __syncthreads();
+    for (int i = threadIdx.x; i < pairs; i += blockDim.x) {
+      const int e = s_ids[i];
+      if (e < n_experts) atomicAdd(&counts[e], 1);
+      else if (mine == 0 && r % tile == 0) pos[i] = -1;       // an identity expert
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {
+      // the expert whose tiles hold this one
+      int before = 0;
+      for (int e0 = 0; e0 < n_experts; e0 += 32) {
+        const int e = e0 + lane, t = e < n_experts ? (counts[e] + tile - 1) / tile : 0;
+        int up_to = t;
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, up_to, o);
-        if (lane >= o) up_to += v;
+        for (int o = 1; o < 32; o <<= 1) {
+          const int v = __shfl_up_sync(0xffffffffu, up_to, o);
+          if (lane >= o) up_to += v;
+        }
+        const int first = before + up_to - t;
+        if (t > 0 && mine >= first && mine < first + t) { s_expert = e; s_rank = r - (n_shared + first) * tile; }
+        before += __shfl_sync(0xffffffffu, up_to, 31);
+        if (mine < before) break;
       }
-      const int first = before + up_to - t;
-      if (t > 0 && mine >= first && mine < first + t) { s_expert = e; s_rank = r - first * tile; }
-      before += __shfl_sync(0xffffffffu, up_to, 31);
-      if (mine < before) break;
+      __syncwarp();
+      // its pair with this row's number
+      const int e = s_expert;
+      int left = e >= 0 ? s_rank : -1;
+      for (int i0 = 0; left >= 0 && i0 < pairs; i0 += 32) {
+        const bool is = i0 + lane < pairs && s_ids[i0 + lane] == e;
+        const unsigned all = __ballot_sync(0xffffffffu, is);
+        if (is && __popc(all & ((1u << lane) - 1u)) == left) s_pair = i0 + lane;
+        left -= __popc(all);
+      }
     }
-    __syncwarp();
-    // its pair with this row's number
-    const int e = s_expert;
-    int left = e >= 0 ? s_rank : -1;
-    for (int i0 = 0; left >= 0 && i0 < pairs; i0 += 32) {
-      const bool is = i0 + lane < pairs && s_ids[i0 + lane] == e;
-      const unsigned all = __ballot_sync(0xffffffffu, is);
-      if (is && __popc(all & ((1u << lane) - 1u)) == left) s_pair = i0 + lane;
-      left -= __popc(all);
+    __syncthreads();
+    const int pair = s_pair;
+    if (threadIdx.x == 0) {
+      if (r % tile == 0) tile_group[r / tile] = s_expert;
+      if (pair >= 0) pos[pair] = r;
     }
-  }
-  __syncthreads();
-  const int pair = s_pair;
-  if (threadIdx.x == 0) {
-    if (r % tile == 0) tile_group[mine] = s_expert;
-    if (pair >= 0) pos[pair] = r;
+    if (pair >= 0) {
+      source = pair / top;
+      if (s_weights != nullptr) w = s_weights[pair];
+    }
   }
   T* dst = xp + (int64_t)r * K;
-  const T* src = h + (int64_t)(pair >= 0 ? pair / top : 0) * ldh;
-  const float w = weights != nullptr && pair >= 0 ? weights[pair] : 1.f;
+  const T* src = h + (int64_t)max(source, 0) * ldh;
   if (vec) {
     for (int k = threadIdx.x * 4; k < K; k += blockDim.x * 4) {
       float v[4] = {0.f, 0.f, 0.f, 0.f};
-      if (pair >= 0) {
+      if (source >= 0) {
         rb_load4(src + k, v);
 #pragma unroll
         for (int j = 0; j < 4; ++j) v[j] *= w;
@@ -483,7 +599,68 @@ __global__ void __launch_bounds__(256) place_kernel(T* xp, int* pos, int* tile_g
     }
     return;
   }
-  for (int k = threadIdx.x; k < K; k += blockDim.x) dst[k] = rb_from_float<T>(pair >= 0 ? w * rb_to_float<T>(src[k]) : 0.f);
+  for (int k = threadIdx.x; k < K; k += blockDim.x) dst[k] = rb_from_float<T>(source >= 0 ? w * rb_to_float<T>(src[k]) : 0.f);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256) place_kernel(T* xp, int* pos, int* tile_group,
+                                                    const T* h, int64_t ldh, const int* ids,
+                                                    const float* weights, int n_tokens, int top, int n_experts, int tile,
+                                                    int n_shared, int K, int vec) {
+  rb_pdl_launch_dependents();
+  extern __shared__ int s_place[];      // ids [PLACE_PAIRS], weights [PLACE_PAIRS], pairs of every expert [n_experts]
+  float* s_weights = reinterpret_cast<float*>(s_place + PLACE_PAIRS);
+  rb_pdl_wait();
+  for (int i = threadIdx.x; i < n_tokens * top; i += blockDim.x) {
+    s_place[i] = ids[i];
+    if (weights != nullptr) s_weights[i] = weights[i];
+  }
+  __syncthreads();
+  place_row<T>(xp, pos, tile_group, h, ldh, s_place, weights != nullptr ? s_weights : nullptr, s_place + 2 * PLACE_PAIRS, n_tokens, top,
+               n_experts, tile, n_shared, K, vec);
+}
+
+// The choice and the placing in one launch, for up to CHOOSE_TOKENS tokens whose sums a product has left: every block makes
+// all tokens' choices for itself (a warp a token, two turns at most), then places its row.  The first block leaves weights and
+// extra sums for the kernels behind.  A decode step pays one launch instead of two: the two took 3.8 + 2.6 us of a step at 8
+// tokens and 32 outputs, this one 4.2.  Many tokens' choices would be made too often: the two kernels again.
+constexpr int CHOOSE_TOKENS = 16, CHOOSE_WARPS = 8;
+struct Choice {
+  const float* sums;          // [tokens, n + n_extra]
+  const float* correction;
+  float* weights;             // [tokens, top]
+  float* extra;               // [tokens, n_extra]
+  int n, n_extra, groups, keep, scoring;
+  RouteWeighing weighing;
+};
+template <typename T>
+__global__ void __launch_bounds__(CHOOSE_WARPS * 32) choose_place_kernel(T* xp, int* pos, int* tile_group, const T* h, int64_t ldh,
+                                                                         Choice c, int weigh, int n_tokens, int top, int n_experts,
+                                                                         int tile, int n_shared, int K, int vec) {
+  rb_pdl_launch_dependents();
+  extern __shared__ int s_place[];      // as above, then 2 n + 2 groups floats a warp
+  float* s_weights = reinterpret_cast<float*>(s_place + PLACE_PAIRS);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, ldz = c.n + c.n_extra;
+  float* z = reinterpret_cast<float*>(s_place + 2 * PLACE_PAIRS + n_experts) + (size_t)warp * (2 * c.n + 2 * c.groups);
+  rb_pdl_wait();
+  for (int t = warp; t < n_tokens; t += CHOOSE_WARPS) {
+    if (blockIdx.x == 0)
+      for (int i = lane; i < c.n_extra; i += 32) c.extra[(int64_t)t * c.n_extra + i] = c.sums[(int64_t)t * ldz + c.n + i];
+    if (c.n <= 32) {
+      route_select32(c.sums + (int64_t)t * ldz, c.correction, c.n, top, c.groups, c.keep, lane, s_place + t * top, s_weights + t * top,
+                     c.scoring, c.weighing);
+      continue;
+    }
+    for (int e = lane; e < c.n; e += 32) z[e] = c.sums[(int64_t)t * ldz + e];
+    __syncwarp();
+    route_select(z, z + c.n, z + 2 * c.n, c.correction, c.n, top, c.groups, c.keep, lane, s_place, s_weights, t, c.scoring, c.weighing);
+    __syncwarp();
+  }
+  __syncthreads();
+  if (blockIdx.x == 0)
+    for (int i = threadIdx.x; i < n_tokens * top; i += blockDim.x) c.weights[i] = s_weights[i];
+  place_row<T>(xp, pos, tile_group, h, ldh, s_place, weigh ? s_weights : nullptr, s_place + 2 * PLACE_PAIRS, n_tokens, top, n_experts, tile,
+               n_shared, K, vec);
 }
 
 // ---------------------------------------------------------------- weighted sum
@@ -641,9 +818,31 @@ __global__ void square_relu_kernel(T* out, const T* in, int64_t n) {
 
 }  // namespace
 
+static int launch_sums(float* z, const void* h, int64_t ldh, int h_dtype, const float* Wr, int T, int K, int n, cudaStream_t stream) {
+  const dim3 grid((n + SUM_WARPS - 1) / SUM_WARPS, T);
+  if (h_dtype == RB_F32)
+    RB_LAUNCH("route_sums_kernel", (route_sums_kernel<float>), grid, SUM_WARPS * 32, 0, stream, z, (const float*)h, ldh, Wr, K, n);
+  else if (h_dtype == RB_BF16)
+    RB_LAUNCH("route_sums_kernel", (route_sums_kernel<__nv_bfloat16>), grid, SUM_WARPS * 32, 0, stream, z, (const __nv_bfloat16*)h, ldh, Wr, K, n);
+  else
+    RB_FAIL("rb_route: unknown dtype %d", h_dtype);
+  RB_CHECK_LAUNCH("rb_route");
+  return 0;
+}
+
+static int select_impl(int* ids, float* weights, const float* z, const float* correction, int T, int n, int top, int groups, int keep,
+                       int scoring, int n_extra, float* extra, const RouteWeighing& weighing, cudaStream_t stream) {
+  const size_t smem = (size_t)4 * (2 * n + 2 * groups) * sizeof(float);
+  RB_REQUIRE(smem <= 48 * 1024, "rb_route: %d router outputs are more than a block's shared memory holds", n);
+  RB_LAUNCH("route_select_kernel", (route_select_kernel), (T + 3) / 4, 128, smem, stream, ids, weights, z, correction, T, n, top,
+            groups, keep, scoring, n_extra, extra, weighing);
+  RB_CHECK_LAUNCH("rb_route");
+  return 0;
+}
+
 // ids, weights: [T, top].  h: the input rows (dtype h_dtype).  Wr: float32 [n, K]; correction: float32 [n] or null.
-// groups <= 1 or keep >= groups: every output can be chosen.  z_scratch: T * n floats (from 64 tokens on, the router's
-// sums are a product of their own that leaves them there), or null.
+// groups <= 1 or keep >= groups: every output can be chosen.  z_scratch: T * n floats (the router's
+// sums are then a kernel of their own that leaves them there), or null.
 static int route_impl(int* ids, float* weights, const void* h, int64_t ldh, int h_dtype, const float* Wr,
                       const float* correction, int T, int K, int n, int top, int groups, int keep, float* z_scratch,
                       int scoring, int n_extra, float* extra, cudaStream_t stream) {
@@ -672,12 +871,16 @@ static int route_impl(int* ids, float* weights, const void* h, int64_t ldh, int 
     RB_CHECK_LAUNCH("rb_route");
     return 0;
   }
+  const int elem = h_dtype == RB_F32 ? 4 : 2;
+  const int vec = K % 4 == 0 && ldh % 4 == 0 && (uintptr_t)h % (4 * elem) == 0 && (uintptr_t)Wr % 16 == 0;
+  if (T < 64 && z_scratch != nullptr && vec && (size_t)4 * (2 * n + 2 * groups) * sizeof(float) <= 48 * 1024) {      // (the choice's scratch)
+    if (launch_sums(z_scratch, h, ldh, h_dtype, Wr, T, K, n_all, stream) != 0) return -1;
+    return select_impl(ids, weights, z_scratch, correction, T, n, top, groups, keep, scoring, n_extra, extra, weighing, stream);
+  }
   const int TB = T >= 64 ? ROUTE_TB : 1;
   const size_t smem = (size_t)TB * (2 * n_all + 2 * groups) * sizeof(float);
   RB_REQUIRE(smem <= 48 * 1024, "rb_route: %d router outputs are more than a block's shared memory holds", n);
   const int blocks = (T + TB - 1) / TB;
-  const int elem = h_dtype == RB_F32 ? 4 : 2;
-  const int vec = K % 4 == 0 && ldh % 4 == 0 && (uintptr_t)h % (4 * elem) == 0 && (uintptr_t)Wr % 16 == 0;
   if (h_dtype == RB_F32)
     RB_LAUNCH("route_kernel", (route_kernel<float>), blocks, 256, smem, stream, ids, weights, (const float*)h, ldh, Wr, correction, T, K, n, top, groups, keep, TB, vec, scoring, n_extra, extra, weighing);
   else if (h_dtype == RB_BF16)
@@ -765,26 +968,83 @@ RB_EXPORT int rb_routed_plan(int* pos, int* row_token, int* tile_group, const in
 // The most pairs that rb_routed_place takes.
 RB_EXPORT int rb_routed_place_pairs() { return PLACE_PAIRS; }
 
+// The next rb_routed_place or rb_route_choose_place call of this thread puts every token's own row, unweighted, into `tiles` tiles
+// ahead of the pairs' (group n_experts: a shared expert whose matrices lie behind the others').
+static thread_local int t_place_shared = 0;
+RB_EXPORT int rb_routed_place_shared(int tiles) {
+  t_place_shared = tiles;
+  return 0;
+}
+
+static int place_impl(void* xp, int* pos, int* tile_group, const void* h, int64_t ldh, int dtype, const int* ids, const float* weights,
+                      const Choice* choice, int weigh, int pairs, int top, int n_experts, int tile, int n_tiles, int K, cudaStream_t stream) {
+  const int n_shared = t_place_shared;
+  t_place_shared = 0;
+  if (pairs == 0) return 0;
+  RB_REQUIRE(pairs <= PLACE_PAIRS && n_experts > 0 && top > 0 && pairs % top == 0 && tile > 0 && n_tiles >= rb_routed_tiles(pairs, n_experts, tile),
+             "rb_routed_place: %d tiles of %d rows for %d pairs over %d experts", n_tiles, tile, pairs, n_experts);
+  const int T = pairs / top;
+  RB_REQUIRE(n_shared == 0 || n_shared * tile >= T, "rb_routed_place: %d tokens in %d shared tiles of %d rows", T, n_shared, tile);
+  size_t smem = (size_t)(2 * PLACE_PAIRS + n_experts) * sizeof(int);
+  RB_REQUIRE(smem <= 40 * 1024, "rb_routed_place: %d experts", n_experts);
+  const size_t four = dtype == RB_F32 ? 16 : 8;
+  const int vec = K % 4 == 0 && ldh % 4 == 0 && (uintptr_t)xp % four == 0 && (uintptr_t)h % four == 0 ? 1 : 0;
+  const int threads = K >= 1024 ? 256 : (K >= 512 ? 128 : 64), blocks = (n_shared + n_tiles) * tile;
+  RB_REQUIRE(dtype == RB_F32 || dtype == RB_BF16, "rb_routed_place: unknown dtype %d", dtype);
+  if (choice != nullptr) {
+    smem += (size_t)CHOOSE_WARPS * (2 * choice->n + 2 * choice->groups) * sizeof(float);
+    RB_REQUIRE(T <= CHOOSE_TOKENS && smem <= 48 * 1024, "rb_route_choose_place: %d tokens, %d outputs", T, choice->n);
+    if (dtype == RB_F32)
+      RB_LAUNCH("choose_place_kernel", (choose_place_kernel<float>), blocks, CHOOSE_WARPS * 32, smem, stream, (float*)xp, pos, tile_group, (const float*)h, ldh, *choice, weigh, T, top, n_experts, tile, n_shared, K, vec);
+    else
+      RB_LAUNCH("choose_place_kernel", (choose_place_kernel<__nv_bfloat16>), blocks, CHOOSE_WARPS * 32, smem, stream, (__nv_bfloat16*)xp, pos, tile_group, (const __nv_bfloat16*)h, ldh, *choice, weigh, T, top, n_experts, tile, n_shared, K, vec);
+  } else if (dtype == RB_F32) {
+    RB_LAUNCH("place_kernel", (place_kernel<float>), blocks, threads, smem, stream, (float*)xp, pos, tile_group, (const float*)h, ldh, ids, weights, T, top, n_experts, tile, n_shared, K, vec);
+  } else {
+    RB_LAUNCH("place_kernel", (place_kernel<__nv_bfloat16>), blocks, threads, smem, stream, (__nv_bfloat16*)xp, pos, tile_group, (const __nv_bfloat16*)h, ldh, ids, weights, T, top, n_experts, tile, n_shared, K, vec);
+  }
+  RB_CHECK_LAUNCH("rb_routed_place");
+  return 0;
+}
+
 // rb_routed_plan and rb_routed_gather (weights null) or rb_routed_gather_scaled in one launch, for few pairs.
 RB_EXPORT int rb_routed_place(void* xp, int* pos, int* tile_group, const void* h, int64_t ldh, int dtype, const int* ids,
                               const float* weights, int pairs, int top, int n_experts, int tile, int n_tiles, int K,
                               cudaStream_t stream) {
-  if (pairs == 0) return 0;
-  RB_REQUIRE(pairs <= PLACE_PAIRS && n_experts > 0 && top > 0 && tile > 0 && n_tiles >= rb_routed_tiles(pairs, n_experts, tile),
-             "rb_routed_place: %d tiles of %d rows for %d pairs over %d experts", n_tiles, tile, pairs, n_experts);
-  const size_t smem = (size_t)(PLACE_PAIRS + n_experts) * sizeof(int);
-  RB_REQUIRE(smem <= 40 * 1024, "rb_routed_place: %d experts", n_experts);
-  const size_t four = dtype == RB_F32 ? 16 : 8;
-  const int vec = K % 4 == 0 && ldh % 4 == 0 && (uintptr_t)xp % four == 0 && (uintptr_t)h % four == 0 ? 1 : 0;
-  const int threads = K >= 1024 ? 256 : (K >= 512 ? 128 : 64);
-  if (dtype == RB_F32)
-    RB_LAUNCH("place_kernel", (place_kernel<float>), n_tiles * tile, threads, smem, stream, (float*)xp, pos, tile_group, (const float*)h, ldh, ids, weights, pairs, top, n_experts, tile, K, vec);
-  else if (dtype == RB_BF16)
-    RB_LAUNCH("place_kernel", (place_kernel<__nv_bfloat16>), n_tiles * tile, threads, smem, stream, (__nv_bfloat16*)xp, pos, tile_group, (const __nv_bfloat16*)h, ldh, ids, weights, pairs, top, n_experts, tile, K, vec);
-  else
-    RB_FAIL("rb_routed_place: unknown dtype %d", dtype);
-  RB_CHECK_LAUNCH("rb_routed_place");
-  return 0;
+  return place_impl(xp, pos, tile_group, h, ldh, dtype, ids, weights, nullptr, 0, pairs, top, n_experts, tile, n_tiles, K, stream);
+}
+
+// Whether the choice and the placing of so many tokens are one launch.
+RB_EXPORT int rb_route_choose_place_supports(int T, int n, int top, int groups, int n_experts) {
+  return T > 0 && T <= CHOOSE_TOKENS && T * top <= PLACE_PAIRS && n_experts > 0 &&
+         (size_t)(2 * PLACE_PAIRS + n_experts) * sizeof(int) <= 40 * 1024 &&
+         (size_t)(2 * PLACE_PAIRS + n_experts) * sizeof(int) + (size_t)CHOOSE_WARPS * (2 * n + 2 * (groups < 1 ? 1 : groups)) * sizeof(float) <= 48 * 1024;
+}
+
+// The choice from sums z [T, n + n_extra] (see rb_route_select_scored; rb_route_next weighs) and the placing of its pairs in one
+// launch.  weigh: rows are multiplied by their pairs' weights.
+RB_EXPORT int rb_route_choose_place(void* xp, int* pos, int* tile_group, const void* h, int64_t ldh, int dtype, float* weights,
+                                    const float* z, const float* correction, int T, int n, int top, int groups, int keep, int scoring,
+                                    int n_extra, float* extra, int weigh, int n_experts, int tile, int n_tiles, int K, cudaStream_t stream) {
+  Choice c;
+  c.weighing = take_weighing();
+  RB_REQUIRE(T > 0 && n > 0 && top > 0 && top <= n && n_extra >= 0 && (n_extra == 0 || extra != nullptr) && scoring >= 0 && scoring <= 2,
+             "rb_route_choose_place: bad sizes tokens=%d outputs=%d top=%d extra=%d scoring=%d", T, n, top, n_extra, scoring);
+  RB_REQUIRE(groups <= 1 || n % groups == 0, "rb_route_choose_place: %d outputs are not %d equal groups", n, groups);
+  c.sums = z; c.correction = correction; c.weights = weights; c.extra = extra;
+  c.n = n; c.n_extra = n_extra; c.groups = groups < 1 ? 1 : groups; c.keep = keep; c.scoring = scoring;
+  return place_impl(xp, pos, tile_group, h, ldh, dtype, nullptr, nullptr, &c, weigh, T * top, top, n_experts, tile, n_tiles, K, stream);
+}
+
+// The router's sums alone: z [T, n] = h Wr^T, float32, for few tokens.
+RB_EXPORT int rb_route_sums_supports(const void* h, int64_t ldh, int h_dtype, const float* Wr, int T, int K) {
+  const int elem = h_dtype == RB_F32 ? 4 : 2;
+  return T > 0 && T < 64 && K % 4 == 0 && ldh % 4 == 0 && (uintptr_t)h % (4 * elem) == 0 && (uintptr_t)Wr % 16 == 0;
+}
+RB_EXPORT int rb_route_sums(float* z, const void* h, int64_t ldh, int h_dtype, const float* Wr, int T, int K, int n, cudaStream_t stream) {
+  if (T == 0) return 0;
+  RB_REQUIRE(n > 0 && K > 0 && rb_route_sums_supports(h, ldh, h_dtype, Wr, T, K), "rb_route_sums: %d tokens of %d values, %d outputs", T, K, n);
+  return launch_sums(z, h, ldh, h_dtype, Wr, T, K, n, stream);
 }
 
 RB_EXPORT int rb_routed_gather(void* xp, const void* h, int64_t ldh, int dtype, const int* row_token, int rows, int K,

@@ -52,6 +52,9 @@ _SIGNATURES = {
     "rb_routed_plan": [P, P, P, P, I, I, I, I, I, P],
     "rb_routed_place": [P, P, P, P, L, I, P, P, I, I, I, I, I, I, P],
     "rb_routed_place_pairs": [],
+    "rb_routed_place_shared": [I],
+    "rb_route_choose_place": [P, P, P, P, L, I, P, P, P, I, I, I, I, I, I, I, P, I, I, I, I, I, P],
+    "rb_route_sums": [P, P, L, I, P, I, I, I, P],
     "rb_routed_gather": [P, P, L, I, P, I, I, P],
     "rb_routed_combine": [P, L, P, P, L, I, P, P, I, I, I, I, P],
     "rb_gemm_grouped_simple": [P, L, I, P, L, P, L, I, P, I, I, I, I, P],
@@ -153,6 +156,8 @@ class KernelLibrary:
         self.declare("rb_gemm_tc_set_workspace", [P, L])
         self.declare("rb_gemm_tc_plan", [I, I, I, I, I, I, P])
         self.declare("rb_gemm_tc_share_for_test", [I])
+        self.declare("rb_route_choose_place_supports", [I, I, I, I, I])
+        self.declare("rb_route_sums_supports", [P, L, I, P, I, I])
         self.declare("rb_f32_tc_plan_of", [I, I, I, I, I, P])
         self.declare("rb_gemm_tc_tail_for_test", [I])
         self.declare("rb_gemm_tc_kernels_launched", [])

@@ -108,6 +108,19 @@ class ExpertGateUp:
 
 
 @dataclass
+class PlacedRows:
+    """A step's (token, choice) pairs sorted by expert (``CudaOps.route_and_place``): ``rows`` holds their input rows in tiles of
+    ``tile``, ``pos`` every pair's row, ``tile_group`` every tile's expert; ``n_shared`` tiles ahead hold the tokens' own rows."""
+    weights: torch.Tensor         # float32 [T, top]
+    extra: Optional[torch.Tensor]
+    rows: torch.Tensor
+    pos: torch.Tensor
+    tile_group: torch.Tensor
+    tile: int
+    n_shared: int
+
+
+@dataclass
 class NormRequest:
     """Asks the product that adds to the residual stream to leave what the norm after it needs
     (``CudaOps.linear(..., then_norm=request)``).  ``result`` is the ``NormedRows`` if it did."""
@@ -199,13 +212,15 @@ class CudaOps:
         #: a decode step's gated addition, norm in groups and filter between two sublayers are one kernel
         self.fuse_norm_filter = True
         #: rows from which a scored router's sums are a tensor-core product (where that product gives the same sums)
-        self.router_tc_from = 1
+        self.router_tc_from = 17
         #: products with one matrix per head of many rows run on the tensor cores where the sizes allow it
         self.per_head_on_tensor_cores = True
         #: gated products of few tokens cut K into parts as the others do
         self.split_gated = True
         #: the plan and the gather of a step's few (token, choice) pairs are one kernel
         self.place_few_pairs = True
+        #: up to 16 tokens' choices are made by the kernel that places their pairs
+        self.choose_and_place = True
         #: so does gated linear attention
         self.gla_in_chunks = True
         #: in bfloat16 mode a state-space mixer takes runs of several tokens in chunks of 64 (else token by token)
@@ -1332,6 +1347,12 @@ class CudaOps:
         w = torch.cat([torch.cat([self.to_compute(g), self.to_compute(u)], dim=0) for g, u in zip(gates, ups)], dim=0)
         return ExpertGateUp(w.contiguous(), inner, K, 2 * inner, 0)
 
+    def expert_of(self, w_up: ExpertGateUp, w_down: LinearWeight, expert: int):
+        """One expert's matrices, sharing the memory of all: what ``gated_linear`` and ``linear`` take."""
+        width = w_up.n_in
+        return (GateUpWeight(w_up.w[expert * w_up.rows:(expert + 1) * w_up.rows], w_up.inner, width, w_up.block),
+                self.rows_of(w_down, expert * width, width))
+
     def route_scored(self, h: torch.Tensor, router: torch.Tensor, correction: Optional[torch.Tensor], top: int, groups: int,
                      keep: int, scoring: str = "softmax", extra_rows: int = 0, router_tc: Optional[LinearWeight] = None,
                      normalize: Optional[float] = None, weight_scale: float = 1.0):
@@ -1349,19 +1370,51 @@ class CudaOps:
         weights = torch.empty((T, top), dtype=torch.float32, device=self.device)
         extra = torch.empty((T, extra_rows), dtype=torch.float32, device=self.device) if extra_rows else None
         if T >= self.router_tc_from and router_tc is not None and self._tensor_core_ok(h, router_tc.w):
-            # the sums (outputs and extra rows) on the tensor cores, then the choice: also for a decode step, where the
-            # kernel that does both has a block per token (20 us at 8 tokens against 7 for the two)
+            # the sums (outputs and extra rows) on the tensor cores, then the choice
             z = self.linear(h, router_tc, out_dtype=torch.float32)
             self.lib.call("rb_route_select_scored", _ptr(ids), _ptr(weights), _ptr(z), _ptr(correction), T, n, int(top),
                           int(groups), int(keep), _SCORING[scoring], int(extra_rows), _ptr(extra),
                           self._stream())
             return ids, weights, extra
-        z = torch.empty((T, n + extra_rows), dtype=torch.float32, device=self.device) if T >= 64 else None
+        z = torch.empty((T, n + extra_rows), dtype=torch.float32, device=self.device)
         self.lib.call("rb_route_scored", _ptr(ids), _ptr(weights), _ptr(h), h.stride(0), self.code, _ptr(router),
                       _ptr(correction), T, K, n, int(top), int(groups), int(keep), _ptr(z),
-                      _SCORING[scoring], int(extra_rows), _ptr(extra), self._stream(),
-                      launches=2 if z is not None else 1)
+                      _SCORING[scoring], int(extra_rows), _ptr(extra), self._stream(), launches=2)
         return ids, weights, extra
+
+    def route_and_place(self, h: torch.Tensor, router: torch.Tensor, correction: Optional[torch.Tensor], top: int, groups: int,
+                        keep: int, n_experts: int, inner: int, scoring: str = "softmax", extra_rows: int = 0,
+                        normalize: Optional[float] = None, weight_scale: float = 1.0, weight_on_input: bool = False,
+                        with_shared: bool = False) -> Optional["PlacedRows"]:
+        """``route_scored`` and the sorting of the pairs by expert that ``routed_experts`` begins with, in two launches for up to 16
+        tokens (None: not for these sizes).  ``with_shared``: the tokens' own rows are placed too, for one more expert whose
+        matrices lie behind the others'."""
+        self._check(h, self.dtype, "route input")
+        T, K = h.shape
+        n = router.shape[0] - extra_rows
+        if not (self.choose_and_place and self.place_few_pairs and n_experts > 0
+                and self.lib.raw("rb_route_choose_place_supports")(T, n, int(top), int(groups), n_experts)
+                and self.lib.raw("rb_route_sums_supports")(_ptr(h), h.stride(0), self.code, _ptr(router), T, K)):
+            return None
+        z = torch.empty((T, n + extra_rows), dtype=torch.float32, device=self.device)
+        weights = torch.empty((T, top), dtype=torch.float32, device=self.device)
+        extra = torch.empty((T, extra_rows), dtype=torch.float32, device=self.device) if extra_rows else None
+        pairs = T * top
+        tile = self.routed_tile(pairs, n_experts, inner, K)
+        n_tiles = self.lib.raw("rb_routed_tiles")(pairs, n_experts, tile)
+        n_shared = -(-T // tile) if with_shared else 0
+        plan = torch.empty((pairs + n_shared + n_tiles,), dtype=torch.int32, device=self.device)
+        placed = PlacedRows(weights, extra, torch.empty(((n_shared + n_tiles) * tile, K), dtype=self.dtype, device=self.device),
+                            plan[:pairs], plan[pairs:], tile, n_shared)
+        self.lib.call("rb_route_sums", _ptr(z), _ptr(h), h.stride(0), self.code, _ptr(router), T, K, n + extra_rows, self._stream())
+        if normalize is not None or weight_scale != 1.0:
+            self.lib.call("rb_route_next", 0 if normalize is None else 1, float(normalize or 0.0), float(weight_scale), launches=0)
+        if n_shared:
+            self.lib.call("rb_routed_place_shared", n_shared, launches=0)
+        self.lib.call("rb_route_choose_place", _ptr(placed.rows), _ptr(placed.pos), _ptr(placed.tile_group), _ptr(h), h.stride(0), self.code,
+                      _ptr(weights), _ptr(z), _ptr(correction), T, n, int(top), int(groups), int(keep), _SCORING[scoring], int(extra_rows),
+                      _ptr(extra), 1 if weight_on_input else 0, n_experts, tile, n_tiles, K, self._stream())
+        return placed
 
     # ------------------------------------------------------------------ routed experts
     def prepare_router(self, router: torch.Tensor) -> Optional[LinearWeight]:
@@ -1392,10 +1445,10 @@ class CudaOps:
             self.lib.call("rb_route_select", _ptr(ids), _ptr(weights), _ptr(z), _ptr(correction), T, n, int(top), int(groups),
                           int(keep), self._stream())
             return ids, weights
-        # from 64 tokens on the router's sums are a tiled product of their own, which leaves them in z
-        z = torch.empty((T, n), dtype=torch.float32, device=self.device) if T >= 64 else None
+        # the router's sums are a kernel of their own (from 64 tokens on a tiled product), which leaves them in z
+        z = torch.empty((T, n), dtype=torch.float32, device=self.device)
         self.lib.call("rb_route", _ptr(ids), _ptr(weights), _ptr(h), h.stride(0), self.code, _ptr(router), _ptr(correction),
-                      T, K, n, int(top), int(groups), int(keep), _ptr(z), self._stream(), launches=2 if z is not None else 1)
+                      T, K, n, int(top), int(groups), int(keep), _ptr(z), self._stream(), launches=2)
         return ids, weights
 
     def routed_tile(self, pairs: int, n_experts: int, inner: int, width: int) -> int:
@@ -1408,9 +1461,34 @@ class CudaOps:
     def _routed_on_tensor_cores(self, inner: int, width: int) -> bool:
         return self.dtype == torch.bfloat16 and inner % 8 == 0 and width % 8 == 0
 
+    def _place(self, h, ids, weights, top: int, n_experts: int, inner: int):
+        """A step's (token, choice) pairs sorted by expert: their input rows (times ``weights``), every pair's row, every tile's
+        expert, rows a tile and rows in all."""
+        T, E = h.shape
+        pairs = T * top
+        tile = self.routed_tile(pairs, n_experts, inner, E)
+        n_tiles = self.lib.raw("rb_routed_tiles")(pairs, n_experts, tile)
+        rows = n_tiles * tile
+        plan = torch.empty((pairs + rows + n_tiles,), dtype=torch.int32, device=self.device)
+        pos, row_token, tile_group = plan[:pairs], plan[pairs:pairs + rows], plan[pairs + rows:]
+        xp = torch.empty((rows, E), dtype=self.dtype, device=self.device)
+        if self.place_few_pairs and pairs <= self.lib.raw("rb_routed_place_pairs")():
+            self.lib.call("rb_routed_place", _ptr(xp), _ptr(pos), _ptr(tile_group), _ptr(h), h.stride(0), self.code, _ptr(ids),
+                          _ptr(weights), pairs, top, n_experts, tile, n_tiles, E, self._stream())
+            return xp, pos, tile_group, tile, rows
+        self.lib.call("rb_routed_plan", _ptr(pos), _ptr(row_token), _ptr(tile_group), _ptr(ids), pairs, top, n_experts,
+                      tile, n_tiles, self._stream())
+        if weights is not None:
+            self.lib.call("rb_routed_gather_scaled", _ptr(xp), _ptr(h), h.stride(0), self.code, _ptr(row_token), _ptr(pos),
+                          _ptr(weights), top, rows, E, self._stream())
+        else:
+            self.lib.call("rb_routed_gather", _ptr(xp), _ptr(h), h.stride(0), self.code, _ptr(row_token), rows, E, self._stream())
+        return xp, pos, tile_group, tile, rows
+
     def routed_experts(self, h: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, w_up, w_down: LinearWeight,
                        n_experts: int, inner: int, accumulate_into: Optional[torch.Tensor] = None, act=None,
-                       weight_on_input: bool = False, shared=None, then_norm: Optional[TanhRequest] = None):
+                       weight_on_input: bool = False, shared=None, then_norm: Optional[TanhRequest] = None,
+                       placed: Optional["PlacedRows"] = None):
         """sum_j weights[t, j] * expert(ids[t, j])(h[t]) with expert e: W_down_e relu2(W_up_e h); ids >= n_experts are
         identity experts (h[t] itself).  ``w_up``: [n_experts * inner, width], ``w_down``: [n_experts * width, inner].
         Added to ``accumulate_into`` (float32), or returned as float32 rows.
@@ -1418,9 +1496,13 @@ class CudaOps:
         g' sigmoid(alpha g') (u' + shift) as in ``gated_linear``.  ``weight_on_input``: sum_j expert(weights[t, j] * h[t])
         instead (the weighted row is rounded to the compute dtype before the expert's first product).
         ``shared`` = (float32 rows, float32 gate logits [T, 1] or None): sigmoid(gate) * rows (None: the rows as they are) is
-        added in the same kernel as the weighted sum; a ``TanhRequest`` is granted there too."""
+        added in the same kernel as the weighted sum; a ``TanhRequest`` is granted there too.  ``placed``: what
+        ``route_and_place`` left, in place of ``ids`` and ``weights``; with the tokens' own rows among them ``w_up`` and ``w_down``
+        hold the shared expert behind the others, and ``shared`` is (None, gate)."""
         T, E = h.shape
-        top = ids.shape[1]
+        if placed is not None:
+            weights = placed.weights
+        top = weights.shape[1]
         pairs = T * top
         if accumulate_into is not None:
             out, acc = accumulate_into, 1
@@ -1428,26 +1510,12 @@ class CudaOps:
             out, acc = torch.empty((T, E), dtype=torch.float32, device=self.device), 0
         y = pos = None
         if n_experts > 0:
-            tile = self.routed_tile(pairs, n_experts, inner, E)
-            n_tiles = self.lib.raw("rb_routed_tiles")(pairs, n_experts, tile)
-            rows = n_tiles * tile
-            plan = torch.empty((pairs + rows + n_tiles,), dtype=torch.int32, device=self.device)
-            pos, row_token, tile_group = plan[:pairs], plan[pairs:pairs + rows], plan[pairs + rows:]
-            xp = torch.empty((rows, E), dtype=self.dtype, device=self.device)
-            place = self.place_few_pairs and pairs <= self.lib.raw("rb_routed_place_pairs")()
-            if place:
-                self.lib.call("rb_routed_place", _ptr(xp), _ptr(pos), _ptr(tile_group), _ptr(h), h.stride(0), self.code, _ptr(ids),
-                              _ptr(weights if weight_on_input else None), pairs, top, n_experts, tile, n_tiles, E, self._stream())
+            groups = n_experts
+            if placed is not None:
+                tile, pos, tile_group, xp, rows = placed.tile, placed.pos, placed.tile_group, placed.rows, placed.rows.shape[0]
+                groups += 1 if placed.n_shared else 0
             else:
-                self.lib.call("rb_routed_plan", _ptr(pos), _ptr(row_token), _ptr(tile_group), _ptr(ids), pairs, top, n_experts,
-                              tile, n_tiles, self._stream())
-            if place:
-                pass
-            elif weight_on_input:
-                self.lib.call("rb_routed_gather_scaled", _ptr(xp), _ptr(h), h.stride(0), self.code, _ptr(row_token), _ptr(pos),
-                              _ptr(weights), top, rows, E, self._stream())
-            else:
-                self.lib.call("rb_routed_gather", _ptr(xp), _ptr(h), h.stride(0), self.code, _ptr(row_token), rows, E, self._stream())
+                xp, pos, tile_group, tile, rows = self._place(h, ids, weights if weight_on_input else None, top, n_experts, inner)
             mid = torch.empty((rows, inner), dtype=self.dtype, device=self.device)
             y = torch.empty((rows, E), dtype=torch.float32, device=self.device)
             if act is not None:
@@ -1461,11 +1529,11 @@ class CudaOps:
                     self._next_gated_act(act)
                     self.lib.call("rb_gemm_tc_grouped", _ptr(tile_group), launches=0)
                     self.lib.call("rb_gemm_tc", _ptr(mid), mid.stride(0), self.code, _ptr(xp), xp.stride(0), rows, _ptr(w_up.w),
-                                  w_up.w.stride(0), n_experts * per, per, E, 3, inner, 1, tile, 1.0, self._stream())
+                                  w_up.w.stride(0), groups * per, per, E, 3, inner, 1, tile, 1.0, self._stream())
                 elif tc:
                     self.lib.call("rb_gemm_tc_grouped", _ptr(tile_group), launches=0)
                     self.lib.call("rb_gemm_tc", _ptr(gu), gu.stride(0), F32, _ptr(xp), xp.stride(0), rows, _ptr(w_up.w),
-                                  w_up.w.stride(0), n_experts * per, per, E, 0, 0, 1, tile, 1.0, self._stream())
+                                  w_up.w.stride(0), groups * per, per, E, 0, 0, 1, tile, 1.0, self._stream())
                 else:
                     self.lib.call("rb_gemm_grouped_simple", _ptr(gu), gu.stride(0), F32, _ptr(xp), xp.stride(0), _ptr(w_up.w),
                                   w_up.w.stride(0), self.code, _ptr(tile_group), rows, per, E, 0, self._stream())
@@ -1474,7 +1542,7 @@ class CudaOps:
                 if tc:
                     self.lib.call("rb_gemm_tc_grouped", _ptr(tile_group), launches=0)
                     self.lib.call("rb_gemm_tc", _ptr(y), y.stride(0), F32, _ptr(mid), mid.stride(0), rows, _ptr(w_down.w),
-                                  w_down.w.stride(0), n_experts * E, E, inner, 0, 0, 1, tile, 1.0, self._stream())
+                                  w_down.w.stride(0), groups * E, E, inner, 0, 0, 1, tile, 1.0, self._stream())
                 else:
                     self.lib.call("rb_gemm_grouped_simple", _ptr(y), y.stride(0), F32, _ptr(mid), mid.stride(0), _ptr(w_down.w),
                                   w_down.w.stride(0), self.code, _ptr(tile_group), rows, E, inner, 0, self._stream())
@@ -1482,10 +1550,10 @@ class CudaOps:
                 self.lib.call("rb_gemm_tc_square_relu", launches=0)
                 self.lib.call("rb_gemm_tc_grouped", _ptr(tile_group), launches=0)
                 self.lib.call("rb_gemm_tc", _ptr(mid), mid.stride(0), self.code, _ptr(xp), xp.stride(0), rows, _ptr(w_up.w),
-                              w_up.w.stride(0), n_experts * inner, inner, E, 0, 0, 1, tile, 1.0, self._stream())
+                              w_up.w.stride(0), groups * inner, inner, E, 0, 0, 1, tile, 1.0, self._stream())
                 self.lib.call("rb_gemm_tc_grouped", _ptr(tile_group), launches=0)
                 self.lib.call("rb_gemm_tc", _ptr(y), y.stride(0), F32, _ptr(mid), mid.stride(0), rows, _ptr(w_down.w),
-                              w_down.w.stride(0), n_experts * E, E, inner, 0, 0, 1, tile, 1.0, self._stream())
+                              w_down.w.stride(0), groups * E, E, inner, 0, 0, 1, tile, 1.0, self._stream())
             else:
                 self.lib.call("rb_gemm_grouped_simple", _ptr(mid), mid.stride(0), self.code, _ptr(xp), xp.stride(0), _ptr(w_up.w),
                               w_up.w.stride(0), self.code, _ptr(tile_group), rows, inner, E, 1, self._stream())
@@ -1495,6 +1563,8 @@ class CudaOps:
             pos = torch.full((pairs,), -1, dtype=torch.int32, device=self.device)
         if shared is not None or isinstance(then_norm, TanhRequest):
             z, gate = shared if shared is not None else (None, None)
+            if placed is not None and placed.n_shared:
+                z = y                                   # the tokens' own rows are the buffer's first
             if z is not None:
                 self._check(z, torch.float32, "shared expert's rows")
             req = then_norm if isinstance(then_norm, TanhRequest) else None

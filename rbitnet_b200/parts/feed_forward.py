@@ -150,7 +150,8 @@ class RoutedExperts(FeedForward):
             if not 1 <= self.keep <= self.groups:
                 raise ValueError(f"routed experts: {self.keep} of {self.groups} groups kept")
         self.router = self.router_tc = self.correction = self.w_up = self.w_down = None
-        self.shared_gate_up = self.shared_down = None
+        self.shared_gate_up = self.shared_down = self.shared_pair = None
+        self.shared_is_expert = False
 
     @property
     def plain(self) -> bool:
@@ -185,23 +186,50 @@ class RoutedExperts(FeedForward):
         # where the operations can make the same float32 sums on the tensor cores, they say so here
         prepare = getattr(ops, "prepare_router", None)
         self.router_tc = prepare(self.router) if prepare is not None else None
+        # a shared expert that is one more of the same form lies behind the others, for steps that take it with them
+        self.shared_is_expert = (self.n_experts > 0 and self.shared is not None and self.act is not None
+                                 and self.shared["inner"] == self.inner and (self.shared["act"] or (1.0, 0.0, 0.0)) == self.act
+                                 and hasattr(ops, "expert_of"))
+        names = [f"e{e}" for e in range(self.n_experts)] + (["shared"] if self.shared_is_expert else [])
         if self.n_experts:
             # the experts' matrices one below the other: [n_experts * rows, width] and [n_experts * width, inner]
             if self.act is None:
-                self.w_up = ops.prepare_linear([weights[f"e{e}.up"] for e in range(self.n_experts)])
+                self.w_up = ops.prepare_linear([weights[f"{e}.up"] for e in names])
             else:
-                self.w_up = ops.prepare_expert_gate_up([weights[f"e{e}.gate"] for e in range(self.n_experts)],
-                                                       [weights[f"e{e}.up"] for e in range(self.n_experts)])
-            self.w_down = ops.prepare_linear([weights[f"e{e}.down"] for e in range(self.n_experts)])
-        if self.shared is not None:
+                self.w_up = ops.prepare_expert_gate_up([weights[f"{e}.gate"] for e in names], [weights[f"{e}.up"] for e in names])
+            self.w_down = ops.prepare_linear([weights[f"{e}.down"] for e in names])
+        if self.shared_is_expert:
+            self.shared_pair = ops.expert_of(self.w_up, self.w_down, self.n_experts)
+        elif self.shared is not None:
             self.shared_gate_up = ops.prepare_gate_up(weights["shared.gate"], weights["shared.up"])
             self.shared_down = ops.prepare_linear([weights["shared.down"]])
+            self.shared_pair = (self.shared_gate_up, self.shared_down)
 
     #: ``then_norm`` is handed to the weighted sum, which grants a norm that needs no sums over the row
     passes_norms = True
 
     def forward(self, ctx, h, accumulate_into=None, then_norm=None):
         ops = ctx.ops
+        extra = 1 if self.shared is not None and self.shared["gate"] else 0
+        weighing = {}
+        if self.normalize is not None or self.weight_scale != 1.0:
+            weighing = {"normalize": self.normalize, "weight_scale": self.weight_scale}
+        kw = {}
+        if then_norm is not None:
+            kw["then_norm"] = then_norm
+        # a few tokens: choice and placing in one, and the shared expert as one more group of the experts' products
+        if hasattr(ops, "route_and_place"):
+            placed = ops.route_and_place(h, self.router, self.correction, self.top, self.groups, self.keep, self.n_experts, self.inner,
+                                         scoring=self.scoring, extra_rows=extra, weight_on_input=self.weight_on == "input",
+                                         with_shared=self.shared_is_expert, **weighing)
+            if placed is not None:
+                if placed.n_shared:
+                    kw["shared"] = (None, placed.extra)
+                elif self.shared is not None:
+                    kw["shared"] = (self._shared(ops, h), placed.extra)
+                return ops.routed_experts(h, None, None, self.w_up, self.w_down, self.n_experts, self.inner,
+                                          accumulate_into=accumulate_into, act=self.act, weight_on_input=self.weight_on == "input",
+                                          placed=placed, **kw)
         if self.plain:
             if self.router_tc is not None:
                 ids, weights = ops.route(h, self.router, self.correction, self.top, self.groups, self.keep, router_tc=self.router_tc)
@@ -209,22 +237,19 @@ class RoutedExperts(FeedForward):
                 ids, weights = ops.route(h, self.router, self.correction, self.top, self.groups, self.keep)
             return ops.routed_experts(h, ids, weights, self.w_up, self.w_down, self.n_experts, self.inner,
                                       accumulate_into=accumulate_into)
-        extra = 1 if self.shared is not None and self.shared["gate"] else 0
-        kw = {}
-        if self.normalize is not None or self.weight_scale != 1.0:
-            kw = {"normalize": self.normalize, "weight_scale": self.weight_scale}
         ids, weights, gate = ops.route_scored(h, self.router, self.correction, self.top, self.groups, self.keep,
-                                              scoring=self.scoring, extra_rows=extra, router_tc=self.router_tc, **kw)
-        kw = {}
+                                              scoring=self.scoring, extra_rows=extra, router_tc=self.router_tc, **weighing)
         if self.shared is not None:
-            t = ops.gated_linear(h, self.shared_gate_up, act=self.shared["act"])
             # sigmoid(gate) * z, one number per row, is added beside the experts' results
-            kw["shared"] = (ops.linear(t, self.shared_down, out_dtype=torch.float32), gate)
-        if then_norm is not None:
-            kw["then_norm"] = then_norm
+            kw["shared"] = (self._shared(ops, h), gate)
         return ops.routed_experts(h, ids, weights, self.w_up, self.w_down, self.n_experts, self.inner,
                                   accumulate_into=accumulate_into, act=self.act,
                                   weight_on_input=self.weight_on == "input", **kw)
+
+    def _shared(self, ops, h):
+        """The shared expert's float32 rows."""
+        gate_up, down = self.shared_pair
+        return ops.linear(ops.gated_linear(h, gate_up, act=self.shared["act"]), down, out_dtype=torch.float32)
 
 
 register_part("feed_forward", "gated_dense", GatedDense)

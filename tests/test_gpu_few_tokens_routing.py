@@ -1,0 +1,119 @@
+"""The router of a few tokens: sums spread over the chip, the choice with a lane per output, the placing that makes the choice itself,
+and a shared expert that is one more group, each against the same thing in float64 or against the kernels apart."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+F32, BF16 = torch.float32, torch.bfloat16
+
+
+@pytest.fixture(scope="module")
+def ops_of():
+    from rbitnet_b200.kernels.ops import CudaOps
+    made = {}
+    return lambda dtype: made.setdefault(dtype, CudaOps(dtype, verbose_build=False))
+
+
+def _choice(z, corr, top, groups, keep, scoring, normalize, scale):
+    """Ids and weights of one token's sums z (float64)."""
+    n = len(z)
+    s = torch.softmax(z, 0) if scoring == "softmax" else torch.sigmoid(z) if scoring == "sigmoid" else z
+    c = s + (corr.double() if corr is not None else 0.0)
+    c = torch.where(torch.isnan(c), torch.tensor(-math.inf, dtype=c.dtype), c)      # not a number: never chosen
+    if groups > 1 and keep < groups:
+        best = c.view(groups, -1).max(1).values
+        order = sorted((g for g in range(groups) if best[g] > -math.inf), key=lambda g: (-float(best[g]), g))[:keep]
+        c = torch.where(torch.tensor([i // (n // groups) in order for i in range(n)]), c, torch.tensor(-math.inf, dtype=c.dtype))
+    ids = sorted((i for i in range(n) if c[i] > -math.inf), key=lambda i: (-float(c[i]), i))[:top]
+    w = [float(s[i]) for i in ids] + [0.0] * (top - len(ids))
+    ids += [0] * (top - len(ids))
+    w = torch.tensor(w, dtype=torch.float64)
+    if scoring == "softmax_chosen":
+        w = torch.softmax(w, 0)
+    if normalize is not None:
+        w = w / (w.sum() + normalize)
+    return ids, w * scale
+
+
+@pytest.mark.parametrize("n,groups,keep", [(1, 1, 1), (5, 0, 0), (32, 8, 4), (30, 3, 2), (31, 31, 5), (32, 1, 1), (32, 2, 1), (33, 0, 0), (48, 4, 2)])
+@pytest.mark.parametrize("scoring,normalize,scale", [("softmax", None, 1.0), ("sigmoid", 1e-20, 2.5), ("softmax_chosen", None, 1.0)])
+@pytest.mark.parametrize("T", [1, 9, 16, 17])
+def test_choices(ops_of, n, groups, keep, scoring, normalize, scale, T):
+    """Up to 32 outputs and more, in groups or not, ties, outputs that cannot be chosen, fewer choosable ones than choices; the
+    same ids and weights from the kernel that also places (up to 16 tokens)."""
+    ops = ops_of(F32)
+    g = torch.Generator(device="cuda").manual_seed(n * 31 + T)
+    K, top = 260, min(4, n)
+    h = torch.randn(T, K, device="cuda", generator=g)
+    router = torch.randn(n, K, device="cuda", generator=g) / math.sqrt(K)
+    h[0] = 0.0                                                   # all sums equal: the lowest outputs
+    corr = 0.3 * torch.randn(n, device="cuda", generator=g)
+    corr[::3] = -math.inf
+    corr[1::5] = float("nan") if n > 10 else 0.0
+    for c in ((None, corr) if groups == 0 or n > 1 else (None,)):
+        ids, w, _ = ops.route_scored(h, router, c, top, groups, keep, scoring=scoring, normalize=normalize, weight_scale=scale)
+        for t in range(T):
+            z = (h[t].double() @ router.double().T).cpu()
+            want_ids, want = _choice(z, None if c is None else c.cpu(), top, groups, keep, scoring, normalize, scale)
+            assert ids[t].tolist() == want_ids
+            # float32 sums of 260 products of about 1/16, an exponential or two, a division
+            assert torch.allclose(w[t].double().cpu(), want, rtol=2e-5, atol=1e-7)
+        placed = ops.route_and_place(h, router, c, top, groups, keep, n, 64, scoring=scoring, normalize=normalize, weight_scale=scale)
+        assert (placed is None) == (T > 16)
+        if placed is not None:
+            assert torch.equal(placed.weights, w)
+            rows = placed.pos.view(T, top)
+            assert torch.equal(placed.rows[rows.flatten().long()], h.repeat_interleave(top, 0))
+            assert torch.equal(placed.tile_group[(rows // placed.tile).long()], ids)
+
+
+@pytest.mark.parametrize("dtype", [F32, BF16])
+@pytest.mark.parametrize("K", [4, 96, 2048, 2052, 4100])
+def test_sums_of_few_tokens(ops_of, dtype, K):
+    """Rows of up to 2,048 values and longer ones.  A float32 sum of K products is within K 2^-24 of the sum of their magnitudes."""
+    from rbitnet_b200.kernels.ops import _ptr
+    ops = ops_of(dtype)
+    g = torch.Generator(device="cuda").manual_seed(K)
+    for T, n in ((1, 1), (7, 33), (63, 130)):
+        h = torch.randn(T, K, device="cuda", generator=g).to(dtype)
+        w = torch.randn(n, K, device="cuda", generator=g)
+        z = torch.empty(T, n, device="cuda")
+        ops.lib.call("rb_route_sums", _ptr(z), _ptr(h), K, ops.code, _ptr(w), T, K, n, ops._stream())
+        bound = (K + 2) * 2.0 ** -24 * (h.double().abs() @ w.double().abs().T)
+        assert ((z.double() - h.double() @ w.double().T).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("dtype", [F32, BF16])
+@pytest.mark.parametrize("T,experts,inner,E,identity", [(1, 32, 88, 128, 0), (5, 6, 40, 96, 0), (16, 3, 64, 200, 0), (3, 40, 24, 64, 8)])
+@pytest.mark.parametrize("weight_on_input", [False, True])
+def test_a_shared_expert_behind_the_others(ops_of, dtype, T, experts, inner, E, identity, weight_on_input):
+    """The shared expert's rows ahead of the pairs' in one buffer, its matrices behind the others', beside the same made apart."""
+    if identity and weight_on_input:
+        pytest.skip("identity experts go with weights on the results")
+    ops = ops_of(dtype)
+    g = torch.Generator(device="cuda").manual_seed(T + experts)
+
+    def m(*shape):
+        return torch.randn(*shape, device="cuda", generator=g).to(dtype) / math.sqrt(shape[-1])
+    gates, ups, downs = ([m(*s) for _ in range(experts + 1)] for s in ((inner, E), (inner, E), (E, inner)))
+    w_up, w_down = ops.prepare_expert_gate_up(gates, ups), ops.prepare_linear(downs)
+    gate_up, down = ops.expert_of(w_up, w_down, experts)
+    h = torch.randn(T, E, device="cuda", generator=g).to(dtype)
+    router = torch.randn(experts + identity + 1, E, device="cuda", generator=g) / math.sqrt(E)
+    act, top = (1.0, 0.0, 0.0), 2
+    ids, w, gate = ops.route_scored(h, router, None, top, 0, 0, scoring="sigmoid", extra_rows=1)
+    shared = ops.linear(ops.gated_linear(h, gate_up, act=act), down, out_dtype=F32)
+    x0 = torch.randn(T, E, device="cuda", generator=g)
+    apart, one = x0.clone(), x0.clone()
+    kw = {"act": act, "weight_on_input": weight_on_input}
+    ops.routed_experts(h, ids, w, w_up, w_down, experts, inner, accumulate_into=apart, shared=(shared, gate), **kw)
+    placed = ops.route_and_place(h, router, None, top, 0, 0, experts, inner, scoring="sigmoid", extra_rows=1,
+                                 weight_on_input=weight_on_input, with_shared=True)
+    assert placed.n_shared == -(-T // placed.tile) and torch.equal(placed.weights, w) and torch.equal(placed.extra, gate)
+    ops.routed_experts(h, None, None, w_up, w_down, experts, inner, accumulate_into=one, shared=(None, placed.extra), placed=placed, **kw)
+    # sums of up to 200 products in another order, one rounding of the inner rows to the compute dtype
+    bound = 1e-5 if dtype == F32 else 1e-2
+    assert float((one - apart).norm() / (apart - x0).norm()) < bound
+    ops.check_errors()
