@@ -74,6 +74,7 @@ struct QkvTail {
 template <bool BY_TMA> struct OutputMap { using type = CUtensorMap; };
 template <> struct OutputMap<false> { struct type { int none; }; };
 template <int BN, int EPI> constexpr bool leaves_by_tma() { return BN >= 128 && EPI != EPI_QKV; }
+template <int N> struct Int { static constexpr int value = N; };
 // Tiles that leave by TMA have two groups of four epilogue warps, the others one.
 constexpr int LEAVE_GROUPS = 2, LEAVE_STAGE_BYTES = 16 * 1024;      // staging room of a group
 template <int BN, int EPI> constexpr int block_threads() { return leaves_by_tma<BN, EPI>() ? 64 + 128 * LEAVE_GROUPS : 192; }
@@ -750,10 +751,6 @@ gemm_wx_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
       const int n = n0 + quarter * 32 + lane;
       const int my = (int)cluster_rank();
       const uint32_t red = smem_u32(smem) + (uint32_t)(quarter * 32 + lane) * 4;
-      uint32_t remote[8];
-#pragma unroll
-      for (int r = 0; r < 8; ++r)
-        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote[r]) : "r"(red), "r"((uint32_t)(r < p.splits ? r : 0)));
       // (every lane walks the loop, also one whose weight row is beyond the matrix: the warp adds up
       // squares together below)
       const bool n_in = n < p.n_out;
@@ -764,12 +761,21 @@ gemm_wx_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
       const float bias_n = p.bias != nullptr && n_in ? p.bias[n] : 0.f;
       const bool emit_tanh = emit && p.emit_b != nullptr;
       const float b_n = emit_tanh && n_in ? p.emit_b[n] : 0.f;
-      {
-        constexpr int CPI = BN >= 64 ? 8 : (BN >= 32 ? 4 : 2);      // columns whose loads are in flight together
+      auto add_up = [&](auto known) {
+        // Tiles of 32 and 64 tokens in 2 or 4 parts: all the loads of the CTA's share in flight at once.  In rounds of eight columns
+        // (four of 32 tokens) each round waited for the others' memory: us before and now, 64 tokens in 2 parts, 2,048 x 2,048 16.7,
+        // 11.1; 4,096 x 4,096 22.6, 16.9; in 4 parts 10.4, 8.5; 14.8, 12.9; two tiles of 32 in 4 parts 7.1, 6.2; 12.3, 11.4.  (8 parts
+        // were one round.  Tiles of 16 tokens gain nothing, and more code costs their short kernels 1-2 %.)
+        constexpr int KNOWN = decltype(known)::value, PARTS = KNOWN > 0 ? KNOWN : 8;
+        constexpr int CPI = KNOWN > 0 && BN <= 64 ? BN / KNOWN : (BN >= 64 ? 8 : (BN >= 32 ? 4 : 2));
+        uint32_t remote[PARTS];
+#pragma unroll
+        for (int r = 0; r < PARTS; ++r)
+          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote[r]) : "r"(red), "r"((uint32_t)(KNOWN > 0 || r < p.splits ? r : 0)));
         for (int cb = 0; cb < BN; cb += CPI * p.splits) {
           int col[CPI];
           bool ok[CPI];
-          float old[CPI], part[CPI][8];
+          float old[CPI], part[CPI][PARTS];
 #pragma unroll
           for (int h = 0; h < CPI; ++h) {
             col[h] = cb + h * p.splits + my;
@@ -780,9 +786,9 @@ gemm_wx_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
 #pragma unroll
           for (int h = 0; h < CPI; ++h)
 #pragma unroll
-            for (int r = 0; r < 8; ++r) {      // all loads first, then the sums in split order
+            for (int r = 0; r < PARTS; ++r) {      // all loads first, then the sums in split order
               part[h][r] = 0.f;
-              if (ok[h] && r < p.splits)
+              if (ok[h] && (KNOWN > 0 || r < p.splits))
                 asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(part[h][r]) : "r"(remote[r] + (uint32_t)(col[h] * BM) * 4));
             }
 #pragma unroll
@@ -793,7 +799,7 @@ gemm_wx_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
               // above): every lane adds up its parts, the halves meet by a shuffle, the lower lanes finish
               float v = part[h][0];
 #pragma unroll
-              for (int r = 1; r < 8; ++r) v += part[h][r];
+              for (int r = 1; r < PARTS; ++r) v += part[h][r];
               if (normed) v *= norm_r[column ? t0 + col[h] : 0];
               v += bias_n;
               const float up = __shfl_xor_sync(0xffffffffu, v, 16);
@@ -806,7 +812,7 @@ gemm_wx_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
             if (ok[h]) {
               float v = part[h][0];
 #pragma unroll
-              for (int r = 1; r < 8; ++r) v += part[h][r];
+              for (int r = 1; r < PARTS; ++r) v += part[h][r];
               v = v * (normed ? p.alpha * norm_r[t0 + col[h]] : p.alpha) + bias_n;
               const int64_t at = (int64_t)(t0 + col[h]) * p.ldc + n;
               if (EPI == EPI_ADD) {
@@ -828,6 +834,13 @@ gemm_wx_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
             }
           }
         }
+      };
+      if constexpr (BN == 32 || BN == 64) {
+        if (p.splits == 2) add_up(Int<2>());
+        else if (p.splits == 4) add_up(Int<4>());
+        else add_up(Int<0>());
+      } else {
+        add_up(Int<0>());
       }
     }
     __syncwarp();
@@ -1065,8 +1078,26 @@ RB_EXPORT int rb_wait_probe(long long limit_ns, int code, int* gave_up, cudaStre
 // piece of it: the tokens go in tiles of at most 64, and when the 128-row tiles of W times the token
 // tiles are fewer than the CTAs that run together (two per SM), K is cut as well: into 2, 4 or 8
 // parts, the sizes clusters schedule well, each of at least four 64-wide blocks.  Beyond 256 tokens: one.
+// 33 to 64 tokens take two tiles of 32 (rb_gemm_tc_few_tile) where that makes a tile's way out, half as long and summed over fewer
+// parts, worth reading W a second time from L2.  us, tiles of 64 and two of 32, each with the best parts, 64 tokens: 2,048 x 2,048 7.0,
+// 6.2; K 5,632 10.2, 9.5; 768 x 2,048 5.9, 5.2; 2,048 x 768 6.2, 5.4; 2,816 gated rows of 2,048 8.4, 7.6; 11,264 16.4, 13.9; with 48
+// tokens 6.3, 6.1; 9.6, 9.3; 11,264 15.5, 13.5.  Not where four parts of 64 fill the chip (5,632 gated rows 11.2, 11.4; 40 tokens 10.2,
+// 11.1; 8,192 stored 11.6, 11.5; 10.8, 11.4), nor where W is larger (4,096 x 14,336 25.3, 26.4; 28,672 x 4,096 43.9, 47.3).
+RB_EXPORT int rb_gemm_tc_few_tile(int n_tokens, int n_out, int K) {
+  const int w_tiles = (n_out + BM - 1) / BM;
+  return n_tokens > 32 && n_tokens <= 64 && (w_tiles <= 24 || (w_tiles >= 80 && w_tiles <= rb_sm_count())) && (int64_t)n_out * K <= (24 << 20) ? 32 : 0;
+}
+
 RB_EXPORT int rb_gemm_tc_splits(int n_tokens, int n_out, int K) {
   if (n_tokens > 256 || n_tokens <= 0 || n_out <= 0 || K <= 0) return 1;
+  if (rb_gemm_tc_few_tile(n_tokens, n_out, K) != 0) {
+    const int both = 2 * ((n_out + BM - 1) / BM), most = K >= 4096 ? 2 * rb_sm_count() : rb_sm_count() + rb_sm_count() / 3;
+    const int of_k = (K + BK - 1) / BK;
+    int parts = 1;
+    while (parts * 2 <= 8 && parts * 2 * both <= most && parts * 2 <= of_k / 4) parts *= 2;
+    const int each = (of_k + parts - 1) / parts;
+    return (of_k + each - 1) / each;
+  }
   const int tiles = ((n_out + BM - 1) / BM) * ((n_tokens + 63) / 64);
   const int blocks = (K + BK - 1) / BK;
   const int together = 2 * rb_sm_count();

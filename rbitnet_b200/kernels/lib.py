@@ -149,6 +149,7 @@ class KernelLibrary:
         self.declare("rb_attention_decode_tma_on_chip", [I, I, I])
         self.declare("rb_attention_decode_parts", [I, I, I])
         self.declare("rb_gemm_tc_splits", [I, I, I])
+        self.declare("rb_gemm_tc_few_tile", [I, I, I])
         self.declare("rb_gemm_tc_workspace_bytes", [], restype=ctypes.c_longlong)
         self.declare("rb_gated_delta_chunk_floats", [I, I], restype=ctypes.c_longlong)
         self.declare("rb_ssd_chunk_floats", [I, I], restype=ctypes.c_longlong)

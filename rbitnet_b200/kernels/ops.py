@@ -396,7 +396,7 @@ class CudaOps:
                 self.lib.call("rb_gemm_tc_bias", _ptr(bias), launches=0)
             self.lib.call("rb_gemm_tc", _ptr(out), out.stride(0), _CODE[out.dtype], _ptr(x), x.stride(0), T,
                           _ptr(weight.w), weight.w.stride(0), N, N, K, acc, 0, splits,
-                          64 if 64 < T <= 256 else 0, float(scale), self._stream())
+                          self._token_tile(T, N, K), float(scale), self._stream())
         else:
             if bias is not None:
                 self.lib.call("rb_gemm_simple_next", _ptr(bias), c_void_p(0), 0, 0, 1, launches=0)
@@ -451,10 +451,14 @@ class CudaOps:
         tokens; else up to 8, so that every SM streams a piece of W)."""
         return self.lib.raw("rb_gemm_tc_splits")(T, N, K)
 
+    def _token_tile(self, T: int, N: int, K: int) -> int:
+        """The token tile to ask for (0: the library's): 64 where K may be cut, two of 32 for the sizes of ``rb_gemm_tc_few_tile``."""
+        return 64 if 64 < T <= 256 else self.lib.raw("rb_gemm_tc_few_tile")(T, N, K)
+
     def _gated_splits(self, T: int, N: int, K: int):
         """(parts of K, token tile) of a gated product: those of ``gated_parts``, and tiles of 64 tokens at most beside them."""
         parts = gated_parts(T, N, K, self._k_splits(T, N, K), self.lib.raw("rb_device_sm_count")()) if self.split_gated else 1
-        return parts, 64 if parts > 1 and T > 64 else 0
+        return parts, self._token_tile(T, N, K) if parts > 1 or T <= 64 else 0
 
     def _tensor_core_ok(self, x: torch.Tensor, w: torch.Tensor) -> bool:
         """The tcgen05 product takes bfloat16 operands whose rows TMA can address: inner size and

@@ -160,3 +160,41 @@ def test_float32_products_that_are_not_finite(ops32, K):
     fin = torch.isfinite(ref)
     mag = torch.where(torch.isfinite(x), x, 0).double().abs() @ torch.where(torch.isfinite(w), w, 0).double().abs().T
     assert ((out.double() - ref).abs()[fin] <= ((K + 8) * 2.0 ** -24 * mag)[fin]).all()      # (K: the sums made by FFMA)
+
+
+@pytest.mark.parametrize("T,tile", [(1, 16), (5, 16), (16, 16), (30, 32), (33, 32), (64, 32), (50, 64), (64, 64)])
+@pytest.mark.parametrize("parts", [2, 3, 4, 5, 8])
+def test_parts_of_a_few_tokens_product(ops, T, tile, parts):
+    """Parts summed with all of a CTA's loads in flight (2, 4, 8) and in rounds (others), tokens that fill no tile, two tiles of 32."""
+    from rbitnet_b200.kernels.ops import _ptr, _CODE
+    g = torch.Generator(device="cuda").manual_seed(T * parts)
+    N, K = 416, 2552                                             # 40 blocks of K: whole parts but with 3
+    x = torch.randn(T, K, device="cuda", generator=g).to(BF16)
+    w = (torch.randn(N, K, device="cuda", generator=g) / math.sqrt(K)).to(BF16)
+    ref = x.double() @ w.double().T
+    pairs = w.view(N // 32, 2, 16, K)
+    gate, up = (x.double() @ pairs[:, h].reshape(-1, K).double().T for h in (0, 1))
+    for epilogue, c, want, bound in ((0, torch.full((T + 2, N), 7.0, device="cuda"), ref, 2e-5), (1, torch.ones((T + 2, N), device="cuda"), 1.0 + ref, 2e-5),
+                                     (3, torch.full((T + 2, N // 2), 7.0, dtype=BF16, device="cuda"), gate / (1 + torch.exp(-gate)) * up, 6e-3)):
+        keep = c[T:].clone()
+        ops.lib.call("rb_gemm_tc", _ptr(c), c.stride(0), _CODE[c.dtype], _ptr(x), K, T, _ptr(w), K, N, N, K, epilogue,
+                     c.shape[1] if epilogue == 3 else 0, parts, tile, 1.0, ops._stream())
+        assert _rel(c[:T], want) < bound and torch.equal(c[T:], keep)
+    ops.check_errors()
+
+
+@pytest.mark.parametrize("T", [33, 48, 64])
+@pytest.mark.parametrize("N,K", [(2048, 2048), (96, 2048), (10304, 520), (2048, 768)])
+def test_two_tiles_of_32_tokens(ops, T, N, K):
+    """What the operations choose for 33 to 64 tokens, stored, added and gated."""
+    assert ops._token_tile(T, N, K) == 32 and ops._token_tile(32, N, K) == 0
+    g = torch.Generator(device="cuda").manual_seed(T)
+    x = torch.randn(T, K, device="cuda", generator=g).to(BF16)
+    w = (torch.randn(N, K, device="cuda", generator=g) / math.sqrt(K)).to(BF16)
+    ref, lw = x.double() @ w.double().T, ops.prepare_linear([w])
+    acc = torch.ones(T, N, device="cuda")
+    ops.linear(x, lw, accumulate_into=acc)
+    assert _rel(ops.linear(x, lw, out_dtype=F32), ref) < 2e-5 and _rel(acc, 1.0 + ref) < 2e-5
+    gate, up = ref[:, :N // 2], ref[:, N // 2:]
+    assert _rel(ops.gated_linear(x, ops.prepare_gate_up(w[:N // 2], w[N // 2:])), gate / (1 + torch.exp(-gate)) * up) < 6e-3
+    ops.check_errors()
