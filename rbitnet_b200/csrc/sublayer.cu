@@ -269,6 +269,73 @@ __global__ void __launch_bounds__(256) norm_filter_rows_kernel(TO* h, TO* hf, fl
   }
 }
 
+// The same for parts of up to 1,024 values and up to four taps: a thread has four neighbouring channels, which stay in registers,
+// the norm's weights, the taps and the bias are asked for before the wait for the kernel before, and the ring's rows as soon as
+// the position is known, not after the norm: 8 rows in 2 parts of 1,024 values 6.3 us of a step above, here 2.7.
+template <typename TO, int K>
+__global__ void __launch_bounds__(256) norm_filter_part_kernel(TO* h, TO* hf, float* x, const float* y, const float* g, int64_t ldg,
+                                                               const float* bias, const float* w, int E, int groups, float eps,
+                                                               const float* taps, float* ring, const int* tok_slot, const int* tok_pos) {
+  rb_pdl_launch_dependents();
+  __shared__ float s_parts[8];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int t = blockIdx.x, per = E / groups, c = blockIdx.y * per + 4 * threadIdx.x;
+  const bool live = 4 * (int)threadIdx.x < per;
+  float ww[4] = {0.f, 0.f, 0.f, 0.f}, bb[4] = {0.f, 0.f, 0.f, 0.f}, tap[4 * K];
+  if (live) {
+    rb_load4(w + c, ww);
+    if (y != nullptr && bias != nullptr) rb_load4(bias + c, bb);
+#pragma unroll
+    for (int i = 0; i < K; ++i) {                    // four channels' K taps are neighbours
+      float four[4];
+      rb_load4(taps + (int64_t)c * K + 4 * i, four);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) tap[4 * i + q] = four[q];
+    }
+  }
+  rb_pdl_wait();
+  const int slot = tok_slot[t], pos = tok_pos[t];
+  float v[4] = {0.f, 0.f, 0.f, 0.f}, back[K][4];
+  float* row = x + (int64_t)t * E;
+  if (live) {
+    rb_load4(row + c, v);
+    if (y != nullptr) {
+      float yy[4], z[4];
+      rb_load4(y + (int64_t)t * E + c, yy);
+      rb_load4(g + (int64_t)t * ldg + c, z);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) v[q] = fmaf(yy[q], sigmoid_(z[q] + bb[q]), v[q]);
+      rb_store4(row + c, v);
+    }
+#pragma unroll
+    for (int d = 1; d < K; ++d)
+      if (pos - d >= 0) rb_load4(ring + ((int64_t)slot * K + (pos - d) % K) * E + c, back[d]);
+  }
+  float ss = fmaf(v[0], v[0], fmaf(v[1], v[1], fmaf(v[2], v[2], fmaf(v[3], v[3], 0.f))));
+  ss = rb_warp_sum(ss);
+  if (lane == 0) s_parts[warp] = ss;
+  __syncthreads();
+  ss = 0.f;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) ss += s_parts[k];
+  if (!live) return;
+  const float r = 1.0f / sqrtf(ss / (float)per + eps);
+  float own[4], acc[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    own[q] = rb_to_float<TO>(rb_from_float<TO>(v[q] * r * ww[q]));    // as the rows leave
+    acc[q] = fmaf(tap[q * K + K - 1], own[q], own[q]);
+  }
+  store4(h + (int64_t)t * E + c, own[0], own[1], own[2], own[3]);
+#pragma unroll
+  for (int d = 1; d < K; ++d)
+    if (pos - d >= 0)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) acc[q] = fmaf(tap[q * K + K - 1 - d], back[d][q], acc[q]);
+  store4(hf + (int64_t)t * E + c, acc[0], acc[1], acc[2], acc[3]);
+  if (K > 1) rb_store4(ring + ((int64_t)slot * K + pos % K) * E + c, own);
+}
+
 // ---------------------------------------------------------------- gated residual
 template <typename TG>
 __global__ void gated_add_kernel(float* x, const float* y, const TG* g, int64_t ldg,
@@ -425,6 +492,16 @@ RB_EXPORT int rb_norm_filter_rows(void* h, void* hf, int dtype, float* x, const 
              "rb_norm_filter_rows: parts of %d values or addresses do not allow 16 bytes a load", E / groups);
   const int threads = 256;
   const size_t smem = 0;
+  RB_REQUIRE(dtype == RB_F32 || dtype == RB_BF16, "rb_norm_filter_rows: unknown dtype %d", dtype);
+  if (E / groups <= 1024 && K <= 4 && groups <= 65535 && (uintptr_t)taps % 16 == 0) {
+#define GO(TO, KT) RB_LAUNCH("norm_filter_part_kernel", (norm_filter_part_kernel<TO, KT>), dim3(T, groups), threads, 0, stream, (TO*)h, (TO*)hf, x, y, g, ldg, bias, w, E, groups, eps, taps, ring, tok_slot, tok_pos)
+#define OF_TAPS(TO) do { if (K == 1) GO(TO, 1); else if (K == 2) GO(TO, 2); else if (K == 3) GO(TO, 3); else GO(TO, 4); } while (0)
+    if (dtype == RB_F32) OF_TAPS(float); else OF_TAPS(__nv_bfloat16);
+#undef OF_TAPS
+#undef GO
+    RB_CHECK_LAUNCH("rb_norm_filter_rows");
+    return 0;
+  }
   const dim3 grid(T, groups < 64 ? groups : 64);
   if (dtype == RB_F32)
     RB_LAUNCH("norm_filter_rows_kernel", (norm_filter_rows_kernel<float>), grid, threads, smem, stream, (float*)h, (float*)hf, x, y, g, ldg, bias, w, E, groups, eps, taps, ring, tok_slot, tok_pos, K);

@@ -186,6 +186,14 @@ class Model:
                 if taps is not None:
                     taps.append(ops.streams_sum(x, s) if s > 1 else x.clone())
                 continue
+            if getattr(block, "chains_results", False):
+                # a block whose last result may wait for the next block's first norm, which adds it (see parts/block.py)
+                after = self.blocks[schedule[e + 1].layer] if e + 1 < len(schedule) else None
+                hand_on = getattr(after, "chains_results", False) and not schedule[e + 1].adds_embedding and taps is None
+                pending = block.run(ctx, x, e, waiting=pending, hand_on=hand_on)
+                if taps is not None:
+                    taps.append(x.clone())
+                continue
             if getattr(block, "chains_rows", False):
                 # a block whose last addition also leaves the rows in the compute dtype, which the block after reads
                 # (see parts/block.py); the last block of the schedule leaves none

@@ -163,7 +163,10 @@ class GatedPreNormBlock:
     "mixer_filter" (role "input_filter"), "mixer_gate" (role "result_gate"); "feed_forward" with "ffn_norm" and
     optionally "ffn_filter", "ffn_gate".  Without a gate the sublayer adds its result itself; without a filter it
     reads the normed rows.  A filter's per-sequence state belongs to the run of the layer
-    (``ctx.part_state(entry, name)``)."""
+    (``ctx.part_state(entry, name)``).  A block's last gated result may be left to the block after it, whose first norm adds it
+    (``chains_results``)."""
+
+    chains_results = True
 
     def __init__(self, spec):
         self.spec = spec
@@ -183,12 +186,13 @@ class GatedPreNormBlock:
     def parts(self):
         return self._parts
 
-    def run(self, ctx, x, entry: int):
+    def run(self, ctx, x, entry: int, waiting=None, hand_on: bool = False):
+        """``waiting``: what the block before has not yet added to x; with ``hand_on`` this block's is returned so."""
         # Where the operations have it, a step of one token per sequence takes what lies between two sublayers (the
         # gated result of the one, the norm and the filter of the next) as one operation; a gated result therefore
-        # waits until the next norm, or the block's end, asks for the residual stream.
+        # waits until the next norm, of this block or of the next, or the last block's end asks for the residual stream.
         rows_between = getattr(ctx.ops, "norm_filter_rows", None)
-        waiting = None                                     # (gate, y, logits) not yet added to x
+        # waiting: (gate, y, logits) not yet added to x
 
         def settle():
             nonlocal waiting
@@ -221,7 +225,10 @@ class GatedPreNormBlock:
             y = part.forward(ctx, hf, entry, accumulate_into=into) if is_mixer else part.forward(ctx, hf, accumulate_into=into)
             if gate is not None:
                 waiting = (gate, y, logits)
+        if hand_on:
+            return waiting
         settle()
+        return None
 
 
 class PostNormBlock:
