@@ -303,28 +303,40 @@ __global__ void __launch_bounds__(FEW_WARPS * 32) per_head_few_rows_kernel(
     TC* C, int64_t ldc, const TA* A, int64_t lda, int head_a, const TA* W, int M, int N,
     int K, Tail tail) {
   rb_pdl_launch_dependents();
-  rb_pdl_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int h = blockIdx.y, n0 = (blockIdx.x * FEW_WARPS + warp) * FEW_OUTS;
   if (n0 >= N) return;
   const TA* w = W + ((int64_t)h * N + n0) * K;
   const TA* a = A + (int64_t)h * head_a;
+  constexpr int V = VEC ? 4 : 1;
+  auto fetch = [&](int k, float (&wv)[FEW_OUTS][4]) {
+#pragma unroll
+    for (int o = 0; o < FEW_OUTS; ++o) {
+      const bool have = n0 + o < N && k < K;
+      if (VEC) {
+        if (have) rb_load4(w + (int64_t)o * K + k, wv[o]);
+        else wv[o][0] = wv[o][1] = wv[o][2] = wv[o][3] = 0.f;
+      } else {
+        wv[o][0] = have ? rb_to_float<TA>(w[(int64_t)o * K + k]) : 0.f;
+      }
+    }
+  };
+  float first[FEW_OUTS][4];                              // the matrices do not depend on the kernel before
+  fetch(lane * V, first);
+  rb_pdl_wait();
   for (int m0 = 0; m0 < M; m0 += FEW_ROWS) {
     float acc[FEW_OUTS * FEW_ROWS];
 #pragma unroll
     for (int i = 0; i < FEW_OUTS * FEW_ROWS; ++i) acc[i] = 0.f;
-    constexpr int V = VEC ? 4 : 1;
     for (int k = lane * V; k < K; k += 32 * V) {
       float wv[FEW_OUTS][4];
+      if (k == lane * V) {
 #pragma unroll
-      for (int o = 0; o < FEW_OUTS; ++o) {
-        const bool have = n0 + o < N;
-        if (VEC) {
-          if (have) rb_load4(w + (int64_t)o * K + k, wv[o]);
-          else wv[o][0] = wv[o][1] = wv[o][2] = wv[o][3] = 0.f;
-        } else {
-          wv[o][0] = have ? rb_to_float<TA>(w[(int64_t)o * K + k]) : 0.f;
-        }
+        for (int o = 0; o < FEW_OUTS; ++o)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) wv[o][j] = first[o][j];
+      } else {
+        fetch(k, wv);
       }
 #pragma unroll
       for (int i = 0; i < FEW_ROWS; ++i) {

@@ -77,9 +77,26 @@ __global__ void __launch_bounds__(FEW_WARPS * 32) latent_queries_few_kernel(
     T* out, const T* q, const T* W, const double* freq, float magnitude,
     int interleaved, const int* tok_pos, int M, int H, int D, int R, int C, int width, int dot_blocks) {
   rb_pdl_launch_dependents();
-  rb_pdl_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int h = blockIdx.y, Dq = D + R;
+  constexpr int V = VEC ? 4 : 1;
+  const int n0 = (blockIdx.x * FEW_WARPS + warp) * FEW_OUTS;      // (of a block that makes dot products)
+  const T* w = W + ((int64_t)h * C + n0) * D;
+  auto fetch = [&](int k, float (&wv)[FEW_OUTS][4]) {
+#pragma unroll
+    for (int o = 0; o < FEW_OUTS; ++o) {
+      const bool have = n0 + o < C && k < D;
+      if (VEC) {
+        if (have) rb_load4(w + (int64_t)o * D + k, wv[o]);
+        else wv[o][0] = wv[o][1] = wv[o][2] = wv[o][3] = 0.f;
+      } else {
+        wv[o][0] = have ? rb_to_float<T>(w[(int64_t)o * D + k]) : 0.f;
+      }
+    }
+  };
+  float first[FEW_OUTS][4];                              // the matrices do not depend on the kernel before
+  if ((int)blockIdx.x < dot_blocks) fetch(lane * V, first);
+  rb_pdl_wait();
   const int64_t ldq = (int64_t)H * Dq, ldo = (int64_t)H * width;
   const T* qh = q + (int64_t)h * Dq;
   T* dst = out + (int64_t)h * width;
@@ -103,25 +120,20 @@ __global__ void __launch_bounds__(FEW_WARPS * 32) latent_queries_few_kernel(
     }
     return;
   }
-  const int n0 = (blockIdx.x * FEW_WARPS + warp) * FEW_OUTS;
   if (n0 >= C) return;
-  const T* w = W + ((int64_t)h * C + n0) * D;
   for (int m0 = 0; m0 < M; m0 += FEW_ROWS) {
     float acc[FEW_OUTS * FEW_ROWS];
 #pragma unroll
     for (int i = 0; i < FEW_OUTS * FEW_ROWS; ++i) acc[i] = 0.f;
-    constexpr int V = VEC ? 4 : 1;
     for (int k = lane * V; k < D; k += 32 * V) {
       float wv[FEW_OUTS][4];
+      if (k == lane * V) {
 #pragma unroll
-      for (int o = 0; o < FEW_OUTS; ++o) {
-        const bool have = n0 + o < C;
-        if (VEC) {
-          if (have) rb_load4(w + (int64_t)o * D + k, wv[o]);
-          else wv[o][0] = wv[o][1] = wv[o][2] = wv[o][3] = 0.f;
-        } else {
-          wv[o][0] = have ? rb_to_float<T>(w[(int64_t)o * D + k]) : 0.f;
-        }
+        for (int o = 0; o < FEW_OUTS; ++o)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) wv[o][j] = first[o][j];
+      } else {
+        fetch(k, wv);
       }
 #pragma unroll
       for (int i = 0; i < FEW_ROWS; ++i) {

@@ -585,7 +585,7 @@ struct Moved {
 template <typename TI, typename TO>
 __global__ void head_norm_gate_kernel(TO* out, const float* o, const float* w,
                                       const TI* proj, int64_t ld, int g_off, int n_rows, int H, int Dv,
-                                      float eps, int w_shared, int gate_silu, int norm_blocks, Moved moved) {
+                                      float eps, int w_shared, int gate_silu, int norm_blocks, int vec, Moved moved) {
   rb_pdl_launch_dependents();
   rb_pdl_wait();
   const int move = (int)blockIdx.x - norm_blocks;         // the blocks behind those take n and m over, one (run, head) each
@@ -602,6 +602,37 @@ __global__ void head_norm_gate_kernel(TO* out, const float* o, const float* w,
   const int t = (int)(item / H), h = (int)(item % H);
   const float* row = o + ((int64_t)t * H + h) * Dv;
   float ss = 0.f;
+  if (vec) {
+    // up to 512 values, four neighbours a load: everything is asked for at once, so a decode step waits for memory once and not
+    // once for the sum and once for every 32 values after it (8 tokens of 8 heads of 256: 8.2 us of a step, so 3.8)
+    float v[4][4], g[4][4], ww[4][4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int j = lane * 4 + u * 128;
+      if (j < Dv) {
+        rb_load4(row + j, v[u]);
+        rb_load4(proj + (int64_t)t * ld + g_off + h * Dv + j, g[u]);
+        rb_load4(w + (w_shared ? j : h * Dv + j), ww[u]);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (lane * 4 + u * 128 < Dv)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) ss += v[u][k] * v[u][k];
+    ss = rb_warp_sum(ss);
+    const float r = 1.0f / sqrtf(ss / (float)Dv + eps);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int j = lane * 4 + u * 128;
+      if (j < Dv) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) v[u][k] = v[u][k] * r * ww[u][k] * (gate_silu ? g[u][k] * sigmoidf_(g[u][k]) : sigmoidf_(g[u][k]));
+        rb_store4(out + ((int64_t)t * H + h) * Dv + j, v[u]);
+      }
+    }
+    return;
+  }
   for (int j = lane; j < Dv; j += 32) ss += row[j] * row[j];
   ss = rb_warp_sum(ss);
   const float r = 1.0f / sqrtf(ss / (float)Dv + eps);
@@ -768,9 +799,12 @@ static int head_norm_gate(void* out, int out_dtype, const float* o, const float*
                           cudaStream_t stream) {
   const int64_t items = (int64_t)T * H;
   const int norm_blocks = (int)((items + 3) / 4), blocks = norm_blocks + (moved.from != nullptr ? moved.n_seq * moved.H : 0);
+  const int pe = proj_dtype == RB_F32 ? 4 : 2, oe = out_dtype == RB_F32 ? 4 : 2;
+  const int vec = Dv % 4 == 0 && Dv <= 512 && ld % 4 == 0 && g_off % 4 == 0 && (uintptr_t)o % 16 == 0 && (uintptr_t)w % 16 == 0 &&
+                  (uintptr_t)proj % (4 * pe) == 0 && (uintptr_t)out % (4 * oe) == 0;
 #define LAUNCH(TI, TO)                                                                                              \
   RB_LAUNCH("head_norm_gate_kernel", (head_norm_gate_kernel<TI, TO>), blocks, 128, 0, stream, (TO*)out, o, w,        \
-            (const TI*)proj, ld, g_off, T, H, Dv, eps, w_shared, gate_silu, norm_blocks, moved)
+            (const TI*)proj, ld, g_off, T, H, Dv, eps, w_shared, gate_silu, norm_blocks, vec, moved)
   if (proj_dtype == RB_F32 && out_dtype == RB_F32) LAUNCH(float, float);
   else if (proj_dtype == RB_F32 && out_dtype == RB_BF16) LAUNCH(float, __nv_bfloat16);
   else if (proj_dtype == RB_BF16 && out_dtype == RB_BF16) LAUNCH(__nv_bfloat16, __nv_bfloat16);

@@ -44,3 +44,24 @@ def test_rows_between_two_sublayers_by_part(ops_of, dtype, E, groups, K):
         for a, b in ((h, want), (hf, want_f), (ring_a[[4, 0, 2]], ring_b[[4, 0, 2]])):
             if K > 1 or b.dim() == 2:
                 assert float((a.double() - b.double()).abs().max()) <= tol * float(b.double().abs().max())
+
+
+@pytest.mark.parametrize("dtype", [F32, BF16])
+@pytest.mark.parametrize("T,H,Dv,pad", [(1, 1, 4, 0), (8, 8, 256, 0), (5, 3, 512, 4), (3, 2, 516, 0), (7, 5, 30, 0), (2, 3, 128, 1)])
+@pytest.mark.parametrize("shared,silu", [(0, 0), (1, 1)])
+def test_norm_and_gate_per_head(ops_of, dtype, T, H, Dv, pad, shared, silu):
+    """Heads in registers (up to 512 values, 16-byte loads) and longer or misaligned ones, in float64."""
+    from rbitnet_b200.kernels.ops import _ptr
+    ops = ops_of(dtype)
+    g = torch.Generator(device="cuda").manual_seed(Dv + T)
+    o = torch.randn(T, H, Dv, device="cuda", generator=g)
+    w = torch.randn(Dv if shared else H * Dv, device="cuda", generator=g)
+    proj = torch.randn(T, 8 + H * Dv + pad, device="cuda", generator=g)
+    out = torch.empty(T, H * Dv, dtype=dtype, device="cuda")
+    off = 4 + pad
+    ops.lib.call("rb_head_norm_gate", _ptr(out), ops.code, _ptr(o), _ptr(w), _ptr(proj), proj.stride(0), 0, off, T, H, Dv, 1e-5, shared, silu,
+                 ops._stream())
+    x, gate = o.double(), proj[:, off:off + H * Dv].double().view(T, H, Dv)
+    n = x / torch.sqrt((x * x).mean(-1, keepdim=True) + 1e-5) * (w.double() if shared else w.double().view(H, Dv))
+    want = (n * torch.sigmoid(gate) * (gate if silu else 1.0)).view(T, H * Dv)
+    assert float((out.double() - want).abs().max()) <= (1e-5 if dtype == F32 else 5e-3) * float(want.abs().max())
