@@ -172,7 +172,7 @@ __global__ void rmsnorm_reg_kernel(TO* out, const float* x, const float* w,
   float ss = 0.f;
 #pragma unroll
   for (int i = 0; i < NV; ++i) ss += v[i].x * v[i].x + v[i].y * v[i].y + v[i].z * v[i].z + v[i].w * v[i].w;
-  ss = rb_block_sum(ss, scratch);
+  ss = rb_block_sum_once(ss, scratch);
   const float r = 1.0f / sqrtf(ss / (float)E + eps);
   TO* o = out + (int64_t)t * E;
 #pragma unroll
@@ -309,19 +309,31 @@ __global__ void __launch_bounds__(256) layernorm_reg_kernel(TO* out, const float
                                                             const float* w, const float* b, int E,
                                                             float eps) {
   rb_pdl_launch_dependents();
-  __shared__ float scratch[33];
-  rb_pdl_wait();
+  __shared__ float scratch[32], scratch2[32];
   const float4* row = reinterpret_cast<const float4*>(x + (int64_t)blockIdx.x * E);
   const int E4 = E >> 2;
-  float4 v[NV];
+  float4 v[NV], ww[NV], bb[NV];
   float s = 0.f;
+  // weights and bias do not depend on the kernel before (up to 4,096 values; more would not stay in registers)
+  constexpr bool AHEAD = NV <= 4;
+  auto fetch = [&](int i) {
+    const int e = threadIdx.x + i * 256;
+    if (e < E4) {
+      ww[i] = reinterpret_cast<const float4*>(w)[e];
+      bb[i] = b != nullptr ? reinterpret_cast<const float4*>(b)[e] : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  };
+  if (AHEAD)
+#pragma unroll
+    for (int i = 0; i < NV; ++i) fetch(i);
+  rb_pdl_wait();
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
     const int e = threadIdx.x + i * 256;
     v[i] = e < E4 ? row[e] : make_float4(0.f, 0.f, 0.f, 0.f);
     s += (v[i].x + v[i].y) + (v[i].z + v[i].w);
   }
-  const float mean = rb_block_sum(s, scratch) / (float)E;
+  const float mean = rb_block_sum_once(s, scratch) / (float)E;
   float q = 0.f;
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
@@ -331,15 +343,15 @@ __global__ void __launch_bounds__(256) layernorm_reg_kernel(TO* out, const float
       q = fmaf(v[i].x, v[i].x, fmaf(v[i].y, v[i].y, fmaf(v[i].z, v[i].z, fmaf(v[i].w, v[i].w, q))));
     }
   }
-  const float r = 1.0f / sqrtf(rb_block_sum(q, scratch) / (float)E + eps);
+  const float r = 1.0f / sqrtf(rb_block_sum_once(q, scratch2) / (float)E + eps);
   TO* dst = out + (int64_t)blockIdx.x * E;
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
     const int e = threadIdx.x + i * 256;
     if (e < E4) {
-      const float4 ww = reinterpret_cast<const float4*>(w)[e];
-      const float4 bb = b != nullptr ? reinterpret_cast<const float4*>(b)[e] : make_float4(0.f, 0.f, 0.f, 0.f);
-      store4<TO>(dst + 4 * e, v[i].x * r * ww.x + bb.x, v[i].y * r * ww.y + bb.y, v[i].z * r * ww.z + bb.z, v[i].w * r * ww.w + bb.w);
+      if (!AHEAD) fetch(i);
+      store4<TO>(dst + 4 * e, v[i].x * r * ww[i].x + bb[i].x, v[i].y * r * ww[i].y + bb[i].y, v[i].z * r * ww[i].z + bb[i].z,
+                 v[i].w * r * ww[i].w + bb[i].w);
     }
   }
 }

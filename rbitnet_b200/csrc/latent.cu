@@ -29,9 +29,18 @@ __global__ void __launch_bounds__(256) latent_norm_append_kernel(
   extern __shared__ float s_mem[];
   float* s_sincos = s_mem;
   float* s_row = s_mem + (rot_dim > 0 ? rot_dim : 1);
-  rb_pdl_wait();
   const int t = blockIdx.x;
+  // positions, pages and weights: no kernel of the step writes them
   const int pos = tok_pos[t];
+  T* dst = reinterpret_cast<T*>(cache.k) + rb_page_offset(cache, tok_slot[t], pos, 0);
+  float wq_ahead[4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) wq_ahead[u] = (int)(threadIdx.x + u * blockDim.x) < q_rank ? wq[threadIdx.x + u * blockDim.x] : 0.f;
+  const float wkv_ahead = (int)threadIdx.x < kv_rank ? wkv[threadIdx.x] : 0.f;
+  // (the block's last threads make the sines and cosines)
+  for (int i = (int)(blockDim.x - 1 - threadIdx.x); i < rot_dim / 2; i += blockDim.x)
+    angle_sincos(pos, freq[i], magnitude, &s_sincos[i], &s_sincos[rot_dim / 2 + i]);
+  rb_pdl_wait();
   const float* q = rows + (int64_t)t * ld + q_off;
   const float* kv = rows + (int64_t)t * ld + kv_off;        // the latent, then the key part
   float sq = 0.f, sk = 0.f;
@@ -47,19 +56,20 @@ __global__ void __launch_bounds__(256) latent_norm_append_kernel(
     if (STAGED) s_row[q_rank + i] = v;
     if (i < kv_rank) sk = fmaf(v, v, sk);
   }
-  // (the block's last threads make the sines and cosines, while the first are still at the latents' ends)
-  for (int i = (int)(blockDim.x - 1 - threadIdx.x); i < rot_dim / 2; i += blockDim.x)
-    angle_sincos(pos, freq[i], magnitude, &s_sincos[i], &s_sincos[rot_dim / 2 + i]);
   const float2 sums = rb_block_sum2(sq, sk, scratch);       // also the barrier after the shared memory's writes
   const float rq = 1.0f / sqrtf(sums.x / (float)q_rank + eps);
   const float rk = 1.0f / sqrtf(sums.y / (float)kv_rank + eps);
   if (STAGED) { q = s_row; kv = s_row + q_rank; }
-  for (int i = threadIdx.x; i < q_rank; i += blockDim.x) cq[(int64_t)t * q_rank + i] = rb_from_float<T>(q[i] * rq * wq[i]);
-  T* dst = reinterpret_cast<T*>(cache.k) + rb_page_offset(cache, tok_slot[t], pos, 0);
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const int i = threadIdx.x + u * blockDim.x;
+    if (i < q_rank) cq[(int64_t)t * q_rank + i] = rb_from_float<T>(q[i] * rq * wq_ahead[u]);
+  }
+  for (int i = threadIdx.x + 4 * blockDim.x; i < q_rank; i += blockDim.x) cq[(int64_t)t * q_rank + i] = rb_from_float<T>(q[i] * rq * wq[i]);
   for (int i = threadIdx.x; i < width; i += blockDim.x) {
     float y = 0.f;
     if (i < kv_rank) {
-      y = kv[i] * rk * wkv[i];
+      y = kv[i] * rk * (i == (int)threadIdx.x ? wkv_ahead : wkv[i]);
     } else if (i < kv_rank + rot_dim) {
       auto val = [&](int e) { return kv[kv_rank + e]; };
       y = turned(val, i - kv_rank, rot_dim, interleaved, s_sincos);

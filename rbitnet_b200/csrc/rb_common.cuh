@@ -203,6 +203,16 @@ __device__ __forceinline__ float2 rb_block_sum2(float a, float b, float* scratch
   return make_float2(ta, tb);
 }
 
+// Sum over a block of up to 1024 threads with one barrier; `scratch` holds 32 floats of shared memory that nothing else has used
+// since the block's last barrier before, and that this call uses alone.  All threads get the result.
+__device__ __forceinline__ float rb_block_sum_once(float v, float* scratch) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = (blockDim.x + 31) >> 5;
+  v = rb_warp_sum(v);
+  if (lane == 0) scratch[warp] = v;
+  __syncthreads();
+  return rb_warp_sum(lane < n_warps ? scratch[lane] : 0.f);
+}
+
 // Sum over a block of up to 1024 threads; `scratch` holds 33 floats of shared
 // memory.  All threads get the result.
 __device__ __forceinline__ float rb_block_sum(float v, float* scratch) {

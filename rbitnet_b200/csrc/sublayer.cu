@@ -387,7 +387,7 @@ __global__ void __launch_bounds__(256) rmsnorm_parts_kernel(TO* out, const float
 #pragma unroll
     for (int k = 0; k < 4; ++k) ss = fmaf(v[i][k], v[i][k], ss);
   }
-  ss = rb_block_sum(ss, scratch);
+  ss = rb_block_sum_once(ss, scratch);
   const float r = 1.0f / sqrtf(ss / (float)per + eps);
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
