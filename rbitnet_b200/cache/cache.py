@@ -22,7 +22,7 @@ import torch
 
 from ..parts.base import CacheNeed, StateNeed
 from .allocator import SlotBook, CacheFull, ContextOverflow  # noqa: F401
-from .upload import upload
+from .upload import upload, upload_into
 
 PAGE_SIZE = 64
 
@@ -136,13 +136,13 @@ class SequenceCache:
         length = self.book.length
         return [length[s] for s in slots]
 
-    def reserve_one_each(self, slots) -> None:
+    def reserve_one_each(self, slots) -> list:
         """Room for one more position in each slot: the decode step's call, which finds room in the
-        last page nearly always and then touches nothing."""
+        last page nearly always and then touches nothing.  Returns the slots' lengths, the new positions."""
         book = self.book
         page, pages, length, most = book.page_size, book.pages, book.length, book.max_seq
-        for s in slots:
-            have = length[s]
+        lengths = [length[s] for s in slots]
+        for s, have in zip(slots, lengths):
             if have % page and have < most:
                 continue                     # the page that holds the last position holds the next one too
             want = have + 1
@@ -153,6 +153,7 @@ class SequenceCache:
                 if want > len(pg) * page:
                     self.reserve(s, 1)
                     break
+        return lengths
 
     def advance_one_each(self, slots) -> None:
         """After ``reserve_one_each``: every slot holds one position more."""
@@ -182,17 +183,26 @@ class SequenceCache:
     def upload_tables(self) -> None:
         """Bring the device page tables up to date (rows that changed since the last call)."""
         for g, grp in enumerate(self.groups):
+            if not grp.dirty:
+                continue
             slots = [s for s in sorted(grp.dirty) if s in self.book.pages and self.book.pages[s][g]]
             # (Entries of pages that were given back behind a window keep their old number: no kernel reads that far back.)
             if slots and slots[-1] + 1 - slots[0] <= 2 * len(slots):
                 lo, hi = slots[0], slots[-1] + 1
                 # neighbours in one copy; rows between them that have not changed get the values they have
-                grp.table[lo:hi].copy_(upload(grp.table_host[lo:hi], grp.table.device))
+                self._bring(grp.table[lo:hi], grp.table_host[lo:hi])
             else:
                 for s in slots:
                     n = len(self.book.pages[s][g])
-                    grp.table[s, :n].copy_(upload(grp.table_host[s, :n], grp.table.device))
+                    self._bring(grp.table[s, :n], grp.table_host[s, :n])
             grp.dirty.clear()                    # once they have been copied: a copy that fails is made up for by the next call
+
+    @staticmethod
+    def _bring(target: torch.Tensor, array) -> None:
+        if target.is_cuda:
+            upload_into(target, array)
+        else:
+            target.copy_(upload(array, target.device))
 
     # ---- views
     def view(self, entry: int) -> CacheLayerView:

@@ -16,7 +16,7 @@ buffers and result buffers are rings of four, of which at most two launches are 
 """
 from __future__ import annotations
 
-from typing import List, Sequence
+from typing import List, Optional, Sequence
 
 import numpy as np
 import torch
@@ -37,6 +37,13 @@ class DecodeGraph:
         for h in self.hosts:
             h.numpy()[3 * B:4 * B] = np.arange(B, dtype=np.int32)
         self.host = self.hosts[0]
+        # per staging buffer its parts as arrays, made once: a step's host time before the launch is the GPU's idle time
+        self.parts = []
+        for h in self.hosts:
+            a = h.numpy()
+            f = a.view(np.float32)
+            self.parts.append((a[0:B], a[B:2 * B], a[2 * B:3 * B], f[4 * B:5 * B], a[5 * B:5 * B + 1], f[5 * B + 1:6 * B + 1]))
+        self.greedy = [True] * self.RING      # the buffer's temperatures and uniform numbers are zeros
         self.token_ids, self.tok_pos, self.tok_slot, self.want = (self.buf[i * B:(i + 1) * B] for i in range(4))
         fl = self.buf.view(torch.float32)
         self.temps, self.uniforms = fl[4 * B:5 * B], fl[5 * B + 1:6 * B + 1]
@@ -87,27 +94,30 @@ class DecodeGraph:
 
     # ---- one step, host tokens in, host ids out
     def stage(self, slots: Sequence[int], tokens: Sequence[int], positions: Sequence[int],
-              temperatures: Sequence[float], uniforms: Sequence[float], n_live: int = -1) -> None:
+              temperatures: Optional[Sequence[float]], uniforms: Optional[Sequence[float]], n_live: int = -1) -> None:
         """Every input of a step, from the host.  ``n_live``: the first so many rows are sequences that
-        go on after the step (the rest belong to the padding sequence); -1: all of them."""
-        B = self.B
-        self.host = self.hosts[self.launched % self.RING]
-        h = self.host.numpy()
-        f = h.view(np.float32)
-        h[0:B] = tokens
-        h[B:2 * B] = positions
-        h[2 * B:3 * B] = slots
-        f[4 * B:5 * B] = temperatures
-        h[5 * B] = B if n_live < 0 else n_live
-        f[5 * B + 1:6 * B + 1] = uniforms
+        go on after the step (the rest belong to the padding sequence); -1: all of them.  ``temperatures`` and
+        ``uniforms`` None: zeros (greedy)."""
+        i = self.launched % self.RING
+        self.host = self.hosts[i]
+        to_tokens, to_positions, to_slots, to_temperatures, to_live, to_uniforms = self.parts[i]
+        to_tokens[:] = tokens
+        to_positions[:] = positions
+        to_slots[:] = slots
+        to_live[0] = self.B if n_live < 0 else n_live
+        if temperatures is not None or uniforms is not None or not self.greedy[i]:
+            to_temperatures[:] = 0.0 if temperatures is None else temperatures
+            to_uniforms[:] = 0.0 if uniforms is None else uniforms
+            self.greedy[i] = temperatures is None and uniforms is None
         self.buf.copy_(self.host, non_blocking=True)
 
     def stage_uniforms(self, uniforms: Sequence[float]) -> None:
         """Only a step's uniform numbers: its tokens and positions are what the step before left on the device."""
         B = self.B
-        self.host = self.hosts[self.launched % self.RING]
-        f = self.host.numpy().view(np.float32)
-        f[5 * B + 1:6 * B + 1] = uniforms
+        i = self.launched % self.RING
+        self.host = self.hosts[i]
+        self.parts[i][5][:] = uniforms
+        self.greedy[i] = False
         self.buf[5 * B + 1:6 * B + 1].copy_(self.host[5 * B + 1:6 * B + 1], non_blocking=True)
 
     def replay(self) -> None:

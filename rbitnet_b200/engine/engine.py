@@ -169,17 +169,16 @@ class Engine:
         ``generate`` uses (CUDA graph, padding rows, arg-max sampling whose ids are dropped) instead of
         kernel by kernel, so that its logits can be compared too."""
         if captured and self.use_graphs and entries:
-            # one pass over the entries: the host's time between two steps is the GPU's too
-            slots, tokens, rows, wants = [], [], [], True
-            for i, e in enumerate(entries):
-                if len(e.tokens) != 1:
-                    return self.stepper.step(entries)
-                slots.append(e.slot)
-                tokens.append(int(e.tokens[0]))
-                if len(e.want):
-                    rows.append(i)
-                    wants = wants and len(e.want) == 1 and e.want[0] == 0
-            n = len(slots)
+            # the host's time between two steps is the GPU's too: few passes over the entries, each of them one expression
+            n = len(entries)
+            given = [e.tokens for e in entries]
+            if any([len(t) != 1 for t in given]):
+                return self.stepper.step(entries)
+            slots = [e.slot for e in entries]
+            tokens = [int(t[0]) for t in given]
+            wanted = [e.want for e in entries]
+            rows = [i for i, w in enumerate(wanted) if len(w)]
+            wants = all([len(w) == 0 or (len(w) == 1 and w[0] == 0) for w in wanted])
             if len(set(slots)) != n:
                 raise ValueError("a slot appears twice in one step")
             V = self.model.vocab_size
@@ -189,7 +188,7 @@ class Engine:
                         raise ValueError(f"slot {e.slot}: token id out of range (vocabulary {V})")
                     if any(w != 0 for w in e.want):
                         raise ValueError(f"slot {e.slot}: wanted place is not among its 1 tokens")
-            ticket = self._launch_rows(slots, tokens, [0.0] * n, [0.0] * n)
+            ticket = self._launch_rows(slots, tokens, None, None)
             logits = self._last_graph.logits
             # asked for before the wait below, so that the copy's launch is not one more thing the GPU waits for
             out = None if not rows else (logits[:n].clone() if len(rows) == n else logits[rows])
@@ -223,24 +222,22 @@ class Engine:
         return self._launch_rows([s for s, _ in feed], [t[0] for _, t in feed], temperatures, uniforms)
 
     def _launch_rows(self, slots, tokens, temperatures, uniforms):
-        """The same with the sequences and their tokens (None: the ones on the device) as two lists."""
+        """The same with the sequences and their tokens (None: the ones on the device) as two lists; temperatures and uniform
+        numbers None: greedy."""
         n = len(slots)
-        positions = self.cache.lengths(slots)
-        self.cache.reserve_one_each(slots)
-        temperatures, uniforms = list(temperatures), list(uniforms)
+        positions = self.cache.reserve_one_each(slots)
         batch = self._graph_batch(n)
         extra = batch - n
-        if extra:
-            temperatures += [0.0] * extra
-            uniforms += [0.0] * extra
+        if temperatures is not None:
+            temperatures, uniforms = list(temperatures) + [0.0] * extra, list(uniforms) + [0.0] * extra
         self.cache.upload_tables()
         g = self.decode_graph(batch)
         if tokens is not None or g.graph is None:
             if tokens is None:
                 raise RuntimeError("a decode step without tokens needs the captured step of the launch before it")
             # rows of the padding sequence fill the step up: they rewrite its position 0 and their results are dropped
-            g.stage(slots + [self._pad_slot] * extra, tokens + [0] * extra, positions + [0] * extra,
-                    temperatures, uniforms, n_live=n)
+            pad = ([self._pad_slot] * extra, [0] * extra) if extra else ([], [])
+            g.stage(slots + pad[0], tokens + pad[1], positions + pad[1], temperatures, uniforms, n_live=n)
             if g.graph is None:
                 g.capture(pool=self._graph_pool)
                 if self._graph_pool is None:

@@ -278,3 +278,27 @@ def test_uploads_behind_a_busy_stream_and_under_capture():
             upload(np.zeros(4, dtype=np.int32), "cuda:0")
         busy + 1.0
     torch.cuda.synchronize()
+
+
+def test_rows_brought_into_a_table_behind_a_busy_stream():
+    """The table's rows hold the values of the call although the host rows change as soon as it returns, on both sides of the size from
+    which the copy goes through pinned memory; under capture it is refused."""
+    import numpy as np
+    from rbitnet_b200.cache.upload import upload_into
+    busy = torch.randn(4096, 4096, device="cuda")
+    for count in (1, 700, 16 << 10, (16 << 10) + 1):
+        table, array = torch.zeros(21, count, dtype=torch.int32, device="cuda"), np.empty(count, dtype=np.int32)
+        for _ in range(4):
+            busy @ busy
+        for k in range(20):
+            array[:] = np.arange(count, dtype=np.int32) + k
+            upload_into(table[k], array)
+            array[:] = -1
+        base = torch.arange(count, dtype=torch.int32, device="cuda")
+        assert all(torch.equal(table[k], base + k) for k in range(20)) and not table[20].any(), count
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        with pytest.raises(RuntimeError, match="captured"):
+            upload_into(table[0], array)
+        busy + 1.0
+    torch.cuda.synchronize()
