@@ -174,8 +174,10 @@ int launch_scan(float* o, const float* rows, int64_t ld, int q_off, int k_off, i
 // (chunk, head) at once; the second walks a run's chunks with the memory: two small products per chunk.  A chunk's
 // missing tokens (the run's end) count as decay 1 and k = q = v = 0.
 constexpr int GCH = 32;          // tokens of a chunk
-constexpr int GCT = 32;          // value columns of a block of the second kernel
-constexpr int GSCAN_NT = 512;
+// second kernel, value columns of a block CT: threads (CT / 4 warps on the memory, eight on the outputs) and row stride of the
+// memory's tile (a phase of eight lanes reads one row of 32 columns, or two rows four apart of 16: those then begin 16 banks apart)
+__host__ __device__ constexpr int gscan_threads(int CT) { return 8 * CT + 256; }
+__host__ __device__ constexpr int gscan_stride(int CT) { return CT == 32 ? 32 : CT + 4; }
 
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
@@ -272,31 +274,36 @@ __global__ void __launch_bounds__(128) gla_chunk_prepare_kernel(float* scratch, 
   for (int d = tid; d < D; d += 128) Eo[d] = expf(Bs[(GCH - 1) * KS + d]);
 }
 
-// grid (runs, H, tiles of 32 value columns), 512 threads.  A run is a chain of its chunks, so what counts is a chunk's time on
-// one SM.  Warps 0..7 move the memory on, 4 x 4 values a thread that stay in registers and are left in shared memory for the
-// others; warps 8..15 make the outputs from what the chunk starts from, beside them.  Shared memory: two buffers of a
-// chunk's item (as the first kernel left it) and the tile's values [32][32], filled a chunk ahead with cp.async; the memory's
-// tile S [D][32] twice: a chunk reads one and writes the other, so that a chunk has one barrier.
-// (With 16 columns and a value or two a thread: 4.6 us a chunk of 128 channels, 3.2 now.)
-__global__ void __launch_bounds__(GSCAN_NT) gla_chunk_scan_kernel(
+// grid (runs, H, tiles of CT value columns), gscan_threads(CT).  A run is a chain of its chunks, so what counts is a chunk's time
+// on one SM.  Warps 0 .. CT / 4 - 1 move the memory on, 4 x 4 values a thread that stay in registers and are left in shared memory
+// for the others; the other eight make the outputs from what the chunk starts from, beside them.  Shared memory: two buffers of a
+// chunk's item (as the first kernel left it) and the tile's values [32][CT], filled a chunk ahead with cp.async; the memory's
+// tile S [D][CT] twice: a chunk reads one and writes the other, so that a chunk has one barrier.
+// What bounds a chunk is the SM's shared memory (loads of both products, all of them from it), which 16 columns halve; where 32
+// leave half of the SMs without a block they are the better ones (1,901 tokens, 8 heads of 128 x 256, so 64 blocks of 32 columns
+// or 128 of 16: 188 us with 32, 124 us with 16, which is 2.1 us a chunk).  With more blocks than that the chunk's item, which every
+// tile copies whole, would be read twice as often for nothing.
+template <int CT>
+__global__ void __launch_bounds__(gscan_threads(CT)) gla_chunk_scan_kernel(
     float* o, const float* scratch, const float* rows, int64_t ld, int v_off,
     float* state, const int* seq_first, const int* seq_count,
     const int* run_chunk0, const int* tok_slot, int H, int D, int Dv) {
   rb_pdl_launch_dependents();
   extern __shared__ __align__(16) float s_gscan[];
+  constexpr int NT = gscan_threads(CT), SS = gscan_stride(CT), QUADS = CT / 4, KSPLIT = 32 / QUADS, OUT = 16 / KSPLIT;
   const int item_floats = gla_item_floats(D);
-  const int per_buf = item_floats + GCH * GCT;
-  float* Sa = s_gscan + 2 * per_buf;    // [D][32]: the memory as this chunk finds it
-  float* Sb = Sa + D * GCT;             // the memory as this chunk leaves it (the two change places after every chunk)
-  const int run = blockIdx.x, h = blockIdx.y, col0 = blockIdx.z * GCT;
+  const int per_buf = item_floats + GCH * CT;
+  float* Sa = s_gscan + 2 * per_buf;    // [D][SS]: the memory as this chunk finds it
+  float* Sb = Sa + D * SS;              // the memory as this chunk leaves it (the two change places after every chunk)
+  const int run = blockIdx.x, h = blockIdx.y, col0 = blockIdx.z * CT;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const bool second = warp >= 8;        // the outputs
-  // outputs: rows 4 (warp - 8) + {0..3}, columns 4 ct + {0..3}; the sum over the channels is shared by four lanes, and part
-  // ks ends up with row 4 (warp - 8) + ks.  (Eight neighbouring lanes, whose 16-byte loads are served together, read one row
-  // of S.)
-  const int ks = lane >> 3, ct = lane & 7, r0 = 4 * (warp & 7), mine_row = r0 + ks;
+  const bool second = warp >= QUADS;    // the outputs
+  // outputs: rows 4 (warp - QUADS) + {0..3}, columns 4 ct + {0..3}; the sum over the channels is shared by KSPLIT lanes, and
+  // share ks ends up with row mine_row, columns c0 .. c0 + OUT - 1
+  const int ks = lane / QUADS, ct = lane % QUADS, r0 = 4 * (warp - QUADS), mine_row = r0 + (ks & 3);
+  const int c0 = 4 * ct + (KSPLIT == 8 ? OUT * (ks >> 2) : 0);
   // the memory's step: channels 4 dt + {0..3}, columns 4 cs + {0..3}
-  const int cs = tid & 7, dt = tid >> 3;
+  const int cs = tid % QUADS, dt = tid / QUADS;
   rb_pdl_wait();
   const int first = seq_first[run], n = seq_count[run], chunk0 = run_chunk0[run];
   const int slot = tok_slot[first];
@@ -304,12 +311,12 @@ __global__ void __launch_bounds__(GSCAN_NT) gla_chunk_scan_kernel(
     const int row0 = first + ci * GCH, m = min(GCH, n - ci * GCH);
     const float* src = scratch + ((int64_t)(chunk0 + ci) * H + h) * item_floats;
     float* dst = s_gscan + (size_t)buf * per_buf;
-    for (int i = tid; i < (item_floats >> 2); i += GSCAN_NT) cp_async16(dst + 4 * i, src + 4 * i);
-    if (tid < GCH * GCT / 4) {
-      const int j = tid >> 3, c4 = (tid & 7) << 2;
+    for (int i = tid; i < (item_floats >> 2); i += NT) cp_async16(dst + 4 * i, src + 4 * i);
+    if (tid < GCH * QUADS) {
+      const int j = tid / QUADS, c4 = (tid % QUADS) << 2;
       const bool real = j < m && col0 + c4 < Dv;
       const float* v = real ? rows + (int64_t)(row0 + j) * ld + v_off + h * Dv + col0 + c4 : rows;
-      cp_async16_or_zeros(dst + item_floats + j * GCT + c4, v, real);
+      cp_async16_or_zeros(dst + item_floats + j * CT + c4, v, real);
     }
   };
   const int n_chunks = (n + GCH - 1) / GCH;
@@ -324,7 +331,7 @@ __global__ void __launch_bounds__(GSCAN_NT) gla_chunk_scan_kernel(
     for (int i = 0; i < 4; ++i) S[i][j] = steps && col0 + 4 * cs + j < Dv ? mine[(int64_t)(4 * cs + j) * D + 4 * dt + i] : 0.f;
   if (steps) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(Sa + (4 * dt + i) * GCT + 4 * cs) = make_float4(S[i][0], S[i][1], S[i][2], S[i][3]);
+    for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(Sa + (4 * dt + i) * SS + 4 * cs) = make_float4(S[i][0], S[i][1], S[i][2], S[i][3]);
   }
   for (int ci = 0, buf = 0; ci < n_chunks; ++ci, buf ^= 1) {
     const int row0 = first + ci * GCH, m = min(GCH, n - ci * GCH);
@@ -350,12 +357,12 @@ __global__ void __launch_bounds__(GSCAN_NT) gla_chunk_scan_kernel(
         for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
       const float* A = Qt + r0 * D;
 #pragma unroll 2
-      for (int d = 4 * ks; d < D; d += 16) {
+      for (int d = 4 * ks; d < D; d += 4 * KSPLIT) {
         float4 a[4], b[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const float4*>(A + i * D + d);
 #pragma unroll
-        for (int x = 0; x < 4; ++x) b[x] = *reinterpret_cast<const float4*>(Ss + (d + x) * GCT + 4 * ct);
+        for (int x = 0; x < 4; ++x) b[x] = *reinterpret_cast<const float4*>(Ss + (d + x) * SS + 4 * ct);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const float ai[4] = {a[i].x, a[i].y, a[i].z, a[i].w};
@@ -368,14 +375,24 @@ __global__ void __launch_bounds__(GSCAN_NT) gla_chunk_scan_kernel(
           }
         }
       }
-      // the four lanes' shares: after two exchanges lane part ks has its row
-      float out[4];
+      // the lanes' shares: an exchange halves the rows, a second leaves one of them, with eight shares a third halves the columns
+      float sum[4], out[OUT];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const float k0 = (ks & 1) ? acc[1][j] : acc[0][j], s0 = (ks & 1) ? acc[0][j] : acc[1][j];
         const float k1 = (ks & 1) ? acc[3][j] : acc[2][j], s1 = (ks & 1) ? acc[2][j] : acc[3][j];
-        const float v0 = k0 + __shfl_xor_sync(0xffffffffu, s0, 8), v1 = k1 + __shfl_xor_sync(0xffffffffu, s1, 8);
-        out[j] = ((ks & 2) ? v1 : v0) + __shfl_xor_sync(0xffffffffu, (ks & 2) ? v0 : v1, 16);
+        const float v0 = k0 + __shfl_xor_sync(0xffffffffu, s0, QUADS), v1 = k1 + __shfl_xor_sync(0xffffffffu, s1, QUADS);
+        sum[j] = ((ks & 2) ? v1 : v0) + __shfl_xor_sync(0xffffffffu, (ks & 2) ? v0 : v1, 2 * QUADS);
+      }
+      if constexpr (KSPLIT == 8) {
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const float other = __shfl_xor_sync(0xffffffffu, (ks & 4) ? sum[j] : sum[2 + j], 16);
+          out[j] = ((ks & 4) ? sum[2 + j] : sum[j]) + other;
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < OUT; ++j) out[j] = sum[j];
       }
       // M is zero above its diagonal: a loop of fixed length whose loads run ahead
 #pragma unroll 4
@@ -384,18 +401,21 @@ __global__ void __launch_bounds__(GSCAN_NT) gla_chunk_scan_kernel(
         const float mj[4] = {m4.x, m4.y, m4.z, m4.w};
 #pragma unroll
         for (int x = 0; x < 4; ++x) {
-          const float4 v4 = *reinterpret_cast<const float4*>(Vs + (j + x) * GCT + 4 * ct);
-          out[0] = fmaf(mj[x], v4.x, out[0]);
-          out[1] = fmaf(mj[x], v4.y, out[1]);
-          out[2] = fmaf(mj[x], v4.z, out[2]);
-          out[3] = fmaf(mj[x], v4.w, out[3]);
+          float v[OUT];
+          if constexpr (OUT == 4) {
+            *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(Vs + (j + x) * CT + c0);
+          } else {
+            *reinterpret_cast<float2*>(v) = *reinterpret_cast<const float2*>(Vs + (j + x) * CT + c0);
+          }
+#pragma unroll
+          for (int c = 0; c < OUT; ++c) out[c] = fmaf(mj[x], v[c], out[c]);
         }
       }
       if (mine_row < m) {
-        float* to = o + ((int64_t)(row0 + mine_row) * H + h) * Dv + col0 + 4 * ct;
+        float* to = o + ((int64_t)(row0 + mine_row) * H + h) * Dv + col0 + c0;
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-          if (col0 + 4 * ct + j < Dv) to[j] = out[j];
+        for (int j = 0; j < OUT; ++j)
+          if (col0 + c0 + j < Dv) to[j] = out[j];
       }
     } else if (steps) {
       // S <- diag(e^{B_end}) S + sum_j Kt_j v_j: the chunk's sum from zero, added once, so that a chunk rounds at the memory's size
@@ -410,7 +430,7 @@ __global__ void __launch_bounds__(GSCAN_NT) gla_chunk_scan_kernel(
 #pragma unroll 4
       for (int j = 0; j < GCH; ++j) {
         const float4 k4 = *reinterpret_cast<const float4*>(Kt + j * D + 4 * dt);
-        const float4 v4 = *reinterpret_cast<const float4*>(Vs + j * GCT + 4 * cs);
+        const float4 v4 = *reinterpret_cast<const float4*>(Vs + j * CT + 4 * cs);
         const float ki[4] = {k4.x, k4.y, k4.z, k4.w};
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -425,7 +445,7 @@ __global__ void __launch_bounds__(GSCAN_NT) gla_chunk_scan_kernel(
 #pragma unroll
         for (int j = 0; j < 4; ++j) S[i][j] = fmaf(e[i], S[i][j], add[i][j]);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(Sn + (4 * dt + i) * GCT + 4 * cs) = make_float4(S[i][0], S[i][1], S[i][2], S[i][3]);
+      for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(Sn + (4 * dt + i) * SS + 4 * cs) = make_float4(S[i][0], S[i][1], S[i][2], S[i][3]);
     }
   }
   if (steps) {
@@ -515,20 +535,28 @@ RB_EXPORT int rb_gla_chunked(float* o, const float* rows, int64_t ld, int q_off,
                  (uintptr_t)scratch % 16 == 0 && (uintptr_t)log_alpha % 16 == 0,
              "rb_gla_chunked: bad sizes H=%d D=%d Dv=%d", H, D, Dv);
   const size_t smem_a = (size_t)(3 * GCH * (D + 4)) * sizeof(float);
-  const size_t smem_b = (size_t)(2 * (gla_item_floats(D) + GCH * GCT) + 2 * GCT * D) * sizeof(float);
+  // tiles of 16 columns where those of 32 would leave half of the SMs without a block
+  const bool narrow = 2ll * n_runs * H * ((Dv + 31) / 32) <= rb_sm_count();
+  const int ct = narrow ? 16 : 32;
+  const size_t smem_b = (size_t)(2 * (gla_item_floats(D) + GCH * ct) + 2 * gscan_stride(ct) * D) * sizeof(float);
   static RbOncePerDevice configured;
   if (configured.first()) {
     RB_CUDA(cudaFuncSetAttribute(gla_chunk_prepare_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
-    RB_CUDA(cudaFuncSetAttribute(gla_chunk_scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024));
+    RB_CUDA(cudaFuncSetAttribute(gla_chunk_scan_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024));
+    RB_CUDA(cudaFuncSetAttribute(gla_chunk_scan_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024));
   }
   RB_REQUIRE(smem_a <= 64 * 1024 && smem_b <= 128 * 1024, "rb_gla_chunked: key size %d needs too much shared memory", D);
   RB_LAUNCH("gla_chunk_prepare_kernel", (gla_chunk_prepare_kernel), dim3(n_chunks, H), 128, smem_a, stream, scratch, rows, ld,
             q_off, k_off, log_alpha, q_scale, chunk_row, chunk_len, H, D, a_ld);
   RB_CHECK_LAUNCH("rb_gla_chunked");
-  const dim3 grid(n_runs, H, (Dv + GCT - 1) / GCT);
+  const dim3 grid(n_runs, H, (Dv + ct - 1) / ct);
   RB_REQUIRE(grid.z <= 65535, "rb_gla_chunked: too many columns");
-  RB_LAUNCH("gla_chunk_scan_kernel", (gla_chunk_scan_kernel), grid, GSCAN_NT, smem_b, stream, o, scratch, rows, ld, v_off, state,
-            seq_first, seq_count, run_chunk0, tok_slot, H, D, Dv);
+  if (narrow)
+    RB_LAUNCH("gla_chunk_scan_kernel", (gla_chunk_scan_kernel<16>), grid, gscan_threads(16), smem_b, stream, o, scratch, rows, ld,
+              v_off, state, seq_first, seq_count, run_chunk0, tok_slot, H, D, Dv);
+  else
+    RB_LAUNCH("gla_chunk_scan_kernel", (gla_chunk_scan_kernel<32>), grid, gscan_threads(32), smem_b, stream, o, scratch, rows, ld,
+              v_off, state, seq_first, seq_count, run_chunk0, tok_slot, H, D, Dv);
   RB_CHECK_LAUNCH("rb_gla_chunked");
   return 0;
 }

@@ -445,3 +445,38 @@ def test_experts_weighted_on_their_inputs(dtype, T, E, F, n, top, shared, fused)
     part.forward(ctx, h.to(dtype).cuda(), accumulate_into=x)
     assert rel_err((x - before).cpu(), want) <= tol
     ops.check_errors()
+
+
+@pytest.mark.parametrize("D,Dv", [(20, 36), (128, 64), (4, 4), (124, 20)])
+@pytest.mark.parametrize("runs", [1, 14])
+def test_gated_linear_attention_in_tiles_of_16_and_32_columns(runs, D, Dv):
+    """The chunks' walk with few blocks (tiles of 16 value columns) and with many (of 32): run lengths around whole chunks, value
+    sizes that end inside a tile, against the definition in 64 bits; the slots of no run stay as they were."""
+    from rbitnet_b200.parts.gla import GatedLinearAttention
+    ops = _ops(torch.float32)
+    g = torch.Generator().manual_seed(runs * 1000 + D)
+    E, H = 24, 6
+    part = GatedLinearAttention(E, H, D, Dv, 4, 4.0, norm_eps=1e-5)
+    w = {k: torch.randn(*shape, generator=g, dtype=torch.float64) * (0.3 if len(shape) > 1 else 1.0)
+         for k, (shape, _) in part.weight_shapes().items()}
+    w["a2.b"] = w["a2.b"] + 3.0
+    part.bind({k: v.float().cuda() for k, v in w.items()}, ops)
+    assert (2 * runs * H * ((Dv + 31) // 32) <= torch.cuda.get_device_properties(0).multi_processor_count) == (runs == 1)
+    lengths = [(97, 64, 33, 31, 2)[i % 5] for i in range(runs)]
+    rows = [torch.randn(n, E, generator=g, dtype=torch.float64) for n in lengths]
+    state = {k: torch.zeros((runs + 2, *n.shape), device="cuda") for k, n in part.state_need().items()}
+    first = [0 if n < 3 else n // 2 for n in lengths]
+    outs = [[] for _ in rows]
+    for a, b in (([0] * runs, first), (first, lengths)):       # two portions: the second starts from what the first left
+        there = [i for i in range(runs) if b[i] > a[i]]
+        ctx = _Ctx(ops, _meta(ops, [(i + 1, a[i], b[i] - a[i]) for i in there]), state=state)
+        out = part.forward(ctx, torch.cat([rows[i][a[i]:b[i]] for i in there]).float().cuda(), 0)
+        at = 0
+        for i in there:
+            outs[i].append(out[at:at + b[i] - a[i]])
+            at += b[i] - a[i]
+    m = {"heads": H, "dim": D, "vdim": Dv, "tau": 4.0}
+    for h, o in zip(rows, outs):
+        assert rel_err(torch.cat(o).cpu(), plain.gla_mixer(h, m, w, 1e-5)) <= 2e-4
+    assert not state["S"][0].any() and not state["S"][runs + 1].any()
+    ops.check_errors()
