@@ -253,9 +253,7 @@ struct QkParams {
 };
 
 // A block per token.  Shared memory: rot_dim sines and cosines, the C = (H + Kh) D convolved q and k values, a factor
-// per head, the norms' weights.  What no kernel of the step writes (positions, pages, weights) is asked for before the wait; the
-// convolution's taps, rows and ring of a few channels at once, not tap after tap.  1 token, 20 heads of 128, norm per head 7.4 us of a
-// step before, 5.3 to 6.9 now; with four taps 12.6 and 6.9.
+// per head, the norms' weights.  Takes what qk_prepare_quads_kernel does not.
 template <typename T>
 __global__ void __launch_bounds__(1024) qk_prepare_kernel(T* q_out, T* gates_out, QkParams p,
                                                          RbPagedLayer cache) {
@@ -278,22 +276,7 @@ __global__ void __launch_bounds__(1024) qk_prepare_kernel(T* q_out, T* gates_out
     angle_sincos(pos, p.freq[i], p.magnitude, &s_sincos[i], &s_sincos[p.rot_dim / 2 + i]);
   rb_pdl_wait();
   const float* row = p.proj + (int64_t)t * p.ld;
-  if (p.conv_w != nullptr && p.tok_first == nullptr && p.K == 4) {
-    // a row that is its own run, four taps
-    const int reach = min(3, pos);
-    const float* ring = p.tail + (int64_t)slot * 4 * C;
-#pragma unroll 3
-    for (int c = threadIdx.x; c < C; c += blockDim.x) {
-      const float* taps = p.conv_w + (int64_t)c * 4;
-      const float own = row[c];
-      float acc = taps[3] * own;
-#pragma unroll
-      for (int back = 1; back <= 3; ++back)
-        if (back <= reach) acc = fmaf(taps[3 - back], ring[(int64_t)((pos - back) & 3) * C + c], acc);
-      s_qk[c] = acc;
-      p.tail[((int64_t)slot * 4 + (pos & 3)) * C + c] = own;
-    }
-  } else if (p.conv_w != nullptr) {
+  if (p.conv_w != nullptr) {
     // tap by tap over all channels, so that a thread's loads of one pass do not wait for one another
     const int K = p.K;
     const int pos0 = p.tok_first != nullptr ? p.tok_pos[p.tok_first[t]] : pos;     // the run's first position
@@ -382,6 +365,177 @@ __global__ void __launch_bounds__(1024) qk_prepare_kernel(T* q_out, T* gates_out
     const int g_at = C + (p.values_are_keys ? 0 : Kh * Dv);
     for (int h = threadIdx.x; h < H; h += blockDim.x) gates_out[(int64_t)t * H + h] = rb_from_float<T>(row[g_at + h]);
   }
+}
+
+// The same in quads of neighbouring values: sizes and strides that are multiples of four, no convolution or one of four taps.
+// A block per token, a chain of dependent reads in a step and, with many tokens, too little of the rows in flight, unless a thread asks
+// for all of its share at once: taps, own row and the three before it (rows of the run, or of the ring before its start), the
+// gates, the values, and only then makes anything of them.  Before the wait: positions, pages, weights, sines.  A warp takes a head,
+// sums its squares (norm per head) and turns it, so that one barrier is all.  20 heads of 128 and 4 of values, of a whole request:
+// a step's token 7.1 -> 5.2 us, 1,901 tokens with four taps 70 -> 31 us, without 36 -> 21 us.
+template <typename T>
+__global__ void __launch_bounds__(1024) qk_prepare_quads_kernel(T* q_out, T* gates_out, QkParams p, RbPagedLayer cache) {
+  rb_pdl_launch_dependents();
+  __shared__ float s_sum[2][32];
+  extern __shared__ __align__(16) float s_mem[];
+  const int H = p.H, D = p.D, Dv = p.Dv, Kh = cache.n_kv_heads, Dc = cache.head_dim;
+  const int C = (H + Kh) * D, rhalf = p.rot_dim >> 1, mode = p.norm_mode;
+  const int nq = mode == 1 ? H * D : (mode == 2 ? D : 0), nk = mode == 1 ? Kh * D : nq;
+  float* s_qk = s_mem;
+  float* s_nw = s_qk + C;                           // [q weights | k weights], of a head or of all
+  float* s_sincos = s_nw + nq + nk;
+  const int t = blockIdx.x, tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, n_warps = nt >> 5;
+  const int pos = p.tok_pos[t], slot = p.tok_slot[t];
+  const bool conv = p.conv_w != nullptr;
+  const int pos0 = conv && p.tok_first != nullptr ? p.tok_pos[p.tok_first[t]] : pos;     // the run's first position
+  const int64_t page0 = rb_page_offset(cache, slot, pos, 0), page_step = (int64_t)cache.page_size * Dc;
+  for (int i = tid; i < nq + nk; i += nt) s_nw[i] = i < nq ? p.q_norm_w[i] : p.k_norm_w[i - nq];
+  for (int i = tid; i < rhalf; i += nt) angle_sincos(pos, p.freq[i], p.magnitude, &s_sincos[i], &s_sincos[rhalf + i]);
+  rb_pdl_wait();
+  const float* row = p.proj + (int64_t)t * p.ld;
+  const int g_at = C + (p.values_are_keys ? 0 : Kh * Dv);
+  const int Dc4 = Dc >> 2, own_quads = p.values_are_keys ? 0 : Kh * Dc4;
+  auto value_quad = [&](int i, float (&y)[4]) {
+    const int kvh = i / Dc4, e = (i - kvh * Dc4) << 2;
+    y[0] = y[1] = y[2] = y[3] = 0.f;
+    if (e >= Dv) return;
+    rb_load4(row + C + kvh * Dv + e, y);
+    if (p.mix_rows != nullptr) {
+      float other[4];
+      rb_load4(p.mix_rows + (int64_t)t * p.mix_ld + kvh * Dv + e, other);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) y[k] = (1.0f - p.mix_weight) * y[k] + p.mix_weight * other[k];
+    }
+  };
+  T* vdst = (T*)cache.v + page0;
+  auto value_to = [&](int i) {
+    const int kvh = i / Dc4;
+    return vdst + kvh * page_step + ((i - kvh * Dc4) << 2);
+  };
+  float v0[4], g0 = 0.f;
+  if (tid < own_quads) value_quad(tid, v0);
+  if (p.gate_heads && tid < H) g0 = row[g_at + tid];
+  const float* before[3];
+  if (conv) {
+#pragma unroll
+    for (int back = 1; back <= 3; ++back) {
+      const int at = pos - back;
+      before[back - 1] = at < 0 ? nullptr : (at >= pos0 ? row - (int64_t)back * p.ld : p.tail + ((int64_t)slot * 4 + (at & 3)) * C);
+    }
+  }
+  float sum_q = 0.f, sum_k = 0.f;
+  for (int c = 4 * tid; c < C; c += 4 * nt) {
+    float own[4], y[4];
+    rb_load4(row + c, own);
+    if (conv) {
+      float taps[4][4], old[3][4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) rb_load4(p.conv_w + (int64_t)(c + j) * 4, taps[j]);
+#pragma unroll
+      for (int back = 0; back < 3; ++back)
+        if (before[back] != nullptr) rb_load4(before[back] + c, old[back]);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        y[j] = taps[j][3] * own[j];
+#pragma unroll
+        for (int back = 0; back < 3; ++back)
+          if (before[back] != nullptr) y[j] = fmaf(taps[j][2 - back], old[back][j], y[j]);
+      }
+      if (p.tok_first == nullptr) rb_store4(p.tail + ((int64_t)slot * 4 + (pos & 3)) * C + c, own);      // a row that is its own run
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) y[j] = own[j];
+    }
+    rb_store4(s_qk + c, y);
+    const float ss = y[0] * y[0] + y[1] * y[1] + y[2] * y[2] + y[3] * y[3];
+    if (c < H * D) sum_q += ss;
+    else sum_k += ss;
+  }
+  if (tid < own_quads) rb_store4(value_to(tid), v0);
+  if (p.gate_heads && tid < H) gates_out[(int64_t)t * H + tid] = rb_from_float<T>(g0);
+  if (mode == 1) {
+    sum_q = rb_warp_sum(sum_q);
+    sum_k = rb_warp_sum(sum_k);
+    if (lane == 0) {
+      s_sum[0][warp] = sum_q;
+      s_sum[1][warp] = sum_k;
+    }
+  }
+  __syncthreads();
+  float rq = 1.f, rk = 1.f;
+  if (mode == 1) {
+    rq = 1.0f / sqrtf(rb_warp_sum(lane < n_warps ? s_sum[0][lane] : 0.f) / (float)(H * D) + p.eps);
+    rk = 1.0f / sqrtf(rb_warp_sum(lane < n_warps ? s_sum[1][lane] : 0.f) / (float)(Kh * D) + p.eps);
+  }
+  const bool apart = !p.interleaved && (rhalf & 3) == 0, within = p.interleaved && (p.rot_dim & 3) == 0;
+  for (int head = warp; head < H + Kh; head += n_warps) {
+    const bool is_q = head < H;
+    T* dst = is_q ? q_out + ((int64_t)t * H + head) * Dc : (T*)cache.k + page0 + (head - H) * page_step;
+    const float* src = s_qk + head * D;
+    const float* nw = s_nw + (is_q ? 0 : nq) + (mode == 1 ? (is_q ? head : head - H) * D : 0);
+    float fac = is_q ? rq : rk;
+    if (mode == 2) {
+      float ss = 0.f;
+      for (int e = 4 * lane; e < D; e += 128) {
+        float y[4];
+        rb_load4(src + e, y);
+        ss += y[0] * y[0] + y[1] * y[1] + y[2] * y[2] + y[3] * y[3];
+      }
+      fac = 1.0f / sqrtf(rb_warp_sum(ss) / (float)D + p.eps);
+    }
+    auto val = [&](int i) { return mode ? src[i] * fac * nw[i] : src[i]; };
+    auto quad = [&](int e, float (&y)[4]) {
+      rb_load4(src + e, y);
+      if (mode) {
+        float w[4];
+        rb_load4(nw + e, w);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) y[k] = y[k] * fac * w[k];
+      }
+    };
+    for (int e = 4 * lane; e < Dc; e += 128) {
+      float y[4] = {0.f, 0.f, 0.f, 0.f};
+      if (e < p.rot_dim && apart) {                 // the other halves of four pairs are neighbours too
+        float me[4], other[4], sn[4], cs[4];
+        const bool first = e < rhalf;
+        const int pair = first ? e : e - rhalf;
+        quad(e, me);
+        quad(first ? e + rhalf : pair, other);
+        rb_load4(s_sincos + pair, sn);
+        rb_load4(s_sincos + rhalf + pair, cs);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) y[k] = first ? me[k] * cs[k] - other[k] * sn[k] : me[k] * cs[k] + other[k] * sn[k];
+      } else if (e < p.rot_dim && within) {         // two whole pairs
+        float me[4];
+        quad(e, me);
+#pragma unroll
+        for (int k = 0; k < 4; k += 2) {
+          const float sn = s_sincos[(e + k) >> 1], cs = s_sincos[rhalf + ((e + k) >> 1)];
+          y[k] = me[k] * cs - me[k + 1] * sn;
+          y[k + 1] = me[k + 1] * cs + me[k] * sn;
+        }
+      } else if (e < p.rot_dim) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) y[k] = turned(val, e + k, p.rot_dim, p.interleaved, s_sincos);
+      } else if (e < D) {
+        quad(e, y);
+      }
+      rb_store4(dst + e, y);
+    }
+  }
+  for (int i = tid + nt; i < own_quads; i += nt) {
+    value_quad(i, v0);
+    rb_store4(value_to(i), v0);
+  }
+  if (p.values_are_keys)
+    for (int i = tid; i < Kh * Dc4; i += nt) {
+      const int kvh = i / Dc4, e = (i - kvh * Dc4) << 2;
+      float y[4] = {0.f, 0.f, 0.f, 0.f};
+      if (e < D) rb_load4(s_qk + (H + kvh) * D + e, y);
+      rb_store4(value_to(i), y);
+    }
+  if (p.gate_heads)
+    for (int h = tid + nt; h < H; h += nt) gates_out[(int64_t)t * H + h] = rb_from_float<T>(row[g_at + h]);
 }
 
 // A block per token.  rows: [H heads of (D + R) | C latent | R shared key part].  q_out [T, H (D + R)]; the cache row
@@ -602,16 +756,35 @@ RB_EXPORT int rb_qk_prepare(void* q_out, void* gates_out, int dtype, const float
     threads = pairs >= 1024 ? 1024 : (pairs >= 512 ? 512 : 256);
   }
   RB_REQUIRE(smem <= 200 * 1024, "rb_qk_prepare: %d q and k values per token do not fit shared memory", (H + Kh) * D);
-#define GO(TT)                                                                                                          \
-  do {                                                                                                                  \
-    if (smem > 48 * 1024)                                                                                               \
-      RB_CUDA(cudaFuncSetAttribute(qk_prepare_kernel<TT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));     \
-    RB_LAUNCH("qk_prepare_kernel", (qk_prepare_kernel<TT>), T, threads, smem, stream, (TT*)q_out, (TT*)gates_out, p, c); \
+  // quads where all sizes, strides and addresses allow it.  Few tokens: a thread for every quad; many: one for five, so that an SM
+  // holds more tokens, each of them the whole chain (1,901 tokens of 20 heads of 128: 44 us with a thread a quad, 24.6 with one for
+  // two, 19.5 with one for five)
+  const uintptr_t all = (uintptr_t)proj | (uintptr_t)q_out | (uintptr_t)cache_k | (uintptr_t)cache_v | (uintptr_t)conv_w |
+                        (conv_w != nullptr ? (uintptr_t)tail : 0) | (uintptr_t)mix_rows;
+  const bool quads = (D | Dv | Dc) % 4 == 0 && ld % 4 == 0 && (mix_rows == nullptr || mix_ld % 4 == 0) && all % 16 == 0 &&
+                     (conv_w == nullptr || K == 4) && (norm_mode == 0 || p.staged);
+  if (quads) {
+    const int n4 = (H + Kh) * D / 4, want = T <= 2 * rb_sm_count() ? n4 : (n4 + 4) / 5;
+    threads = want >= 1024 ? 1024 : (want <= 128 ? 128 : (want + 31) / 32 * 32);
+  }
+#define GO_AS(NAME, KERNEL)                                                                              \
+  do {                                                                                                   \
+    if (smem > 48 * 1024)                                                                                \
+      RB_CUDA(cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));     \
+    RB_LAUNCH(NAME, (KERNEL), T, threads, smem, stream, (decltype(q))q_out, (decltype(q))gates_out, p, c); \
+  } while (0)
+#define GO(TT)                                                                 \
+  do {                                                                         \
+    TT* q = nullptr;                                                           \
+    if (quads) GO_AS("qk_prepare_quads_kernel", qk_prepare_quads_kernel<TT>);  \
+    else GO_AS("qk_prepare_kernel", qk_prepare_kernel<TT>);                    \
+    (void)q;                                                                   \
   } while (0)
   if (dtype == RB_BF16) GO(__nv_bfloat16);
   else if (dtype == RB_F32) GO(float);
   else RB_FAIL("rb_qk_prepare: unknown dtype %d", dtype);
 #undef GO
+#undef GO_AS
   RB_CHECK_LAUNCH("rb_qk_prepare");
   return 0;
 }

@@ -65,3 +65,59 @@ def test_norm_and_gate_per_head(ops_of, dtype, T, H, Dv, pad, shared, silu):
     n = x / torch.sqrt((x * x).mean(-1, keepdim=True) + 1e-5) * (w.double() if shared else w.double().view(H, Dv))
     want = (n * torch.sigmoid(gate) * (gate if silu else 1.0)).view(T, H * Dv)
     assert float((out.double() - want).abs().max()) <= (1e-5 if dtype == F32 else 5e-3) * float(want.abs().max())
+
+
+@pytest.mark.parametrize("dtype", [F32, BF16])
+@pytest.mark.parametrize("H,Kh,D,Dv,rot,interleaved,norm,taps,keys,mix,gates", [
+    (16, 4, 128, 128, 64, True, "head_weight", 4, False, False, False), (20, 4, 64, 72, 24, False, "projection", 4, False, True, True),
+    (5, 1, 12, 4, 6, True, None, 4, False, False, True), (3, 1, 260, 260, 12, False, "head_weight", 0, True, False, True),
+    (300, 1, 4, 4, 4, False, None, 0, False, False, True), (2, 60, 4, 132, 2, False, "projection", 0, False, True, False)])
+def test_q_and_k_preparation_in_quads(ops_of, dtype, H, Kh, D, Dv, rot, interleaved, norm, taps, keys, mix, gates):
+    """Quads of values against the form that takes any size and address (rows that begin one value late), over runs of several rows
+    and single rows, from the first position: the ring, the cache's pages, q and the gates."""
+    from rbitnet_b200.cache import SequenceCache
+    from rbitnet_b200.parts.base import CacheNeed
+    from rbitnet_b200.engine.step import SeqChunk, build_meta
+    ops = ops_of(dtype)
+    g = torch.Generator(device="cuda").manual_seed(H + D)
+    dev = {"device": "cuda", "generator": g}
+    C, Dc = (H + Kh) * D, max(D, Dv)
+    width = C + (0 if keys else Kh * Dv) + (H if gates else 0)
+    table = (10000.0 ** (-2.0 * torch.arange(rot // 2, dtype=torch.float64, device="cuda") / rot), 1.25, interleaved, rot)
+    qw, kw = {"projection": (torch.randn(H * D, **dev), torch.randn(Kh * D, **dev)), "head_weight": (torch.randn(D, **dev), torch.randn(D, **dev)),
+              None: (None, None)}[norm]
+    conv = torch.randn(C, taps, **dev) if taps else None
+    made = []
+    for late in (0, 1):
+        cache = SequenceCache({0: CacheNeed(Kh, Dc)}, reads={}, state_needs={}, max_tokens=16 * 64, max_seq=256, dtype=dtype,
+                              device="cuda", page_size=16, n_slots=4)
+        for pages in (cache.view(0).k, cache.view(0).v):
+            pages.zero_()
+        slots = [cache.alloc() for _ in range(3)]
+        made.append((cache, slots, torch.zeros(4, max(taps, 1), C, device="cuda")))
+    at = [0, 0, 0]
+    for lengths in ((1, 1, 1), (5, 1, 40), (1, 1, 1), (1, 1, 1), (2, 33, 1), (1, 1, 1)):
+        T = sum(lengths)
+        rows, other = torch.randn(T, (width + 7) // 4 * 4, **dev), torch.randn(T, Kh * Dv + 8, **dev)
+        got = []
+        for late, (cache, slots, ring) in enumerate(made):
+            chunks, first = [], 0
+            for s, p, n in zip(slots, at, lengths):
+                cache.reserve(s, n)
+                cache.advance(s, n)
+                chunks.append(SeqChunk(s, p, n, first))
+                first += n
+            cache.upload_tables()
+            meta = build_meta(chunks, np.zeros(T, dtype=np.int32), np.zeros(0, dtype=np.int32), ops.device)
+            x = torch.empty(rows.numel() + late, device="cuda")[late:].view(rows.shape)
+            x.copy_(rows)
+            got.append(ops.qk_prepare(x, meta, cache.view(0), H, D, Dv, table, norm, qw, kw, 1e-5, conv=conv, tail=ring if taps else None,
+                                      values_are_keys=keys, v_mix=(0.3, other, 4) if mix else None, gate_heads=gates))
+        at = [a + n for a, n in zip(at, lengths)]
+        (q, gate), (q1, gate1) = got
+        a, b = made[0][0].view(0), made[1][0].view(0)
+        tol = 2e-6 if dtype == F32 else 8e-3               # sums of squares in another order; a rounding to 8 bits
+        for one, two in ((q, q1), (a.k, b.k), (a.v, b.v)):
+            assert float((one.double() - two.double()).abs().max()) <= tol * float(two.double().abs().max())
+        assert torch.equal(made[0][2], made[1][2]) and (gate is None or torch.equal(gate, gate1))
+    ops.check_errors()
