@@ -117,3 +117,38 @@ def test_a_shared_expert_behind_the_others(ops_of, dtype, T, experts, inner, E, 
     bound = 1e-5 if dtype == F32 else 1e-2
     assert float((one - apart).norm() / (apart - x0).norm()) < bound
     ops.check_errors()
+
+
+@pytest.mark.parametrize("dtype", [F32, BF16])
+@pytest.mark.parametrize("T,E,top,accumulate,shared,gated,norm", [
+    (1, 4, 1, 1, False, False, False), (3, 1028, 4, 1, True, True, True), (300, 2052, 5, 0, True, False, True), (2, 2048, 9, 1, False, False, True),
+    (148, 256, 4, 1, True, True, False), (5, 30, 3, 1, True, True, True), (7, 2048, 4, 0, False, False, False)])
+def test_weighted_sum_of_the_experts_rows(ops_of, dtype, T, E, top, accumulate, shared, gated, norm):
+    """Few tokens and many, four columns a thread and one (widths that are no multiple of four), choices around groups of four, some of
+    them the token's own row; the row of infinities is nobody's.  In float64."""
+    from rbitnet_b200.kernels.ops import _ptr
+    ops = ops_of(dtype)
+    g = torch.Generator(device="cuda").manual_seed(T * 10 + top)
+    dev = {"device": "cuda", "generator": g}
+    y, h = torch.randn(T * top + 1, E, **dev), torch.randn(T, E, **dev).to(dtype)
+    y[0] = math.inf
+    pos = torch.randint(1, T * top + 1, (T, top), dtype=torch.int32, **dev)
+    pos[torch.rand(T, top, **dev) < 0.3] = -1
+    w, x = torch.rand(T, top, **dev), torch.randn(T, E, **dev)
+    z = torch.randn(T, E, **dev) if shared else None
+    gate = torch.randn(T, 3, **dev)[:, 1:2] if gated else None
+    nw, nb = torch.randn(E, **dev), torch.randn(E, **dev)
+    out = torch.empty(T, E, dtype=dtype, device="cuda")
+    rows = torch.where((pos >= 0)[..., None], y[pos.clamp(min=1).long()].double(), h.double()[:, None])
+    want = (w.double()[..., None] * rows).sum(1) + (x.double() if accumulate else 0.0)
+    if shared:
+        want = want + z.double() * (torch.sigmoid(gate.double()) if gated else 1.0)
+    if shared or norm:
+        ops.lib.call("rb_routed_combine_next", _ptr(z), _ptr(gate), gate.stride(0) if gated else 0, _ptr(nw if norm else None),
+                     _ptr(nb if norm else None), 0.4, _ptr(out if norm else None), launches=0)
+    ops.lib.call("rb_routed_combine", _ptr(x), x.stride(0), _ptr(y), _ptr(h), h.stride(0), ops.code, _ptr(pos), _ptr(w), T, top, E, accumulate,
+                 ops._stream())
+    assert float((x.double() - want).abs().max()) <= 1e-6 * float(want.abs().max()) * (top + 3)
+    if norm:
+        after = nw.double() * torch.tanh(0.4 * want) + nb.double()
+        assert float((out.double() - after).abs().max()) <= (2e-5 if dtype == F32 else 8e-3) * float(after.abs().max())
