@@ -1032,23 +1032,14 @@ RB_EXPORT int rb_routed_plan(int* pos, int* row_token, int* tile_group, const in
 // The most pairs that rb_routed_place takes.
 RB_EXPORT int rb_routed_place_pairs() { return PLACE_PAIRS; }
 
-// The next rb_routed_place or rb_route_choose_place call of this thread puts every token's own row, unweighted, into `tiles` tiles
-// ahead of the pairs' (group n_experts: a shared expert whose matrices lie behind the others').
-static thread_local int t_place_shared = 0;
-RB_EXPORT int rb_routed_place_shared(int tiles) {
-  t_place_shared = tiles;
-  return 0;
-}
-
 static int place_impl(void* xp, int* pos, int* tile_group, const void* h, int64_t ldh, int dtype, const int* ids, const float* weights,
-                      const Choice* choice, int weigh, int pairs, int top, int n_experts, int tile, int n_tiles, int K, cudaStream_t stream) {
-  const int n_shared = t_place_shared;
-  t_place_shared = 0;
+                      const Choice* choice, int weigh, int pairs, int top, int n_experts, int tile, int n_shared, int n_tiles, int K,
+                      cudaStream_t stream) {
   if (pairs == 0) return 0;
   RB_REQUIRE(pairs <= PLACE_PAIRS && n_experts > 0 && top > 0 && pairs % top == 0 && tile > 0 && n_tiles >= rb_routed_tiles(pairs, n_experts, tile),
              "rb_routed_place: %d tiles of %d rows for %d pairs over %d experts", n_tiles, tile, pairs, n_experts);
   const int T = pairs / top;
-  RB_REQUIRE(n_shared == 0 || n_shared * tile >= T, "rb_routed_place: %d tokens in %d shared tiles of %d rows", T, n_shared, tile);
+  RB_REQUIRE(n_shared == 0 || (n_shared > 0 && (int64_t)n_shared * tile >= T), "rb_routed_place: %d tokens in %d shared tiles of %d rows", T, n_shared, tile);
   size_t smem = (size_t)(2 * PLACE_PAIRS + n_experts) * sizeof(int);
   RB_REQUIRE(smem <= 40 * 1024, "rb_routed_place: %d experts", n_experts);
   const size_t four = dtype == RB_F32 ? 16 : 8;
@@ -1075,7 +1066,7 @@ static int place_impl(void* xp, int* pos, int* tile_group, const void* h, int64_
 RB_EXPORT int rb_routed_place(void* xp, int* pos, int* tile_group, const void* h, int64_t ldh, int dtype, const int* ids,
                               const float* weights, int pairs, int top, int n_experts, int tile, int n_tiles, int K,
                               cudaStream_t stream) {
-  return place_impl(xp, pos, tile_group, h, ldh, dtype, ids, weights, nullptr, 0, pairs, top, n_experts, tile, n_tiles, K, stream);
+  return place_impl(xp, pos, tile_group, h, ldh, dtype, ids, weights, nullptr, 0, pairs, top, n_experts, tile, 0, n_tiles, K, stream);
 }
 
 // Whether the choice and the placing of so many tokens are one launch.
@@ -1086,10 +1077,12 @@ RB_EXPORT int rb_route_choose_place_supports(int T, int n, int top, int groups, 
 }
 
 // The choice from sums z [T, n + n_extra] (see rb_route_select_scored; rb_route_next weighs) and the placing of its pairs in one
-// launch.  weigh: rows are multiplied by their pairs' weights.
+// launch.  weigh: rows are multiplied by their pairs' weights.  n_shared: every token's own row, unweighted, goes into so many tiles
+// ahead of the pairs' n_tiles (group n_experts: a shared expert whose matrices lie behind the others').
 RB_EXPORT int rb_route_choose_place(void* xp, int* pos, int* tile_group, const void* h, int64_t ldh, int dtype, float* weights,
                                     const float* z, const float* correction, int T, int n, int top, int groups, int keep, int scoring,
-                                    int n_extra, float* extra, int weigh, int n_experts, int tile, int n_tiles, int K, cudaStream_t stream) {
+                                    int n_extra, float* extra, int weigh, int n_experts, int tile, int n_shared, int n_tiles, int K,
+                                    cudaStream_t stream) {
   Choice c;
   c.weighing = take_weighing();
   RB_REQUIRE(T > 0 && n > 0 && top > 0 && top <= n && n_extra >= 0 && (n_extra == 0 || extra != nullptr) && scoring >= 0 && scoring <= 2,
@@ -1097,7 +1090,7 @@ RB_EXPORT int rb_route_choose_place(void* xp, int* pos, int* tile_group, const v
   RB_REQUIRE(groups <= 1 || n % groups == 0, "rb_route_choose_place: %d outputs are not %d equal groups", n, groups);
   c.sums = z; c.correction = correction; c.weights = weights; c.extra = extra;
   c.n = n; c.n_extra = n_extra; c.groups = groups < 1 ? 1 : groups; c.keep = keep; c.scoring = scoring;
-  return place_impl(xp, pos, tile_group, h, ldh, dtype, nullptr, nullptr, &c, weigh, T * top, top, n_experts, tile, n_tiles, K, stream);
+  return place_impl(xp, pos, tile_group, h, ldh, dtype, nullptr, nullptr, &c, weigh, T * top, top, n_experts, tile, n_shared, n_tiles, K, stream);
 }
 
 // The router's sums alone: z [T, n] = h Wr^T, float32, for few tokens.

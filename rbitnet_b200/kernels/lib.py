@@ -52,8 +52,7 @@ _SIGNATURES = {
     "rb_routed_plan": [P, P, P, P, I, I, I, I, I, P],
     "rb_routed_place": [P, P, P, P, L, I, P, P, I, I, I, I, I, I, P],
     "rb_routed_place_pairs": [],
-    "rb_routed_place_shared": [I],
-    "rb_route_choose_place": [P, P, P, P, L, I, P, P, P, I, I, I, I, I, I, I, P, I, I, I, I, I, P],
+    "rb_route_choose_place": [P, P, P, P, L, I, P, P, P, I, I, I, I, I, I, I, P, I, I, I, I, I, I, P],
     "rb_route_sums": [P, P, L, I, P, I, I, I, P],
     "rb_routed_gather": [P, P, L, I, P, I, I, P],
     "rb_routed_combine": [P, L, P, P, L, I, P, P, I, I, I, I, P],

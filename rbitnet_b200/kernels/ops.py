@@ -1413,11 +1413,9 @@ class CudaOps:
         self.lib.call("rb_route_sums", _ptr(z), _ptr(h), h.stride(0), self.code, _ptr(router), T, K, n + extra_rows, self._stream())
         if normalize is not None or weight_scale != 1.0:
             self.lib.call("rb_route_next", 0 if normalize is None else 1, float(normalize or 0.0), float(weight_scale), launches=0)
-        if n_shared:
-            self.lib.call("rb_routed_place_shared", n_shared, launches=0)
         self.lib.call("rb_route_choose_place", _ptr(placed.rows), _ptr(placed.pos), _ptr(placed.tile_group), _ptr(h), h.stride(0), self.code,
                       _ptr(weights), _ptr(z), _ptr(correction), T, n, int(top), int(groups), int(keep), _SCORING[scoring], int(extra_rows),
-                      _ptr(extra), 1 if weight_on_input else 0, n_experts, tile, n_tiles, K, self._stream())
+                      _ptr(extra), 1 if weight_on_input else 0, n_experts, tile, n_shared, n_tiles, K, self._stream())
         return placed
 
     # ------------------------------------------------------------------ routed experts

@@ -152,3 +152,35 @@ def test_weighted_sum_of_the_experts_rows(ops_of, dtype, T, E, top, accumulate, 
     if norm:
         after = nw.double() * torch.tanh(0.4 * want) + nb.double()
         assert float((out.double() - after).abs().max()) <= (2e-5 if dtype == F32 else 8e-3) * float(after.abs().max())
+
+
+def test_a_refused_choice_leaves_nothing_for_the_next_placing(ops_of):
+    """A choice with the tokens' own rows that is refused (more choices than outputs, unequal groups, an unknown scoring) and then a
+    plain placing: its rows, places and tiles, and nothing behind them."""
+    from rbitnet_b200.kernels.lib import KernelError
+    from rbitnet_b200.kernels.ops import _ptr
+    ops = ops_of(F32)
+    g = torch.Generator(device="cuda").manual_seed(3)
+    T, K, experts, top = 5, 64, 6, 2
+    h, router = (torch.randn(n, K, device="cuda", generator=g) for n in (T, experts))
+    pairs, tile, guard = T * top, 64, 256
+    n_tiles = ops.lib.raw("rb_routed_tiles")(pairs, experts, tile)
+    ids = torch.randint(0, experts, (T, top), dtype=torch.int32, device="cuda", generator=g)
+
+    def placed():
+        xp = torch.full((n_tiles * tile + guard, K), 7.0, device="cuda")
+        pos, groups = (torch.full((n + guard,), 77, dtype=torch.int32, device="cuda") for n in (pairs, n_tiles))
+        ops.lib.call("rb_routed_place", _ptr(xp), _ptr(pos), _ptr(groups), _ptr(h), K, ops.code, _ptr(ids), None, pairs, top, experts, tile,
+                     n_tiles, K, ops._stream())
+        return xp, pos, groups
+    want = placed()
+    for refused, error in (({"top": experts + 1, "groups": 0, "keep": 0}, KernelError), ({"top": top, "groups": 4, "keep": 1}, KernelError),
+                           ({"top": top, "groups": 0, "keep": 0, "scoring": "?"}, KeyError)):
+        with pytest.raises(error):
+            ops.route_and_place(h, router, None, n_experts=experts, inner=64, with_shared=True, **refused)
+        for got, expected in zip(placed(), want):
+            assert torch.equal(got, expected)
+    xp, pos, groups = want
+    assert bool((xp[n_tiles * tile:] == 7.0).all()) and bool((pos[pairs:] == 77).all()) and bool((groups[n_tiles:] == 77).all())
+    assert torch.equal(xp[pos[:pairs].long()], h.repeat_interleave(top, 0))
+    ops.check_errors()
