@@ -1366,8 +1366,7 @@ class CudaOps:
         None without).  ``normalize`` (a small number): the chosen outputs' weights are divided by their sum + it; then
         they are multiplied by ``weight_scale``.  Returns (ids, weights, extra)."""
         self._check(h, self.dtype, "route input")
-        if normalize is not None or weight_scale != 1.0:
-            self.lib.call("rb_route_next", 0 if normalize is None else 1, float(normalize or 0.0), float(weight_scale), launches=0)
+        scored = _SCORING[scoring]
         T, K = h.shape
         n = router.shape[0] - extra_rows
         ids = torch.empty((T, top), dtype=torch.int32, device=self.device)
@@ -1376,15 +1375,22 @@ class CudaOps:
         if T >= self.router_tc_from and router_tc is not None and self._tensor_core_ok(h, router_tc.w):
             # the sums (outputs and extra rows) on the tensor cores, then the choice
             z = self.linear(h, router_tc, out_dtype=torch.float32)
+            self._next_weighing(normalize, weight_scale)
             self.lib.call("rb_route_select_scored", _ptr(ids), _ptr(weights), _ptr(z), _ptr(correction), T, n, int(top),
-                          int(groups), int(keep), _SCORING[scoring], int(extra_rows), _ptr(extra),
+                          int(groups), int(keep), scored, int(extra_rows), _ptr(extra),
                           self._stream())
             return ids, weights, extra
         z = torch.empty((T, n + extra_rows), dtype=torch.float32, device=self.device)
+        self._next_weighing(normalize, weight_scale)
         self.lib.call("rb_route_scored", _ptr(ids), _ptr(weights), _ptr(h), h.stride(0), self.code, _ptr(router),
                       _ptr(correction), T, K, n, int(top), int(groups), int(keep), _ptr(z),
-                      _SCORING[scoring], int(extra_rows), _ptr(extra), self._stream(), launches=2)
+                      scored, int(extra_rows), _ptr(extra), self._stream(), launches=2)
         return ids, weights, extra
+
+    def _next_weighing(self, normalize: Optional[float], weight_scale: float):
+        """For the library's choice that is called right after this: whatever is called next takes it."""
+        if normalize is not None or weight_scale != 1.0:
+            self.lib.call("rb_route_next", 0 if normalize is None else 1, float(normalize or 0.0), float(weight_scale), launches=0)
 
     def route_and_place(self, h: torch.Tensor, router: torch.Tensor, correction: Optional[torch.Tensor], top: int, groups: int,
                         keep: int, n_experts: int, inner: int, scoring: str = "softmax", extra_rows: int = 0,
@@ -1394,6 +1400,7 @@ class CudaOps:
         tokens (None: not for these sizes).  ``with_shared``: the tokens' own rows are placed too, for one more expert whose
         matrices lie behind the others'."""
         self._check(h, self.dtype, "route input")
+        scored = _SCORING[scoring]
         T, K = h.shape
         n = router.shape[0] - extra_rows
         if not (self.choose_and_place and self.place_few_pairs and n_experts > 0
@@ -1411,10 +1418,9 @@ class CudaOps:
         placed = PlacedRows(weights, extra, torch.empty(((n_shared + n_tiles) * tile, K), dtype=self.dtype, device=self.device),
                             plan[:pairs], plan[pairs:], tile, n_shared)
         self.lib.call("rb_route_sums", _ptr(z), _ptr(h), h.stride(0), self.code, _ptr(router), T, K, n + extra_rows, self._stream())
-        if normalize is not None or weight_scale != 1.0:
-            self.lib.call("rb_route_next", 0 if normalize is None else 1, float(normalize or 0.0), float(weight_scale), launches=0)
+        self._next_weighing(normalize, weight_scale)
         self.lib.call("rb_route_choose_place", _ptr(placed.rows), _ptr(placed.pos), _ptr(placed.tile_group), _ptr(h), h.stride(0), self.code,
-                      _ptr(weights), _ptr(z), _ptr(correction), T, n, int(top), int(groups), int(keep), _SCORING[scoring], int(extra_rows),
+                      _ptr(weights), _ptr(z), _ptr(correction), T, n, int(top), int(groups), int(keep), scored, int(extra_rows),
                       _ptr(extra), 1 if weight_on_input else 0, n_experts, tile, n_shared, n_tiles, K, self._stream())
         return placed
 

@@ -184,3 +184,18 @@ def test_a_refused_choice_leaves_nothing_for_the_next_placing(ops_of):
     assert bool((xp[n_tiles * tile:] == 7.0).all()) and bool((pos[pairs:] == 77).all()) and bool((groups[n_tiles:] == 77).all())
     assert torch.equal(xp[pos[:pairs].long()], h.repeat_interleave(top, 0))
     ops.check_errors()
+
+
+@pytest.mark.parametrize("T", [3, 20, 70])
+def test_a_refused_scoring_leaves_no_weighing_for_the_next_choice(ops_of, T):
+    """Weights as they are after a call that asked for others and was refused."""
+    ops = ops_of(F32)
+    g = torch.Generator(device="cuda").manual_seed(T)
+    h, router = (torch.randn(n, 64, device="cuda", generator=g) for n in (T, 8))
+    ids, want, _ = ops.route_scored(h, router, None, 2, 0, 0)
+    for refused in (lambda: ops.route_scored(h, router, None, 2, 0, 0, scoring="?", normalize=1e-20, weight_scale=3.0),
+                    lambda: ops.route_and_place(h, router, None, 2, 0, 0, 8, 64, scoring="?", normalize=1e-20, weight_scale=3.0)):
+        with pytest.raises(KeyError):
+            refused()
+        again, weights, _ = ops.route_scored(h, router, None, 2, 0, 0)
+        assert torch.equal(again, ids) and torch.equal(weights, want)
