@@ -522,7 +522,7 @@ __global__ void gather_scaled_kernel(T* xp, const T* h, int64_t ldh, const int* 
 // chosen, rows of 2,048: the two took 5.1 us of a step, this one 2.1; 8 tokens, weighed rows 7.1 and 3.6).
 // A shared expert whose matrices lie behind the others' (group n_experts) takes the first `n_shared` tiles: row r of them is
 // token r's row, unweighted.
-constexpr int PLACE_PAIRS = 256;
+constexpr int PLACE_PAIRS = 256, PLACE_EXPERTS = 9984;      // (41 KB of shared memory with the pairs' ids and weights)
 // What a block does with its row once the ids (and, if rows are weighed, the weights) of all pairs are in shared memory.
 template <typename T>
 __device__ __forceinline__ void place_row(T* xp, int* pos, int* tile_group, const T* h, int64_t ldh, const int* s_ids,
@@ -1040,8 +1040,8 @@ static int place_impl(void* xp, int* pos, int* tile_group, const void* h, int64_
              "rb_routed_place: %d tiles of %d rows for %d pairs over %d experts", n_tiles, tile, pairs, n_experts);
   const int T = pairs / top;
   RB_REQUIRE(n_shared == 0 || (n_shared > 0 && (int64_t)n_shared * tile >= T), "rb_routed_place: %d tokens in %d shared tiles of %d rows", T, n_shared, tile);
+  RB_REQUIRE(n_experts <= PLACE_EXPERTS, "rb_routed_place: %d experts", n_experts);
   size_t smem = (size_t)(2 * PLACE_PAIRS + n_experts) * sizeof(int);
-  RB_REQUIRE(smem <= 40 * 1024, "rb_routed_place: %d experts", n_experts);
   const size_t four = dtype == RB_F32 ? 16 : 8;
   const int vec = K % 4 == 0 && ldh % 4 == 0 && (uintptr_t)xp % four == 0 && (uintptr_t)h % four == 0 ? 1 : 0;
   const int threads = K >= 1024 ? 256 : (K >= 512 ? 128 : 64), blocks = (n_shared + n_tiles) * tile;
@@ -1071,8 +1071,7 @@ RB_EXPORT int rb_routed_place(void* xp, int* pos, int* tile_group, const void* h
 
 // Whether the choice and the placing of so many tokens are one launch.
 RB_EXPORT int rb_route_choose_place_supports(int T, int n, int top, int groups, int n_experts) {
-  return T > 0 && T <= CHOOSE_TOKENS && T * top <= PLACE_PAIRS && n_experts > 0 &&
-         (size_t)(2 * PLACE_PAIRS + n_experts) * sizeof(int) <= 40 * 1024 &&
+  return T > 0 && T <= CHOOSE_TOKENS && T * top <= PLACE_PAIRS && n_experts > 0 && n_experts <= PLACE_EXPERTS &&
          (size_t)(2 * PLACE_PAIRS + n_experts) * sizeof(int) + (size_t)CHOOSE_WARPS * (2 * n + 2 * (groups < 1 ? 1 : groups)) * sizeof(float) <= 48 * 1024;
 }
 

@@ -199,3 +199,29 @@ def test_a_refused_scoring_leaves_no_weighing_for_the_next_choice(ops_of, T):
             refused()
         again, weights, _ = ops.route_scored(h, router, None, 2, 0, 0)
         assert torch.equal(again, ids) and torch.equal(weights, want)
+
+
+@pytest.mark.parametrize("weighed", [False, True])
+def test_few_pairs_of_as_many_experts_as_are_counted(ops_of, weighed):
+    """9,984 experts are placed (more than the plan for many pairs takes), one more is refused."""
+    from rbitnet_b200.kernels.lib import KernelError
+    from rbitnet_b200.kernels.ops import _ptr
+    ops = ops_of(F32)
+    T, K, top, tile, experts = 3, 64, 2, 16, 9984
+    g = torch.Generator(device="cuda").manual_seed(1)
+    h, w = torch.randn(T, K, device="cuda", generator=g), torch.rand(T, top, device="cuda", generator=g)
+    ids = torch.tensor([[9983, 0], [5, 9983], [9728, 9984]], dtype=torch.int32, device="cuda")        # the last is an identity expert
+    n_tiles = ops.lib.raw("rb_routed_tiles")(T * top, experts, tile)
+    xp, pos, groups = torch.full((n_tiles * tile, K), 7.0, device="cuda"), *(torch.full((n,), -7, dtype=torch.int32, device="cuda") for n in (T * top, n_tiles))
+
+    def place(n):
+        ops.lib.call("rb_routed_place", _ptr(xp), _ptr(pos), _ptr(groups), _ptr(h), K, ops.code, _ptr(ids), _ptr(w if weighed else None),
+                     T * top, top, n, tile, n_tiles, K, ops._stream())
+    place(experts)
+    assert groups.tolist() == [0, 5, 9728, 9983, -1, -1] and pos.tolist() == [48, 0, 16, 49, 32, -1]
+    rows = torch.zeros_like(xp)
+    at = pos[pos >= 0].long()
+    rows[at] = (h.repeat_interleave(top, 0) * (w.view(-1, 1) if weighed else 1.0))[pos >= 0]
+    assert torch.equal(xp, rows)
+    with pytest.raises(KernelError, match="9985 experts"):
+        place(experts + 1)
