@@ -623,7 +623,7 @@ __global__ void __launch_bounds__(256) place_kernel(T* xp, int* pos, int* tile_g
 // The choice and the placing in one launch, for up to CHOOSE_TOKENS tokens whose sums a product has left: every block makes
 // all tokens' choices for itself (a warp a token, two turns at most), then places its row.  The first block leaves weights and
 // extra sums for the kernels behind.  A decode step pays one launch instead of two: the two took 3.8 + 2.6 us of a step at 8
-// tokens and 32 outputs, this one 4.2.  Many tokens' choices would be made too often: the two kernels again.
+// tokens and 32 outputs, this one 4.2.  Many tokens' choices would be made too often: the two kernels again (rb_route_choose_place_pays).
 constexpr int CHOOSE_TOKENS = 16, CHOOSE_WARPS = 8;
 struct Choice {
   const float* sums;          // [tokens, n + n_extra]
@@ -1069,10 +1069,28 @@ RB_EXPORT int rb_routed_place(void* xp, int* pos, int* tile_group, const void* h
   return place_impl(xp, pos, tile_group, h, ldh, dtype, ids, weights, nullptr, 0, pairs, top, n_experts, tile, 0, n_tiles, K, stream);
 }
 
-// Whether the choice and the placing of so many tokens are one launch.
+// The same with every token's own row, unweighted, in n_shared tiles ahead of the pairs' n_tiles (group n_experts: a shared expert
+// whose matrices lie behind the others').
+RB_EXPORT int rb_routed_place_shared(void* xp, int* pos, int* tile_group, const void* h, int64_t ldh, int dtype, const int* ids,
+                                     const float* weights, int pairs, int top, int n_experts, int tile, int n_shared, int n_tiles,
+                                     int K, cudaStream_t stream) {
+  return place_impl(xp, pos, tile_group, h, ldh, dtype, ids, weights, nullptr, 0, pairs, top, n_experts, tile, n_shared, n_tiles, K, stream);
+}
+
+// Whether the choice and the placing of so many tokens can be one launch.
 RB_EXPORT int rb_route_choose_place_supports(int T, int n, int top, int groups, int n_experts) {
   return T > 0 && T <= CHOOSE_TOKENS && T * top <= PLACE_PAIRS && n_experts > 0 && n_experts <= PLACE_EXPERTS &&
          (size_t)(2 * PLACE_PAIRS + n_experts) * sizeof(int) + (size_t)CHOOSE_WARPS * (2 * n + 2 * (groups < 1 ? 1 : groups)) * sizeof(float) <= 48 * 1024;
+}
+
+// Whether one launch is also the faster way, for so many blocks (rows of all tiles): every block makes every token's choice again.
+// us of a step of rows of 2,048 values, sums, choice and placing, one launch against two, tiles of 16 (64 in float32) rows: 32 outputs,
+// top 4, no groups: 1 token 5.8, 6.5 (6.2, 7.1), 4 6.1, 6.7 (8.3, 7.5), 8 7.2, 7.3 (11.6, 9.5), 16 9.2, 7.4 (15.3, 9.8); in 8 groups
+// 4 7.7, 7.6, 8 9.4, 8.3; 64 outputs, top 8: 2 9.9, 10.3 (15.2, 10.9), 4 11.4, 10.6, 16 31, 12 (94, 18); 128 outputs, top 8: 2 10.0, 10.5
+// (15.7, 10.9), 16 53, 15 (187, 28); 256 in 8 groups, top 8: 1 13.5, 14.5, 2 16.2, 14.9, 16 106, 22 (363, 38).
+RB_EXPORT int rb_route_choose_place_pays(int T, int n, int groups, int blocks) {
+  if (n <= 32 && groups <= 1) return T <= 8 && blocks <= 640;
+  return (int64_t)blocks * T * ((n + 63) / 64) <= 1152;
 }
 
 // The choice from sums z [T, n + n_extra] (see rb_route_select_scored; rb_route_next weighs) and the placing of its pairs in one

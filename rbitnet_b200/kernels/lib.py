@@ -51,6 +51,7 @@ _SIGNATURES = {
     "rb_routed_tiles": [I, I, I],
     "rb_routed_plan": [P, P, P, P, I, I, I, I, I, P],
     "rb_routed_place": [P, P, P, P, L, I, P, P, I, I, I, I, I, I, P],
+    "rb_routed_place_shared": [P, P, P, P, L, I, P, P, I, I, I, I, I, I, I, P],
     "rb_routed_place_pairs": [],
     "rb_route_choose_place": [P, P, P, P, L, I, P, P, P, I, I, I, I, I, I, I, P, I, I, I, I, I, I, P],
     "rb_route_sums": [P, P, L, I, P, I, I, I, P],
@@ -157,6 +158,7 @@ class KernelLibrary:
         self.declare("rb_gemm_tc_plan", [I, I, I, I, I, I, P])
         self.declare("rb_gemm_tc_share_for_test", [I])
         self.declare("rb_route_choose_place_supports", [I, I, I, I, I])
+        self.declare("rb_route_choose_place_pays", [I, I, I, I])
         self.declare("rb_route_sums_supports", [P, L, I, P, I, I])
         self.declare("rb_f32_tc_plan_of", [I, I, I, I, I, P])
         self.declare("rb_gemm_tc_tail_for_test", [I])

@@ -1396,8 +1396,8 @@ class CudaOps:
                         keep: int, n_experts: int, inner: int, scoring: str = "softmax", extra_rows: int = 0,
                         normalize: Optional[float] = None, weight_scale: float = 1.0, weight_on_input: bool = False,
                         with_shared: bool = False) -> Optional["PlacedRows"]:
-        """``route_scored`` and the sorting of the pairs by expert that ``routed_experts`` begins with, in two launches for up to 16
-        tokens (None: not for these sizes).  ``with_shared``: the tokens' own rows are placed too, for one more expert whose
+        """``route_scored`` and the sorting of the pairs by expert that ``routed_experts`` begins with, for up to 16 tokens (None: not
+        for these sizes), in two launches where the choice costs less than a third.  ``with_shared``: the tokens' own rows are placed too, for one more expert whose
         matrices lie behind the others'."""
         self._check(h, self.dtype, "route input")
         scored = _SCORING[scoring]
@@ -1419,6 +1419,14 @@ class CudaOps:
                             plan[:pairs], plan[pairs:], tile, n_shared)
         self.lib.call("rb_route_sums", _ptr(z), _ptr(h), h.stride(0), self.code, _ptr(router), T, K, n + extra_rows, self._stream())
         self._next_weighing(normalize, weight_scale)
+        if not self.lib.raw("rb_route_choose_place_pays")(T, n, int(groups), placed.rows.shape[0]):
+            ids = torch.empty((T, top), dtype=torch.int32, device=self.device)
+            self.lib.call("rb_route_select_scored", _ptr(ids), _ptr(weights), _ptr(z), _ptr(correction), T, n, int(top), int(groups), int(keep),
+                          scored, int(extra_rows), _ptr(extra), self._stream())
+            self.lib.call("rb_routed_place_shared", _ptr(placed.rows), _ptr(placed.pos), _ptr(placed.tile_group), _ptr(h), h.stride(0),
+                          self.code, _ptr(ids), _ptr(weights if weight_on_input else None), pairs, top, n_experts, tile, n_shared, n_tiles,
+                          K, self._stream())
+            return placed
         self.lib.call("rb_route_choose_place", _ptr(placed.rows), _ptr(placed.pos), _ptr(placed.tile_group), _ptr(h), h.stride(0), self.code,
                       _ptr(weights), _ptr(z), _ptr(correction), T, n, int(top), int(groups), int(keep), scored, int(extra_rows),
                       _ptr(extra), 1 if weight_on_input else 0, n_experts, tile, n_shared, n_tiles, K, self._stream())

@@ -183,6 +183,17 @@ def test_float32_products_that_go_to_the_tensor_cores(lib):
     assert plan(4000, 64, 256, 64) == (0, 0) and plan(2048, 128, 128, 16) == (128, 1) and plan(300, 512, 192) == (0, 0)
 
 
+def test_when_few_tokens_choices_are_made_by_the_kernel_that_places(lib):
+    """Every block makes every token's choice: few blocks times tokens, fewer with more outputs than a warp has lanes or in groups."""
+    def pays(T, n, groups, top, tile, shared=0):
+        n_tiles = lib.raw("rb_routed_tiles")(T * top, n, tile) + shared
+        return bool(lib.raw("rb_route_choose_place_pays")(T, n, groups, n_tiles * tile))
+    assert pays(8, 32, 0, 4, 16, 1) and not pays(16, 32, 0, 4, 16) and not pays(4, 32, 0, 4, 64) and pays(2, 32, 0, 4, 64, 1)
+    assert pays(4, 32, 8, 4, 16, 1) and not pays(8, 32, 8, 4, 16) and pays(2, 32, 8, 4, 16, 1)
+    assert pays(2, 128, 0, 8, 16) and not pays(4, 64, 0, 8, 16) and not pays(2, 64, 0, 8, 64)
+    assert pays(1, 256, 8, 8, 16) and not pays(2, 256, 8, 8, 16) and not pays(16, 256, 8, 8, 64)
+
+
 def test_when_a_matrix_memory_goes_in_chunks():
     """The longest run decides where the runs are few, not their average; small memories and short runs stay token by token."""
     from rbitnet_b200.kernels.ops import memory_chunks_pay

@@ -86,7 +86,8 @@ def test_sums_of_few_tokens(ops_of, dtype, K):
 
 
 @pytest.mark.parametrize("dtype", [F32, BF16])
-@pytest.mark.parametrize("T,experts,inner,E,identity", [(1, 32, 88, 128, 0), (5, 6, 40, 96, 0), (16, 3, 64, 200, 0), (3, 40, 24, 64, 8)])
+@pytest.mark.parametrize("T,experts,inner,E,identity", [(1, 32, 88, 128, 0), (5, 6, 40, 96, 0), (16, 3, 64, 200, 0), (3, 40, 24, 64, 8),
+                                                        (9, 32, 88, 128, 0), (16, 70, 24, 64, 8)])
 @pytest.mark.parametrize("weight_on_input", [False, True])
 def test_a_shared_expert_behind_the_others(ops_of, dtype, T, experts, inner, E, identity, weight_on_input):
     """The shared expert's rows ahead of the pairs' in one buffer, its matrices behind the others', beside the same made apart."""
