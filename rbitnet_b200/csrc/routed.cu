@@ -295,16 +295,19 @@ __global__ void __launch_bounds__(256) route_kernel(int* ids, float* weights,
   route_select(z, z + n, z + 2 * n, correction, n_out, top, groups, keep, lane, ids, weights, t0 + warp, scoring, weighing);
 }
 
-// Few tokens: a warp makes one output of one token, so that a step's sums run on many SMs, with the same sums as above (lane l
-// takes every 32nd group of four values, then the lanes' shares in a fixed tree).  Up to 2,048 values of the warp's row of Wr are
-// asked for before the wait for the kernel before.  2 tokens, 32 outputs in 8 groups, 2,048 values: the kernel that makes sums and
-// choice in one block a token and the placing took 14.6 + 3.1 us of a step, this and the choice with the placing (below) 3.7 + 5.3;
-// 8 tokens: a tensor-core product with K in 8 parts 3.8, this 4.4 at twice the precision, and less where the kernel before ends early.
+// Few tokens: a warp makes one output of one token, or of two where there are many of both, so that a step's sums run on many SMs,
+// with the same sums as above (lane l takes every 32nd group of four values, then the lanes' shares in a fixed tree).  Up to 2,048
+// values of the warp's row of Wr are asked for before the wait for the kernel before.  2 tokens, 32 outputs in 8 groups, 2,048 values:
+// the kernel that makes sums and choice in one block a token and the placing took 14.6 + 3.1 us of a step, this and the choice with the
+// placing (below) 3.7 + 5.3; 8 tokens: a tensor-core product with K in 8 parts 3.8, this 4.4 at twice the precision, and less where
+// the kernel before ends early.  16 tokens of 256 outputs, sums and choice, with a token and with two a warp, and the tensor-core
+// product instead (which a scored router takes from 17 tokens on): K 2,048 11.3, 8.8, 9.1; 4,096 13.8, 10.6, 10.1; 7,168 17.3, 13.0,
+// 11.6; float32 63 tokens of K 2,048 22.6, 16.0 (four tokens a warp: 9.5 to 10.4 for the first; eight 11.4).
 constexpr int SUM_WARPS = 4, SUM_AHEAD = 16;
-template <typename TI>
-__global__ void __launch_bounds__(SUM_WARPS * 32) route_sums_kernel(float* z, const TI* h, int64_t ldh, const float* Wr, int K, int n) {
+template <typename TI, int TOKENS>
+__global__ void __launch_bounds__(SUM_WARPS * 32) route_sums_kernel(float* z, const TI* h, int64_t ldh, const float* Wr, int T, int K, int n) {
   rb_pdl_launch_dependents();
-  const int lane = threadIdx.x & 31, e = blockIdx.x * SUM_WARPS + (threadIdx.x >> 5), t = blockIdx.y;
+  const int lane = threadIdx.x & 31, e = blockIdx.x * SUM_WARPS + (threadIdx.x >> 5), t0 = blockIdx.y * TOKENS;
   if (e >= n) return;
   const float* w = Wr + (int64_t)e * K;
   float ahead[SUM_AHEAD][4];
@@ -315,27 +318,38 @@ __global__ void __launch_bounds__(SUM_WARPS * 32) route_sums_kernel(float* z, co
     else ahead[u][0] = ahead[u][1] = ahead[u][2] = ahead[u][3] = 0.f;
   }
   rb_pdl_wait();
-  const TI* row = h + (int64_t)t * ldh;
-  float acc = 0.f;
+  const TI* row[TOKENS];                                 // (the last token's again behind it: a sum that nobody keeps)
+  float acc[TOKENS];
+#pragma unroll
+  for (int i = 0; i < TOKENS; ++i) {
+    row[i] = h + (int64_t)min(t0 + i, T - 1) * ldh;
+    acc[i] = 0.f;
+  }
+  auto add = [&](int k, const float (&wv)[4]) {
+    float hv[TOKENS][4];
+#pragma unroll
+    for (int i = 0; i < TOKENS; ++i) rb_load4(row[i] + k, hv[i]);
+#pragma unroll
+    for (int i = 0; i < TOKENS; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[i] = fmaf(hv[i][j], wv[j], acc[i]);
+  };
 #pragma unroll
   for (int u = 0; u < SUM_AHEAD; ++u) {
     const int k = lane * 4 + u * 128;
-    if (k < K) {
-      float hv[4];
-      rb_load4(row + k, hv);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) acc = fmaf(hv[i], ahead[u][i], acc);
-    }
+    if (k < K) add(k, ahead[u]);
   }
+#pragma unroll 8
   for (int k = lane * 4 + SUM_AHEAD * 128; k < K; k += 128) {
-    float hv[4], wv[4];
-    rb_load4(row + k, hv);
+    float wv[4];
     rb_load4(w + k, wv);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) acc = fmaf(hv[i], wv[i], acc);
+    add(k, wv);
   }
-  acc = rb_warp_sum(acc);
-  if (lane == 0) z[(int64_t)t * n + e] = acc;
+#pragma unroll
+  for (int i = 0; i < TOKENS; ++i) {
+    const float sum = rb_warp_sum(acc[i]);
+    if (lane == 0 && t0 + i < T) z[(int64_t)(t0 + i) * n + e] = sum;
+  }
 }
 
 // Many tokens: the router's sums as a tiled float32 product (16 tokens by 64 outputs a block, k in steps of 32 through
@@ -883,13 +897,19 @@ __global__ void square_relu_kernel(T* out, const T* in, int64_t n) {
 }  // namespace
 
 static int launch_sums(float* z, const void* h, int64_t ldh, int h_dtype, const float* Wr, int T, int K, int n, cudaStream_t stream) {
-  const dim3 grid((n + SUM_WARPS - 1) / SUM_WARPS, T);
-  if (h_dtype == RB_F32)
-    RB_LAUNCH("route_sums_kernel", (route_sums_kernel<float>), grid, SUM_WARPS * 32, 0, stream, z, (const float*)h, ldh, Wr, K, n);
-  else if (h_dtype == RB_BF16)
-    RB_LAUNCH("route_sums_kernel", (route_sums_kernel<__nv_bfloat16>), grid, SUM_WARPS * 32, 0, stream, z, (const __nv_bfloat16*)h, ldh, Wr, K, n);
-  else
-    RB_FAIL("rb_route: unknown dtype %d", h_dtype);
+  const int tokens = T * n <= 2048 ? 1 : 2;            // (16 tokens of 128 outputs, a token a warp: 7.9 us, the tensor-core product 8.8)
+  const dim3 grid((n + SUM_WARPS - 1) / SUM_WARPS, (T + tokens - 1) / tokens);
+#define GO(TI)                                                                                                                    \
+  do {                                                                                                                            \
+    if (tokens == 1)                                                                                                              \
+      RB_LAUNCH("route_sums_kernel", (route_sums_kernel<TI, 1>), grid, SUM_WARPS * 32, 0, stream, z, (const TI*)h, ldh, Wr, T, K, n); \
+    else                                                                                                                          \
+      RB_LAUNCH("route_sums_kernel", (route_sums_kernel<TI, 2>), grid, SUM_WARPS * 32, 0, stream, z, (const TI*)h, ldh, Wr, T, K, n); \
+  } while (0)
+  if (h_dtype == RB_F32) GO(float);
+  else if (h_dtype == RB_BF16) GO(__nv_bfloat16);
+  else RB_FAIL("rb_route: unknown dtype %d", h_dtype);
+#undef GO
   RB_CHECK_LAUNCH("rb_route");
   return 0;
 }
