@@ -924,6 +924,19 @@ static int select_impl(int* ids, float* weights, const float* z, const float* co
   return 0;
 }
 
+// rows of 16-byte (float32) or 8-byte loads
+static bool route_rows_vec(const void* h, int64_t ldh, int h_dtype, const float* Wr, int K) {
+  const int elem = h_dtype == RB_F32 ? 4 : 2;
+  return K % 4 == 0 && ldh % 4 == 0 && (uintptr_t)h % (4 * elem) == 0 && (uintptr_t)Wr % 16 == 0;
+}
+// the choice by itself (four tokens a block) has room for its scratch
+static bool choice_fits(int n, int groups) { return (size_t)4 * (2 * n + 2 * (groups < 1 ? 1 : groups)) * sizeof(float) <= 48 * 1024; }
+
+// The kernels of rb_route and rb_route_scored for these sizes: 2 (sums, then choice), which want z_scratch, or 1.
+RB_EXPORT int rb_route_kernels(const void* h, int64_t ldh, int h_dtype, const float* Wr, int T, int K, int n, int groups) {
+  return T >= 64 || (route_rows_vec(h, ldh, h_dtype, Wr, K) && choice_fits(n, groups)) ? 2 : 1;
+}
+
 // ids, weights: [T, top].  h: the input rows (dtype h_dtype).  Wr: float32 [n, K]; correction: float32 [n] or null.
 // groups <= 1 or keep >= groups: every output can be chosen.  z_scratch: T * n floats (the router's
 // sums are then a kernel of their own that leaves them there), or null.
@@ -955,9 +968,8 @@ static int route_impl(int* ids, float* weights, const void* h, int64_t ldh, int 
     RB_CHECK_LAUNCH("rb_route");
     return 0;
   }
-  const int elem = h_dtype == RB_F32 ? 4 : 2;
-  const int vec = K % 4 == 0 && ldh % 4 == 0 && (uintptr_t)h % (4 * elem) == 0 && (uintptr_t)Wr % 16 == 0;
-  if (T < 64 && z_scratch != nullptr && vec && (size_t)4 * (2 * n + 2 * groups) * sizeof(float) <= 48 * 1024) {      // (the choice's scratch)
+  const int vec = route_rows_vec(h, ldh, h_dtype, Wr, K) ? 1 : 0;
+  if (T < 64 && z_scratch != nullptr && vec && choice_fits(n, groups)) {
     if (launch_sums(z_scratch, h, ldh, h_dtype, Wr, T, K, n_all, stream) != 0) return -1;
     return select_impl(ids, weights, z_scratch, correction, T, n, top, groups, keep, scoring, n_extra, extra, weighing, stream);
   }
@@ -1132,8 +1144,7 @@ RB_EXPORT int rb_route_choose_place(void* xp, int* pos, int* tile_group, const v
 
 // The router's sums alone: z [T, n] = h Wr^T, float32, for few tokens.
 RB_EXPORT int rb_route_sums_supports(const void* h, int64_t ldh, int h_dtype, const float* Wr, int T, int K) {
-  const int elem = h_dtype == RB_F32 ? 4 : 2;
-  return T > 0 && T < 64 && K % 4 == 0 && ldh % 4 == 0 && (uintptr_t)h % (4 * elem) == 0 && (uintptr_t)Wr % 16 == 0;
+  return T > 0 && T < 64 && route_rows_vec(h, ldh, h_dtype, Wr, K);
 }
 RB_EXPORT int rb_route_sums(float* z, const void* h, int64_t ldh, int h_dtype, const float* Wr, int T, int K, int n, cudaStream_t stream) {
   if (T == 0) return 0;

@@ -159,6 +159,7 @@ class KernelLibrary:
         self.declare("rb_gemm_tc_share_for_test", [I])
         self.declare("rb_route_choose_place_supports", [I, I, I, I, I])
         self.declare("rb_route_choose_place_pays", [I, I, I, I])
+        self.declare("rb_route_kernels", [P, L, I, P, I, I, I, I])
         self.declare("rb_route_sums_supports", [P, L, I, P, I, I])
         self.declare("rb_f32_tc_plan_of", [I, I, I, I, I, P])
         self.declare("rb_gemm_tc_tail_for_test", [I])

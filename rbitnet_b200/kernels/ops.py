@@ -1380,11 +1380,12 @@ class CudaOps:
                           int(groups), int(keep), scored, int(extra_rows), _ptr(extra),
                           self._stream())
             return ids, weights, extra
-        z = torch.empty((T, n + extra_rows), dtype=torch.float32, device=self.device)
+        kernels = self.lib.raw("rb_route_kernels")(_ptr(h), h.stride(0), self.code, _ptr(router), T, K, n, int(groups))
+        z = torch.empty((T, n + extra_rows), dtype=torch.float32, device=self.device) if kernels == 2 else None
         self._next_weighing(normalize, weight_scale)
         self.lib.call("rb_route_scored", _ptr(ids), _ptr(weights), _ptr(h), h.stride(0), self.code, _ptr(router),
                       _ptr(correction), T, K, n, int(top), int(groups), int(keep), _ptr(z),
-                      scored, int(extra_rows), _ptr(extra), self._stream(), launches=2)
+                      scored, int(extra_rows), _ptr(extra), self._stream(), launches=kernels)
         return ids, weights, extra
 
     def _next_weighing(self, normalize: Optional[float], weight_scale: float):
@@ -1461,10 +1462,12 @@ class CudaOps:
             self.lib.call("rb_route_select", _ptr(ids), _ptr(weights), _ptr(z), _ptr(correction), T, n, int(top), int(groups),
                           int(keep), self._stream())
             return ids, weights
-        # the router's sums are a kernel of their own (from 64 tokens on a tiled product), which leaves them in z
-        z = torch.empty((T, n), dtype=torch.float32, device=self.device)
+        # the router's sums are a kernel of their own (from 64 tokens on a tiled product), which leaves them in z; rows without wide
+        # loads and more outputs than the choice has room for go through one kernel
+        kernels = self.lib.raw("rb_route_kernels")(_ptr(h), h.stride(0), self.code, _ptr(router), T, K, n, int(groups))
+        z = torch.empty((T, n), dtype=torch.float32, device=self.device) if kernels == 2 else None
         self.lib.call("rb_route", _ptr(ids), _ptr(weights), _ptr(h), h.stride(0), self.code, _ptr(router), _ptr(correction),
-                      T, K, n, int(top), int(groups), int(keep), _ptr(z), self._stream(), launches=2)
+                      T, K, n, int(top), int(groups), int(keep), _ptr(z), self._stream(), launches=kernels)
         return ids, weights
 
     def routed_tile(self, pairs: int, n_experts: int, inner: int, width: int) -> int:

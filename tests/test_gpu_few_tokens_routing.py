@@ -226,3 +226,23 @@ def test_few_pairs_of_as_many_experts_as_are_counted(ops_of, weighed):
     assert torch.equal(xp, rows)
     with pytest.raises(KernelError, match="9985 experts"):
         place(experts + 1)
+
+
+@pytest.mark.parametrize("T,K,n,kernels", [(3, 64, 8, 2), (3, 66, 8, 1), (70, 66, 8, 2), (3, 64, 1600, 1), (63, 64, 1500, 2)])
+def test_as_many_launches_are_counted_as_there_are(ops_of, T, K, n, kernels):
+    """Few tokens with rows of wide loads, without, and with more outputs than the choice by itself has room for."""
+    from torch.profiler import profile, ProfilerActivity
+    ops = ops_of(F32)
+    g = torch.Generator(device="cuda").manual_seed(n)
+    h, router = torch.randn(T, K, device="cuda", generator=g), torch.randn(n, K, device="cuda", generator=g) / math.sqrt(K)
+    for choose in (lambda: ops.route_scored(h, router, None, 2, 0, 0)[:2], lambda: ops.route(h, router, None, 2, 0, 0)):
+        choose()
+        torch.cuda.synchronize()
+        before = ops.lib.launches
+        with profile(activities=[ProfilerActivity.CUDA]) as seen:
+            ids, w = choose()
+            torch.cuda.synchronize()
+        assert sum("route" in e.name and "kernel" in e.name for e in seen.events()) == kernels == ops.lib.launches - before
+        z = torch.softmax(h.double() @ router.double().T, 1)
+        best = z.topk(2, dim=1)
+        assert torch.equal(ids.long(), best.indices) and torch.allclose(w.double(), best.values, rtol=2e-5, atol=1e-7)
