@@ -762,12 +762,15 @@ gemm_wx_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
       const bool emit_tanh = emit && p.emit_b != nullptr;
       const float b_n = emit_tanh && n_in ? p.emit_b[n] : 0.f;
       auto add_up = [&](auto known) {
-        // Tiles of 32 and 64 tokens in 2 or 4 parts: all the loads of the CTA's share in flight at once.  In rounds of eight columns
-        // (four of 32 tokens) each round waited for the others' memory: us before and now, 64 tokens in 2 parts, 2,048 x 2,048 16.7,
-        // 11.1; 4,096 x 4,096 22.6, 16.9; in 4 parts 10.4, 8.5; 14.8, 12.9; two tiles of 32 in 4 parts 7.1, 6.2; 12.3, 11.4.  (8 parts
-        // were one round.  Tiles of 16 tokens gain nothing, and more code costs their short kernels 1-2 %.)
+        // The parts of 2 and 4 are known to the code of tiles of 32 and 64 tokens, which leaves out the loads of parts that are not there
+        // (us of a product whose W comes from memory, before this and the issuing warps, and with both: 2,048 x 2,048, 64 tokens 6.8, 5.8, 256 tokens 11.8, 8.8; 4,096 x 4,096
+        // 128 tokens 15.6, 12.6, 256 23.9, 16.7; 11,264 gated rows of 2,048, 64 tokens 16.5, 12.9).  Up to eight columns in flight: with a CTA's
+        // whole share of 32 columns the added product takes 165 registers, two CTAs of it all of an SM's, and no block of the kernel
+        // behind it gets in before it ends; the 32-layer 8B shape at batch 64 then decodes 9,180 tokens/s instead of 9,500, and 192
+        // tokens of 4,096 x 4,096 take 17.3 us instead of 16.6.  (Tiles of 16 tokens gain nothing, and more code costs their short
+        // kernels 1-2 %.)
         constexpr int KNOWN = decltype(known)::value, PARTS = KNOWN > 0 ? KNOWN : 8;
-        constexpr int CPI = KNOWN > 0 && BN <= 64 ? BN / KNOWN : (BN >= 64 ? 8 : (BN >= 32 ? 4 : 2));
+        constexpr int CPI = KNOWN > 0 ? (BN / KNOWN < 8 ? BN / KNOWN : 8) : (BN >= 64 ? 8 : (BN >= 32 ? 4 : 2));
         uint32_t remote[PARTS];
 #pragma unroll
         for (int r = 0; r < PARTS; ++r)
