@@ -200,7 +200,12 @@ __device__ __forceinline__ void cluster_sync_all() {
 // that holds the tile's first k blocks and is taken first; so the part that everybody else waits
 // for waits for nobody, all CTAs of the launch are resident (one per SM at most), and every wait is
 // bounded like the others.  The last part sets the count back to zero.
-template <int BN, int STAGES, int EPI, typename OutT, int MINB>
+//
+// GROUPED (see GemmParams::tile_group) is a kernel of its own: a tile's place and group then come out of counts and loads, which
+// the compiler takes for different in every lane, and the plain products' loads would take their coordinates through
+// vector registers too.  One kernel for both cost the 32-layer 8B shape's steps 2.7 % (batch 8: 2,406 and 2,470 tokens/s, batch 1
+// 336 and 347); the shuffles make the values the warp's again (with them in one kernel for both 2,455 and 345).
+template <int BN, int STAGES, int EPI, typename OutT, int MINB, bool GROUPED>
 __global__ void __launch_bounds__((block_threads<BN, EPI>()), MINB)
 gemm_wx_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX,
                const __grid_constant__ typename OutputMap<leaves_by_tma<BN, EPI>()>::type tmC, GemmParams p) {
@@ -281,11 +286,12 @@ gemm_wx_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
   // without, so the items of the former go first, and the CTAs share them out evenly: taken as they lie, 21 of 32 tiles gave a
   // third of the CTAs three of them and another third one.
   int n_filled = 0;
-  if (p.tile_group != nullptr) {
+  if (GROUPED) {
     rb_pdl_wait();
     if (BN < 128)
       for (int i = 0; i < p.n_t_tiles; i += blockDim.x)
         n_filled += __syncthreads_count(i + (int)threadIdx.x < p.n_t_tiles && p.tile_group[i + (int)threadIdx.x] >= 0);
+    n_filled = __shfl_sync(0xffffffffu, n_filled, 0);
   }
   // Barriers and tensor memory are ready.  Whoever touches memory that an earlier kernel may
   // still be writing or reading calls rb_pdl_wait() first: the loader before it loads X, the
@@ -333,7 +339,7 @@ gemm_wx_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
       const int width = min(p.t_band, p.n_t_tiles - band * p.t_band);
       s.w_tile = in_band / width;
       t_tile = band * p.t_band + in_band - s.w_tile * width;
-    } else if (p.tile_group != nullptr) {
+    } else if (GROUPED) {
       const int filled = p.n_w_tiles * n_filled, rest = p.n_t_tiles - n_filled;
       if (tile < filled) { s.w_tile = tile / n_filled; t_tile = tile - s.w_tile * n_filled; }
       else { s.w_tile = (tile - filled) / rest; t_tile = n_filled + (tile - filled) - s.w_tile * rest; }
@@ -346,8 +352,8 @@ gemm_wx_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
     s.kb_begin = split * p.kb_per_split;
     s.nkb = max(0, min(nkb_total, s.kb_begin + p.kb_per_split) - s.kb_begin);
     s.w0 = s.n0;
-    if (p.tile_group != nullptr) {
-      const int g = p.tile_group[t_tile];
+    if (GROUPED) {
+      const int g = __shfl_sync(0xffffffffu, p.tile_group[t_tile], 0);
       if (g < 0) s.nkb = 0;
       else s.w0 = g * p.group_rows + s.n0;
     }
@@ -762,13 +768,13 @@ gemm_wx_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
       const bool emit_tanh = emit && p.emit_b != nullptr;
       const float b_n = emit_tanh && n_in ? p.emit_b[n] : 0.f;
       auto add_up = [&](auto known) {
-        // The parts of 2 and 4 are known to the code of tiles of 32 and 64 tokens, which leaves out the loads of parts that are not there
-        // (us of a product whose W comes from memory, before this and the issuing warps, and with both: 2,048 x 2,048, 64 tokens 6.8, 5.8, 256 tokens 11.8, 8.8; 4,096 x 4,096
-        // 128 tokens 15.6, 12.6, 256 23.9, 16.7; 11,264 gated rows of 2,048, 64 tokens 16.5, 12.9).  Up to eight columns in flight: with a CTA's
-        // whole share of 32 columns the added product takes 165 registers, two CTAs of it all of an SM's, and no block of the kernel
-        // behind it gets in before it ends; the 32-layer 8B shape at batch 64 then decodes 9,180 tokens/s instead of 9,500, and 192
-        // tokens of 4,096 x 4,096 take 17.3 us instead of 16.6.  (Tiles of 16 tokens gain nothing, and more code costs their short
-        // kernels 1-2 %.)
+        // The parts of 2 and 4 are known to the code of tiles of 32 and 64 tokens, which leaves out the loads of parts that are not
+        // there (us of a product whose W comes from memory, before this and the issuing warps, and with both: 2,048 x 2,048, 64 tokens
+        // 6.8, 5.8, 256 tokens 11.8, 8.8; 4,096 x 4,096 128 tokens 15.6, 12.6, 256 23.9, 16.7; 11,264 gated rows of 2,048, 64 tokens
+        // 16.5, 12.9).  Up to eight columns in flight: with a CTA's whole share of 32 columns the added product takes 165 registers, two
+        // CTAs of it all of an SM's, and no block of the kernel behind it gets in before it ends; the 32-layer 8B shape at batch 64
+        // then decodes 9,160 tokens/s instead of 9,500, and 192 tokens of 4,096 x 4,096 take 17.3 us instead of 16.6.  (Tiles of 16
+        // tokens gain nothing, and more code costs their short kernels 1-2 %.)
         constexpr int KNOWN = decltype(known)::value, PARTS = KNOWN > 0 ? KNOWN : 8;
         constexpr int CPI = KNOWN > 0 ? (BN / KNOWN < 8 ? BN / KNOWN : 8) : (BN >= 64 ? 8 : (BN >= 32 ? 4 : 2));
         uint32_t remote[PARTS];
@@ -952,12 +958,12 @@ namespace {
 
 thread_local int t_kernels_launched = 0;     // by this thread's product calls, for tests
 
-template <int BN, int STAGES, int EPI, typename OutT, int MINB>
-int launch(const CUtensorMap& tw, const CUtensorMap& tx, const CUtensorMap& tc, const GemmParams& p, cudaStream_t stream) {
+template <int BN, int STAGES, int EPI, typename OutT, int MINB, bool GROUPED>
+int launch_as(const CUtensorMap& tw, const CUtensorMap& tx, const CUtensorMap& tc, const GemmParams& p, cudaStream_t stream) {
   constexpr int stage_bytes = W_TILE_BYTES + BN * BK * 2;
   constexpr int smem = STAGES * stage_bytes + 1024 + (leaves_by_tma<BN, EPI>() ? LEAVE_GROUPS * LEAVE_STAGE_BYTES : 0);
   static_assert(smem * MINB <= 227 * 1024, "shared memory");
-  auto kernel = gemm_wx_kernel<BN, STAGES, EPI, OutT, MINB>;
+  auto kernel = gemm_wx_kernel<BN, STAGES, EPI, OutT, MINB, GROUPED>;
   ++t_kernels_launched;
   typename OutputMap<leaves_by_tma<BN, EPI>()>::type out_map;
   if constexpr (leaves_by_tma<BN, EPI>()) out_map = tc; else out_map.none = 0;
@@ -993,6 +999,14 @@ int launch(const CUtensorMap& tw, const CUtensorMap& tx, const CUtensorMap& tc, 
   RB_LAUNCH("kernel", (kernel), grid, (block_threads<BN, EPI>()), smem, stream, tw, tx, out_map, p);
   RB_CHECK_LAUNCH("rb_gemm_tc");
   return 0;
+}
+
+template <int BN, int STAGES, int EPI, typename OutT, int MINB>
+int launch(const CUtensorMap& tw, const CUtensorMap& tx, const CUtensorMap& tc, const GemmParams& p, cudaStream_t stream) {
+  if constexpr (EPI == EPI_STORE || EPI == EPI_GATED) {
+    if (p.tile_group != nullptr) return launch_as<BN, STAGES, EPI, OutT, MINB, true>(tw, tx, tc, p, stream);
+  }
+  return launch_as<BN, STAGES, EPI, OutT, MINB, false>(tw, tx, tc, p, stream);
 }
 
 template <int EPI, typename OutT>
