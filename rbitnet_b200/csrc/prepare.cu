@@ -50,8 +50,8 @@ __global__ void __launch_bounds__(256) round_rows_kernel(T* out, const float* x,
 }
 
 // A block per row.  VEC: a thread holds NV times four values of both rows in registers (blockDim.x * NV * 4 >= E), all asked for at
-// once, the weights before the wait for the kernel before; else the rows go through memory.  1 row of 2,048 values took 3.0 us
-// of a step with a load of y for its sum and one of everything after it, so 1.8.
+// once, the weights before the wait for the kernel before; else the rows go through memory, with NV 0 four values at a time.  1 row
+// of 2,048 values took 3.0 us of a step with a load of y for its sum and one of everything after it, so 1.8.
 template <typename T, bool VEC, int NV>
 __global__ void __launch_bounds__(1024) norm_add_kernel(float* x, const float* y,
                                                         const float* w, float eps, int E,
@@ -61,7 +61,7 @@ __global__ void __launch_bounds__(1024) norm_add_kernel(float* x, const float* y
   const int64_t row = blockIdx.x;
   const float* yr = y + row * E;
   float* xr = x + row * E;
-  if (VEC) {
+  if constexpr (VEC) {
     float ww[NV][4], v[NV][4], o[NV][4];
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
@@ -97,6 +97,28 @@ __global__ void __launch_bounds__(1024) norm_add_kernel(float* x, const float* y
   }
   rb_pdl_wait();
   float ss = 0.f;
+  if (NV == 0) {
+    for (int e = threadIdx.x * 4; e < E; e += blockDim.x * 4) {
+      float v[4];
+      rb_load4(yr + e, v);
+      ss += v[0] * v[0] + v[1] * v[1] + v[2] * v[2] + v[3] * v[3];
+    }
+    ss = rb_block_sum(ss, scratch);
+    const float r = 1.0f / sqrtf(ss / (float)E + eps);
+    for (int e = threadIdx.x * 4; e < E; e += blockDim.x * 4) {
+      float v[4], ww[4], o[4];
+      rb_load4(yr + e, v);
+      rb_load4(w + e, ww);
+      rb_load4(xr + e, o);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) o[k] += v[k] * r * ww[k];
+      rb_store4(xr + e, o);
+      if (rounded != nullptr)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) rounded[row * E + e + k] = rb_from_float<T>(o[k]);
+    }
+    return;
+  }
   for (int e = threadIdx.x; e < E; e += blockDim.x) ss += yr[e] * yr[e];
   ss = rb_block_sum(ss, scratch);
   const float r = 1.0f / sqrtf(ss / (float)E + eps);
@@ -636,13 +658,15 @@ RB_EXPORT int rb_norm_add(float* x, const float* y, const float* w, float eps, i
                           cudaStream_t stream) {
   if (T == 0) return 0;
   RB_REQUIRE(E > 0, "rb_norm_add: bad width %d", E);
-  const bool vec = E % 4 == 0 && E <= 16384 && (uintptr_t)x % 16 == 0 && (uintptr_t)y % 16 == 0 && (uintptr_t)w % 16 == 0 && (uintptr_t)rounded % 16 == 0;
+  const bool wide = E % 4 == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)y % 16 == 0 && (uintptr_t)w % 16 == 0;
+  const bool vec = wide && E <= 16384 && (uintptr_t)rounded % 16 == 0;        // (more than 16 values a thread do not fit its registers)
   const int n4 = E / 4, nv = n4 <= 256 ? 1 : (n4 <= 1024 ? 2 : 4);
   const int threads = vec ? ((n4 + nv - 1) / nv + 31) / 32 * 32 : (E >= 1024 ? 256 : 128);
 #define GO(TT, V, N) RB_LAUNCH("norm_add_kernel", (norm_add_kernel<TT, V, N>), T, threads, 0, stream, x, y, w, eps, E, (TT*)rounded)
 #define PICK(TT)                         \
   do {                                   \
-    if (!vec) GO(TT, false, 1);          \
+    if (!wide) GO(TT, false, 1);         \
+    else if (!vec) GO(TT, false, 0);     \
     else if (nv == 1) GO(TT, true, 1);   \
     else if (nv == 2) GO(TT, true, 2);   \
     else GO(TT, true, 4);                \

@@ -121,3 +121,22 @@ def test_q_and_k_preparation_in_quads(ops_of, dtype, H, Kh, D, Dv, rot, interlea
             assert float((one.double() - two.double()).abs().max()) <= tol * float(two.double().abs().max())
         assert torch.equal(made[0][2], made[1][2]) and (gate is None or torch.equal(gate, gate1))
     ops.check_errors()
+
+
+@pytest.mark.parametrize("dtype", [F32, BF16])
+@pytest.mark.parametrize("E,shift", [(4096, 0), (4100, 0), (16384, 0), (16388, 0), (20000, 0), (32772, 0), (16390, 0), (2048, 2), (5120, 2)])
+def test_normed_result_added_to_wide_rows(ops_of, dtype, E, shift):
+    """Rows in registers, wider ones four values at a time, no multiple of four; ``shift``: rounded rows that begin between two places
+    of a wide store.  A sum of E squares and a division are within a few units of float32."""
+    from rbitnet_b200.kernels.ops import _ptr
+    ops = ops_of(dtype)
+    g = torch.Generator(device="cuda").manual_seed(E)
+    T = 3
+    x, y = torch.randn(T, E, device="cuda", generator=g), 30.0 * torch.randn(T, E, device="cuda", generator=g)
+    w = torch.randn(E, device="cuda", generator=g)
+    want = x.double() + y.double() / (y.double().square().mean(1, keepdim=True) + 1e-5).sqrt() * w.double()
+    to = torch.full((T * E + 8,), 9.0, dtype=dtype, device="cuda")
+    ops.lib.call("rb_norm_add", _ptr(x), _ptr(y), _ptr(w), 1e-5, T, E, _ptr(to[shift:]), ops.code, ops._stream())
+    assert float((x.double() - want).norm() / want.norm()) <= 1e-6
+    assert torch.equal(to[shift:shift + T * E].view(T, E), x.to(dtype))
+    assert bool((to[:shift] == 9.0).all()) and bool((to[shift + T * E:] == 9.0).all())
