@@ -140,3 +140,26 @@ def test_normed_result_added_to_wide_rows(ops_of, dtype, E, shift):
     assert float((x.double() - want).norm() / want.norm()) <= 1e-6
     assert torch.equal(to[shift:shift + T * E].view(T, E), x.to(dtype))
     assert bool((to[:shift] == 9.0).all()) and bool((to[shift + T * E:] == 9.0).all())
+
+
+@pytest.mark.parametrize("dtype", [F32, BF16])
+@pytest.mark.parametrize("E", [4100, 5120, 16384])
+@pytest.mark.parametrize("fresh", [False, True])
+def test_a_results_norm_and_the_norm_after_it_of_few_and_many_wide_rows(ops_of, dtype, E, fresh):
+    """Sixteen values a thread, the second weights asked for before the rows (as many rows as SMs) and after their first sum (more):
+    the same bits, and those of float64 within a few units of float32."""
+    ops = ops_of(dtype)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    g = torch.Generator(device="cuda").manual_seed(E)
+    x, y = torch.randn(sms + 1, E, device="cuda", generator=g), 30.0 * torch.randn(sms + 1, E, device="cuda", generator=g)
+    w, w2 = torch.randn(E, device="cuda", generator=g), torch.randn(E, device="cuda", generator=g)
+    many, h_many = ops.norm_add_norm(None if fresh else x.clone(), y, w, 1e-5, w2, 1e-5)
+    few, h_few = ops.norm_add_norm(None if fresh else x[:sms].clone(), y[:sms], w, 1e-5, w2, 1e-5)
+    assert torch.equal(many[:sms], few) and torch.equal(h_many[:sms], h_few)
+
+    def rms(v):
+        return v / (v.square().mean(1, keepdim=True) + 1e-5).sqrt()
+    want = (0.0 if fresh else x.double()) + rms(y.double()) * w.double()
+    assert float((many.double() - want).norm() / want.norm()) <= 1e-6
+    rows = rms(want) * w2.double()
+    assert float((h_many.double() - rows).norm() / rows.norm()) <= (2e-6 if dtype == F32 else 4e-3)
