@@ -10,6 +10,9 @@
 //
 // A sum that is not finite is made again by FFMA (an infinity's parts are infinite and not a number, and a value above the largest
 // bfloat16 rounds to infinity), so infinities, NaN and sums near the largest float32 come out as the plain tiles leave them.
+// What that costs, us of 600 x 2,048 (2,048 x 2,048 with K 5,632), 66 (342) with finite sums only: 128 tokens with a NaN 73 (636), all
+// of them 89 (1,070); 128 tokens with an infinity and no NaN 1,310 (13,700), whose sums are really made again, a thread each.  (All
+// sums that are not finite made again, value by value: 128 tokens 4,520 (49,700), all of them 13,400 (98,900); FFMA tiles 145 (1,090).)
 // Parts below 2^-133 vanish: values under 2^-110 keep fewer than 24 digits.
 //
 // A CTA makes a tile of 128 rows of W (the instruction's M side) times BN tokens, or a part of its K.  Sixteen warps fetch float32
@@ -89,18 +92,30 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_kernel(const F32Product p
   __syncthreads();
   tcgen05_fence_after();
   const uint32_t tmem_base = tmem_holder;
-  // a sum made by FFMA over all of K, in its order
-  auto plain_sum = [&](int m, int n) -> float {
+  // A sum that is not finite as FFMA leaves it over all of K, in its order; called by whole warps, one token each.  A token with a NaN
+  // among its values (what a row looks like once anything in it has overflowed) has no other sums, and is known by one look at the row.
+  auto settled = [&](float v, bool in, int m, int n) -> float {
+    const bool bad = in && !(fabsf(v) <= 3.402823466e+38f);
+    if (!__any_sync(0xffffffffu, bad)) return v;
     const float* a = A + (int64_t)m * p.lda;
+    bool nan = false;
+    for (int k = lane * 4; k < p.K; k += 128) {
+      const float4 x = *reinterpret_cast<const float4*>(a + k);
+      nan |= x.x != x.x || x.y != x.y || x.z != x.z || x.w != x.w;
+    }
+    nan = __any_sync(0xffffffffu, nan);
+    if (!bad) return v;
+    if (nan) return __uint_as_float(0x7fffffffu);
     const float* w = W + (int64_t)n * p.ldw;
-    float v = 0.f;
-    for (int k = 0; k < p.K; ++k) v = fmaf(a[k], w[k], v);
+    v = 0.f;
+#pragma unroll 4
+    for (int k = 0; k < p.K; k += 4) {
+      const float4 x = *reinterpret_cast<const float4*>(a + k), y = *reinterpret_cast<const float4*>(w + k);
+      v = fmaf(x.w, y.w, fmaf(x.z, y.z, fmaf(x.y, y.y, fmaf(x.x, y.x, v))));
+    }
     return v;
   };
-  auto value = [&](float v, int m, int n) -> float {
-    if (!(fabsf(v) <= 3.402823466e+38f)) v = plain_sum(m, n);
-    return finished(p.tail, p.alpha == 1.0f ? v : v * p.alpha, m, n, z);
-  };
+  auto value = [&](float v, int m, int n) -> float { return finished(p.tail, p.alpha == 1.0f ? v : v * p.alpha, m, n, z); };
 
   const int my_row = warp * 2 + (lane >> 4), my_k = (lane & 15) * 4;
   // a row's 128 bytes lie at row * 128, its 16-byte pieces exchanged by the row's number modulo 8 (rows STEP apart: the same)
@@ -212,19 +227,23 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_kernel(const F32Product p
     float* red = reinterpret_cast<float*>(smem);          // [token column][row of W]
 #pragma unroll
     for (int j = 0; j < COLS; ++j) red[(c0 + j) * BM + row] = sum[j];
-  } else if (n < p.N) {
+  } else {
     float* dst = C + (int64_t)(t0 + c0) * p.ldc + n;
     const int left = p.M - (t0 + c0);
+    const bool in = n < p.N;
 #pragma unroll
     for (int c = 0; c < COLS; c += 16) {
       float old[16];
 #pragma unroll
-      for (int j = 0; j < 16; ++j) old[j] = p.accumulate && c + j < left ? dst[(int64_t)(c + j) * p.ldc] : 0.f;
+      for (int j = 0; j < 16; ++j) old[j] = in && p.accumulate && c + j < left ? dst[(int64_t)(c + j) * p.ldc] : 0.f;
 #pragma unroll
       for (int j = 0; j < 16; ++j)
         if (c + j < left) {
-          const float v = value(sum[c + j], t0 + c0 + c + j, n);
-          dst[(int64_t)(c + j) * p.ldc] = p.accumulate ? old[j] + v : v;
+          const float v = settled(sum[c + j], in, t0 + c0 + c + j, n);
+          if (in) {
+            const float done = value(v, t0 + c0 + c + j, n);
+            dst[(int64_t)(c + j) * p.ldc] = p.accumulate ? old[j] + done : done;
+          }
         }
     }
   }
@@ -233,23 +252,25 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_kernel(const F32Product p
     cluster_sync_all();
     const int my = (int)cluster_rank(), srow = threadIdx.x % BM, sn = n0 + srow;
     const uint32_t red = smem_u32(smem) + (uint32_t)srow * 4;
-    if (sn < p.N) {
-      for (int col = my + parts * (threadIdx.x / BM); col < BN && t0 + col < p.M; col += parts * (THREADS / BM)) {
-        float* dst = C + (int64_t)(t0 + col) * p.ldc + sn;
-        const float old = p.accumulate ? *dst : 0.f;
-        float from[8];
+    const bool in = sn < p.N;
+    for (int col = my + parts * (threadIdx.x / BM); col < BN && t0 + col < p.M; col += parts * (THREADS / BM)) {
+      float* dst = C + (int64_t)(t0 + col) * p.ldc + sn;
+      const float old = in && p.accumulate ? *dst : 0.f;
+      float from[8];
 #pragma unroll
-        for (int r = 0; r < 8; ++r) {
-          from[r] = 0.f;
-          if (r < parts) {
-            uint32_t there;
-            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"(red + (uint32_t)(col * BM) * 4), "r"((uint32_t)r));
-            asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(from[r]) : "r"(there));
-          }
+      for (int r = 0; r < 8; ++r) {
+        from[r] = 0.f;
+        if (r < parts) {
+          uint32_t there;
+          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"(red + (uint32_t)(col * BM) * 4), "r"((uint32_t)r));
+          asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(from[r]) : "r"(there));
         }
-        float v = from[0];
+      }
+      float v = from[0];
 #pragma unroll
-        for (int r = 1; r < 8; ++r) v += from[r];
+      for (int r = 1; r < 8; ++r) v += from[r];
+      v = settled(v, in, t0 + col, sn);
+      if (in) {
         v = value(v, t0 + col, sn);
         *dst = p.accumulate ? old + v : v;
       }
