@@ -76,7 +76,14 @@ template <> struct OutputMap<false> { struct type { int none; }; };
 template <int BN, int EPI> constexpr bool leaves_by_tma() { return BN >= 128 && EPI != EPI_QKV; }
 template <int N> struct Int { static constexpr int value = N; };
 // Tiles that leave by TMA have two groups of four epilogue warps, the others one.
-constexpr int LEAVE_GROUPS = 2, LEAVE_STAGE_BYTES = 16 * 1024;      // staging room of a group
+constexpr int LEAVE_GROUPS = 2;
+// Staging room of a group.  Token tiles of 192 have room for a fifth stage of the ring where it is half as large, which takes two boxes of
+// bfloat16 and more but only one of float32; the fused q/k/v needs none.  us of gated products of 192 and 960 tokens, one group and five
+// stages, two and four, two and five: 11,264 x 2,048 22.4, 16.9, 15.8; 51.2, 39.4, 37.3; 4,096 x 11,008 58.5, 61.4, 50.4; 107, 123, 100;
+// 22,016 x 4,096 146, 141, 129 (960).  Float32 keeps four: 2,048 x 2,048 18.6, 16.0; 17.5, 15.9; 11,264 x 2,048 39.9, 40.9 (960); a long
+// K pays for it, 4,096 x 11,008 57.6, 65.4; 118, 118, but not where it is added (192 tokens 42.6, 38.1).
+template <int BN, typename OutT> constexpr int leave_bytes() { return BN == 192 && sizeof(OutT) == 2 ? 8 * 1024 : 16 * 1024; }
+template <int BN, int EPI, typename OutT> constexpr int stages_of_192() { return leaves_by_tma<BN, EPI>() && sizeof(OutT) == 4 ? 4 : 5; }
 template <int BN, int EPI> constexpr int block_threads() { return leaves_by_tma<BN, EPI>() ? 64 + 128 * LEAVE_GROUPS : 192; }
 
 struct GemmParams {
@@ -227,7 +234,6 @@ gemm_wx_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
   // 128 x 256 gated tile took 19 us to leave, more than its products with K 2,048.  11,264 gated rows of 2,048, us before and
   // now: 600 tokens 50, 30; 2,048 106, 70; 3,001 157, 106; 6,140 279, 195; 2,048 x 2,048 float32 of 3,001 tokens 43, 27.
   // With K 4,096 the products hide either, and only a launch's last tiles show (2,048 tokens of 28,672 gated rows 343, 337).
-  // (Token tiles of 192 gave a stage of their ring for the room.)
   constexpr bool TMA_EPI = leaves_by_tma<BN, EPI>();
   constexpr int GROUPS = TMA_EPI ? LEAVE_GROUPS : 1;
   // A pending norm of the input rows and what a later norm needs (see GemmParams) are compiled for the
@@ -236,14 +242,15 @@ gemm_wx_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
   constexpr bool PENDING_NORM = BN <= 16;
   constexpr int OUT_COLS = EPI == EPI_GATED ? BM / 2 : BM;          // values per token row of a staged box
   constexpr int BOX_BYTES = 16 * OUT_COLS * (int)sizeof(OutT);
-  constexpr int BOXES = LEAVE_STAGE_BYTES / BOX_BYTES < 4 ? LEAVE_STAGE_BYTES / BOX_BYTES : 4;
+  constexpr int LEAVE_BYTES = leave_bytes<BN, OutT>();
+  constexpr int BOXES = LEAVE_BYTES / BOX_BYTES < 4 ? LEAVE_BYTES / BOX_BYTES : 4;
   static_assert(BOXES >= 2, "a group's boxes alternate");
   static_assert(BN % 16 == 0 && BN >= 16 && BN <= 256, "UMMA N");
   static_assert(WANT_COLS <= 512, "tensor memory has 512 columns");
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  uint8_t* out_stage = smem + (size_t)STAGES * STAGE_BYTES;          // TMA_EPI: LEAVE_STAGE_BYTES per group
+  uint8_t* out_stage = smem + (size_t)STAGES * STAGE_BYTES;          // TMA_EPI: LEAVE_BYTES per group
   __shared__ uint64_t full_bar[STAGES];
   __shared__ uint64_t empty_bar[STAGES];
   __shared__ uint64_t accum_full[NBUF];
@@ -554,7 +561,7 @@ gemm_wx_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
           ask_acc(c + 16 * GROUPS < c_end ? c + 16 * GROUPS : c, next);
           // The 16 token rows of the chunk go to shared memory as [token][OUT_COLS values] and leave as
           // one box; rows and columns beyond the matrix are dropped by the tensor map.
-          OutT* box = reinterpret_cast<OutT*>(out_stage + group * LEAVE_STAGE_BYTES + n_boxes % BOXES * BOX_BYTES);
+          OutT* box = reinterpret_cast<OutT*>(out_stage + group * LEAVE_BYTES + n_boxes % BOXES * BOX_BYTES);
           ++n_boxes;
           if (EPI == EPI_GATED) {
             // Lanes 0..15 hold gate rows, lanes 16..31 the up rows of the same 16 features (feature =
@@ -961,7 +968,7 @@ thread_local int t_kernels_launched = 0;     // by this thread's product calls, 
 template <int BN, int STAGES, int EPI, typename OutT, int MINB, bool GROUPED>
 int launch_as(const CUtensorMap& tw, const CUtensorMap& tx, const CUtensorMap& tc, const GemmParams& p, cudaStream_t stream) {
   constexpr int stage_bytes = W_TILE_BYTES + BN * BK * 2;
-  constexpr int smem = STAGES * stage_bytes + 1024 + (leaves_by_tma<BN, EPI>() ? LEAVE_GROUPS * LEAVE_STAGE_BYTES : 0);
+  constexpr int smem = STAGES * stage_bytes + 1024 + (leaves_by_tma<BN, EPI>() ? LEAVE_GROUPS * leave_bytes<BN, OutT>() : 0);
   static_assert(smem * MINB <= 227 * 1024, "shared memory");
   auto kernel = gemm_wx_kernel<BN, STAGES, EPI, OutT, MINB, GROUPED>;
   ++t_kernels_launched;
@@ -1018,7 +1025,7 @@ int dispatch(int bn, const CUtensorMap& tw, const CUtensorMap& tx, const CUtenso
     case 64: return launch<64, 4, EPI, OutT, 2>(tw, tx, tc, p, stream);
     case 128: return launch<128, 6, EPI, OutT, 1>(tw, tx, tc, p, stream);
     case 160: return launch<160, 5, EPI, OutT, 1>(tw, tx, tc, p, stream);
-    case 192: return launch<192, 4, EPI, OutT, 1>(tw, tx, tc, p, stream);
+    case 192: return launch<192, stages_of_192<192, EPI, OutT>(), EPI, OutT, 1>(tw, tx, tc, p, stream);
     case 224: return launch<224, 4, EPI, OutT, 1>(tw, tx, tc, p, stream);
     case 256: return launch<256, 4, EPI, OutT, 1>(tw, tx, tc, p, stream);
   }
@@ -1096,10 +1103,13 @@ RB_EXPORT int rb_wait_probe(long long limit_ns, int code, int* gave_up, cudaStre
 // tiles are fewer than the CTAs that run together (two per SM), K is cut as well: into 2, 4 or 8
 // parts, the sizes clusters schedule well, each of at least four 64-wide blocks.  Beyond 256 tokens: one.
 // 33 to 64 tokens take two tiles of 32 (rb_gemm_tc_few_tile) where that makes a tile's way out, half as long and summed over fewer
-// parts, worth reading W a second time from L2.  us, tiles of 64 and two of 32, each with the best parts, 64 tokens: 2,048 x 2,048 7.0,
-// 6.2; K 5,632 10.2, 9.5; 768 x 2,048 5.9, 5.2; 2,048 x 768 6.2, 5.4; 2,816 gated rows of 2,048 8.4, 7.6; 11,264 16.4, 13.9; with 48
-// tokens 6.3, 6.1; 9.6, 9.3; 11,264 15.5, 13.5.  Not where four parts of 64 fill the chip (5,632 gated rows 11.2, 11.4; 40 tokens 10.2,
-// 11.1; 8,192 stored 11.6, 11.5; 10.8, 11.4), nor where W is larger (4,096 x 14,336 25.3, 26.4; 28,672 x 4,096 43.9, 47.3).
+// parts, worth reading W a second time from L2.  us, two tiles of 32 and tiles of 64, each with the best parts, 64 tokens added and
+// gated, W from memory: 16 weight tiles K 2,048 5.8, 6.7; 6.5, 7.3; K 5,632 9.2, 10.3; 9.1, 10.6; 24 K 2,048 6.7, 7.8; 7.2, 8.3; K 8,192
+// 13.8, 14.2; 14.4, 14.4.  25 to 32 tiles gain with a short K (32, K 2,048 7.7, 8.3; 8.1, 9.5) and with K 4,096 no longer always (25
+// tiles 9.7, 10.4; 10.3, 10.6; 33 tokens gated 10.1, 9.5), and are left as they were.  40 to 72 tiles, whose four parts of 64 fill the chip:
+// 40 K 2,048 9.7, 9.2; 10.8, 10.4; 64 10.8, 10.8; 11.3, 11.8; K 4,096 40 13.7, 12.8; 14.7, 14.2.  From 80 on a tile is made whole: 80 K 2,048
+// 12.0, 14.4; 12.5, 15.4; 88 12.3, 14.5; 12.9, 15.6; K 1,024 148 10.1, 11.0; 10.6, 12.2.  Not where W is larger (4,096 x 14,336 25.3,
+// 26.4 so; 28,672 x 4,096 43.9, 47.3).
 RB_EXPORT int rb_gemm_tc_few_tile(int n_tokens, int n_out, int K) {
   const int w_tiles = (n_out + BM - 1) / BM;
   return n_tokens > 32 && n_tokens <= 64 && (w_tiles <= 24 || (w_tiles >= 80 && w_tiles <= rb_sm_count())) && (int64_t)n_out * K <= (24 << 20) ? 32 : 0;
@@ -1107,6 +1117,9 @@ RB_EXPORT int rb_gemm_tc_few_tile(int n_tokens, int n_out, int K) {
 
 RB_EXPORT int rb_gemm_tc_splits(int n_tokens, int n_out, int K) {
   if (n_tokens > 256 || n_tokens <= 0 || n_out <= 0 || K <= 0) return 1;
+  // Two tiles of 32: up to a CTA and a third per SM; from K 4,096 on up to two, the longer chain being worth the clusters of eight.
+  // us of added products in 4 and 8 parts: 16 weight tiles K 2,048 5.8, 6.6; 3,072 6.9, 7.4; 4,096 8.1, 8.1; 5,632 9.4, 9.2; 8,192 11.8,
+  // 11.4; gated 2,048 6.5, 6.6; 4,096 8.8, 8.0; 8,192 12.5, 11.3.  24 tiles in 8 parts are more than two: 9.6, 13.9.
   if (rb_gemm_tc_few_tile(n_tokens, n_out, K) != 0) {
     const int both = 2 * ((n_out + BM - 1) / BM), most = K >= 4096 ? 2 * rb_sm_count() : rb_sm_count() + rb_sm_count() / 3;
     const int of_k = (K + BK - 1) / BK;
