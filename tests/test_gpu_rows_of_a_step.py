@@ -71,7 +71,8 @@ def test_norm_and_gate_per_head(ops_of, dtype, T, H, Dv, pad, shared, silu):
 @pytest.mark.parametrize("H,Kh,D,Dv,rot,interleaved,norm,taps,keys,mix,gates", [
     (16, 4, 128, 128, 64, True, "head_weight", 4, False, False, False), (20, 4, 64, 72, 24, False, "projection", 4, False, True, True),
     (5, 1, 12, 4, 6, True, None, 4, False, False, True), (3, 1, 260, 260, 12, False, "head_weight", 0, True, False, True),
-    (300, 1, 4, 4, 4, False, None, 0, False, False, True), (2, 60, 4, 132, 2, False, "projection", 0, False, True, False)])
+    (300, 1, 4, 4, 4, False, None, 0, False, False, True), (2, 60, 4, 132, 2, False, "projection", 0, False, True, False),
+    (97, 3, 128, 128, 32, False, "projection", 4, False, False, True)])
 def test_q_and_k_preparation_in_quads(ops_of, dtype, H, Kh, D, Dv, rot, interleaved, norm, taps, keys, mix, gates):
     """Quads of values against the form that takes any size and address (rows that begin one value late), over runs of several rows
     and single rows, from the first position: the ring, the cache's pages, q and the gates."""
