@@ -1,7 +1,8 @@
 // float32 products on the tensor cores (included by gemm_tcgen05.cu): C[M,N] (+)= alpha * A[M,K] * W[N,K]^T in 32 bits.
 //
 // A float32 value is the sum of three bfloat16 values: h = bf16(x), m = bf16(x - h), l = x - h - m, the differences exact
-// and l too, for 3 times 8 digits hold all 24.  A product of two values is then hh + (hm + mh) + (hl + mm + lh) but for
+// and l too, for 3 times 8 digits hold all 24 (the method of Henry, Tang and Heinecke, "Leveraging the bfloat16 Artificial
+// Intelligence Datatype For Higher-Precision Computations", 2019).  A product of two values is then hh + (hm + mh) + (hl + mm + lh) but for
 // ml + lm + ll, at most 2^-26 of it, and every product of two parts is exact in the tensor cores' float32.  What they
 // lose is in their sums, which are cut off and not rounded, so the large term is summed there over no more than one block of K
 // (64 values), into one of two accumulators in tensor memory, and the blocks' sums are added up in registers, rounded.

@@ -229,8 +229,9 @@ gemm_wx_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
   // flight per thread, about 8 KB an SM, and an epilogue of a 128 x 256 tile then takes longer than
   // the products of a short tile.  What bounds the way out is the chain of a box: out of tensor memory, into
   // shared memory, a barrier of its warps, the box read again before its room is used twice.  So two
-  // groups of four warps take every other box, each with up to four boxes in flight in its 16 KB, and the
-  // next box's values come out of tensor memory while the one before is finished.  With one group and two boxes a
+  // groups of four warps take every other box, each with boxes of its own in turn (BOXES: four of bfloat16 and gated values, of
+  // which three may still be read while one is filled; two of float32, so one; see leave_bytes), and the next box's values
+  // come out of tensor memory while the one before is finished.  With one group and two boxes a
   // 128 x 256 gated tile took 19 us to leave, more than its products with K 2,048.  11,264 gated rows of 2,048, us before and
   // now: 600 tokens 50, 30; 2,048 106, 70; 3,001 157, 106; 6,140 279, 195; 2,048 x 2,048 float32 of 3,001 tokens 43, 27.
   // With K 4,096 the products hide either, and only a launch's last tiles show (2,048 tokens of 28,672 gated rows 343, 337).

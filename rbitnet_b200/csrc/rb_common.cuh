@@ -41,11 +41,17 @@ void rb_set_error(const char* fmt, ...);
 
 // ---------------------------------------------------------------- programmatic dependent launch
 // Every kernel of the library is launched with the attribute that lets it start while the
-// kernel before it in the stream is still running.  A kernel therefore calls rb_pdl_wait()
-// before its first access to global memory (after the wait, everything earlier in the stream
-// has completed and is visible), and rb_pdl_launch_dependents() as early as it can, so that
-// the next kernel's launch and set-up overlap this kernel's work.  Inside a captured graph the
-// same launches become programmatic edges.
+// kernel before it in the stream is still running, and calls rb_pdl_launch_dependents() as early as it
+// can, so that the next kernel's launch and set-up overlap its work.  Inside a captured graph the same
+// launches become programmatic edges.  A kernel calls rb_pdl_wait() before it touches global memory: after the
+// wait, everything earlier in the stream has completed and is visible.
+//
+// Before the wait a kernel may read only what no kernel has written since the stream's last full boundary
+// (a copy, a synchronisation, the start of a graph launch).  That the kernel right before it does not
+// write it is not enough: every kernel lets the next one start at its own top, so a read ahead of the wait can overlap
+// several kernels before that.  What qualifies: weights, taps, biases and frequencies (written when a model
+// is bound; a step begins with copies), page tables, and a step's positions and slots (brought by copies).  rb_decode_advance moves the
+// positions of a captured step on and is therefore its last kernel: what comes after it is a copy or a graph launch.
 //
 // No pointer of a kernel is declared restrict.  Behind such a pointer the compiler takes the data for its own, or, if it is
 // const, for constant while the kernel runs, and may load it before the wait, whose clobber says nothing about it: the tiled

@@ -70,6 +70,43 @@ def test_choices(ops_of, n, groups, keep, scoring, normalize, scale, T):
 
 
 @pytest.mark.parametrize("dtype", [F32, BF16])
+@pytest.mark.parametrize("n,groups,keep,top", [(3, 0, 0, 2), (30, 3, 2, 4), (32, 0, 0, 4), (33, 0, 0, 1), (64, 8, 3, 8)])
+@pytest.mark.parametrize("T", [2, 8, 9, 16])
+def test_choices_made_by_the_kernel_that_places_and_apart(ops_of, dtype, n, groups, keep, top, T):
+    """The same weights, extra sums, places and rows both ways, whatever the rule between them says: a turn of eight tokens and two."""
+    ops = ops_of(dtype)
+    lib = ops.lib
+
+    class Ruled:
+        def __init__(self, pays):
+            self.pays = pays
+
+        def raw(self, name):
+            return (lambda *sizes: self.pays) if name == "rb_route_choose_place_pays" else lib.raw(name)
+
+        def call(self, name, *args, launches=1):
+            assert name != "rb_route_choose_place" or self.pays
+            lib.call(name, *args, launches=launches)
+    g = torch.Generator(device="cuda").manual_seed(T * n)
+    K = 128
+    h = torch.randn(T, K, device="cuda", generator=g).to(dtype)
+    router, corr = torch.randn(n + 1, K, device="cuda", generator=g), 0.3 * torch.randn(n, device="cuda", generator=g)
+    made = []
+    for pays in (0, 1):
+        ops.lib = Ruled(pays)
+        try:
+            made.append(ops.route_and_place(h, router, corr, top, groups, keep, n, 64, scoring="sigmoid", extra_rows=1, normalize=1e-20,
+                                            weight_scale=1.5, weight_on_input=True, with_shared=True))
+        finally:
+            ops.lib = lib
+    a, b = made
+    for one, two in ((a.weights, b.weights), (a.extra, b.extra), (a.rows, b.rows), (a.pos, b.pos), (a.tile_group, b.tile_group)):
+        assert torch.equal(one, two)
+    assert a.n_shared == b.n_shared == 1 and torch.equal(a.rows[:T], h) and int(a.tile_group[0]) == n
+    ops.check_errors()
+
+
+@pytest.mark.parametrize("dtype", [F32, BF16])
 @pytest.mark.parametrize("K", [4, 96, 2048, 2052, 4100])
 def test_sums_of_few_tokens(ops_of, dtype, K):
     """Rows of up to 2,048 values and longer ones.  A float32 sum of K products is within K 2^-24 of the sum of their magnitudes."""
