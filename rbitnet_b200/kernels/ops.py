@@ -1397,9 +1397,9 @@ class CudaOps:
                         keep: int, n_experts: int, inner: int, scoring: str = "softmax", extra_rows: int = 0,
                         normalize: Optional[float] = None, weight_scale: float = 1.0, weight_on_input: bool = False,
                         with_shared: bool = False) -> Optional["PlacedRows"]:
-        """``route_scored`` and the sorting of the pairs by expert that ``routed_experts`` begins with, for up to 16 tokens (None: not
-        for these sizes), in two launches where the choice costs less than a third.  ``with_shared``: the tokens' own rows are placed too, for one more expert whose
-        matrices lie behind the others'."""
+        """``route_scored`` and the sorting of the pairs by expert that ``routed_experts`` begins with, for up to 16 tokens (None:
+        not for these sizes), in two launches where the choice costs less than a third.  ``with_shared``: the tokens' own rows are
+        placed too, for one more expert whose matrices lie behind the others'."""
         self._check(h, self.dtype, "route input")
         scored = _SCORING[scoring]
         T, K = h.shape
